@@ -201,6 +201,174 @@ PM_HD void zfp_decode_block(const uint32_t* words, float* f, int maxbits) {
   for (int i = 0; i < 16; ++i) f[i] = zfp_ldexp((float)q[i], emax - 30);
 }
 
+// ---- the same block coder, bit planes at a time -------------------------------------------------
+// Writes and reads exactly the stream of zfp_encode_block / zfp_decode_block (the serial form, which the CPU twin runs
+// and the tests compare with).  What the serial form spends its instructions on is collecting one bit of each of the 16
+// coefficients per plane and moving the code bit by bit; here all planes come from one 16 x 32 bit-matrix transpose,
+// and a group test with the run of zeros and the one that follow it is one append (or one look at the next 17 bits).
+// `planes` is room for 16 words and `words` for the block's code words, both `stride` words apart, so that a
+// thread block can keep one column per thread in shared memory.
+
+// Transposes the 16 x 16 bit matrices in the low and in the high halves of a[0..15]: afterwards bit i of a[r] is what
+// bit r of a[i] was, and bit 16 + i what bit 16 + r was.  Its own inverse.
+PM_HD void bit_transpose16(uint32_t* a) {
+  const uint32_t mask[4] = {0x00ff00ffu, 0x0f0f0f0fu, 0x33333333u, 0x55555555u};
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+  for (int st = 0; st < 4; ++st) {
+    const int sh = 8 >> st;
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+    for (int i = 0; i < 16; ++i) {
+      if (i & sh) continue;
+      const uint32_t t = ((a[i] >> sh) ^ a[i + sh]) & mask[st];
+      a[i + sh] ^= t;
+      a[i] ^= t << sh;
+    }
+  }
+}
+
+PM_HD int low_zeros(uint32_t x) {            // number of zero bits below the lowest one; x != 0
+#if defined(__CUDA_ARCH__)
+  return __ffs((int)x) - 1;
+#else
+  return __builtin_ctz(x);
+#endif
+}
+
+PM_HD void zfp_encode_block_planes(const float* f, uint32_t* planes, uint32_t* words, int stride, int maxbits) {
+  const int nwords = maxbits / 32;
+  float amax = 0.f;
+  for (int i = 0; i < 16; ++i) { const float a = f[i] < 0 ? -f[i] : f[i]; if (a > amax) amax = a; }
+  int widx = 0;
+  if (amax > 0.f && amax < 3.0e38f) {
+    const int emax = zfp_exponent(amax);
+    int32_t q[16];
+    for (int i = 0; i < 16; ++i) q[i] = (int32_t)zfp_ldexp(f[i], 30 - emax);
+    for (int y = 0; y < 4; ++y) zfp_fwd_lift(q + 4 * y, 1);
+    for (int x = 0; x < 4; ++x) zfp_fwd_lift(q + x, 4);
+    uint32_t u[16];
+    for (int i = 0; i < 16; ++i) u[i] = ((uint32_t)q[zfp_perm(i)] + 0xaaaaaaaau) ^ 0xaaaaaaaau;
+    bit_transpose16(u);
+    for (int i = 0; i < 16; ++i) planes[i * stride] = u[i];   // plane k: bits (k & 16) .. +15 of word k & 15
+    uint64_t acc = (2u * (uint32_t)(emax + 127) + 1u) & 0x1ffu;   // pending code bits, LSB first; below 32 between rounds
+    int nacc = 9, bits = maxbits - 9, n = 0, k = 31;
+    uint32_t x = planes[15 * stride] >> 16;
+    bool fresh = true;                                        // x is a plane whose first n bits are not written yet
+    while (true) {
+      uint32_t val = 0;
+      int len = 0;
+      if (fresh) {
+        len = n < bits ? n : bits;
+        val = x & ((1u << len) - 1u);
+        x >>= n;
+        bits -= len;
+      }
+      bool next = true;
+      if (n < 16 && bits > 0) {
+        if (x == 0u) {                                        // group test: nothing more in this plane
+          ++len;
+          --bits;
+        } else {                                              // group test, z zeros and, unless it is the last place, a one
+          const int z = low_zeros(x);
+          int l = z + 2 - (n + z == 15 ? 1 : 0);
+          l = l < bits ? l : bits;
+          val |= ((1u | (2u << z)) & ((1u << l) - 1u)) << len;
+          len += l;
+          bits -= l;
+          x >>= z + 1;
+          n += z + 1;
+          next = n >= 16;
+        }
+      }
+      acc |= (uint64_t)val << nacc;                           // at most 17 bits a round
+      nacc += len;
+      if (nacc >= 32) {
+        words[widx * stride] = (uint32_t)acc;
+        ++widx;
+        acc >>= 32;
+        nacc -= 32;
+      }
+      if (bits == 0) break;
+      fresh = next;
+      if (next) {
+        if (--k < 0) break;
+        x = (planes[(k & 15) * stride] >> (k & 16)) & 0xffffu;
+      }
+    }
+    if (nacc > 0) { words[widx * stride] = (uint32_t)acc; ++widx; }
+  }
+  for (; widx < nwords; ++widx) words[widx * stride] = 0u;
+}
+
+PM_HD void zfp_decode_block_planes(const uint32_t* words, float* f, uint32_t* planes, int stride, int maxbits) {
+  const int nwords = maxbits / 32;
+  uint64_t acc = words[0] | ((uint64_t)words[stride] << 32);   // fetched bits; at least 32 at the start of a round
+  int nacc = 64, widx = 2;
+  if (!(acc & 1u)) {
+    for (int i = 0; i < 16; ++i) f[i] = 0.f;
+    return;
+  }
+  const int emax = (int)((acc >> 1) & 255u) - 127;
+  acc >>= 9;
+  nacc -= 9;
+  for (int i = 0; i < 16; ++i) planes[i * stride] = 0u;
+  int bits = maxbits - 9, n = 0, k = 31;
+  uint32_t x = 0;
+  bool fresh = true;
+  while (true) {
+    if (nacc < 32) {
+      const uint32_t next = widx < nwords ? words[widx * stride] : 0u;
+      ++widx;
+      acc |= (uint64_t)next << nacc;
+      nacc += 32;
+    }
+    uint32_t p = (uint32_t)acc;                               // a round takes at most 17 bits
+    int used = 0;
+    if (fresh) {
+      used = n < bits ? n : bits;
+      x = p & ((1u << used) - 1u);
+      p >>= used;
+      bits -= used;
+    }
+    bool next = true;
+    if (n < 16 && bits > 0) {
+      const bool any = p & 1u;
+      p >>= 1;
+      ++used;
+      --bits;
+      if (any) {
+        const int room = 15 - n;
+        const int lim = room < bits ? room : bits;
+        const int z = low_zeros(p | (1u << lim));             // zeros before a one, or all that may be read
+        const int took = z + (z < lim ? 1 : 0);
+        used += took;
+        bits -= took;
+        x |= 1u << (n + z);
+        n += z + 1;
+        next = n >= 16;
+      }
+    }
+    acc >>= used;
+    nacc -= used;
+    if (next || bits == 0) {
+      planes[(k & 15) * stride] |= x << (k & 16);
+      if (bits == 0 || --k < 0) break;
+    }
+    fresh = next;
+  }
+  uint32_t u[16];
+  for (int i = 0; i < 16; ++i) u[i] = planes[i * stride];
+  bit_transpose16(u);
+  int32_t q[16];
+  for (int i = 0; i < 16; ++i) q[zfp_perm(i)] = (int32_t)((u[i] ^ 0xaaaaaaaau) - 0xaaaaaaaau);
+  for (int x4 = 0; x4 < 4; ++x4) zfp_inv_lift(q + x4, 4);
+  for (int y = 0; y < 4; ++y) zfp_inv_lift(q + 4 * y, 1);
+  for (int i = 0; i < 16; ++i) f[i] = zfp_ldexp((float)q[i], emax - 30);
+}
+
 // ------------------------------------------------------------------------------------------------
 // LZ block coder
 // ------------------------------------------------------------------------------------------------

@@ -1,8 +1,7 @@
 // ZFP fixed-rate 2-D and LZ codec kernels (sm_100a) plus their CPU twins.
 //
 // ZFP: one thread per 4x4 block; a thread reads four 4-element row segments (neighbouring threads
-// read neighbouring segments, so rows are read coalesced) and writes its 2*rate-byte code word with
-// 16-byte stores.  LZ: one warp per 2 KiB block for both directions, then a per-slice scan and a
+// read neighbouring segments, so rows are read coalesced) and writes its 2*rate-byte code word.  LZ: one warp per 2 KiB block for both directions, then a per-slice scan and a
 // compaction copy pack the blocks back to back.  Both reuse the host/device block coders of
 // codec_core.h, so the CUDA streams are bit-identical to the CPU oracle.
 //
@@ -46,7 +45,8 @@ __host__ __device__ inline void store_elem(void* base, int elem, long long i, fl
   reinterpret_cast<__half*>(base)[i] = __float2half_rn(f);
 }
 
-__host__ __device__ inline void zfp_block_io(bool encode, const void* x_in, void* x_out, int elem, uint8_t* stream,
+// One block of the CPU twins.
+inline void zfp_block_io(bool encode, const void* x_in, void* x_out, int elem, uint8_t* stream,
                                              long long b, long long rows, long long M, int rate) {
   const long long bx = M / 4, by = (rows + 3) / 4;
   const long long per_slice = bx * by;
@@ -57,20 +57,8 @@ __host__ __device__ inline void zfp_block_io(bool encode, const void* x_in, void
   float f[16];
   uint32_t* dst = reinterpret_cast<uint32_t*>(stream + b * (long long)(2 * rate));
   if (encode) {
-#pragma unroll
     for (int r = 0; r < 4; ++r) {
       const long long row = yb * 4 + r;
-#if defined(__CUDA_ARCH__)
-      if (elem == 1 && row < rows) {              // bf16: the block's four values of this row in one 8-byte load
-        const uint2 raw = *reinterpret_cast<const uint2*>(
-            reinterpret_cast<const __nv_bfloat16*>(x_in) + (slice * rows + row) * M + xb * 4);
-        f[r * 4 + 0] = __uint_as_float(raw.x << 16);
-        f[r * 4 + 1] = __uint_as_float(raw.x & 0xffff0000u);
-        f[r * 4 + 2] = __uint_as_float(raw.y << 16);
-        f[r * 4 + 3] = __uint_as_float(raw.y & 0xffff0000u);
-        continue;
-      }
-#endif
       for (int c = 0; c < 4; ++c)
         f[r * 4 + c] = row < rows ? load_elem(x_in, elem, (slice * rows + row) * M + xb * 4 + c) : 0.f;
     }
@@ -80,31 +68,151 @@ __host__ __device__ inline void zfp_block_io(bool encode, const void* x_in, void
   } else {
     for (int i = 0; i < words_n; ++i) words[i] = dst[i];
     zfp_decode_block(words, f, 16 * rate);
-#pragma unroll
     for (int r = 0; r < 4; ++r) {
       const long long row = yb * 4 + r;
       if (row >= rows) break;
-#if defined(__CUDA_ARCH__)
-      if (elem == 1) {                            // bf16: one 8-byte store per row of the block
-        const __nv_bfloat162 lo = __floats2bfloat162_rn(f[r * 4 + 0], f[r * 4 + 1]);
-        const __nv_bfloat162 hi = __floats2bfloat162_rn(f[r * 4 + 2], f[r * 4 + 3]);
-        uint2 raw;
-        raw.x = *reinterpret_cast<const uint32_t*>(&lo);
-        raw.y = *reinterpret_cast<const uint32_t*>(&hi);
-        *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(x_out) + (slice * rows + row) * M + xb * 4) = raw;
-        continue;
-      }
-#endif
       for (int c = 0; c < 4; ++c) store_elem(x_out, elem, (slice * rows + row) * M + xb * 4 + c, f[r * 4 + c]);
     }
   }
 }
 
-__global__ void __launch_bounds__(128)
-zfp_kernel(bool encode, const void* x_in, void* x_out, int elem, uint8_t* stream, long long nblocks, long long rows,
-           long long M, int rate) {
-  const long long b = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (b < nblocks) zfp_block_io(encode, x_in, x_out, elem, stream, b, rows, M, rate);
+// One thread per block, the bit planes of its 16 coefficients and its code words in its own column of shared memory.
+// Bound by integer issue: the serial bit-plane coder took 4685 warp instructions per 32 blocks (318 us to encode 8192 x
+// 4096 bf16, 84 % of the issue slots); see zfp_encode_block_planes for what replaced it.  VEC: rows of a block are
+// moved as one 4-element vector, which needs the tensor's base to lie on such a vector (rows are multiples of four
+// elements); other bases take the element loop.
+constexpr int kZfpThreads = 128;
+
+template <int ELEM> struct ZfpElem { using type = float; };
+template <> struct ZfpElem<1> { using type = __nv_bfloat16; };
+template <> struct ZfpElem<2> { using type = __half; };
+
+template <int ELEM, bool VEC>
+__device__ __forceinline__ void zfp_load_row(const void* x, long long at, float* f) {
+  if constexpr (!VEC) {
+    for (int c = 0; c < 4; ++c) f[c] = load_elem(x, ELEM, at + c);
+  } else if constexpr (ELEM == 0) {
+    const float4 v = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(x) + at);
+    f[0] = v.x; f[1] = v.y; f[2] = v.z; f[3] = v.w;
+  } else {
+    using T = typename ZfpElem<ELEM>::type;
+    const uint2 raw = *reinterpret_cast<const uint2*>(reinterpret_cast<const T*>(x) + at);
+    T v[4];
+    *reinterpret_cast<uint2*>(v) = raw;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) f[c] = (float)v[c];
+  }
+}
+template <int ELEM, bool VEC>
+__device__ __forceinline__ void zfp_store_row(void* x, long long at, const float* f) {
+  if constexpr (!VEC) {
+    for (int c = 0; c < 4; ++c) store_elem(x, ELEM, at + c, f[c]);
+  } else if constexpr (ELEM == 0) {
+    *reinterpret_cast<float4*>(reinterpret_cast<float*>(x) + at) = make_float4(f[0], f[1], f[2], f[3]);
+  } else {
+    using T = typename ZfpElem<ELEM>::type;
+    T v[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) v[c] = (T)f[c];
+    *reinterpret_cast<uint2*>(reinterpret_cast<T*>(x) + at) = *reinterpret_cast<const uint2*>(v);
+  }
+}
+
+// Slice, block row and block column of block b (32-bit divisions wherever the block numbers fit).
+__device__ __forceinline__ void zfp_block_at(long long b, long long nblocks, long long rows, long long M, long long& slice,
+                                             long long& yb, long long& xb) {
+  const long long bx = M / 4, per_slice = bx * ((rows + 3) / 4);
+  if (nblocks <= 0xffffffffll) {
+    const uint32_t s = (uint32_t)b / (uint32_t)per_slice, bb = (uint32_t)b - s * (uint32_t)per_slice;
+    const uint32_t y = bb / (uint32_t)bx;
+    slice = s; yb = y; xb = bb - y * (uint32_t)bx;
+  } else {
+    slice = b / per_slice;
+    const long long bb = b - slice * per_slice;
+    yb = bb / bx;
+    xb = bb - yb * bx;
+  }
+}
+
+template <int ELEM, bool VEC>
+__global__ void __launch_bounds__(kZfpThreads)
+zfp_encode_kernel(const void* __restrict__ x, uint8_t* __restrict__ stream, long long nblocks, long long rows, long long M,
+                  int rate) {
+  __shared__ uint32_t planes[16 * kZfpThreads];
+  __shared__ uint32_t words[kZfpMaxWords * kZfpThreads];
+  const long long b = (long long)blockIdx.x * kZfpThreads + threadIdx.x;
+  if (b >= nblocks) return;                       // no barrier below: every thread uses its own column only
+  long long slice, yb, xb;
+  zfp_block_at(b, nblocks, rows, M, slice, yb, xb);
+  float f[16];
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const long long row = yb * 4 + r;
+    if (row < rows) {
+      zfp_load_row<ELEM, VEC>(x, (slice * rows + row) * M + xb * 4, f + r * 4);
+    } else {
+      f[r * 4] = f[r * 4 + 1] = f[r * 4 + 2] = f[r * 4 + 3] = 0.f;
+    }
+  }
+  uint32_t* w = words + threadIdx.x;
+  zfp_encode_block_planes(f, planes + threadIdx.x, w, kZfpThreads, 16 * rate);
+  uint8_t* dst = stream + b * (2 * rate);         // the stream is a fresh allocation: 8-byte stores are aligned
+  for (int i = 0; i < rate / 2; i += 2)
+    *reinterpret_cast<uint2*>(dst + 4 * i) = make_uint2(w[i * kZfpThreads], w[(i + 1) * kZfpThreads]);
+}
+
+template <int ELEM, bool VEC, bool WIDE>
+__global__ void __launch_bounds__(kZfpThreads)
+zfp_decode_kernel(const uint8_t* __restrict__ stream, void* __restrict__ x, long long nblocks, long long rows, long long M,
+                  int rate) {
+  __shared__ uint32_t planes[16 * kZfpThreads];
+  __shared__ uint32_t words[kZfpMaxWords * kZfpThreads];
+  const long long b = (long long)blockIdx.x * kZfpThreads + threadIdx.x;
+  if (b >= nblocks) return;
+  uint32_t* w = words + threadIdx.x;
+  const uint8_t* src = stream + b * (2 * rate);
+  for (int i = 0; i < rate / 2; i += 2) {
+    if constexpr (WIDE) {                         // the stream starts on an 8-byte boundary
+      const uint2 v = *reinterpret_cast<const uint2*>(src + 4 * i);
+      w[i * kZfpThreads] = v.x;
+      w[(i + 1) * kZfpThreads] = v.y;
+    } else {
+      w[i * kZfpThreads] = reinterpret_cast<const uint32_t*>(src)[i];
+      w[(i + 1) * kZfpThreads] = reinterpret_cast<const uint32_t*>(src)[i + 1];
+    }
+  }
+  float f[16];
+  zfp_decode_block_planes(w, f, planes + threadIdx.x, kZfpThreads, 16 * rate);
+  long long slice, yb, xb;
+  zfp_block_at(b, nblocks, rows, M, slice, yb, xb);
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const long long row = yb * 4 + r;
+    if (row < rows) zfp_store_row<ELEM, VEC>(x, (slice * rows + row) * M + xb * 4, f + r * 4);
+  }
+}
+
+template <int ELEM>
+void zfp_launch(bool encode, const void* x_in, void* x_out, uint8_t* stream, long long nblocks, long long rows, long long M,
+                int rate, cudaStream_t s) {
+  const unsigned grid = (unsigned)((nblocks + kZfpThreads - 1) / kZfpThreads);
+  const uintptr_t base = reinterpret_cast<uintptr_t>(encode ? x_in : x_out);
+  const bool vec = base % (4 * sizeof(typename ZfpElem<ELEM>::type)) == 0;
+  const bool wide = reinterpret_cast<uintptr_t>(stream) % 8 == 0;
+  if (encode) {
+    if (vec) zfp_encode_kernel<ELEM, true><<<grid, kZfpThreads, 0, s>>>(x_in, stream, nblocks, rows, M, rate);
+    else zfp_encode_kernel<ELEM, false><<<grid, kZfpThreads, 0, s>>>(x_in, stream, nblocks, rows, M, rate);
+  } else {
+    if (vec && wide) zfp_decode_kernel<ELEM, true, true><<<grid, kZfpThreads, 0, s>>>(stream, x_out, nblocks, rows, M, rate);
+    else zfp_decode_kernel<ELEM, false, false><<<grid, kZfpThreads, 0, s>>>(stream, x_out, nblocks, rows, M, rate);
+  }
+}
+void zfp_launch_elem(bool encode, const void* x_in, void* x_out, int elem, uint8_t* stream, long long n, long long rows,
+                     long long M, int rate, cudaStream_t s) {
+  if (n <= 0) return;
+  if (elem == 0) zfp_launch<0>(encode, x_in, x_out, stream, n, rows, M, rate, s);
+  else if (elem == 1) zfp_launch<1>(encode, x_in, x_out, stream, n, rows, M, rate, s);
+  else zfp_launch<2>(encode, x_in, x_out, stream, n, rows, M, rate, s);
 }
 
 }  // namespace
@@ -124,16 +232,11 @@ void zfp_decode_cpu(const uint8_t* stream, void* x, int elem, long long lead, lo
 }
 void launch_zfp_encode(const void* x, int elem, uint8_t* stream, long long lead, long long rows, long long M, int rate,
                        cudaStream_t s) {
-  const long long n = lead * ((rows + 3) / 4) * (M / 4);
-  if (n <= 0) return;
-  zfp_kernel<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(true, x, nullptr, elem, stream, n, rows, M, rate);
+  zfp_launch_elem(true, x, nullptr, elem, stream, lead * ((rows + 3) / 4) * (M / 4), rows, M, rate, s);
 }
 void launch_zfp_decode(const uint8_t* stream, void* x, int elem, long long lead, long long rows, long long M, int rate,
                        cudaStream_t s) {
-  const long long n = lead * ((rows + 3) / 4) * (M / 4);
-  if (n <= 0) return;
-  zfp_kernel<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(false, nullptr, x, elem, const_cast<uint8_t*>(stream), n, rows, M,
-                                                        rate);
+  zfp_launch_elem(false, nullptr, x, elem, const_cast<uint8_t*>(stream), lead * ((rows + 3) / 4) * (M / 4), rows, M, rate, s);
 }
 
 // ------------------------------------------------------------------------------------------------
