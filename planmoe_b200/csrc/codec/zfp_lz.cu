@@ -260,180 +260,159 @@ __host__ __device__ inline void lz_decode_one(const uint8_t* packed, uint8_t* ra
   else lz_decode_block<uint32_t>(packed, reinterpret_cast<uint32_t*>(raw + off), bytes / 4);
 }
 
-// scratch layout: [slices][nb] slots of kLzSlotBytes, then int sizes [slices][nb]
+// Warp-parallel block coder.  One warp codes one 2 KiB block, 32 positions ("a row") at a time, and produces exactly
+// the bytes of the serial coder lz_encode_block (the CPU twin, which the tests compare against).  A row's symbols are
+// held bit-sliced: B[b] is the ballot of bit b over the row.
+//   1. lane d compares the row with the symbols d + 1 positions back: all 32 positions at once, by and-ing, over the
+//      symbol's bits, B[b] with itself shifted across the row boundary.  A 32 x 32 bit transpose over the warp turns
+//      that into one mask of candidate distances per position (bit d set: in[p] == in[p - d - 1]).
+//   2. a candidate at distance d matches L symbols from p exactly when the masks of p .. p + L - 1 all have bit d, so
+//      the longest match comes from and-ing masks until nothing survives, and the first candidate of maximal length
+//      (the serial coder's choice) is the largest surviving distance.  Matches are at most 32 long: the masks of this
+//      row and the next are enough.
+//   3. token starts are the positions reachable from 0 by p + (match ? length : 1).  Every lane gets, by pointer doubling
+//      over the row, the set of starts a walk from it visits and where that walk enters the next row; the row's own
+//      entry picks one of them.
+//   4. the row's tokens are written at their ordinals; their flags are compressed by one or-reduction.
+// Bound by issue: the former coder compared through shared memory, 32 loads a position, then walked its tokens
+// serially per lane (13.7 k warp instructions a block; 537 us for 8192 x 4096 bf16).
 //
-// Warp-parallel block coder.  One warp codes one 2 KiB block and produces exactly the bytes of the
-// serial coder lz_encode_block (the CPU twin, which the tests compare against):
-//   1. every lane finds, for its positions p = lane, lane + 32, ..., the longest match in the 32-symbol
-//      window (first candidate of maximal length), as the serial coder would if a token started at p, from
-//      per-position candidate bit masks;
-//   2. the token starts are the positions reachable from 0 by next(p) = p + (match ? length : 1): each lane
-//      owns a segment of 32 positions, computes where a walk from each of them leaves the segment, the exits
-//      are chained from position 0 to give every segment its entry, and each lane walks its own segment;
-//   3. token ordinals and data offsets come from a warp scan over the per-segment counts of that walk;
-//   4. a second walk assembles flags and data in shared memory, which are then copied to the block's slot.
+// scratch layout: [slices][nb] slots of kLzScratchSlot bytes {token data, flag words, token count}, then int sizes
+// [slices][nb] (bytes of the block's code)
 constexpr int kLzWarps = 4;                       // blocks coded per CTA
-constexpr int kLzMaxSym = kLzBlockBytes / 2;      // symbols per block with 16-bit symbols
+constexpr int kLzScratchFlags = kLzBlockBytes;
+constexpr int kLzScratchCount = kLzScratchFlags + 128;
+constexpr int kLzScratchSlot = kLzScratchCount + 16;
+static_assert(kLzWindow == 32 && kLzMaxMatch == 32 && kLzScratchSlot % 16 == 0, "lz encoder: rows of 32, distance masks");
 
-constexpr int kLzInfoWords = 32 * 33;             // position p lives at word (p % 32) * 33 + p / 32 (see lz_tp)
-
-template <class Sym>
-struct LzEncSmem {
-  Sym in[kLzBlockBytes / sizeof(Sym)];
-  // One word per position, written at the end of step 1: bits 0-10 next(p) = p + (match ? length : 1), bit 31
-  // match; a match has its length in bits 11-16 and its distance in bits 17-22, a 16-bit literal its symbol in
-  // bits 11-26.
-  uint32_t info[kLzInfoWords];
-  uint32_t flagw[kLzMaxSym / 32];                 // one bit per token: 1 = match
-  // step 1: candidate masks eq[1024]; afterwards: exit positions (u16 [kLzInfoWords]) and the token payload
-  uint32_t scratch[(kLzInfoWords * 2 + kLzBlockBytes + 3) / 4];
-  __device__ uint32_t* eq() { return scratch; }
-  __device__ uint16_t* exits() { return reinterpret_cast<uint16_t*>(scratch); }
-  __device__ uint8_t* data() { return reinterpret_cast<uint8_t*>(scratch) + kLzInfoWords * 2; }
-};
-static_assert(kLzWindow == 32 && kLzMaxMatch <= 32 && kLzMaxSym <= 1024, "lz encoder: masks, info fields and segments");
-static_assert(sizeof(LzEncSmem<uint16_t>::scratch) >= kLzMaxSym * 4, "eq() needs one word per position");
-
-// Positions are handed to lanes in two ways: strided (p = k * 32 + lane, steps 1) and in segments of 32 consecutive
-// positions per lane (steps 2-4).  This index keeps both conflict-free or nearly so: strided writes hit 32 banks,
-// and lanes walking their segments in lock-step (same offset) do too.
-__device__ __forceinline__ int lz_tp(int p) { return (p & 31) * 33 + (p >> 5); }
+// Bit c of lane r becomes bit r of lane c.
+__device__ __forceinline__ uint32_t warp_transpose32(uint32_t x, int lane) {
+#pragma unroll
+  for (int s = 16; s > 0; s >>= 1) {
+    const uint32_t m = s == 16 ? 0x0000ffffu : s == 8 ? 0x00ff00ffu : s == 4 ? 0x0f0f0f0fu : s == 2 ? 0x33333333u : 0x55555555u;
+    const uint32_t keep = (lane & s) ? ~m : m;
+    const uint32_t y = __shfl_xor_sync(0xffffffffu, x, s);
+    const uint32_t rot = __funnelshift_l(y, y, (lane & s) ? 32 - s : s);
+    x = (x & keep) | (rot & ~keep);
+  }
+  return x;
+}
 
 template <class Sym>
-__device__ __forceinline__ void lz_encode_block_warp(const Sym* __restrict__ g_in, int nsym, uint8_t* __restrict__ out,
-                                                     int* __restrict__ out_size, LzEncSmem<Sym>& sm, int lane) {
+__device__ __forceinline__ void lz_encode_block_warp(const Sym* __restrict__ in, int nsym, uint8_t* __restrict__ slot,
+                                                     int* __restrict__ out_size, uint32_t* eqs, int lane) {
+  constexpr int kBits = 8 * (int)sizeof(Sym);
   constexpr int min_match = sizeof(Sym) == 2 ? 2 : 1;
-  for (int i = lane; i < nsym; i += 32) sm.in[i] = g_in[i];
-  for (int i = lane; i < kLzMaxSym / 32; i += 32) sm.flagw[i] = 0u;
-  __syncwarp();
-
-  // 1. longest match per position.  eq[q] has bit d-1 set when in[q - d] == in[q] (d = 1 .. 32): a candidate at
-  // distance d matches L symbols from p exactly when eq[p] & eq[p + 1] & ... & eq[p + L - 1] keeps bit d-1, so the
-  // longest match is found by and-ing masks until nothing survives, and the first candidate of maximal length
-  // (the serial coder's choice) is the largest surviving distance.
-  uint32_t* eq = sm.eq();
-  for (int p = lane; p < nsym; p += 32) {
-    const Sym v = sm.in[p];
-    uint32_t m = 0u;
-    const int dmax = p < kLzWindow ? p : kLzWindow;
-#pragma unroll 8
-    for (int d = 1; d <= dmax; ++d) m |= (sm.in[p - d] == v ? 1u : 0u) << (d - 1);
-    eq[p] = m;
-  }
-  __syncwarp();
-  uint32_t info_r[kLzMaxSym / 32];                  // eq shares its memory with later steps: results wait in registers
+  const uint32_t lt = (1u << lane) - 1u;
+  uint16_t* data = reinterpret_cast<uint16_t*>(slot);
+  uint32_t* flag_words = reinterpret_cast<uint32_t*>(slot + kLzScratchFlags);
+  uint32_t prev[kBits];                           // the row before, bit-sliced
 #pragma unroll
-  for (int k = 0; k < kLzMaxSym / 32; ++k) {
-    const int p = k * 32 + lane;
-    uint32_t w = 0u;
-    if (p < nsym) {
-      const int lim = nsym - p < kLzMaxMatch ? nsym - p : kLzMaxMatch;
-      uint32_t m = eq[p];
-      int best = 0;
-      if (m != 0u) {
-        best = 1;
-        while (best < lim) {
-          const uint32_t m2 = m & eq[p + best];
-          if (m2 == 0u) break;
-          m = m2;
-          ++best;
-        }
-      }
-      if (best >= min_match && best > 0) {
-        w = 0x80000000u | (uint32_t)(p + best) | ((uint32_t)best << 11) | ((uint32_t)(32 - __clz(m)) << 17);
-      } else {
-        w = (uint32_t)(p + 1);
-        if (sizeof(Sym) == 2) w |= (uint32_t)sm.in[p] << 11;
+  for (int b = 0; b < kBits; ++b) prev[b] = 0u;
+  const int rows = (nsym + 31) >> 5;
+  auto row_mask = [&](int k) { const int left = nsym - k * 32; return left >= 32 ? 0xffffffffu : (1u << left) - 1u; };
+  auto load = [&](int k) { const int p = k * 32 + lane; return p < nsym ? in[p] : (Sym)0; };
+  auto candidates = [&](Sym v, int k) {
+    uint32_t acc = row_mask(k);
+    if (k == 0) acc &= ~((2u << lane) - 1u);      // nothing lies before position 0
+#pragma unroll
+    for (int b = 0; b < kBits; ++b) {
+      const uint32_t cur = __ballot_sync(0xffffffffu, (v >> b) & 1u);
+      acc &= ~(cur ^ __funnelshift_lc(prev[b], cur, lane + 1));
+      prev[b] = cur;
+    }
+    return warp_transpose32(acc, lane);
+  };
+
+  Sym v = load(0);
+  uint32_t eq = candidates(v, 0);                 // this lane's mask of row k
+  eqs[lane] = eq;
+  int entry = 0, ntok = 0, dbytes = 0;
+  uint64_t facc = 0;                              // flags not yet written, first token lowest
+  int fbits = 0;
+  Sym v_ahead = rows > 1 ? load(1) : (Sym)0;
+  for (int k = 0; k < rows; ++k) {
+    const Sym v_next = v_ahead;
+    uint32_t eq_next = 0u;
+    if (k + 1 < rows) eq_next = candidates(v_next, k + 1);
+    if (k + 2 < rows) v_ahead = load(k + 2);
+    eqs[((k + 1) & 1) * 32 + lane] = eq_next;
+    __syncwarp();
+
+    // 2. longest match (the first four symbols without a branch)
+    const int at = (k & 1) * 32 + lane;           // masks of positions p .. p + 31 lie at (at + i) & 63
+    const uint32_t m1 = eq & eqs[(at + 1) & 63];
+    const uint32_t m2 = m1 & eqs[(at + 2) & 63];
+    const uint32_t m3 = m2 & eqs[(at + 3) & 63];
+    int best = (eq != 0u) + (m1 != 0u) + (m2 != 0u) + (m3 != 0u);
+    uint32_t m = m1 ? m1 : eq;
+    m = m2 ? m2 : m;
+    if (m3) {
+      m = m3;
+      while (best < kLzMaxMatch) {
+        const uint32_t t = m & eqs[(at + best) & 63];
+        if (t == 0u) break;
+        m = t;
+        ++best;
       }
     }
-    info_r[k] = w;
-  }
-  __syncwarp();                                   // every lane is done reading eq
-#pragma unroll
-  for (int k = 0; k < kLzMaxSym / 32; ++k) {
-    const int p = k * 32 + lane;
-    if (p < nsym) sm.info[lz_tp(p)] = info_r[k];
-  }
-  __syncwarp();
+    const bool match = best >= min_match;
+    __syncwarp();                                 // the masks of row k are overwritten in the next round
 
-  // 2. token starts = positions reachable from 0 by next().  Lane l owns the segment [32 l, 32 l + 32).  (a) Going
-  // backwards through its segment every lane finds, for each position, where a walk from there leaves the
-  // segment; (b) following these exits from position 0, segment by segment, gives every segment its entry
-  // point (a jump is at most 32 long, so a walk enters each segment it does not end in); (c) each lane then
-  // walks its segment from its entry.
-  const int p0 = lane * 32, p1 = p0 + 32 < nsym ? p0 + 32 : nsym;
-  uint16_t* exits = sm.exits();
-  for (int o = p1 - p0 - 1; o >= 0; --o) {
-    const int nx = (int)(sm.info[o * 33 + lane] & 0x7ffu);
-    exits[o * 33 + lane] = (uint16_t)(nx >= p1 ? nx : exits[(nx & 31) * 33 + lane]);
-  }
-  __syncwarp();
-  int entry = -1;
-  {
-    int e = 0;
-    for (int l = 0; l < 32 && e < nsym; ++l) {
-      const int end = (l + 1) * 32 < nsym ? (l + 1) * 32 : nsym;
-      if (e < end) {
-        if (l == lane) entry = e;
-        e = exits[(e & 31) * 33 + l];
-      }
+    // 3. starts of this row and the entry into the next
+    uint32_t visits = 1u << lane;
+    int to = lane + (match ? best : 1);           // 32 and above: a position of the next row
+#pragma unroll
+    for (int r = 0; r < 5; ++r) {
+      const uint32_t vo = __shfl_sync(0xffffffffu, visits, to & 31);
+      const int too = __shfl_sync(0xffffffffu, to, to & 31);
+      if (to < 32) { visits |= vo; to = too; }
     }
-  }
+    const uint32_t starts = __shfl_sync(0xffffffffu, visits, entry) & row_mask(k);
+    entry = __shfl_sync(0xffffffffu, to, entry) & 31;
 
-  // 3. ordinals and data offsets from a first walk
-  int ntok_l = 0, bytes_l = 0;
-  for (int p = entry; p >= 0 && p < p1;) {
-    const uint32_t w = sm.info[(p & 31) * 33 + lane];
-    ++ntok_l;
-    bytes_l += (w >> 31) ? 2 : (int)sizeof(Sym);
-    p = (int)(w & 0x7ffu);
-  }
-  int tok_incl = ntok_l, byt_incl = bytes_l;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int t = __shfl_up_sync(0xffffffffu, tok_incl, o);
-    const int b = __shfl_up_sync(0xffffffffu, byt_incl, o);
-    if (lane >= o) { tok_incl += t; byt_incl += b; }
-  }
-  const int ntok = __shfl_sync(0xffffffffu, tok_incl, 31);
-  const int dbytes = __shfl_sync(0xffffffffu, byt_incl, 31);
-  int t = tok_incl - ntok_l, dpos = byt_incl - bytes_l;
-
-  // 4. flags + data from a second walk
-  uint8_t* data = sm.data();
-  for (int p = entry; p >= 0 && p < p1; ++t) {
-    const uint32_t w = sm.info[(p & 31) * 33 + lane];
-    if (w >> 31) {
-      atomicOr(&sm.flagw[t >> 5], 1u << (t & 31));
-      data[dpos++] = (uint8_t)((w >> 11) & 63u);
-      data[dpos++] = (uint8_t)((w >> 17) & 63u);
+    // 4. tokens
+    const bool is = (starts >> lane) & 1u;
+    const int r = __popc(starts & lt), cnt = __popc(starts);
+    const uint32_t flags = __reduce_or_sync(0xffffffffu, is && match ? 1u << r : 0u);
+    const uint32_t pair = (uint32_t)best | ((uint32_t)(32 - __clz(m)) << 8);
+    if constexpr (sizeof(Sym) == 2) {
+      if (is) data[ntok + r] = match ? (uint16_t)pair : (uint16_t)v;
+      dbytes += 2 * cnt;
     } else {
-      const uint32_t v = sizeof(Sym) == 2 ? ((w >> 11) & 0xffffu) : (uint32_t)sm.in[p];
-#pragma unroll
-      for (unsigned b = 0; b < sizeof(Sym); ++b) data[dpos++] = (uint8_t)(v >> (8 * b));
+      const uint32_t matches = __ballot_sync(0xffffffffu, is && match);
+      if (is) {
+        uint16_t* d = data + dbytes / 2 + 2 * r - __popc(matches & lt);
+        d[0] = match ? (uint16_t)pair : (uint16_t)v;
+        if (!match) d[1] = (uint16_t)(v >> 16);
+      }
+      dbytes += 4 * cnt - 2 * __popc(matches);
     }
-    p = (int)(w & 0x7ffu);
+    ntok += cnt;
+    facc |= (uint64_t)flags << fbits;
+    fbits += cnt;
+    if (fbits >= 32) {
+      if (lane == 0) *flag_words = (uint32_t)facc;
+      ++flag_words;
+      facc >>= 32;
+      fbits -= 32;
+    }
+    v = v_next;
+    eq = eq_next;
   }
-  __syncwarp();
-  const int flag_bytes = (ntok + 7) >> 3;
   if (lane == 0) {
-    out[0] = (uint8_t)(ntok & 0xff);
-    out[1] = (uint8_t)(ntok >> 8);
-    *out_size = 2 + flag_bytes + dbytes;
+    if (fbits > 0) *flag_words = (uint32_t)facc;
+    *reinterpret_cast<uint32_t*>(slot + kLzScratchCount) = (uint32_t)ntok;
+    *out_size = 2 + ((ntok + 7) >> 3) + dbytes;
   }
-  const uint8_t* fb = reinterpret_cast<const uint8_t*>(sm.flagw);
-  for (int i = lane; i < flag_bytes; i += 32) out[2 + i] = fb[i];
-  uint8_t* od = out + 2 + flag_bytes;
-  for (int i = lane; i < dbytes; i += 32) od[i] = data[i];
-  __syncwarp();
 }
 
 template <class Sym>
 __global__ void __launch_bounds__(kLzWarps * 32)
-lz_encode_blocks_kernel(const uint8_t* raw, uint8_t* slots, int* blk_sizes, long long slices, long long raw_bytes) {
-  extern __shared__ __align__(16) uint8_t lz_smem[];
+lz_encode_blocks_kernel(const uint8_t* __restrict__ raw, uint8_t* __restrict__ slots, int* __restrict__ blk_sizes,
+                        long long slices, long long raw_bytes) {
+  __shared__ uint32_t eqs[kLzWarps][64];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  LzEncSmem<Sym>& sm = reinterpret_cast<LzEncSmem<Sym>*>(lz_smem)[warp];
   const long long nb = lz_blocks(raw_bytes);
   const long long i = (long long)blockIdx.x * kLzWarps + warp;
   if (i >= slices * nb) return;
@@ -441,24 +420,27 @@ lz_encode_blocks_kernel(const uint8_t* raw, uint8_t* slots, int* blk_sizes, long
   const long long off = b * kLzBlockBytes;
   const int bytes = (int)(raw_bytes - off < kLzBlockBytes ? raw_bytes - off : kLzBlockBytes);
   lz_encode_block_warp<Sym>(reinterpret_cast<const Sym*>(raw + s * raw_bytes + off), bytes / (int)sizeof(Sym),
-                            slots + i * kLzSlotBytes, blk_sizes + i, sm, lane);
+                            slots + i * kLzScratchSlot, blk_sizes + i, eqs[warp], lane);
 }
 
-// one CTA per slice: exclusive scan of the block sizes -> header of the slice payload
-__global__ void __launch_bounds__(256)
-lz_scan_kernel(const int* blk_sizes, uint8_t* payload, int* sizes, long long raw_bytes, long long payload_stride) {
-  __shared__ unsigned carry;
-  __shared__ unsigned warp_tot[8];
+// One CTA per slice: exclusive scan of the block sizes -> header of the slice payload.  Four sizes a thread, so that a
+// slice of 8 MiB (4096 blocks) is one round.
+constexpr int kLzScanThreads = 1024;
+__global__ void __launch_bounds__(kLzScanThreads)
+lz_scan_kernel(const int* __restrict__ blk_sizes, uint8_t* __restrict__ payload, int* __restrict__ sizes, long long raw_bytes,
+               long long payload_stride) {
+  __shared__ unsigned warp_tot[32];
   const long long nb = lz_blocks(raw_bytes);
   const long long s = blockIdx.x;
   uint32_t* hdr = reinterpret_cast<uint32_t*>(payload + s * payload_stride);
-  if (threadIdx.x == 0) { carry = 0; hdr[0] = (uint32_t)nb; }
-  __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (long long base = 0; base < nb; base += 256) {
-    const long long i = base + threadIdx.x;
-    unsigned v = i < nb ? (unsigned)blk_sizes[s * nb + i] : 0u;
-    unsigned incl = v;
+  unsigned carry = 0;
+  for (long long base = 0; base < nb; base += 4 * kLzScanThreads) {
+    const long long i = base + 4 * threadIdx.x;
+    unsigned v[4], sum = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) { v[j] = i + j < nb ? (unsigned)blk_sizes[s * nb + i + j] : 0u; sum += v[j]; }
+    unsigned incl = sum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const unsigned t = __shfl_up_sync(0xffffffffu, incl, o);
@@ -466,112 +448,161 @@ lz_scan_kernel(const int* blk_sizes, uint8_t* payload, int* sizes, long long raw
     }
     if (lane == 31) warp_tot[warp] = incl;
     __syncthreads();
-    unsigned before = carry;
-    for (int w = 0; w < warp; ++w) before += warp_tot[w];
-    if (i < nb) hdr[1 + i] = before + incl - v;
-    __syncthreads();
-    if (threadIdx.x == 255) carry = before + incl;
-    __syncthreads();
+    unsigned tot = warp_tot[lane], wincl = tot;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned t = __shfl_up_sync(0xffffffffu, wincl, o);
+      if (lane >= o) wincl += t;
+    }
+    const unsigned before_warp = __shfl_sync(0xffffffffu, wincl - tot, warp);
+    unsigned at = carry + before_warp + incl - sum;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (i + j < nb) hdr[1 + i + j] = at;
+      at += v[j];
+    }
+    carry += __shfl_sync(0xffffffffu, wincl, 31);
+    __syncthreads();                              // warp_tot is written again in the next round
   }
   if (threadIdx.x == 0) {
+    hdr[0] = (uint32_t)nb;
     hdr[1 + nb] = carry;
     for (long long w = 2 + nb; w < lz_header_bytes(nb) / 4; ++w) hdr[w] = 0;   // header padding
     sizes[s] = (int)(lz_header_bytes(nb) + carry);
   }
 }
 
+// n bytes from a 4-byte aligned source to any address: byte stores up to the destination's next word, then whole words
+// put together from two source words (the word behind the last one that is copied may be read, not used).
+__device__ __forceinline__ void warp_copy_to_bytes(uint8_t* __restrict__ dst, const uint8_t* __restrict__ src, int n, int lane) {
+  const int head = min(n, (int)((4 - (reinterpret_cast<uintptr_t>(dst) & 3)) & 3));
+  if (lane < head) dst[lane] = src[lane];
+  const int words = (n - head) >> 2;
+  const uint32_t* s32 = reinterpret_cast<const uint32_t*>(src);
+  uint32_t* d32 = reinterpret_cast<uint32_t*>(dst + head);
+  for (int i = lane; i < words; i += 32) d32[i] = __funnelshift_r(s32[i], s32[i + 1], 8 * head);
+  const int done = head + 4 * words;
+  if (lane < n - done) dst[done + lane] = src[done + lane];
+}
+
+// One warp per block: {token count, flags, data} of its scratch slot to its place in the payload.  Word copies: byte
+// copies took 61 us for 8192 x 4096 bf16.
 __global__ void __launch_bounds__(128)
-lz_compact_kernel(const uint8_t* slots, const int* blk_sizes, uint8_t* payload, long long raw_bytes, long long payload_stride) {
-  // one warp per block: byte copy of the block's code into its packed position
+lz_compact_kernel(const uint8_t* __restrict__ slots, const int* __restrict__ blk_sizes, uint8_t* __restrict__ payload,
+                  long long raw_bytes, long long payload_stride) {
   const long long nb = lz_blocks(raw_bytes);
   const long long i = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
   const long long s = blockIdx.y;
+  const int lane = threadIdx.x & 31;
   if (i >= nb) return;
   const uint32_t* hdr = reinterpret_cast<const uint32_t*>(payload + s * payload_stride);
   uint8_t* dst = payload + s * payload_stride + lz_header_bytes(nb) + hdr[1 + i];
-  const uint8_t* src = slots + (s * nb + i) * kLzSlotBytes;
+  const uint8_t* src = slots + (s * nb + i) * kLzScratchSlot;
   const int n = blk_sizes[s * nb + i];
-  for (int k = threadIdx.x & 31; k < n; k += 32) dst[k] = src[k];
+  const int ntok = (int)*reinterpret_cast<const uint32_t*>(src + kLzScratchCount);
+  const int flag_bytes = (ntok + 7) >> 3;
+  if (lane < 2) dst[lane] = (uint8_t)(ntok >> (8 * lane));
+  warp_copy_to_bytes(dst + 2, src + kLzScratchFlags, flag_bytes, lane);
+  warp_copy_to_bytes(dst + 2 + flag_bytes, src, n - 2 - flag_bytes, lane);
 }
 
-// Warp-parallel block decoder (same output as lz_decode_block).  Tokens are expanded to a source map
-// (a literal is its own source; symbol i of a match sources position p - distance) from a warp scan of
-// token lengths; sources are resolved to literals with ten rounds of pointer doubling, because a match
-// may copy symbols that an earlier (or the same, overlapping) match produced.
-template <class Sym>
+// Warp-parallel block decoder (same output as lz_decode_block).  Tokens are laid out first, 32 at a time: a scan of
+// their lengths gives each its position, where it leaves one word {start mark, literal or distance}.  Positions are then
+// resolved a row of 32 at a time: a position belongs to the last start at or before it; a source in an earlier row is
+// already known, a source in the same row (matches may copy what an earlier or the same match produced) is reached by
+// five rounds of pointer doubling in registers.  The former decoder doubled pointers ten times over the whole block
+// in shared memory (285 us for 8192 x 4096 bf16).
+constexpr int kLzCodeWords = (3 + kLzSlotBytes + 3) / 4;
+constexpr int kLzMaxSym = kLzBlockBytes / 2;
 struct LzDecSmem {
-  uint8_t code[kLzSlotBytes + 2];                 // the block's code bytes
-  Sym val[kLzBlockBytes / sizeof(Sym)];           // literal value at p (defined where src[p] == p)
-  uint16_t src[2][kLzMaxSym];
+  uint32_t code[kLzCodeWords + 1];                // the block's code, as it lies in global words
+  uint32_t info[kLzMaxSym];                       // token words, then the decoded symbols
 };
 
 template <class Sym>
 __device__ __forceinline__ void lz_decode_block_warp(const uint8_t* __restrict__ g_code, int code_bytes,
-                                                     Sym* __restrict__ g_out, int nsym, LzDecSmem<Sym>& sm, int lane) {
-  for (int i = lane; i < code_bytes; i += 32) sm.code[i] = g_code[i];
-  for (int q = lane; q < nsym; q += 32) { sm.src[0][q] = (uint16_t)q; sm.val[q] = (Sym)0; }   // defined even for a short code
+                                                     Sym* __restrict__ g_out, int nsym, LzDecSmem& sm, int lane) {
+  const int mis = (int)(reinterpret_cast<uintptr_t>(g_code) & 3);
+  const uint32_t* g_words = reinterpret_cast<const uint32_t*>(g_code - mis);
+  const int whole = (mis + code_bytes) >> 2, tail = (mis + code_bytes) & 3;
+  for (int i = lane; i < whole; i += 32) sm.code[i] = g_words[i];
+  uint8_t* code = reinterpret_cast<uint8_t*>(sm.code) + mis;
+  if (lane < tail) reinterpret_cast<uint8_t*>(sm.code + whole)[lane] = reinterpret_cast<const uint8_t*>(g_words + whole)[lane];
+  const int rows = (nsym + 31) >> 5;
+  for (int k = 0; k < rows; ++k) sm.info[k * 32 + lane] = 0u;
   __syncwarp();
-  const int ntok = (int)sm.code[0] | ((int)sm.code[1] << 8);
-  const uint8_t* flags = sm.code + 2;
-  const uint8_t* data = flags + ((ntok + 7) >> 3);
+  const uint32_t lt = (1u << lane) - 1u;
+  const int ntok = min((int)code[0] | ((int)code[1] << 8), nsym);
+  const int flag_bytes = (ntok + 7) >> 3;
+  const int data_at = 2 + flag_bytes;
+  const int last = code_bytes - 1;                // reads of a damaged code stay inside it
 
-  // lane owns tokens [t0, t1): first their data bytes, then (needs the lengths) their output symbols
-  const int seg = (ntok + 31) / 32;
-  const int t0 = lane * seg < ntok ? lane * seg : ntok, t1 = t0 + seg < ntok ? t0 + seg : ntok;
-  int byt_l = 0;
-  for (int t = t0; t < t1; ++t) byt_l += ((flags[t >> 3] >> (t & 7)) & 1u) ? 2 : (int)sizeof(Sym);
-  int byt_incl = byt_l;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int b = __shfl_up_sync(0xffffffffu, byt_incl, o);
-    if (lane >= o) byt_incl += b;
-  }
-  int dpos = byt_incl - byt_l;
-  int sym_l = 0;
-  {
-    int d = dpos;
-    for (int t = t0; t < t1; ++t) {
-      if ((flags[t >> 3] >> (t & 7)) & 1u) { sym_l += data[d]; d += 2; }
-      else { sym_l += 1; d += (int)sizeof(Sym); }
+  int total = 0, lits = 0;
+  for (int t0 = 0; t0 < ntok; t0 += 32) {
+    const int t = t0 + lane;
+    const bool live = t < ntok;
+    const bool match = live && ((code[min(2 + (t >> 3), last)] >> (t & 7)) & 1u);
+    int off = data_at + 2 * t;
+    if constexpr (sizeof(Sym) == 4) {
+      const uint32_t lit = __ballot_sync(0xffffffffu, live && !match);
+      off += 2 * (lits + __popc(lit & lt));
+      lits += __popc(lit);
     }
-  }
-  int sym_incl = sym_l;
+    const uint32_t b0 = code[min(off, last)], b1 = code[min(off + 1, last)];
+    const int len = !live ? 0 : match ? (int)b0 : 1;
+    int incl = len;
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int b = __shfl_up_sync(0xffffffffu, sym_incl, o);
-    if (lane >= o) sym_incl += b;
-  }
-  int p = sym_incl - sym_l;
-  for (int t = t0; t < t1; ++t) {
-    if ((flags[t >> 3] >> (t & 7)) & 1u) {
-      const int len = data[dpos], dist = data[dpos + 1];
-      dpos += 2;
-      for (int i = 0; i < len && p < nsym; ++i, ++p) sm.src[0][p] = (uint16_t)(p - dist > 0 ? p - dist : 0);
-    } else {
-      uint32_t v = 0;
-#pragma unroll
-      for (unsigned b = 0; b < sizeof(Sym); ++b) v |= (uint32_t)data[dpos++] << (8 * b);
-      if (p < nsym) { sm.val[p] = (Sym)v; sm.src[0][p] = (uint16_t)p; }
-      ++p;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int n = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += n;
     }
+    const int p = total + incl - len;
+    if (live && p < nsym)
+      sm.info[p] = match ? 0xc0000000u | b1 : 0x80000000u | (sizeof(Sym) == 2 ? b0 | (b1 << 8) : (uint32_t)off);
+    total += __shfl_sync(0xffffffffu, incl, 31);
   }
   __syncwarp();
-  int cur = 0;
-  for (int hop = 1; hop < nsym; hop <<= 1) {
-    for (int q = lane; q < nsym; q += 32) sm.src[cur ^ 1][q] = sm.src[cur][sm.src[cur][q]];
+  uint32_t carry = 0u;                            // the last token that starts before the row
+  for (int k = 0; k < rows; ++k) {
+    const int p = k * 32 + lane;
+    const uint32_t w = sm.info[p];
+    const uint32_t starts = __ballot_sync(0xffffffffu, w >> 31);
+    const uint32_t upto = starts & (lt | (1u << lane));
+    uint32_t own = __shfl_sync(0xffffffffu, w, upto ? 31 - __clz(upto) : 0);
+    if (upto == 0u) own = carry;
+    if (starts != 0u) carry = __shfl_sync(0xffffffffu, w, 31 - __clz(starts));
+    uint32_t val = 0u;
+    int from = lane;
+    if (p < total) {
+      if (own & 0x40000000u) {
+        const int src = max(p - (int)(own & 0xffu), 0);
+        if (src < k * 32) val = sm.info[src];
+        else from = src & 31;
+      } else if (w >> 31) {
+        if constexpr (sizeof(Sym) == 2) {
+          val = w & 0xffffu;
+        } else {
+          const int off = (int)(w & 0xffffu);
+#pragma unroll
+          for (int b = 0; b < 4; ++b) val |= (uint32_t)code[min(off + b, last)] << (8 * b);
+        }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < 5; ++r) from = __shfl_sync(0xffffffffu, from, from);
+    val = __shfl_sync(0xffffffffu, val, from);
+    sm.info[p] = val;
+    if (p < nsym) g_out[p] = (Sym)val;
     __syncwarp();
-    cur ^= 1;
   }
-  for (int q = lane; q < nsym; q += 32) g_out[q] = sm.val[sm.src[cur][q]];
-  __syncwarp();
 }
 
 template <class Sym>
 __global__ void __launch_bounds__(kLzWarps * 32)
-lz_decode_blocks_kernel(const uint8_t* payload, uint8_t* raw, long long slices, long long raw_bytes, long long payload_stride) {
-  extern __shared__ __align__(16) uint8_t lz_smem[];
+lz_decode_blocks_kernel(const uint8_t* __restrict__ payload, uint8_t* __restrict__ raw, long long slices, long long raw_bytes,
+                        long long payload_stride) {
+  __shared__ LzDecSmem smem[kLzWarps];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  LzDecSmem<Sym>& sm = reinterpret_cast<LzDecSmem<Sym>*>(lz_smem)[warp];
   const long long nb = lz_blocks(raw_bytes);
   const long long i = (long long)blockIdx.x * kLzWarps + warp;
   if (i >= slices * nb) return;
@@ -583,7 +614,7 @@ lz_decode_blocks_kernel(const uint8_t* payload, uint8_t* raw, long long slices, 
   const int code_bytes = (int)(hdr[2 + b] - hdr[1 + b]);
   if (code_bytes < 2 || code_bytes > kLzSlotBytes) return;       // corrupt header: leave the block untouched
   lz_decode_block_warp<Sym>(base + lz_header_bytes(nb) + hdr[1 + b], code_bytes,
-                            reinterpret_cast<Sym*>(raw + s * raw_bytes + off), bytes / (int)sizeof(Sym), sm, lane);
+                            reinterpret_cast<Sym*>(raw + s * raw_bytes + off), bytes / (int)sizeof(Sym), smem[warp], lane);
 }
 
 }  // namespace
@@ -599,7 +630,7 @@ void lz_slice_layout(long long raw_bytes, long long* len_off, long long* header_
 }
 size_t lz_scratch_bytes(long long slices, long long raw_bytes) {
   const long long nb = lz_blocks(raw_bytes);
-  return (size_t)(slices * nb * (kLzSlotBytes + 4) + 16);
+  return (size_t)(slices * nb * (kLzScratchSlot + 4));
 }
 
 void lz_encode_cpu(const uint8_t* raw, uint8_t* payload, int* sizes, long long slices, long long raw_bytes,
@@ -639,20 +670,13 @@ void launch_lz_encode(const uint8_t* raw, uint8_t* payload, int* sizes, uint8_t*
   const long long total = slices * nb;
   if (total <= 0) return;
   uint8_t* slots = scratch;
-  int* blk_sizes = reinterpret_cast<int*>(scratch + (total * kLzSlotBytes + 15) / 16 * 16);
+  int* blk_sizes = reinterpret_cast<int*>(scratch + total * kLzScratchSlot);
   const unsigned ctas = (unsigned)((total + kLzWarps - 1) / kLzWarps);
-  if (sym == 2) {
-    constexpr int smem = kLzWarps * (int)sizeof(LzEncSmem<uint16_t>);
-    static bool once = false;
-    if (!once) { cudaFuncSetAttribute(lz_encode_blocks_kernel<uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); once = true; }
-    lz_encode_blocks_kernel<uint16_t><<<ctas, kLzWarps * 32, smem, stream>>>(raw, slots, blk_sizes, slices, raw_bytes);
-  } else {
-    constexpr int smem = kLzWarps * (int)sizeof(LzEncSmem<uint32_t>);
-    static bool once = false;
-    if (!once) { cudaFuncSetAttribute(lz_encode_blocks_kernel<uint32_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); once = true; }
-    lz_encode_blocks_kernel<uint32_t><<<ctas, kLzWarps * 32, smem, stream>>>(raw, slots, blk_sizes, slices, raw_bytes);
-  }
-  lz_scan_kernel<<<(unsigned)slices, 256, 0, stream>>>(blk_sizes, payload, sizes, raw_bytes, payload_stride);
+  if (sym == 2)
+    lz_encode_blocks_kernel<uint16_t><<<ctas, kLzWarps * 32, 0, stream>>>(raw, slots, blk_sizes, slices, raw_bytes);
+  else
+    lz_encode_blocks_kernel<uint32_t><<<ctas, kLzWarps * 32, 0, stream>>>(raw, slots, blk_sizes, slices, raw_bytes);
+  lz_scan_kernel<<<(unsigned)slices, kLzScanThreads, 0, stream>>>(blk_sizes, payload, sizes, raw_bytes, payload_stride);
   dim3 grid((unsigned)((nb + 3) / 4), (unsigned)slices);
   lz_compact_kernel<<<grid, 128, 0, stream>>>(slots, blk_sizes, payload, raw_bytes, payload_stride);
 }
@@ -661,17 +685,10 @@ void launch_lz_decode(const uint8_t* payload, uint8_t* raw, long long slices, lo
   const long long total = slices * lz_blocks(raw_bytes);
   if (total <= 0) return;
   const unsigned ctas = (unsigned)((total + kLzWarps - 1) / kLzWarps);
-  if (sym == 2) {
-    constexpr int smem = kLzWarps * (int)sizeof(LzDecSmem<uint16_t>);
-    static bool once = false;
-    if (!once) { cudaFuncSetAttribute(lz_decode_blocks_kernel<uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); once = true; }
-    lz_decode_blocks_kernel<uint16_t><<<ctas, kLzWarps * 32, smem, stream>>>(payload, raw, slices, raw_bytes, payload_stride);
-  } else {
-    constexpr int smem = kLzWarps * (int)sizeof(LzDecSmem<uint32_t>);
-    static bool once = false;
-    if (!once) { cudaFuncSetAttribute(lz_decode_blocks_kernel<uint32_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); once = true; }
-    lz_decode_blocks_kernel<uint32_t><<<ctas, kLzWarps * 32, smem, stream>>>(payload, raw, slices, raw_bytes, payload_stride);
-  }
+  if (sym == 2)
+    lz_decode_blocks_kernel<uint16_t><<<ctas, kLzWarps * 32, 0, stream>>>(payload, raw, slices, raw_bytes, payload_stride);
+  else
+    lz_decode_blocks_kernel<uint32_t><<<ctas, kLzWarps * 32, 0, stream>>>(payload, raw, slices, raw_bytes, payload_stride);
 }
 
 }  // namespace planmoe

@@ -46,3 +46,36 @@ def test_zfp_forms_match_the_serial_coder(dtype, offset, kind):
         assert torch.equal(y_gpu.cpu(), y_cpu)
         shifted = torch.empty(s_gpu.numel() + 4, dtype=torch.uint8, device='cuda')[4:].view_as(s_gpu).copy_(s_gpu)
         assert torch.equal(lib.zfp_decode(shifted, lead, rows, cols, rate, dtype), y_gpu)
+
+
+@pytest.mark.parametrize('sym', [2, 4])
+@pytest.mark.parametrize('nbytes', [16, 48, 2032, 2048, 2064, 6160, 40960])
+@pytest.mark.parametrize('kind', ['zeros', 'period', 'few', 'relu', 'random', 'runs'])
+def test_lz_forms_match_the_serial_coder(sym, nbytes, kind):
+    """Tail blocks of every raggedness, matches of the greatest length and distance, codes that start on any byte."""
+    lib = _lib()
+    gen = torch.Generator().manual_seed(3)
+    slices, n = 3, nbytes // sym
+    if kind == 'zeros':
+        v = torch.zeros(slices, n, dtype=torch.int32)
+    elif kind == 'period':                       # matches reach back exactly 32 symbols, and 33 (too far)
+        v = torch.stack([torch.arange(n) % p for p in (32, 33, 31)]).int()
+    elif kind == 'few':
+        v = torch.randint(0, 3, (slices, n), generator=gen).int()
+    elif kind == 'relu':
+        x = torch.relu(torch.randn(slices, n, generator=gen))
+        v = x.view(torch.int32) if sym == 4 else x.bfloat16().view(torch.int16).int()
+    elif kind == 'random':
+        v = torch.randint(-2 ** 31, 2 ** 31 - 1, (slices, n), generator=gen, dtype=torch.int64).int()
+    else:                                        # runs of uneven length, some longer than a match can be
+        v = torch.repeat_interleave(torch.arange(slices * n), torch.randint(1, 90, (slices * n,), generator=gen))
+        v = v[:slices * n].view(slices, n).int()
+    raw = (v if sym == 4 else v.to(torch.int16)).contiguous().view(torch.uint8).view(slices, -1)
+    p_cpu, n_cpu = lib.lz_encode(raw, sym)
+    p_gpu, n_gpu = lib.lz_encode(raw.cuda(), sym)
+    assert torch.equal(n_gpu.cpu(), n_cpu)
+    for s in range(slices):
+        used = int(n_cpu[s])
+        assert torch.equal(p_gpu[s, :used].cpu(), p_cpu[s, :used])
+    assert torch.equal(lib.lz_decode(p_gpu, n_gpu, raw.size(1), sym).cpu(), raw)
+    assert torch.equal(lib.lz_decode(p_cpu.cuda(), n_cpu.cuda(), raw.size(1), sym).cpu(), raw)
