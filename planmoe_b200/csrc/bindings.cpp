@@ -7,6 +7,7 @@
 // becomes the symmetric-heap runtime, the FIFO compress/comm/decompress triple becomes explicit
 // handles on the Python side.
 
+#include <climits>
 #include <torch/extension.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAStream.h>
@@ -228,6 +229,9 @@ void remap_slot_map_op(Tensor& slot_map, const Tensor& perm, int64_t K) {
 
 // ---- fused gate -------------------------------------------------------------------------------
 // returns (idx[K,S] i32, loc[K,S] i32, gates[K,S] f32, slot_map[E*C] i32, top1_count[E] i32, l_aux[1] f32)
+constexpr float kFloatEps = 1.1920929e-07f;
+float gate_eps(at::ScalarType t) { return t == at::kFloat ? kFloatEps : (t == at::kHalf ? 9.765625e-04f : 7.8125e-03f); }
+
 std::vector<Tensor> gate_forward_op(const Tensor& logits, int64_t K, int64_t C, bool normalize) {
   count_launch(2);
   TORCH_CHECK(logits.is_cuda() && logits.dim() == 2 && logits.is_contiguous());
@@ -236,22 +240,22 @@ std::vector<Tensor> gate_forward_op(const Tensor& logits, int64_t K, int64_t C, 
   c10::cuda::CUDAGuard guard(logits.device());
   auto iopt = logits.options().dtype(at::kInt);
   auto fopt = logits.options().dtype(at::kFloat);
+  const int nblk = gate_workspace_blocks(S);
   Tensor idx = torch::empty({K, S}, iopt), loc = torch::empty({K, S}, iopt);
-  Tensor gates = torch::empty({K, S}, fopt), raw = torch::empty({K, S}, fopt);
+  Tensor gates = torch::empty({K, S}, fopt);
   Tensor smap = torch::empty({(int64_t)E * C}, iopt);
   Tensor top1 = torch::empty({E}, iopt), laux = torch::empty({1}, fopt);
-  const int nblk = gate_workspace_blocks(S);
-  Tensor ws_rank = torch::empty({K, S}, iopt);
-  Tensor ws_cnt = torch::empty({nblk, K, E}, iopt);
-  Tensor ws_score = torch::empty({nblk, E}, fopt);
-  const float eps = logits.scalar_type() == at::kFloat ? 1.1920929e-07f
-                    : (logits.scalar_type() == at::kHalf ? 9.765625e-04f : 7.8125e-03f);
+  // scratch of this call: raw gates, in-block ranks, per-block histograms and score sums
+  Tensor ws = torch::empty({2 * K * S + (K + 1) * (int64_t)nblk * E}, iopt);
+  int* w = ws.data_ptr<int>();
+  GatePtrs gp{};
+  for (int k = 0; k < K; ++k) gp.p[k] = gates.data_ptr<float>() + (int64_t)k * S;
   DISPATCH_FLOAT(logits, "gate_forward", [&] {
-    launch_gate_forward<scalar_t>(reinterpret_cast<const scalar_t*>(logits.data_ptr()), S, E, K, C, normalize, eps,
-                                  idx.data_ptr<int>(), loc.data_ptr<int>(), gates.data_ptr<float>(),
-                                  raw.data_ptr<float>(), smap.data_ptr<int>(), top1.data_ptr<int>(),
-                                  laux.data_ptr<float>(), ws_rank.data_ptr<int>(), ws_cnt.data_ptr<int>(),
-                                  ws_score.data_ptr<float>(), cur_stream());
+    launch_gate_forward<scalar_t, false>(reinterpret_cast<const scalar_t*>(logits.data_ptr()), S, E, K, C, normalize,
+                                         gate_eps(logits.scalar_type()), idx.data_ptr<int>(), loc.data_ptr<int>(), gp,
+                                         reinterpret_cast<float*>(w), smap.data_ptr<int>(), top1.data_ptr<int>(),
+                                         laux.data_ptr<float>(), w + K * S, w + 2 * K * S,
+                                         reinterpret_cast<float*>(w + 2 * K * S + K * (int64_t)nblk * E), cur_stream());
   });
   return {idx, loc, gates, smap, top1, laux};
 }
@@ -262,13 +266,64 @@ Tensor gate_backward_op(const Tensor& logits, const Tensor& idx, const c10::opti
   const int S = logits.size(0), E = logits.size(1), K = idx.size(0);
   c10::cuda::CUDAGuard guard(logits.device());
   Tensor out = torch::empty_like(logits);
-  const float eps = logits.scalar_type() == at::kFloat ? 1.1920929e-07f
-                    : (logits.scalar_type() == at::kHalf ? 9.765625e-04f : 7.8125e-03f);
+  GatePtrs gp{};
+  if (opt_f32(dgates) != nullptr)
+    for (int k = 0; k < K; ++k) gp.p[k] = dgates->data_ptr<float>() + (int64_t)k * S;
   DISPATCH_FLOAT(logits, "gate_backward", [&] {
-    launch_gate_backward<scalar_t>(reinterpret_cast<const scalar_t*>(logits.data_ptr()), S, E, K, normalize, eps,
-                                   idx.data_ptr<int>(), opt_f32(dgates), opt_f32(dl_aux), top1.data_ptr<int>(),
-                                   reinterpret_cast<scalar_t*>(out.data_ptr()), cur_stream());
+    launch_gate_backward<scalar_t, false>(reinterpret_cast<const scalar_t*>(logits.data_ptr()), S, E, K, normalize,
+                                          gate_eps(logits.scalar_type()), idx.data_ptr<int>(), gp, opt_f32(dl_aux),
+                                          top1.data_ptr<int>(), reinterpret_cast<scalar_t*>(out.data_ptr()), cur_stream());
   });
+  return out;
+}
+
+// Routing from a [S, E] fp32 score matrix (extract_critical): {idx, loc, slot_map, top1, loss, gate of pick 0, 1, ...}.
+std::vector<Tensor> route_scores_op(const Tensor& scores, int64_t K, int64_t C, bool normalize) {
+  count_launch(2);
+  TORCH_CHECK(scores.is_cuda() && scores.dim() == 2 && scores.is_contiguous() && scores.scalar_type() == at::kFloat);
+  const int64_t S = scores.size(0), E = scores.size(1);
+  TORCH_CHECK(S > 0 && E >= 1 && E <= 64 && K >= 1 && K <= 4 && K <= E && C >= 0 && K * S <= INT_MAX,
+              "route_scores supports up to 64 experts and top-4");
+  c10::cuda::CUDAGuard guard(scores.device());
+  auto iopt = scores.options().dtype(at::kInt);
+  const int64_t nblk = gate_workspace_blocks(S);
+  Tensor idx = torch::empty({K, S}, iopt), loc = torch::empty({K, S}, iopt), smap = torch::empty({E * C}, iopt);
+  Tensor top1 = torch::empty({E}, iopt), loss = torch::empty({}, scores.options());
+  Tensor ws = torch::empty({2 * K * S + (K + 1) * nblk * E}, iopt);
+  int* w = ws.data_ptr<int>();
+  std::vector<Tensor> out{idx, loc, smap, top1, loss};
+  GatePtrs gp{};
+  for (int k = 0; k < K; ++k) {
+    out.push_back(torch::empty({S}, scores.options()));
+    gp.p[k] = out.back().data_ptr<float>();
+  }
+  launch_gate_forward<float, true>(scores.data_ptr<float>(), S, E, K, C, normalize, kFloatEps, idx.data_ptr<int>(),
+                                   loc.data_ptr<int>(), gp, reinterpret_cast<float*>(w), smap.data_ptr<int>(),
+                                   top1.data_ptr<int>(), loss.data_ptr<float>(), w + K * S, w + 2 * K * S,
+                                   reinterpret_cast<float*>(w + 2 * K * S + K * nblk * E), cur_stream());
+  return out;
+}
+
+Tensor route_scores_backward_op(const Tensor& scores, const Tensor& idx, const std::vector<c10::optional<Tensor>>& dgates,
+                                const c10::optional<Tensor>& dloss, const Tensor& top1, bool normalize) {
+  count_launch(1);
+  const int S = scores.size(0), E = scores.size(1), K = idx.size(0);
+  c10::cuda::CUDAGuard guard(scores.device());
+  TORCH_CHECK((int)dgates.size() == K);
+  Tensor out = torch::empty_like(scores);
+  std::vector<Tensor> keep;
+  GatePtrs gp{};
+  for (int k = 0; k < K; ++k) {
+    if (!dgates[k].has_value() || !dgates[k]->defined()) continue;
+    keep.push_back(dgates[k]->to(at::kFloat).contiguous());
+    TORCH_CHECK(keep.back().numel() == S);
+    gp.p[k] = keep.back().data_ptr<float>();
+  }
+  Tensor dl;
+  if (dloss.has_value() && dloss->defined()) dl = dloss->to(at::kFloat).contiguous();
+  launch_gate_backward<float, true>(scores.data_ptr<float>(), S, E, K, normalize, kFloatEps, idx.data_ptr<int>(), gp,
+                                    dl.defined() ? dl.data_ptr<float>() : nullptr, top1.data_ptr<int>(),
+                                    out.data_ptr<float>(), cur_stream());
   return out;
 }
 
@@ -708,6 +763,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("importance_order", &importance_order_op);
   m.def("remap_slot_map", &remap_slot_map_op);
   m.def("gate_backward", &gate_backward_op);
+  m.def("route_scores", &route_scores_op);
+  m.def("route_scores_backward", &route_scores_backward_op);
   m.def("cumsum_sub_one", &cumsum_sub_one_op);
   m.def("int8_encode", &int8_encode_op);
   m.def("int8_decode", &int8_decode_op);

@@ -5,8 +5,9 @@
 // custom/custom_kernel.cpp:338-383).  Slot ordering is the reference's: within an expert, every
 // k-th pick ranks after all (k-1)-th picks, and picks of equal k rank by token index.
 //
-//   gate_stats   per token: softmax, top-k (ties -> lower expert id), raw gate scores; per block:
-//                (k, expert) histograms, in-block ranks, per-expert score sums.
+//   gate_stats   per token: softmax (or scores taken as they are), top-k (ties -> lower expert id, NaN before every
+//                number), raw gate scores; per block: (k, expert) histograms, in-block ranks, per-expert score sums;
+//                marks every slot of the map as empty.
 //   gate_assign  per block: base offsets from the histograms of preceding blocks / lower k,
 //                locations, normalised gates, slot map; block 0 also reduces the loss.
 //   gate_bwd     per token: d(logits) from d(gates) and d(l_aux) (softmax recomputed).
@@ -19,7 +20,9 @@
 
 namespace planmoe {
 
-constexpr int kGateThreads = 64;    // small blocks: 8192 tokens still fill most SMs
+// Threads (= tokens) per block.  The assign kernel of every block sums the histograms of the blocks before it, so half as
+// many blocks is a quarter of that work: with 64 threads it took 14 us for 16384 tokens and 8 experts.
+constexpr int kGateThreads = 128;
 constexpr int kGateWarps = kGateThreads / 32;
 constexpr int kMaxE = 64;   // experts handled by the fused gate (per-thread register row)
 constexpr int kMaxK = 4;
@@ -30,14 +33,28 @@ __device__ __forceinline__ void load_row(const T* row, int E, float* v) {
   for (int e = 0; e < ME; ++e) v[e] = (e < E) ? to_f32(row[e]) : -INFINITY;
 }
 
-template <class T, int ME>
+template <int ME>
+__device__ __forceinline__ void softmax_row(float* p, int E) {
+  float mx = -INFINITY;
+#pragma unroll
+  for (int e = 0; e < ME; ++e) mx = fmaxf(mx, p[e]);
+  float sum = 0.f;
+#pragma unroll
+  for (int e = 0; e < ME; ++e) { p[e] = (e < E) ? expf(p[e] - mx) : 0.f; sum += p[e]; }
+  const float inv = 1.f / sum;
+#pragma unroll
+  for (int e = 0; e < ME; ++e) p[e] *= inv;
+}
+
+template <class T, int ME, bool SCORES>
 __global__ void __launch_bounds__(kGateThreads)
-gate_stats_kernel(const T* __restrict__ logits, int S, int E, int K,
+gate_stats_kernel(const T* __restrict__ logits, int S, int E, int K, int nblk,
                   int* __restrict__ idx,          // [K][S]
                   float* __restrict__ raw_gate,   // [K][S] un-normalised softmax score of pick k
                   int* __restrict__ rank_in_blk,  // [K][S]
-                  int* __restrict__ blk_count,    // [nblk][K][E]
-                  float* __restrict__ blk_score)  // [nblk][E]  sum of softmax scores
+                  int* __restrict__ blk_count,    // [K][E][nblk]
+                  float* __restrict__ blk_score,  // [E][nblk]  sum of softmax scores
+                  int* __restrict__ slot_map, long long slots)
 {
   __shared__ int warp_cnt[kGateWarps][kMaxK][kMaxE];
   __shared__ float score_sum[kGateWarps][kMaxE];
@@ -46,21 +63,14 @@ gate_stats_kernel(const T* __restrict__ logits, int S, int E, int K,
   const bool live = t < S;
 
   for (int i = tid; i < kGateWarps * kMaxK * kMaxE; i += kGateThreads) (&warp_cnt[0][0][0])[i] = 0;
+  for (long long i = t; i < slots; i += (long long)gridDim.x * kGateThreads) slot_map[i] = -1;
   __syncthreads();
 
   float p[ME];
   int pick[kMaxK];
   if (live) {
     load_row<T, ME>(logits + (size_t)t * E, E, p);
-    float mx = -INFINITY;
-#pragma unroll
-    for (int e = 0; e < ME; ++e) mx = fmaxf(mx, p[e]);
-    float sum = 0.f;
-#pragma unroll
-    for (int e = 0; e < ME; ++e) { p[e] = (e < E) ? expf(p[e] - mx) : 0.f; sum += p[e]; }
-    const float inv = 1.f / sum;
-#pragma unroll
-    for (int e = 0; e < ME; ++e) p[e] *= inv;
+    if constexpr (!SCORES) softmax_row<ME>(p, E);
   } else {
 #pragma unroll
     for (int e = 0; e < ME; ++e) p[e] = 0.f;
@@ -77,14 +87,14 @@ gate_stats_kernel(const T* __restrict__ logits, int S, int E, int K,
 
   unsigned long long taken = 0ull;
   for (int k = 0; k < K; ++k) {
-    int best = -1;
-    float bv = -1.f;
+    int best = -1;                               // K <= E: one expert is always left
+    float bv = 0.f;
 #pragma unroll
     for (int e = 0; e < ME; ++e) {
-      if (e < E && !((taken >> e) & 1ull) && p[e] > bv) { bv = p[e]; best = e; }
+      if (e < E && !((taken >> e) & 1ull) && (best < 0 || p[e] > bv || (isnan(p[e]) && !isnan(bv)))) { bv = p[e]; best = e; }
     }
     pick[k] = live ? best : -1;
-    taken |= (best >= 0) ? (1ull << best) : 0ull;
+    taken |= 1ull << best;
     if (live) {
       idx[(size_t)k * S + t] = best;
       raw_gate[(size_t)k * S + t] = bv;
@@ -108,12 +118,12 @@ gate_stats_kernel(const T* __restrict__ logits, int S, int E, int K,
     const int k = i / E, e = i - k * E;
     int c = 0;
     for (int w = 0; w < kGateWarps; ++w) c += warp_cnt[w][k][e];
-    blk_count[((size_t)blockIdx.x * K + k) * E + e] = c;
+    blk_count[(size_t)i * nblk + blockIdx.x] = c;
   }
   for (int e = tid; e < E; e += kGateThreads) {
     float s = 0.f;
     for (int w = 0; w < kGateWarps; ++w) s += score_sum[w][e];
-    blk_score[(size_t)blockIdx.x * E + e] = s;
+    blk_score[(size_t)e * nblk + blockIdx.x] = s;
   }
 }
 
@@ -122,7 +132,7 @@ gate_assign_kernel(int S, int E, int K, int C, int normalize, float eps,
                    const int* __restrict__ idx, const float* __restrict__ raw_gate,
                    const int* __restrict__ rank_in_blk, const int* __restrict__ blk_count,
                    const float* __restrict__ blk_score, int nblk,
-                   int* __restrict__ loc, float* __restrict__ gates, int* __restrict__ slot_map,
+                   int* __restrict__ loc, GatePtrs gates, int* __restrict__ slot_map,
                    int* __restrict__ top1_count,  // [E] tokens whose first pick is e
                    float* __restrict__ l_aux)     // [1]
 {
@@ -134,11 +144,11 @@ gate_assign_kernel(int S, int E, int K, int C, int normalize, float eps,
   // then the k-th picks of the blocks before this one.  One warp per (k, e), lanes strided over that list.
   for (int i = warp; i < K * E; i += kGateWarps) {
     const int k = i / E, e = i - k * E;
-    const int n = k * nblk + b;
     int acc = 0;
-    for (int j = lane; j < n; j += 32) {
-      const int kk = j / nblk, bb = j - kk * nblk;
-      acc += blk_count[((size_t)bb * K + kk) * E + e];
+    for (int kk = 0; kk <= k; ++kk) {
+      const int* row = blk_count + (size_t)(kk * E + e) * nblk;
+      const int n = kk < k ? nblk : b;
+      for (int bb = lane; bb < n; bb += 32) acc += row[bb];
     }
     acc = __reduce_add_sync(0xffffffffu, acc);
     if (lane == 0) base[k][e] = acc;
@@ -150,12 +160,13 @@ gate_assign_kernel(int S, int E, int K, int C, int normalize, float eps,
     float g[kMaxK];
     float denom = 0.f;
     for (int k = 0; k < K; ++k) { g[k] = raw_gate[(size_t)k * S + t]; denom += g[k]; }
-    const float scale = (normalize && K > 1) ? 1.f / fmaxf(denom, eps) : 1.f;
+    const bool norm = normalize && K > 1;
+    denom = fmaxf(denom, eps);
     for (int k = 0; k < K; ++k) {
       const int e = idx[(size_t)k * S + t];
       const int l = base[k][e] + rank_in_blk[(size_t)k * S + t];
       loc[(size_t)k * S + t] = l;
-      gates[(size_t)k * S + t] = g[k] * scale;
+      gates.p[k][t] = norm ? g[k] / denom : g[k];
       if (l < C) slot_map[(size_t)e * C + l] = t * K + k;
     }
   }
@@ -167,8 +178,8 @@ gate_assign_kernel(int S, int E, int K, int C, int normalize, float eps,
       float s = 0.f;
       int c = 0;
       for (int bb = lane; bb < nblk; bb += 32) {
-        s += blk_score[(size_t)bb * E + e];
-        c += blk_count[((size_t)bb * K + 0) * E + e];
+        s += blk_score[(size_t)e * nblk + bb];
+        c += blk_count[(size_t)e * nblk + bb];
       }
       s = warp_sum(s);
       c = __reduce_add_sync(0xffffffffu, c);
@@ -186,25 +197,17 @@ gate_assign_kernel(int S, int E, int K, int C, int normalize, float eps,
   }
 }
 
-template <class T, int ME>
+template <class T, int ME, bool SCORES>
 __global__ void __launch_bounds__(kGateThreads)
 gate_bwd_kernel(const T* __restrict__ logits, int S, int E, int K, int normalize, float eps,
-                const int* __restrict__ idx, const float* __restrict__ dgates,   // [K][S] or null
+                const int* __restrict__ idx, GatePtrs dgates,                     // K rows of S, null = zeros
                 const float* __restrict__ dl_aux,                                 // [1] or null
                 const int* __restrict__ top1_count, T* __restrict__ dlogits) {
   const int t = blockIdx.x * kGateThreads + threadIdx.x;
   if (t >= S) return;
   float p[ME];
   load_row<T, ME>(logits + (size_t)t * E, E, p);
-  float mx = -INFINITY;
-#pragma unroll
-  for (int e = 0; e < ME; ++e) mx = fmaxf(mx, p[e]);
-  float sum = 0.f;
-#pragma unroll
-  for (int e = 0; e < ME; ++e) { p[e] = (e < E) ? expf(p[e] - mx) : 0.f; sum += p[e]; }
-  const float inv = 1.f / sum;
-#pragma unroll
-  for (int e = 0; e < ME; ++e) p[e] *= inv;
+  if constexpr (!SCORES) softmax_row<ME>(p, E);
 
   // d(score): loss part for every expert, gate part for the picked ones
   const float lw = dl_aux ? dl_aux[0] * (float)E / ((float)S * (float)S) : 0.f;
@@ -221,11 +224,11 @@ gate_bwd_kernel(const T* __restrict__ logits, int S, int E, int K, int normalize
   }
   const bool norm = normalize && K > 1;
   for (int k = 0; k < K; ++k) {
-    const float dg = dgates ? dgates[(size_t)k * S + t] : 0.f;
+    const float dg = dgates.p[k] ? dgates.p[k][t] : 0.f;
     dot += dg * ds_pick[k];
   }
   for (int k = 0; k < K; ++k) {
-    const float dg = dgates ? dgates[(size_t)k * S + t] : 0.f;
+    const float dg = dgates.p[k] ? dgates.p[k][t] : 0.f;
     if (norm) {
       if (denom > eps) ds_pick[k] = dg / denom - dot / (denom * denom);
       else ds_pick[k] = dg / eps;
@@ -248,43 +251,32 @@ gate_bwd_kernel(const T* __restrict__ logits, int S, int E, int K, int normalize
   T* out = dlogits + (size_t)t * E;
 #pragma unroll
   for (int e = 0; e < ME; ++e)
-    if (e < E) out[e] = from_f32<T>(p[e] * (ds[e] - inner));
+    if (e < E) out[e] = from_f32<T>(SCORES ? ds[e] : p[e] * (ds[e] - inner));
 }
 
-template <class T>
+template <class T, bool SCORES>
 void launch_gate_forward(const T* logits, int S, int E, int K, int C, bool normalize, float eps,
-                         int* idx, int* loc, float* gates, float* raw_gate, int* slot_map,
+                         int* idx, int* loc, GatePtrs gates, float* raw_gate, int* slot_map,
                          int* top1_count, float* l_aux, int* ws_rank, int* ws_blk_count,
                          float* ws_blk_score, cudaStream_t stream) {
   const int nblk = (S + kGateThreads - 1) / kGateThreads;
-  cudaMemsetAsync(slot_map, 0xFF, sizeof(int) * (size_t)E * C, stream);
-  if (E <= 8)
-    gate_stats_kernel<T, 8><<<nblk, kGateThreads, 0, stream>>>(logits, S, E, K, idx, raw_gate, ws_rank, ws_blk_count, ws_blk_score);
-  else if (E <= 16)
-    gate_stats_kernel<T, 16><<<nblk, kGateThreads, 0, stream>>>(logits, S, E, K, idx, raw_gate, ws_rank, ws_blk_count, ws_blk_score);
-  else if (E <= 32)
-    gate_stats_kernel<T, 32><<<nblk, kGateThreads, 0, stream>>>(logits, S, E, K, idx, raw_gate, ws_rank, ws_blk_count, ws_blk_score);
-  else
-    gate_stats_kernel<T, 64><<<nblk, kGateThreads, 0, stream>>>(logits, S, E, K, idx, raw_gate, ws_rank, ws_blk_count, ws_blk_score);
+  auto stats = E <= 8 ? gate_stats_kernel<T, 8, SCORES> : E <= 16 ? gate_stats_kernel<T, 16, SCORES>
+             : E <= 32 ? gate_stats_kernel<T, 32, SCORES> : gate_stats_kernel<T, 64, SCORES>;
+  stats<<<nblk, kGateThreads, 0, stream>>>(logits, S, E, K, nblk, idx, raw_gate, ws_rank, ws_blk_count, ws_blk_score,
+                                           slot_map, (long long)E * C);
   gate_assign_kernel<<<nblk, kGateThreads, 0, stream>>>(S, E, K, C, normalize ? 1 : 0, eps, idx,
                                                       raw_gate, ws_rank, ws_blk_count, ws_blk_score,
                                                       nblk, loc, gates, slot_map, top1_count, l_aux);
 }
 
-template <class T>
+template <class T, bool SCORES>
 void launch_gate_backward(const T* logits, int S, int E, int K, bool normalize, float eps,
-                          const int* idx, const float* dgates, const float* dl_aux,
+                          const int* idx, GatePtrs dgates, const float* dl_aux,
                           const int* top1_count, T* dlogits, cudaStream_t stream) {
   const int nblk = (S + kGateThreads - 1) / kGateThreads;
-  const int nz = normalize ? 1 : 0;
-  if (E <= 8)
-    gate_bwd_kernel<T, 8><<<nblk, kGateThreads, 0, stream>>>(logits, S, E, K, nz, eps, idx, dgates, dl_aux, top1_count, dlogits);
-  else if (E <= 16)
-    gate_bwd_kernel<T, 16><<<nblk, kGateThreads, 0, stream>>>(logits, S, E, K, nz, eps, idx, dgates, dl_aux, top1_count, dlogits);
-  else if (E <= 32)
-    gate_bwd_kernel<T, 32><<<nblk, kGateThreads, 0, stream>>>(logits, S, E, K, nz, eps, idx, dgates, dl_aux, top1_count, dlogits);
-  else
-    gate_bwd_kernel<T, 64><<<nblk, kGateThreads, 0, stream>>>(logits, S, E, K, nz, eps, idx, dgates, dl_aux, top1_count, dlogits);
+  auto bwd = E <= 8 ? gate_bwd_kernel<T, 8, SCORES> : E <= 16 ? gate_bwd_kernel<T, 16, SCORES>
+           : E <= 32 ? gate_bwd_kernel<T, 32, SCORES> : gate_bwd_kernel<T, 64, SCORES>;
+  bwd<<<nblk, kGateThreads, 0, stream>>>(logits, S, E, K, normalize ? 1 : 0, eps, idx, dgates, dl_aux, top1_count, dlogits);
 }
 
 int gate_workspace_blocks(int S) { return (S + kGateThreads - 1) / kGateThreads; }
@@ -354,15 +346,16 @@ void launch_remap_slot_map(int* slot_map, long long n, const int* perm, int K, c
   if (n > 0) remap_slot_map_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(slot_map, n, perm, K);
 }
 
-#define INSTANTIATE(T)                                                                            \
-  template void launch_gate_forward<T>(const T*, int, int, int, int, bool, float, int*, int*,     \
-                                       float*, float*, int*, int*, float*, int*, int*, float*,    \
-                                       cudaStream_t);                                             \
-  template void launch_gate_backward<T>(const T*, int, int, int, bool, float, const int*,         \
-                                        const float*, const float*, const int*, T*, cudaStream_t);
-INSTANTIATE(float)
-INSTANTIATE(__nv_bfloat16)
-INSTANTIATE(__half)
+#define INSTANTIATE(T, SCORES)                                                                    \
+  template void launch_gate_forward<T, SCORES>(const T*, int, int, int, int, bool, float, int*, int*,     \
+                                               GatePtrs, float*, int*, int*, float*, int*, int*, float*,  \
+                                               cudaStream_t);                                             \
+  template void launch_gate_backward<T, SCORES>(const T*, int, int, int, bool, float, const int*, GatePtrs, \
+                                                const float*, const int*, T*, cudaStream_t);
+INSTANTIATE(float, false)
+INSTANTIATE(__nv_bfloat16, false)
+INSTANTIATE(__half, false)
+INSTANTIATE(float, true)
 
 // ---- stand-alone cumsum - 1 -----------------------------------------------------------------
 // Two passes over [S, E] int32: per-tile column sums, then each tile scans with the carried base.

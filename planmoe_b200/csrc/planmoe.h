@@ -64,14 +64,18 @@ void launch_gate_grad(const T* disp, const T* dy, const int* idx, const int* loc
 
 // ---- kernels/gate.cu -------------------------------------------------------------------------
 int gate_workspace_blocks(int S);
-template <class T>
+// One fp32 row of S values per pick (gates, or their gradients; null = zeros).
+struct GatePtrs { float* p[4]; };
+// SCORES: the input is a [S, E] matrix of scores to pick from as they are; otherwise logits, softmax first.
+// slot_map: [E * C], written completely.
+template <class T, bool SCORES>
 void launch_gate_forward(const T* logits, int S, int E, int K, int C, bool normalize, float eps,
-                         int* idx, int* loc, float* gates, float* raw_gate, int* slot_map,
+                         int* idx, int* loc, GatePtrs gates, float* raw_gate, int* slot_map,
                          int* top1_count, float* l_aux, int* ws_rank, int* ws_blk_count,
                          float* ws_blk_score, cudaStream_t stream);
-template <class T>
+template <class T, bool SCORES>
 void launch_gate_backward(const T* logits, int S, int E, int K, bool normalize, float eps,
-                          const int* idx, const float* dgates, const float* dl_aux,
+                          const int* idx, GatePtrs dgates, const float* dl_aux,
                           const int* top1_count, T* dlogits, cudaStream_t stream);
 // order of tokens for batch-prioritised routing: rank[t] = position of token t (best top score first, ties by index),
 // perm[position] = token; `key` is an fp32 [S] workspace

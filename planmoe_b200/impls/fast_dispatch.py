@@ -22,8 +22,10 @@ import torch
 
 from . import losses
 from .communicate import simple_all_reduce
+from ..jit_kernels import gating
 from ..jit_kernels.gating import fast_cumsum_sub_one
 from ..ops import dispatch as D
+from ..ops import native
 
 
 class RoutingPlan(tuple):
@@ -32,12 +34,23 @@ class RoutingPlan(tuple):
 
     def __new__(cls, num_experts, indices_s, locations_s, gates_s, capacity, slots=None):
         self = super().__new__(cls, (num_experts, indices_s, locations_s, gates_s, capacity))
-        self._slots = slots
+        self._slots = self._made = None
+        if slots is not None and not slots.idx.is_inference():
+            self._made = (slots, tuple(indices_s), tuple(locations_s), slots.idx._version, slots.loc._version)
         return self
 
     @property
     def slots(self):
         if self._slots is None:
+            if self._made is not None:
+                # the routing kernels' own stacked tensors, unless the lists were changed since
+                slots, indices, locations, vi, vl = self._made
+                if len(self[1]) == len(indices) and len(self[2]) == len(locations) \
+                        and all(a is b for a, b in zip(self[1], indices)) \
+                        and all(a is b for a, b in zip(self[2], locations)) \
+                        and slots.idx._version == vi and slots.loc._version == vl:
+                    self._slots = slots
+                    return slots
             idx = torch.stack([x.to(torch.int32).view(-1) for x in self[1]])
             loc = torch.stack([x.to(torch.int32).view(-1) for x in self[2]])
             self._slots = D.SlotPlan(idx, loc, self[0], self[4])
@@ -64,10 +77,96 @@ def compute_sorted_location(x, importance_scores):
     return out
 
 
+def _gates_of(gates_all, normalize_gate):
+    """Per-pick gate lists from the picked scores ``[S, k]``."""
+    gates_s = [gates_all[:, k] for k in range(gates_all.size(1))]
+    if gates_all.size(1) > 1 and normalize_gate:
+        denom = torch.clamp(gates_all.sum(dim=1), min=torch.finfo(gates_all.dtype).eps)
+        gates_s = [g / denom for g in gates_s]
+    return gates_s
+
+
+class _RouteScores(torch.autograd.Function):
+    """Top-k, gates, locations, slot map and the value of the GShard loss of fp32 scores in two launches; the gates'
+    gradient in one."""
+
+    @staticmethod
+    def forward(ctx, scores, top_k, capacity, normalize):
+        ctx.set_materialize_grads(False)
+        idx, loc, slot_map, top1, loss, *gates = native.lib().route_scores(scores, top_k, capacity, normalize)
+        ctx.save_for_backward(scores, idx, top1)
+        ctx.normalize = normalize
+        ctx.mark_non_differentiable(loss, top1, idx, loc, slot_map)
+        return (loss, top1, idx, loc, slot_map, *gates)
+
+    @staticmethod
+    def backward(ctx, _loss, _top1, _idx, _loc, _map, *dgates):
+        scores, idx, top1 = ctx.saved_tensors
+        if all(d is None for d in dgates):
+            return None, None, None, None
+        if torch.is_grad_enabled():             # create_graph: the same gradient as differentiable operations
+            pairs = [(g, d) for g, d in zip(_gates_of(scores.gather(1, idx.t().long()), ctx.normalize), dgates)
+                     if d is not None]
+            return torch.autograd.grad([g for g, _ in pairs], scores, [d for _, d in pairs], create_graph=True)[0], \
+                None, None, None
+        return native.lib().route_scores_backward(scores, idx, list(dgates), None, top1, ctx.normalize), None, None, None
+
+
+class _RouteLoss(torch.autograd.Function):
+    """The GShard loss that ``_RouteScores`` computed, as a node of its own: its backward can run before, after or without
+    the gates'."""
+
+    @staticmethod
+    def forward(ctx, scores, value, top1, idx):
+        ctx.save_for_backward(scores, idx, top1)
+        return value.clone()
+
+    @staticmethod
+    def backward(ctx, dloss):
+        scores, idx, top1 = ctx.saved_tensors
+        if torch.is_grad_enabled():
+            return torch.autograd.grad(losses.gshard_loss(scores, idx.t()), scores, dloss, create_graph=True)[0], \
+                None, None, None
+        return native.lib().route_scores_backward(scores, idx, [None] * idx.size(0), dloss, top1, False), None, None, None
+
+
+def _route_on_kernels(scores, top_k, loss_fn):
+    """Whether the routing kernels take this call.  They pick from fp32 scores (a tie goes to the lower expert id) and
+    know the GShard loss; other losses and types, batch-prioritised order, function transforms (vmap, forward-mode),
+    tracing and tensor subclasses take the ATen composition."""
+    return (scores.is_cuda and scores.dtype == torch.float32 and scores.dim() == 2 and scores.size(0) > 0
+            and 1 <= scores.size(1) <= 64 and 1 <= top_k <= 4 and scores.size(0) * top_k < 2 ** 31
+            and (loss_fn is None or loss_fn is losses.gshard_loss)
+            and type(scores) in (torch.Tensor, torch.nn.Parameter) and gating.use_fast_cumsum
+            and not torch._C._are_functorch_transforms_active()
+            and torch.autograd.forward_ad._current_level < 0
+            and not torch.compiler.is_compiling() and not torch.jit.is_tracing()
+            and torch.utils._python_dispatch._get_current_dispatch_mode() is None)
+
+
+def _align(capacity, alignment):
+    return capacity + -capacity % alignment
+
+
 def extract_critical(scores, top_k, loss_fn=losses.gshard_loss, capacity_factor=1.0,
                      batch_prioritized_routing=False, normalize_gate=True, group=None, alignment=1):
     S, E = int(scores.size(0)), int(scores.size(1))
     top_k = min(int(top_k), E)
+    per_expert = (S + E - 1) // E
+    if not batch_prioritized_routing and _route_on_kernels(scores, top_k, loss_fn):
+        capacity = _align(top_k * int(capacity_factor * per_expert), alignment) if capacity_factor > 0 else 0
+        scores = scores.contiguous()
+        l_loss, top1, idx, loc, slot_map, *gates_s = _RouteScores.apply(scores, top_k, capacity, bool(normalize_gate))
+        l_loss = _RouteLoss.apply(scores, l_loss, top1, idx) if loss_fn is not None else None
+        if capacity_factor <= 0:
+            peak = simple_all_reduce(loc.max(), group=group, op=torch.distributed.ReduceOp.MAX)
+            capacity = int(peak) + 1
+            if capacity_factor < 0:
+                capacity = min(capacity, top_k * int(-capacity_factor * per_expert))
+            capacity, slot_map = _align(capacity, alignment), None
+        plan = RoutingPlan(E, list(idx.unbind(0)), list(loc.unbind(0)), gates_s, capacity,
+                           D.SlotPlan(idx, loc, E, capacity, slot_map))
+        return plan, l_loss
     topk_indices = torch.topk(scores, top_k, dim=1).indices
     gates_all = scores.gather(1, topk_indices)                      # [S, k], differentiable
 
@@ -92,12 +191,7 @@ def extract_critical(scores, top_k, loss_fn=losses.gshard_loss, capacity_factor=
         counts = mask.sum(dim=0, keepdim=True)
         base = counts if base is None else base + counts
 
-    gates_s = [gates_all[:, k] for k in range(top_k)]
-    if top_k > 1 and normalize_gate:
-        denom = torch.clamp(gates_all.sum(dim=1), min=torch.finfo(scores.dtype).eps)
-        gates_s = [g / denom for g in gates_s]
-
-    per_expert = (S + E - 1) // E
+    gates_s = _gates_of(gates_all, normalize_gate)
     if capacity_factor > 0:
         capacity = top_k * int(capacity_factor * per_expert)
     else:
@@ -105,9 +199,7 @@ def extract_critical(scores, top_k, loss_fn=losses.gshard_loss, capacity_factor=
         capacity = int(simple_all_reduce(peak, group=group, op=torch.distributed.ReduceOp.MAX)) + 1
         if capacity_factor < 0:
             capacity = min(capacity, top_k * int(-capacity_factor * per_expert))
-    if capacity % alignment:
-        capacity += alignment - capacity % alignment
-
+    capacity = _align(capacity, alignment)
     return RoutingPlan(E, indices_s, locations_s, gates_s, capacity), l_loss
 
 

@@ -1,0 +1,93 @@
+"""``extract_critical`` on the routing kernels against its ATen composition: every form that the kernels accept."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _both(scores, monkeypatch, **kw):
+    """(kernel result, composition result), each with its own leaf."""
+    from planmoe_b200.impls import fast_dispatch as FD
+    from planmoe_b200.jit_kernels import gating
+    out = []
+    for fast in (True, False):
+        monkeypatch.setattr(gating, 'use_fast_cumsum', fast)
+        leaf = scores.detach().clone().requires_grad_()
+        view = leaf.t() if kw.get('transposed') else leaf
+        args = {k: v for k, v in kw.items() if k != 'transposed'}
+        out.append((leaf, *FD.extract_critical(view, **args)))
+    return out
+
+
+@pytest.mark.parametrize('S,E,k', [(1, 1, 1), (5, 3, 2), (127, 8, 2), (128, 9, 1), (129, 16, 4), (1000, 33, 3), (4097, 64, 2)])
+@pytest.mark.parametrize('cf', [1.0, 0.4, 0.0, -0.5])
+@pytest.mark.parametrize('normalize', [True, False])
+def test_matches_composition(S, E, k, cf, normalize, monkeypatch):
+    torch.manual_seed(S + E)
+    scores = torch.softmax(torch.randn(S, E, device='cuda'), dim=1)
+    transposed = S == 129
+    if transposed:
+        scores = scores.t().contiguous()
+    (a, pa, la), (b, pb, lb) = _both(scores, monkeypatch, top_k=k, capacity_factor=cf, normalize_gate=normalize, alignment=4,
+                                     transposed=transposed)
+    assert pa[0] == pb[0] and pa[4] == pb[4]
+    for i in (1, 2):
+        assert len(pa[i]) == len(pb[i]) == k
+        for u, v in zip(pa[i], pb[i]):
+            assert u.dtype == v.dtype and torch.equal(u, v)
+    for u, v in zip(pa[3], pb[3]):
+        torch.testing.assert_close(u, v, rtol=4e-7, atol=0)          # a division of sums of at most four scores
+    torch.testing.assert_close(la, lb, rtol=2e-6, atol=0)            # S * E positive terms, another order
+    assert torch.equal(pa.slots.slot_map, pb.slots.slot_map)
+    weights = [torch.randn(S, device='cuda') for _ in range(k)]
+    for leaf, p, l in ((a, pa, la), (b, pb, lb)):
+        (sum((g * w).sum() for g, w in zip(p[3], weights)) + 0.3 * l).backward()
+    torch.testing.assert_close(a.grad, b.grad, rtol=1e-5, atol=1e-5 * float(b.grad.abs().max()))
+
+
+def test_partial_and_second_gradients(monkeypatch):
+    torch.manual_seed(0)
+    scores = torch.softmax(torch.randn(300, 8, device='cuda'), dim=1)
+    got = []
+    for leaf, p, l in _both(scores, monkeypatch, top_k=2):
+        first, = torch.autograd.grad(p[3][1].square().sum(), leaf, create_graph=True)     # pick 0 and the loss get none
+        second, = torch.autograd.grad(first.square().sum(), leaf)
+        only_loss, = torch.autograd.grad(l, leaf)              # the gates' graph is gone, the loss has its own
+        got.append((first.detach(), second, only_loss))
+    for u, v in zip(*got):
+        torch.testing.assert_close(u, v, rtol=1e-4, atol=1e-5 * float(v.abs().max()))
+
+
+def test_unusual_scores(monkeypatch):
+    """Scores that are no probabilities, NaN rows and infinities stay inside the experts' range."""
+    from planmoe_b200.impls import fast_dispatch as FD
+    scores = torch.randn(400, 6, device='cuda')
+    scores[3] = float('nan')
+    scores[4, 2] = float('nan')
+    scores[5] = -float('inf')
+    scores[6, 1] = float('inf')
+    plan, _ = FD.extract_critical(scores, 3)
+    idx = torch.stack(plan[1]).long()
+    assert int(idx.min()) >= 0 and int(idx.max()) < 6
+    assert all(len(set(r)) == 3 for r in idx.t().tolist())
+    assert idx[0, 4] == 2 and idx[0, 6] == 1
+    loc = torch.stack(plan[2])
+    for e in range(6):
+        assert sorted(loc[idx == e].tolist()) == list(range(int((idx == e).sum())))
+
+
+def test_changed_lists_and_other_forms_take_the_composition(monkeypatch):
+    from planmoe_b200.impls import fast_dispatch as FD, losses
+    scores = torch.softmax(torch.randn(64, 4, device='cuda'), dim=1)
+    plan, _ = FD.extract_critical(scores, 2)
+    plan[2][1].add_(1)                                                # in place: the made slot map no longer fits
+    ref = FD.RoutingPlan(plan[0], [x.clone() for x in plan[1]], [x.clone() for x in plan[2]], plan[3], plan[4])
+    assert torch.equal(plan.slots.slot_map, ref.slots.slot_map)
+    for kw in (dict(loss_fn=lambda s, i: losses.gshard_loss(s, i) * 2), dict(batch_prioritized_routing=True)):
+        FD.extract_critical(scores, 2, **kw)
+    FD.extract_critical(scores.half(), 2)
+    from planmoe_b200.jit_kernels import gating
+    monkeypatch.setattr(gating, 'use_fast_cumsum', False)             # the cumsum kernel knows no function transforms
+    grad = torch.func.grad(lambda s: FD.extract_critical(s, 2)[1])(scores)
+    assert torch.isfinite(grad).all()
