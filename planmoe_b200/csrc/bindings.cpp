@@ -232,7 +232,8 @@ void remap_slot_map_op(Tensor& slot_map, const Tensor& perm, int64_t K) {
 constexpr float kFloatEps = 1.1920929e-07f;
 float gate_eps(at::ScalarType t) { return t == at::kFloat ? kFloatEps : (t == at::kHalf ? 9.765625e-04f : 7.8125e-03f); }
 
-std::vector<Tensor> gate_forward_op(const Tensor& logits, int64_t K, int64_t C, bool normalize) {
+// {idx, loc, gates, slot_map, top1, l_aux, used}
+std::vector<Tensor> gate_forward_used_op(const Tensor& logits, int64_t K, int64_t C, bool normalize) {
   count_launch(2);
   TORCH_CHECK(logits.is_cuda() && logits.dim() == 2 && logits.is_contiguous());
   const int S = logits.size(0), E = logits.size(1);
@@ -244,7 +245,7 @@ std::vector<Tensor> gate_forward_op(const Tensor& logits, int64_t K, int64_t C, 
   Tensor idx = torch::empty({K, S}, iopt), loc = torch::empty({K, S}, iopt);
   Tensor gates = torch::empty({K, S}, fopt);
   Tensor smap = torch::empty({(int64_t)E * C}, iopt);
-  Tensor top1 = torch::empty({E}, iopt), laux = torch::empty({1}, fopt);
+  Tensor top1 = torch::empty({2, E}, iopt), laux = torch::empty({1}, fopt);   // first picks, used slots of every expert
   // scratch of this call: raw gates, in-block ranks, per-block histograms and score sums
   Tensor ws = torch::empty({2 * K * S + (K + 1) * (int64_t)nblk * E}, iopt);
   int* w = ws.data_ptr<int>();
@@ -254,10 +255,15 @@ std::vector<Tensor> gate_forward_op(const Tensor& logits, int64_t K, int64_t C, 
     launch_gate_forward<scalar_t, false>(reinterpret_cast<const scalar_t*>(logits.data_ptr()), S, E, K, C, normalize,
                                          gate_eps(logits.scalar_type()), idx.data_ptr<int>(), loc.data_ptr<int>(), gp,
                                          reinterpret_cast<float*>(w), smap.data_ptr<int>(), top1.data_ptr<int>(),
-                                         laux.data_ptr<float>(), w + K * S, w + 2 * K * S,
+                                         top1.data_ptr<int>() + E, laux.data_ptr<float>(), w + K * S, w + 2 * K * S,
                                          reinterpret_cast<float*>(w + 2 * K * S + K * (int64_t)nblk * E), cur_stream());
   });
-  return {idx, loc, gates, smap, top1, laux};
+  return {idx, loc, gates, smap, top1[0], laux, top1[1]};
+}
+std::vector<Tensor> gate_forward_op(const Tensor& logits, int64_t K, int64_t C, bool normalize) {
+  std::vector<Tensor> r = gate_forward_used_op(logits, K, C, normalize);
+  r.pop_back();
+  return r;
 }
 
 Tensor gate_backward_op(const Tensor& logits, const Tensor& idx, const c10::optional<Tensor>& dgates,
@@ -299,7 +305,7 @@ std::vector<Tensor> route_scores_op(const Tensor& scores, int64_t K, int64_t C, 
   }
   launch_gate_forward<float, true>(scores.data_ptr<float>(), S, E, K, C, normalize, kFloatEps, idx.data_ptr<int>(),
                                    loc.data_ptr<int>(), gp, reinterpret_cast<float*>(w), smap.data_ptr<int>(),
-                                   top1.data_ptr<int>(), loss.data_ptr<float>(), w + K * S, w + 2 * K * S,
+                                   top1.data_ptr<int>(), nullptr, loss.data_ptr<float>(), w + K * S, w + 2 * K * S,
                                    reinterpret_cast<float*>(w + 2 * K * S + K * nblk * E), cur_stream());
   return out;
 }
@@ -386,6 +392,7 @@ struct GemmOpts {
   // de-quantiser role (int8 wire): local landing buffer, arrival flags (set by peers), ready flags (set by the role)
   int64_t dq_ptr = 0, dq_arrival_ptr = 0, dq_ready_ptr = 0;
   int64_t trace_ptr = 0;                     // optional u64 [grid][8] role trace (see GemmArgs::trace)
+  c10::optional<Tensor> rows_used;           // optional int32 [groups] (see GemmArgs::rows_used)
 };
 
 GemmOperand operand_of(const Tensor& t, bool mn_major) {
@@ -458,6 +465,11 @@ Tensor grouped_gemm_op(const Tensor& A, bool a_mn, const Tensor& B, bool b_mn, c
   g.budget_ns = (unsigned long long)o.budget_ms * 1000000ull;
   g.status = reinterpret_cast<int*>(o.status_ptr);
   g.trace = reinterpret_cast<unsigned long long*>(o.trace_ptr);
+  if (o.rows_used.has_value() && o.rows_used->defined()) {
+    const Tensor& u = *o.rows_used;
+    TORCH_CHECK(u.is_cuda() && u.scalar_type() == at::kInt && u.is_contiguous() && u.numel() == groups, "rows_used: int32 [groups]");
+    g.rows_used = u.data_ptr<int>();
+  }
   g.max_ctas = o.max_ctas;
   g.cta_group = o.cta_group;
   if (o.epilogue == kEpiPush) TORCH_CHECK(g.heap_bases != nullptr, "push epilogue needs heap bases");
@@ -502,7 +514,7 @@ static void colsum_check(const Tensor& x, int64_t fold) {
 }
 
 // scratch of one job: [out][partials][counters]; fills `j`, returns the buffer
-static Tensor colsum_job(const Tensor& x, int64_t fold, bool as_bf16, ColsumJob& j, Tensor& ob) {
+static Tensor colsum_job(const Tensor& x, int64_t fold, bool as_bf16, ColsumJob& j, Tensor& ob, const int* rows_used = nullptr) {
   const int groups = x.size(0), N = x.size(2);
   const int64_t rows = x.size(1), slabs = colsum_slabs(rows), out_groups = groups / fold;
   const int64_t counters = out_groups * colsum_colblocks(N);
@@ -512,7 +524,7 @@ static Tensor colsum_job(const Tensor& x, int64_t fold, bool as_bf16, ColsumJob&
   j.partial = j.out + out_groups * N;
   j.counters = reinterpret_cast<unsigned*>(j.partial + (int64_t)groups * N * slabs);
   j.rows = rows; j.row_stride = x.stride(1); j.group_stride = x.stride(0);
-  j.N = N; j.groups = groups; j.fold = (int)fold;
+  j.N = N; j.groups = groups; j.fold = (int)fold; j.rows_used = rows_used;
   return buf;
 }
 
@@ -544,6 +556,149 @@ std::vector<Tensor> colsum2_op(const Tensor& xa, const Tensor& xb, int64_t fold,
   if (as_bf16) return {oa, ob};
   const int64_t ga = xa.size(0) / fold, gb = xb.size(0) / fold;
   return {ba.narrow(0, 0, ga * xa.size(2)).view({ga, xa.size(2)}), bb.narrow(0, 0, gb * xb.size(2)).view({gb, xb.size(2)})};
+}
+
+// ---- one rank: the experts' forward and backward in one call each --------------------------------
+// A stage of the pass for the per-stage timers: `stages` is None, or a callable that makes a context manager of a name.
+struct Stage {
+  py::object cm;
+  Stage(const py::object& stages, const char* name) {
+    if (!stages.is_none()) { cm = stages(name); cm.attr("__enter__")(); }
+  }
+  ~Stage() {
+    if (!cm) return;
+    try { cm.attr("__exit__")(py::none(), py::none(), py::none()); } catch (...) {}
+  }
+};
+
+// Routing of a pass: idx, loc int32 [K, S]; slot_map int32 [E * C]; used int32 [E]; gates fp32 [K, S].
+struct LocalRoute {
+  Tensor idx, loc, slot_map, used, gates;
+  int64_t C, act;
+  bool postscore;
+  int64_t budget_ms, status_ptr;
+};
+
+static void local_check(const Tensor& x, const LocalRoute& r, const Tensor& w1) {
+  const int64_t K = r.idx.size(0), S = r.idx.size(1), E = w1.size(0);
+  auto i32 = [&](const Tensor& t, int64_t n) {
+    return t.is_cuda() && t.scalar_type() == at::kInt && t.is_contiguous() && t.numel() == n;
+  };
+  TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.dim() == 2 && x.is_contiguous() && x.size(0) == S);
+  TORCH_CHECK(reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0 && x.size(1) % 8 == 0, "rows must be 16-byte aligned");
+  TORCH_CHECK(i32(r.idx, K * S) && i32(r.loc, K * S) && i32(r.slot_map, E * r.C) && i32(r.used, E) && K <= 4 && E <= 64);
+  TORCH_CHECK(r.gates.is_cuda() && r.gates.scalar_type() == at::kFloat && r.gates.is_contiguous() && r.gates.numel() == K * S);
+}
+
+static GemmOpts local_opts(const LocalRoute& r, int64_t epilogue) {
+  GemmOpts o;
+  o.epilogue = epilogue; o.activation = r.act; o.budget_ms = r.budget_ms; o.status_ptr = r.status_ptr;
+  o.rows_used = r.used;
+  return o;
+}
+
+static const void* rows16(const Tensor& t) {      // a row tensor the vector kernels may read
+  TORCH_CHECK(t.is_contiguous() && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0, "rows must be 16-byte aligned");
+  return t.data_ptr();
+}
+
+// {y [S, O], xs [E, C, M], dact [E, C, H], h [E, C, H], ys [E, C, O]}; without `want_grad` no derivative is saved (dact
+// is empty)
+std::vector<Tensor> local_forward_op(const Tensor& x, const LocalRoute& r, const Tensor& w1, const Tensor& b1, const Tensor& w2,
+                                     const Tensor& b2, bool want_grad, const py::object& stages) {
+  local_check(x, r, w1);
+  c10::cuda::CUDAGuard guard(x.device());
+  const int64_t K = r.idx.size(0), S = x.size(0), M = x.size(1), E = w1.size(0), C = r.C, H = w1.size(2), O = w2.size(2);
+  Tensor xs = torch::empty({E, C, M}, x.options()), dact, h, ys, y = torch::empty({S, O}, x.options());
+  {
+    Stage st(stages, "fwd.slots");
+    count_launch(1);
+    launch_slots_fill(x.data_ptr(), r.slot_map.data_ptr<int>(), r.postscore ? nullptr : r.gates.data_ptr<float>(),
+                      r.used.data_ptr<int>(), xs.data_ptr(), K, S, M, E, C, cur_stream());
+  }
+  {
+    Stage st(stages, "fwd.gemm1");
+    GemmOpts o = local_opts(r, kEpiBiasAct);
+    o.bias = b1;
+    if (want_grad) o.aux = dact = torch::empty({E, C, H}, x.options());
+    h = grouped_gemm_op(xs, false, w1, true, o);
+  }
+  {
+    Stage st(stages, "fwd.gemm2");
+    GemmOpts o = local_opts(r, kEpiStore);
+    o.bias = b2;
+    ys = grouped_gemm_op(h, false, w2, true, o);
+  }
+  {
+    Stage st(stages, "fwd.combine");
+    count_launch(1);
+    launch_gather_rows<__nv_bfloat16>(ys.data_ptr(), nullptr, r.idx.data_ptr<int>(), r.loc.data_ptr<int>(),
+                                      r.postscore ? r.gates.data_ptr<float>() : nullptr,
+                                      reinterpret_cast<__nv_bfloat16*>(y.data_ptr()), K, S, O, C, nullptr, cur_stream());
+  }
+  return {y, xs, dact, h, ys};
+}
+
+// {dx, dgates, dw1, db1, dw2, db2}; the weights' gradients only where `need_w` says so ([w1, b1, w2, b2])
+std::vector<Tensor> local_backward_op(const Tensor& dy, const Tensor& x, const LocalRoute& r, const Tensor& w1, const Tensor& w2,
+                                      const Tensor& xs, const Tensor& dact, const Tensor& h, const Tensor& ys,
+                                      const std::vector<bool>& need_w, const py::object& stages) {
+  local_check(x, r, w1);
+  c10::cuda::CUDAGuard guard(x.device());
+  const int64_t K = r.idx.size(0), S = x.size(0), M = x.size(1), E = w1.size(0), C = r.C, O = w2.size(2);
+  TORCH_CHECK(dy.is_cuda() && dy.scalar_type() == at::kBFloat16 && dy.dim() == 2 && dy.size(0) == S && dy.size(1) == O);
+  const void* dyp = rows16(dy);
+  const int *idx = r.idx.data_ptr<int>(), *loc = r.loc.data_ptr<int>(), *used = r.used.data_ptr<int>();
+  const float* gates = r.gates.data_ptr<float>();
+  Tensor dgates = torch::empty({K, S}, r.gates.options()), dys = torch::empty({E, C, O}, x.options());
+  Tensor dx = torch::empty_like(x), dh, dxs, dw1, dw2, db1, db2;
+  {
+    Stage st(stages, "bwd.gate_grad");
+    count_launch(1);
+    if (r.postscore)
+      launch_slots_gate_grad(ys.data_ptr(), dyp, idx, loc, gates, used, dgates.data_ptr<float>(), dys.data_ptr(), K, S, O, E, C,
+                             cur_stream());
+    else
+      launch_slots_fill(dyp, r.slot_map.data_ptr<int>(), nullptr, used, dys.data_ptr(), K, S, O, E, C, cur_stream());
+  }
+  {
+    Stage st(stages, "bwd.dgrad2");               // dH = (dY . W2^T) * act'
+    GemmOpts o = local_opts(r, kEpiDAct);
+    o.aux = dact;
+    dh = grouped_gemm_op(dys, false, w2, false, o);
+  }
+  {
+    Stage st(stages, "bwd.dgrad1");               // dX slots = dH . W1^T
+    dxs = grouped_gemm_op(dh, false, w1, false, local_opts(r, kEpiStore));
+  }
+  {
+    Stage st(stages, "bwd.dispatch");
+    count_launch(1);
+    launch_gather_rows<__nv_bfloat16>(dxs.data_ptr(), nullptr, idx, loc, r.postscore ? nullptr : gates,
+                                      reinterpret_cast<__nv_bfloat16*>(dx.data_ptr()), K, S, M, C, nullptr, cur_stream());
+    if (!r.postscore) {
+      count_launch(1);
+      launch_gate_grad<__nv_bfloat16>(reinterpret_cast<const __nv_bfloat16*>(dxs.data_ptr()),
+                                      reinterpret_cast<const __nv_bfloat16*>(x.data_ptr()), idx, loc, dgates.data_ptr<float>(),
+                                      nullptr, nullptr, K, S, M, C, cur_stream());
+    }
+  }
+  if (need_w[2]) {
+    Stage st(stages, "bwd.wgrad2");
+    dw2 = grouped_gemm_op(h, true, dys, true, local_opts(r, kEpiStore));
+  }
+  if (need_w[0]) {
+    Stage st(stages, "bwd.wgrad1");
+    dw1 = grouped_gemm_op(xs, true, dh, true, local_opts(r, kEpiStore));
+  }
+  if (need_w[1] || need_w[3]) {
+    Stage st(stages, "bwd.bias_grads");
+    count_launch(2);
+    ColsumJob j[2] = {};
+    Tensor b2s = colsum_job(dys, 1, true, j[0], db2, used), b1s = colsum_job(dh, 1, true, j[1], db1, used);
+    launch_colsum_jobs(j, 2, cur_stream());
+  }
+  return {dx, dgates, dw1, db1, dw2, db2};
 }
 
 // rows [R, M] -> uint8 [R, M + 16]: M quantised bytes + {scale, low, 0, 0} (the wire rows of the fused send)
@@ -760,6 +915,14 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("dispatch_gate_grad_scaled", &dispatch_gate_grad_scaled_op);
   m.def("dispatch_gate_grad_q8", &dispatch_gate_grad_q8_op);
   m.def("gate_forward", &gate_forward_op);
+  m.def("gate_forward_used", &gate_forward_used_op);
+  py::class_<LocalRoute>(m, "LocalRoute")
+      .def(py::init([](Tensor idx, Tensor loc, Tensor slot_map, Tensor used, Tensor gates, int64_t C, int64_t act, bool postscore,
+                       int64_t budget_ms, int64_t status_ptr) {
+        return LocalRoute{idx, loc, slot_map, used, gates, C, act, postscore, budget_ms, status_ptr};
+      }));
+  m.def("local_forward", &local_forward_op);
+  m.def("local_backward", &local_backward_op);
   m.def("importance_order", &importance_order_op);
   m.def("remap_slot_map", &remap_slot_map_op);
   m.def("gate_backward", &gate_backward_op);
@@ -820,6 +983,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def_readwrite("perm_seg_rows", &GemmOpts::perm_seg_rows)
       .def_readwrite("perm_local_first", &GemmOpts::perm_local_first)
       .def_readwrite("copy_nblk", &GemmOpts::copy_nblk)
+      .def_readwrite("rows_used", &GemmOpts::rows_used)
       .def_readwrite("trace_ptr", &GemmOpts::trace_ptr)
       .def_readwrite("dq_ptr", &GemmOpts::dq_ptr)
       .def_readwrite("dq_arrival_ptr", &GemmOpts::dq_arrival_ptr)

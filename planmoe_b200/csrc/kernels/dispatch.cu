@@ -444,6 +444,155 @@ void launch_gate_grad(const T* disp, const T* dy, const int* idx, const int* loc
                                                         disp_scales, group_rows, scaled_q);
 }
 
+// ------------------------------------------------------------------------------------------
+// One rank: rows go straight into the experts' slots (bf16), no receive buffer, no flags.
+// ------------------------------------------------------------------------------------------
+namespace {
+
+// Rows of expert e that have to be written: used[e] tokens, then zeros to the end of their block.
+__device__ __forceinline__ int slots_end(int used, int C) {
+  return min(C, (max(used, 1) + kSlotBlock - 1) / kSlotBlock * kSlotBlock);
+}
+constexpr int kRowUnroll = 4;                      // 16-byte loads a lane has in flight per row
+
+// One warp per slot.  Bound by memory: 34 MB read and 67 MB written for 8192 tokens of 2048, top-2.
+template <bool SCALE>
+__global__ void __launch_bounds__(kRowThreads)
+slots_fill_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ slot_map, const float* __restrict__ gates,
+                  const int* __restrict__ used, __nv_bfloat16* __restrict__ out, int K, int S, int M, int E, int C) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nvec = M / 8;
+  const long long rows = (long long)E * C;
+  for (long long r = (long long)blockIdx.x * kRowWarps + warp; r < rows; r += (long long)gridDim.x * kRowWarps) {
+    const int e = (int)(r / C), c = (int)(r - (long long)e * C);
+    const int n = used[e];
+    if (c >= slots_end(n, C)) continue;
+    uint4* dst = reinterpret_cast<uint4*>(out + r * M);
+    const int owner = c < n ? slot_map[r] : -1;
+    if (owner < 0) {
+      for (int v = lane; v < nvec; v += 32) dst[v] = make_uint4(0, 0, 0, 0);
+      continue;
+    }
+    const int t = owner / K;
+    const uint4* src = reinterpret_cast<const uint4*>(x + (long long)t * M);
+    const float gw = SCALE ? gates[(size_t)(owner - t * K) * S + t] : 1.f;
+    for (int v0 = lane; v0 < nvec; v0 += 32 * kRowUnroll) {
+      uint4 raw[kRowUnroll];
+#pragma unroll
+      for (int i = 0; i < kRowUnroll; ++i)
+        if (v0 + 32 * i < nvec) raw[i] = __ldg(src + v0 + 32 * i);
+#pragma unroll
+      for (int i = 0; i < kRowUnroll; ++i) {
+        if (v0 + 32 * i >= nvec) break;
+        if constexpr (SCALE) {
+          Pack<__nv_bfloat16> q = *reinterpret_cast<Pack<__nv_bfloat16>*>(&raw[i]);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) q.v[j] = __float2bfloat16_rn(gw * __bfloat162float(q.v[j]));
+          raw[i] = *reinterpret_cast<uint4*>(&q);
+        }
+        dst[v0 + 32 * i] = raw[i];
+      }
+    }
+  }
+}
+
+// One warp per token: the token's dy row is read once for all its picks (the exchange form reads it once per pick and
+// writes token-major copies that a send then moves).  The warps behind the tokens' write the zero rows.
+template <int MAXK>
+__global__ void __launch_bounds__(kRowThreads)
+slots_gate_grad_kernel(const __nv_bfloat16* __restrict__ disp, const __nv_bfloat16* __restrict__ dy,
+                       const int* __restrict__ idx, const int* __restrict__ loc, const float* __restrict__ gates,
+                       const int* __restrict__ used, float* __restrict__ dgates, __nv_bfloat16* __restrict__ ddisp, int K,
+                       int S, int M, int E, int C) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nvec = M / 8;
+  const long long items = (long long)S + (long long)E * kSlotBlock;
+  for (long long it = (long long)blockIdx.x * kRowWarps + warp; it < items; it += (long long)gridDim.x * kRowWarps) {
+    if (it >= S) {
+      const int q = (int)(it - S), e = q / kSlotBlock;
+      const int n = used[e], c = n + (q - e * kSlotBlock);
+      if (c >= slots_end(n, C)) continue;
+      uint4* dst = reinterpret_cast<uint4*>(ddisp + ((long long)e * C + c) * M);
+      for (int v = lane; v < nvec; v += 32) dst[v] = make_uint4(0, 0, 0, 0);
+      continue;
+    }
+    const int t = (int)it;
+    const uint4* b = reinterpret_cast<const uint4*>(dy + (long long)t * M);
+    long long slot[MAXK];
+    float gw[MAXK], acc[MAXK];
+#pragma unroll
+    for (int k = 0; k < MAXK; ++k) {
+      slot[k] = -1; gw[k] = 0.f; acc[k] = 0.f;
+      if (k < K) {
+        const int e = idx[(size_t)k * S + t], l = loc[(size_t)k * S + t];
+        if (e >= 0 && l >= 0 && l < C) { slot[k] = ((long long)e * C + l) * nvec; gw[k] = gates[(size_t)k * S + t]; }
+      }
+    }
+    constexpr int U = MAXK <= 2 ? 2 : 1;
+    for (int v0 = lane; v0 < nvec; v0 += 32 * U) {
+      uint4 rb[U], ra[U][MAXK];
+#pragma unroll
+      for (int i = 0; i < U; ++i) {
+        const int v = v0 + 32 * i;
+        if (v >= nvec) break;
+        rb[i] = __ldg(b + v);
+#pragma unroll
+        for (int k = 0; k < MAXK; ++k)
+          if (slot[k] >= 0) ra[i][k] = __ldg(reinterpret_cast<const uint4*>(disp) + slot[k] + v);
+      }
+#pragma unroll
+      for (int i = 0; i < U; ++i) {
+        const int v = v0 + 32 * i;
+        if (v >= nvec) break;
+        float fb[8];
+        const Pack<__nv_bfloat16> pb = *reinterpret_cast<const Pack<__nv_bfloat16>*>(&rb[i]);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) fb[j] = __bfloat162float(pb.v[j]);
+#pragma unroll
+        for (int k = 0; k < MAXK; ++k) {
+          if (slot[k] < 0) continue;
+          const Pack<__nv_bfloat16> pa = *reinterpret_cast<const Pack<__nv_bfloat16>*>(&ra[i][k]);
+          Pack<__nv_bfloat16> o;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            acc[k] += __bfloat162float(pa.v[j]) * fb[j];
+            o.v[j] = __float2bfloat16_rn(gw[k] * fb[j]);
+          }
+          reinterpret_cast<uint4*>(ddisp)[slot[k] + v] = *reinterpret_cast<const uint4*>(&o);
+        }
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < MAXK; ++k) {
+      const float a = warp_sum(acc[k]);
+      if (k < K && lane == 0) dgates[(size_t)k * S + t] = a;
+    }
+  }
+}
+
+unsigned row_grid(long long rows) {
+  const long long ctas = (rows + kRowWarps - 1) / kRowWarps;
+  return (unsigned)(ctas < 1 ? 1 : ctas > 148 * 8 ? 148 * 8 : ctas);
+}
+
+}  // namespace
+
+void launch_slots_fill(const void* x, const int* slot_map, const float* gates, const int* used, void* out, int K, int S,
+                       int M, int E, int C, cudaStream_t stream) {
+  auto kern = gates != nullptr ? slots_fill_kernel<true> : slots_fill_kernel<false>;
+  kern<<<row_grid((long long)E * C), kRowThreads, 0, stream>>>(reinterpret_cast<const __nv_bfloat16*>(x), slot_map, gates,
+                                                               used, reinterpret_cast<__nv_bfloat16*>(out), K, S, M, E, C);
+}
+
+void launch_slots_gate_grad(const void* disp, const void* dy, const int* idx, const int* loc, const float* gates,
+                            const int* used, float* dgates, void* ddisp, int K, int S, int M, int E, int C,
+                            cudaStream_t stream) {
+  auto kern = K <= 1 ? slots_gate_grad_kernel<1> : K <= 2 ? slots_gate_grad_kernel<2> : slots_gate_grad_kernel<4>;
+  kern<<<row_grid((long long)S + (long long)E * kSlotBlock), kRowThreads, 0, stream>>>(
+      reinterpret_cast<const __nv_bfloat16*>(disp), reinterpret_cast<const __nv_bfloat16*>(dy), idx, loc, gates, used, dgates,
+      reinterpret_cast<__nv_bfloat16*>(ddisp), K, S, M, E, C);
+}
+
 #define INSTANTIATE(T)                                                                             \
   template void launch_scatter_rows<T>(const T*, const int*, const float*, T*, int, int, int, int, \
                                        int, const PushArgs*, bool, cudaStream_t);                  \

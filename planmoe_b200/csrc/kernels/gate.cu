@@ -134,6 +134,7 @@ gate_assign_kernel(int S, int E, int K, int C, int normalize, float eps,
                    const float* __restrict__ blk_score, int nblk,
                    int* __restrict__ loc, GatePtrs gates, int* __restrict__ slot_map,
                    int* __restrict__ top1_count,  // [E] tokens whose first pick is e
+                   int* __restrict__ used,        // [E] slots of expert e that hold a token, or null
                    float* __restrict__ l_aux)     // [1]
 {
   __shared__ int base[kMaxK][kMaxE];
@@ -183,6 +184,13 @@ gate_assign_kernel(int S, int E, int K, int C, int normalize, float eps,
       }
       s = warp_sum(s);
       c = __reduce_add_sync(0xffffffffu, c);
+      if (used != nullptr) {
+        int n = 0;
+        for (int kk = 1; kk < K; ++kk)
+          for (int bb = lane; bb < nblk; bb += 32) n += blk_count[(size_t)(kk * E + e) * nblk + bb];
+        n = __reduce_add_sync(0xffffffffu, n);
+        if (lane == 0) used[e] = min(C, c + n);
+      }
       if (lane == 0) {
         top1_count[e] = c;
         red[e] = s * (float)c;
@@ -257,7 +265,7 @@ gate_bwd_kernel(const T* __restrict__ logits, int S, int E, int K, int normalize
 template <class T, bool SCORES>
 void launch_gate_forward(const T* logits, int S, int E, int K, int C, bool normalize, float eps,
                          int* idx, int* loc, GatePtrs gates, float* raw_gate, int* slot_map,
-                         int* top1_count, float* l_aux, int* ws_rank, int* ws_blk_count,
+                         int* top1_count, int* used, float* l_aux, int* ws_rank, int* ws_blk_count,
                          float* ws_blk_score, cudaStream_t stream) {
   const int nblk = (S + kGateThreads - 1) / kGateThreads;
   auto stats = E <= 8 ? gate_stats_kernel<T, 8, SCORES> : E <= 16 ? gate_stats_kernel<T, 16, SCORES>
@@ -266,7 +274,7 @@ void launch_gate_forward(const T* logits, int S, int E, int K, int C, bool norma
                                            slot_map, (long long)E * C);
   gate_assign_kernel<<<nblk, kGateThreads, 0, stream>>>(S, E, K, C, normalize ? 1 : 0, eps, idx,
                                                       raw_gate, ws_rank, ws_blk_count, ws_blk_score,
-                                                      nblk, loc, gates, slot_map, top1_count, l_aux);
+                                                      nblk, loc, gates, slot_map, top1_count, used, l_aux);
 }
 
 template <class T, bool SCORES>
@@ -348,7 +356,7 @@ void launch_remap_slot_map(int* slot_map, long long n, const int* perm, int K, c
 
 #define INSTANTIATE(T, SCORES)                                                                    \
   template void launch_gate_forward<T, SCORES>(const T*, int, int, int, int, bool, float, int*, int*,     \
-                                               GatePtrs, float*, int*, int*, float*, int*, int*, float*,  \
+                                               GatePtrs, float*, int*, int*, int*, float*, int*, int*, float*, \
                                                cudaStream_t);                                             \
   template void launch_gate_backward<T, SCORES>(const T*, int, int, int, bool, float, const int*, GatePtrs, \
                                                 const float*, const int*, T*, cudaStream_t);

@@ -62,16 +62,29 @@ void launch_gate_grad(const T* disp, const T* dy, const int* idx, const int* loc
                       const float* gates, T* scaled, int K, int S, int M, int C, cudaStream_t stream,
                       const float* disp_scales = nullptr, long long group_rows = 0, unsigned char* scaled_q = nullptr);
 
+// ---- one rank: tokens straight into the experts' slots ----
+// Of an expert's C slots only the first used[e] hold tokens.  What computes on slots does so in blocks of at most
+// kSlotBlock rows and stops behind the block with the last token; the rows of that block behind it are zeros.
+constexpr int kSlotBlock = 256;
+// out[e * C + c] = (gate *) row of the token that holds the slot
+void launch_slots_fill(const void* x, const int* slot_map, const float* gates, const int* used, void* out, int K, int S,
+                       int M, int E, int C, cudaStream_t stream);
+// dgates[k][t] = <disp[slot_k(t)], dy[t]>, ddisp[slot_k(t)] = gates[k][t] * dy[t]
+void launch_slots_gate_grad(const void* disp, const void* dy, const int* idx, const int* loc, const float* gates,
+                            const int* used, float* dgates, void* ddisp, int K, int S, int M, int E, int C,
+                            cudaStream_t stream);
+
 // ---- kernels/gate.cu -------------------------------------------------------------------------
 int gate_workspace_blocks(int S);
 // One fp32 row of S values per pick (gates, or their gradients; null = zeros).
 struct GatePtrs { float* p[4]; };
 // SCORES: the input is a [S, E] matrix of scores to pick from as they are; otherwise logits, softmax first.
-// slot_map: [E * C], written completely.
+// slot_map: [E * C], written completely.  used (optional): [E] slots of every expert that hold a token; an expert's
+// slots are handed out from 0 on, so these are its first ones.
 template <class T, bool SCORES>
 void launch_gate_forward(const T* logits, int S, int E, int K, int C, bool normalize, float eps,
                          int* idx, int* loc, GatePtrs gates, float* raw_gate, int* slot_map,
-                         int* top1_count, float* l_aux, int* ws_rank, int* ws_blk_count,
+                         int* top1_count, int* used, float* l_aux, int* ws_rank, int* ws_blk_count,
                          float* ws_blk_score, cudaStream_t stream);
 template <class T, bool SCORES>
 void launch_gate_backward(const T* logits, int S, int E, int K, bool normalize, float eps,
@@ -171,6 +184,11 @@ struct GemmArgs {
   // gate_flags[chunk * W + s]; pushed rows land at column offset chunk * push_rows and signal
   // flag [chunk * W + my_rank].  One launch then covers all pipeline chunks.
   int chunk_groups;
+  // Optional device [groups]: only the first rows_used[g] token rows of group g hold anything.  The token rows are the M
+  // dim, or the contraction of a weight gradient (MN-major A).  Row blocks (M) or K blocks behind them are left out;
+  // at least one is computed, so rows up to the end of the last block (kSlotBlock) have to be finite, and zero in
+  // one operand of a weight gradient.  At most 64 groups, one chunk, no flag gate, no push, no copy role.
+  const int* rows_used;
   unsigned long long budget_ns; int* status;
   // Optional role trace, device u64 [grid][32] (ns of %globaltimer): [0] kernel entry, [1] / [2] copy role begin / end,
   // [3] time the TMA producer spent waiting on gate flags, [4] kernel exit, [5] de-quantiser role end; in SM clocks,
@@ -227,6 +245,7 @@ struct ColsumJob {
   const void* x; float* out; void* out_bf16; float* partial; unsigned* counters;
   long long rows, row_stride, group_stride;
   int N, groups, fold;
+  const int* rows_used;            // optional device [groups]: rows behind the first rows_used[g] are left out
 };
 int colsum_colblocks(int N);
 void launch_colsum_jobs(const ColsumJob* jobs, int n, cudaStream_t stream);

@@ -20,8 +20,9 @@ Backward mirrors it (combine-backward is a dispatch-like push of dY, the two dgr
 flag-gated / pushing in the same way, dispatch-backward is a flag-waiting gather) and the two
 weight-gradient GEMMs contract over all chunks of the receive buffers in one launch each.
 
-No NCCL call and no library GEMM is on this path; with one rank the "peer" is the local heap and
-the same kernels run.  The receive buffers are laid out ``[chunk][E_local][W_src][C/chunks][M]``,
+No NCCL call and no library GEMM is on this path.  With one rank there is nothing to exchange: rows go straight into the
+experts' slots and the same GEMM kernels run on them, without flags, receive buffers or pipeline chunks
+(``_LocalExperts``).  The receive buffers are laid out ``[chunk][E_local][W_src][C/chunks][M]``,
 i.e. they *are* the grouped-GEMM operands: the reference's permute copies, chunk splits and
 concatenations (``PlanMoE/impls/overlap.py:55-75``, ``impls/communicate.py:604-623``) have no
 counterpart here.
@@ -41,6 +42,7 @@ import torch.nn.functional as F
 from . import native
 from .gemm import ACT_CODES, EPI_BIAS_ACT, EPI_DACT, EPI_PUSH, EPI_STORE, grouped_gemm
 from ..parallel import transport as T
+from ..utils import stage_timer
 from ..utils.stage_timer import stage
 
 MAX_CHUNKS = 32      # largest pipeline degree (flag slots per phase are sized for it)
@@ -276,11 +278,11 @@ class _FusedGate(torch.autograd.Function):
     def forward(ctx, logits, top_k, capacity, normalize):
         lib = native.lib()
         logits = logits.contiguous()
-        idx, loc, gates, slot_map, top1, l_aux = lib.gate_forward(logits, top_k, capacity, normalize)
+        idx, loc, gates, slot_map, top1, l_aux, used = lib.gate_forward_used(logits, top_k, capacity, normalize)
         ctx.save_for_backward(logits, idx, top1)
         ctx.normalize = normalize
-        ctx.mark_non_differentiable(idx, loc, slot_map)
-        return gates, l_aux.view(()), idx, loc, slot_map
+        ctx.mark_non_differentiable(idx, loc, slot_map, used)
+        return gates, l_aux.view(()), idx, loc, slot_map, used
 
     @staticmethod
     def backward(ctx, dgates, dl_aux, *_):
@@ -293,6 +295,11 @@ class _FusedGate(torch.autograd.Function):
 
 def fused_gate(logits, top_k, capacity, normalize):
     """(gates [K,S] fp32, l_aux scalar fp32, idx, loc, slot_map) — differentiable in logits."""
+    return fused_gate_used(logits, top_k, capacity, normalize)[:5]
+
+
+def fused_gate_used(logits, top_k, capacity, normalize):
+    """The same, and ``used [E]``: how many of an expert's slots hold a token (its first ones)."""
     return _FusedGate.apply(logits, int(top_k), int(capacity), bool(normalize))
 
 
@@ -444,6 +451,61 @@ class _FusedExperts(torch.autograd.Function):
         return dx, dgates, dw1, db1, dw2, db2, None
 
 
+def _local_path(tr, q8):
+    """Whether a layer's experts run without the exchange: one rank and bf16 rows.  PLANMOE_LOCAL=0, a choice of the send's
+    form (PLANMOE_FUSE_SEND), the debug guards and the role trace keep the exchange, which is what they are about."""
+    return (tr.world == 1 and not tr.emulated and not q8 and os.environ.get('PLANMOE_LOCAL', '1') != '0'
+            and 'PLANMOE_FUSE_SEND' not in os.environ and not T.debug_guards()
+            and os.environ.get('PLANMOE_GEMM_TRACE', '0') != '1')
+
+
+def _aligned(t):
+    """``t`` contiguous, its first element on a 16-byte boundary (the kernels move rows as 16-byte vectors)."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
+def _stages():
+    return stage if stage_timer.enabled() else None
+
+
+class _LocalExperts(torch.autograd.Function):
+    """Dispatch, experts and combine of one rank.  Slots are ``[E, C]``; what lies behind an expert's last used row block is
+    neither written nor computed (``used``)."""
+
+    @staticmethod
+    def forward(ctx, x, gates, w1, b1, w2, b2, meta):
+        y, xs, dact, h, ys = _local_forward(x, gates, w1, b1, w2, b2, meta, True)
+        ctx.save_for_backward(x, gates, w1, w2, xs, dact, h, ys, meta['idx'], meta['loc'], meta['slot_map'], meta['used'])
+        ctx.meta = {k: meta[k] for k in ('C', 'act', 'postscore', 'budget_ms', 'status')}
+        return y
+
+    @staticmethod
+    def backward(ctx, dy):
+        x, gates, w1, w2, xs, dact, h, ys, idx, loc, slot_map, used = ctx.saved_tensors
+        route = _local_route(gates, dict(ctx.meta, idx=idx, loc=loc, slot_map=slot_map, used=used))
+        dx, dgates, dw1, db1, dw2, db2 = native.lib().local_backward(
+            _aligned(dy), x, route, w1, w2, xs, dact, h, ys, list(ctx.needs_input_grad[2:6]), _stages())
+        return dx, dgates, dw1, db1, dw2, db2, None
+
+
+def _local_route(gates, m):
+    return native.lib().LocalRoute(m['idx'], m['loc'], m['slot_map'], m['used'], gates, m['C'], m['act'], m['postscore'],
+                                   m['budget_ms'], m['status'].device_ptr())
+
+
+def _local_forward(x, gates, w1, b1, w2, b2, meta, want_grad):
+    route = _local_route(gates, meta)
+    return native.lib().local_forward(x, route, w1, b1, w2, b2, want_grad, _stages())
+
+
+def _local_experts(x, gates, w1, b1, w2, b2, meta):
+    x, gates = _aligned(x), gates.contiguous()
+    if torch.is_grad_enabled() and any(t.requires_grad for t in (x, gates, w1, b1, w2, b2)):
+        return _LocalExperts.apply(x, gates, w1, b1, w2, b2, meta)
+    return _local_forward(x, gates, w1, b1, w2, b2, meta, False)[0]
+
+
 def _dynamic_capacity(lib, logits, top_k, normalize, group, align):
     """Capacity for ``capacity_factor == 0``: the largest slot any expert hands out, over all ranks, plus one
     (reference: PlanMoE/impls/fast_dispatch.py:183-184, including its one host read of the all-reduced value).
@@ -522,14 +584,14 @@ def forward(layer, x, gctx, top_k, capacity_factor, degree):
     with stage('fwd.gate_topk_scan'):
         if layer.batch_prioritized_routing:
             rank, perm = lib.importance_order(logits.detach())
-            gates_p, l_aux, idx_p, loc_p, slot_map = fused_gate(logits.index_select(0, perm.long()), top_k, capacity,
-                                                                layer.normalize_gate)
+            gates_p, l_aux, idx_p, loc_p, slot_map, used = fused_gate_used(logits.index_select(0, perm.long()), top_k, capacity,
+                                                                      layer.normalize_gate)
             pos = rank.long()
             gates = gates_p.index_select(1, pos)
             idx, loc = idx_p.index_select(1, pos).contiguous(), loc_p.index_select(1, pos).contiguous()
             lib.remap_slot_map(slot_map, perm, top_k)
         else:
-            gates, l_aux, idx, loc, slot_map = fused_gate(logits, top_k, capacity, layer.normalize_gate)
+            gates, l_aux, idx, loc, slot_map, used = fused_gate_used(logits, top_k, capacity, layer.normalize_gate)
     if not layer.is_gshard_loss:
         from ..impls import losses
         topk_logits = logits.float().gather(1, idx.t().long())
@@ -537,13 +599,19 @@ def forward(layer, x, gctx, top_k, capacity_factor, degree):
     if T.debug_guards():
         check_routing_bounds(idx, loc, slot_map, S, E, capacity, top_k)
     ex = layer.experts
-    meta = dict(state=st, idx=idx, loc=loc, slot_map=slot_map, E=E, C=capacity, degree=degree, K=top_k,
-                act=ACT_CODES[ex.act_name], postscore=layer.is_postscore, q8=(layer.compress_name == 'int8'))
-    y = _FusedExperts.apply(x.contiguous(), gates, ex.batched_fc1_w, ex.batched_fc1_bias,
-                            ex.batched_fc2_w, ex.batched_fc2_bias, meta)
+    q8 = layer.compress_name == 'int8'
+    args = (gates, ex.batched_fc1_w, ex.batched_fc1_bias, ex.batched_fc2_w, ex.batched_fc2_bias)
+    if _local_path(st.tr, q8):
+        y = _local_experts(x, *args, dict(idx=idx, loc=loc, slot_map=slot_map, used=used, C=capacity,
+                                          act=ACT_CODES[ex.act_name], postscore=layer.is_postscore,
+                                          budget_ms=st.tr.budget_ms, status=st.tr.status))
+    else:
+        meta = dict(state=st, idx=idx, loc=loc, slot_map=slot_map, E=E, C=capacity, degree=degree, K=top_k,
+                    act=ACT_CODES[ex.act_name], postscore=layer.is_postscore, q8=q8)
+        y = _FusedExperts.apply(x.contiguous(), *args, meta)
     # both 'naive' and 'pipe' run as the flat push of the copy role / push epilogue: say so instead of echoing the name
     layer.last_stats = dict(capacity=capacity, degree=degree, path='fused', comm='flat-push',
-                            wire=('int8' if meta['q8'] else 'bf16'))
+                            wire=('int8' if q8 else 'bf16'))
     if getattr(layer, 'collect_stats', False):
         from ..utils import metrics
         layer.last_stats.update(metrics.routing_stats(idx, loc, E, capacity))

@@ -36,6 +36,8 @@ ENV = {
     'STRICT_FMT / PTYPE / CONFIG / DEVICE / MODE / CONFIG_STORE_PATH / HOSTS / VERBOSE': ('', 'parted (auto-SPMD tool)'),
     # ---- this package --------------------------------------------------------------------------------------------
     'PLANMOE_FUSED': ('1', '0: every layer takes the generic path (ATen routing, codec objects, stand-alone all-to-all)'),
+    'PLANMOE_LOCAL': ('1', '0: a single rank runs the exchange (receive buffers, flags, dispatch send) like any other instead of '
+                      'filling the slots directly'),
     'PLANMOE_FUSE_SEND': ('1', '0: the dispatch send is a separate copy kernel in front of the flag-gated GEMM instead of a '
                           'copy warp inside it (the int8 wire needs 1)'),
     'PLANMOE_GEMM': ('tcgen05', "'cublas': FFN experts use torch.matmul (and layers leave the fused path)"),
