@@ -23,6 +23,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <algorithm>
 #include <atomic>
 
 namespace py = pybind11;
@@ -558,7 +559,7 @@ std::vector<Tensor> colsum2_op(const Tensor& xa, const Tensor& xb, int64_t fold,
   return {ba.narrow(0, 0, ga * xa.size(2)).view({ga, xa.size(2)}), bb.narrow(0, 0, gb * xb.size(2)).view({gb, xb.size(2)})};
 }
 
-// ---- one rank: the experts' forward and backward in one call each --------------------------------
+// ---- one rank: a pass of the layer, or of its experts, in one call --------------------------------
 // A stage of the pass for the per-stage timers: `stages` is None, or a callable that makes a context manager of a name.
 struct Stage {
   py::object cm;
@@ -571,7 +572,8 @@ struct Stage {
   }
 };
 
-// Routing of a pass: idx, loc int32 [K, S]; slot_map int32 [E * C]; used int32 [E]; gates fp32 [K, S].
+// What a pass is done with, and its routing: idx, loc int32 [K, S]; slot_map int32 [E * C]; used int32 [E]; gates fp32
+// [K, S].
 struct LocalRoute {
   Tensor idx, loc, slot_map, used, gates;
   int64_t C, act;
@@ -579,13 +581,18 @@ struct LocalRoute {
   int64_t budget_ms, status_ptr;
 };
 
+static const void* rows16(const Tensor& t) {      // a row tensor the vector kernels may read
+  TORCH_CHECK(t.is_contiguous() && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0, "rows must be 16-byte aligned");
+  return t.data_ptr();
+}
+
 static void local_check(const Tensor& x, const LocalRoute& r, const Tensor& w1) {
   const int64_t K = r.idx.size(0), S = r.idx.size(1), E = w1.size(0);
   auto i32 = [&](const Tensor& t, int64_t n) {
     return t.is_cuda() && t.scalar_type() == at::kInt && t.is_contiguous() && t.numel() == n;
   };
-  TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.dim() == 2 && x.is_contiguous() && x.size(0) == S);
-  TORCH_CHECK(reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0 && x.size(1) % 8 == 0, "rows must be 16-byte aligned");
+  TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.dim() == 2 && x.size(0) == S && x.size(1) % 8 == 0);
+  rows16(x);
   TORCH_CHECK(i32(r.idx, K * S) && i32(r.loc, K * S) && i32(r.slot_map, E * r.C) && i32(r.used, E) && K <= 4 && E <= 64);
   TORCH_CHECK(r.gates.is_cuda() && r.gates.scalar_type() == at::kFloat && r.gates.is_contiguous() && r.gates.numel() == K * S);
 }
@@ -595,11 +602,6 @@ static GemmOpts local_opts(const LocalRoute& r, int64_t epilogue) {
   o.epilogue = epilogue; o.activation = r.act; o.budget_ms = r.budget_ms; o.status_ptr = r.status_ptr;
   o.rows_used = r.used;
   return o;
-}
-
-static const void* rows16(const Tensor& t) {      // a row tensor the vector kernels may read
-  TORCH_CHECK(t.is_contiguous() && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0, "rows must be 16-byte aligned");
-  return t.data_ptr();
 }
 
 // {y [S, O], xs [E, C, M], dact [E, C, H], h [E, C, H], ys [E, C, O]}; without `want_grad` no derivative is saved (dact
@@ -639,10 +641,38 @@ std::vector<Tensor> local_forward_op(const Tensor& x, const LocalRoute& r, const
   return {y, xs, dact, h, ys};
 }
 
-// {dx, dgates, dw1, db1, dw2, db2}; the weights' gradients only where `need_w` says so ([w1, b1, w2, b2])
-std::vector<Tensor> local_backward_op(const Tensor& dy, const Tensor& x, const LocalRoute& r, const Tensor& w1, const Tensor& w2,
-                                      const Tensor& xs, const Tensor& dact, const Tensor& h, const Tensor& ys,
-                                      const std::vector<bool>& need_w, const py::object& stages) {
+// The linear gate of a pass: logits fp32 [S, E] and what its backward needs.
+struct LocalGate {
+  Tensor w, logits, top1;
+  bool normalize, bf16_logits;
+  float eps() const { return bf16_logits ? 7.8125e-03f : kFloatEps; }
+};
+
+static Tensor local_gate_backward(const LocalGate& g, const LocalRoute& r, const Tensor& dgates,
+                                  const c10::optional<Tensor>& dl_aux) {
+  const int S = g.logits.size(0), E = g.logits.size(1), K = r.idx.size(0);
+  Tensor dl = torch::empty_like(g.logits);
+  GatePtrs gp{};
+  for (int k = 0; k < K; ++k) gp.p[k] = dgates.data_ptr<float>() + (int64_t)k * S;
+  const float* f = nullptr;
+  const void* h = nullptr;
+  if (dl_aux.has_value() && dl_aux->defined()) {
+    TORCH_CHECK(dl_aux->is_cuda() && dl_aux->numel() == 1);
+    if (dl_aux->scalar_type() == at::kBFloat16) h = dl_aux->data_ptr();
+    else f = dl_aux->data_ptr<float>();
+  }
+  count_launch(1);
+  launch_gate_backward<float, false>(g.logits.data_ptr<float>(), S, E, K, g.normalize, g.eps(), r.idx.data_ptr<int>(), gp, f,
+                                     g.top1.data_ptr<int>(), dl.data_ptr<float>(), cur_stream(), h);
+  return dl;
+}
+
+// {dx, dgates or dwg, dw1, db1, dw2, db2}: with `gate` the second is the gradient of the gate's weight and dx has the
+// gate's part in it, without it the gradient of the gates.  `need`: which of x, (gates or wg), w1, b1, w2, b2 are asked for.
+static std::vector<Tensor> local_backward(const Tensor& dy, const Tensor& x, const LocalRoute& r, const Tensor& w1,
+                                          const Tensor& w2, const Tensor& xs, const Tensor& dact, const Tensor& h,
+                                          const Tensor& ys, const std::vector<bool>& need, const LocalGate* gate,
+                                          const c10::optional<Tensor>& dl_aux, const py::object& stages) {
   local_check(x, r, w1);
   c10::cuda::CUDAGuard guard(x.device());
   const int64_t K = r.idx.size(0), S = x.size(0), M = x.size(1), E = w1.size(0), C = r.C, O = w2.size(2);
@@ -651,7 +681,7 @@ std::vector<Tensor> local_backward_op(const Tensor& dy, const Tensor& x, const L
   const int *idx = r.idx.data_ptr<int>(), *loc = r.loc.data_ptr<int>(), *used = r.used.data_ptr<int>();
   const float* gates = r.gates.data_ptr<float>();
   Tensor dgates = torch::empty({K, S}, r.gates.options()), dys = torch::empty({E, C, O}, x.options());
-  Tensor dx = torch::empty_like(x), dh, dxs, dw1, dw2, db1, db2;
+  Tensor dx, dh, dxs, dl, dwg, dw1, dw2, db1, db2;
   {
     Stage st(stages, "bwd.gate_grad");
     count_launch(1);
@@ -660,6 +690,7 @@ std::vector<Tensor> local_backward_op(const Tensor& dy, const Tensor& x, const L
                              cur_stream());
     else
       launch_slots_fill(dyp, r.slot_map.data_ptr<int>(), nullptr, used, dys.data_ptr(), K, S, O, E, C, cur_stream());
+    if (gate != nullptr && r.postscore) dl = local_gate_backward(*gate, r, dgates, dl_aux);
   }
   {
     Stage st(stages, "bwd.dgrad2");               // dH = (dY . W2^T) * act'
@@ -667,38 +698,150 @@ std::vector<Tensor> local_backward_op(const Tensor& dy, const Tensor& x, const L
     o.aux = dact;
     dh = grouped_gemm_op(dys, false, w2, false, o);
   }
-  {
+  const bool gate_from_dx = !r.postscore && (need[1] || gate != nullptr);
+  if (need[0] || gate_from_dx) {
     Stage st(stages, "bwd.dgrad1");               // dX slots = dH . W1^T
     dxs = grouped_gemm_op(dh, false, w1, false, local_opts(r, kEpiStore));
   }
   {
     Stage st(stages, "bwd.dispatch");
-    count_launch(1);
-    launch_gather_rows<__nv_bfloat16>(dxs.data_ptr(), nullptr, idx, loc, r.postscore ? nullptr : gates,
-                                      reinterpret_cast<__nv_bfloat16*>(dx.data_ptr()), K, S, M, C, nullptr, cur_stream());
-    if (!r.postscore) {
+    if (gate_from_dx) {
       count_launch(1);
       launch_gate_grad<__nv_bfloat16>(reinterpret_cast<const __nv_bfloat16*>(dxs.data_ptr()),
                                       reinterpret_cast<const __nv_bfloat16*>(x.data_ptr()), idx, loc, dgates.data_ptr<float>(),
                                       nullptr, nullptr, K, S, M, C, cur_stream());
+      if (gate != nullptr) dl = local_gate_backward(*gate, r, dgates, dl_aux);
+    }
+    if (need[0]) {
+      dx = torch::empty_like(x);
+      count_launch(1);
+      if (gate != nullptr)
+        launch_gather_gate(dxs.data_ptr(), idx, loc, r.postscore ? nullptr : gates, dl.data_ptr<float>(), gate->w.data_ptr(),
+                           gate->w.scalar_type() == at::kBFloat16, dx.data_ptr(), K, S, M, E, C, cur_stream());
+      else
+        launch_gather_rows<__nv_bfloat16>(dxs.data_ptr(), nullptr, idx, loc, r.postscore ? nullptr : gates,
+                                          reinterpret_cast<__nv_bfloat16*>(dx.data_ptr()), K, S, M, C, nullptr, cur_stream());
     }
   }
-  if (need_w[2]) {
+  if (need[4]) {
     Stage st(stages, "bwd.wgrad2");
     dw2 = grouped_gemm_op(h, true, dys, true, local_opts(r, kEpiStore));
   }
-  if (need_w[0]) {
+  if (need[2]) {
     Stage st(stages, "bwd.wgrad1");
     dw1 = grouped_gemm_op(xs, true, dh, true, local_opts(r, kEpiStore));
   }
-  if (need_w[1] || need_w[3]) {
+  {
     Stage st(stages, "bwd.bias_grads");
-    count_launch(2);
-    ColsumJob j[2] = {};
-    Tensor b2s = colsum_job(dys, 1, true, j[0], db2, used), b1s = colsum_job(dh, 1, true, j[1], db1, used);
-    launch_colsum_jobs(j, 2, cur_stream());
+    ColsumJob j[3] = {};
+    Tensor keep[3];
+    int n = 0;
+    if (need[5]) { keep[n] = colsum_job(dys, 1, true, j[n], db2, used); ++n; }
+    if (need[3]) { keep[n] = colsum_job(dh, 1, true, j[n], db1, used); ++n; }
+    if (n > 0) count_launch(1);
+    if (gate != nullptr && need[1]) {
+      const int chunks = gate_wgrad_chunks(S, M);
+      keep[n] = torch::empty({(int64_t)chunks + 1, E * M}, r.gates.options());
+      const bool bf16 = gate->w.scalar_type() == at::kBFloat16;
+      dwg = torch::empty_like(gate->w);
+      float* partial = keep[n].data_ptr<float>();
+      count_launch(1);
+      launch_gate_wgrad(x.data_ptr(), dl.data_ptr<float>(), partial, S, E, M, cur_stream());
+      j[n].partial = partial;
+      j[n].out = bf16 ? partial + (int64_t)chunks * E * M : dwg.data_ptr<float>();
+      j[n].out_bf16 = bf16 ? dwg.data_ptr() : nullptr;
+      j[n].rows = (long long)chunks * 128; j[n].N = (int)(E * M); j[n].groups = j[n].fold = 1;
+      ++n;
+    }
+    if (n > 0) {
+      count_launch(1);
+      launch_colsum_jobs(j, n, cur_stream());
+    }
   }
-  return {dx, dgates, dw1, db1, dw2, db2};
+  return {dx, gate != nullptr ? dwg : dgates, dw1, db1, dw2, db2};
+}
+
+std::vector<Tensor> local_backward_op(const Tensor& dy, const Tensor& x, const LocalRoute& r, const Tensor& w1, const Tensor& w2,
+                                      const Tensor& xs, const Tensor& dact, const Tensor& h, const Tensor& ys,
+                                      const std::vector<bool>& need, const py::object& stages) {
+  return local_backward(dy, x, r, w1, w2, xs, dact, h, ys, need, nullptr, c10::nullopt, stages);
+}
+
+// The whole layer with a linear gate `wg` [E, M].  capacity < 0: as many slots as the busiest expert needs, rounded up by
+// `round_up` (one host read).  Returns {y, l_aux, logits, top1, slot_map, used, idx, loc, gates, xs, dact, h, ys} and the
+// capacity.
+std::tuple<std::vector<Tensor>, int64_t> local_moe_forward_op(
+    const Tensor& x, const Tensor& wg, const Tensor& w1, const Tensor& b1, const Tensor& w2, const Tensor& b2, int64_t K,
+    int64_t capacity, const py::object& round_up, bool normalize, bool bf16_logits, bool prio, int64_t act, bool postscore,
+    int64_t budget_ms, int64_t status_ptr, bool want_grad, const py::object& stages) {
+  TORCH_CHECK(x.is_cuda() && x.dim() == 2 && x.scalar_type() == at::kBFloat16);
+  const int64_t S = x.size(0), M = x.size(1), E = w1.size(0);
+  TORCH_CHECK(wg.is_cuda() && wg.is_contiguous() && wg.dim() == 2 && wg.size(0) == E && wg.size(1) == M && M % 32 == 0 &&
+              (wg.scalar_type() == at::kFloat || wg.scalar_type() == at::kBFloat16) && E <= kProjMaxE && K >= 1 && K <= 4 &&
+              K <= E && S > 0 && S * K <= INT_MAX, "linear gate outside the kernels' range");
+  rows16(wg);
+  c10::cuda::CUDAGuard guard(x.device());
+  auto iopt = x.options().dtype(at::kInt);
+  auto fopt = x.options().dtype(at::kFloat);
+  const int64_t nblk = gate_workspace_blocks(S);
+  LocalRoute r{torch::empty({K, S}, iopt), torch::empty({K, S}, iopt), {}, {}, torch::empty({K, S}, fopt), capacity, act,
+               postscore, budget_ms, status_ptr};
+  Tensor logits = torch::empty({S, E}, fopt), counts = torch::empty({2, E}, iopt);
+  Tensor laux = torch::empty({}, fopt), laux_bf16;
+  if (bf16_logits) laux_bf16 = torch::empty({}, x.options());
+  Tensor ws = torch::empty({2 * K * S + (K + 1) * nblk * E}, iopt), order;
+  const int* perm = nullptr;
+  {
+    Stage st(stages, "fwd.gate_linear");
+    count_launch(1);
+    launch_gate_project(rows16(x), wg.data_ptr(), wg.scalar_type() == at::kBFloat16, logits.data_ptr<float>(), S, E, M,
+                        bf16_logits, cur_stream());
+  }
+  {
+    Stage st(stages, "fwd.gate_topk_scan");
+    if (prio) {
+      order = torch::empty({3, S}, iopt);         // keys, ranks, permutation
+      int* o = order.data_ptr<int>();
+      count_launch(2);
+      launch_importance_order<float>(logits.data_ptr<float>(), S, E, reinterpret_cast<float*>(o), o + S, o + 2 * S, cur_stream());
+      perm = o + 2 * S;
+    }
+    const bool dynamic = capacity < 0;
+    if (!dynamic) r.slot_map = torch::empty({E * capacity}, iopt);
+    GatePtrs gp{};
+    for (int k = 0; k < K; ++k) gp.p[k] = r.gates.data_ptr<float>() + (int64_t)k * S;
+    int* w = ws.data_ptr<int>();
+    count_launch(2);
+    launch_gate_forward<float, false>(logits.data_ptr<float>(), S, E, K, dynamic ? INT_MAX : (int)capacity, normalize,
+                                      bf16_logits ? 7.8125e-03f : kFloatEps, r.idx.data_ptr<int>(), r.loc.data_ptr<int>(), gp,
+                                      reinterpret_cast<float*>(w), dynamic ? nullptr : r.slot_map.data_ptr<int>(),
+                                      counts.data_ptr<int>(), counts.data_ptr<int>() + E, laux.data_ptr<float>(), w + K * S,
+                                      w + 2 * K * S, reinterpret_cast<float*>(w + 2 * K * S + K * nblk * E), cur_stream(), perm,
+                                      bf16_logits ? laux_bf16.data_ptr() : nullptr);
+    if (dynamic) {
+      const Tensor host = counts[1].cpu();
+      int peak = 0;
+      for (int64_t e = 0; e < E; ++e) peak = std::max(peak, host.data_ptr<int>()[e]);
+      r.C = round_up(peak).cast<int64_t>();
+      TORCH_CHECK(r.C >= peak);
+      r.slot_map = torch::empty({E * r.C}, iopt);
+      count_launch(1);
+      launch_build_slot_map(r.idx.data_ptr<int>(), r.loc.data_ptr<int>(), r.slot_map.data_ptr<int>(), K, S, E, r.C, cur_stream());
+    }
+  }
+  r.used = counts[1];
+  std::vector<Tensor> e = local_forward_op(x, r, w1, b1, w2, b2, want_grad, stages);
+  return {{e[0], bf16_logits ? laux_bf16 : laux, logits, counts[0], r.slot_map, r.used, r.idx, r.loc, r.gates, e[1], e[2], e[3],
+           e[4]}, r.C};
+}
+
+std::vector<Tensor> local_moe_backward_op(const Tensor& dy, const c10::optional<Tensor>& dl_aux, const Tensor& x, const Tensor& wg,
+                                          const LocalRoute& r, const Tensor& w1, const Tensor& w2, const Tensor& logits,
+                                          const Tensor& top1, const Tensor& xs, const Tensor& dact, const Tensor& h,
+                                          const Tensor& ys, bool normalize, bool bf16_logits, const std::vector<bool>& need,
+                                          const py::object& stages) {
+  const LocalGate g{wg, logits, top1, normalize, bf16_logits};
+  return local_backward(dy, x, r, w1, w2, xs, dact, h, ys, need, &g, dl_aux, stages);
 }
 
 // rows [R, M] -> uint8 [R, M + 16]: M quantised bytes + {scale, low, 0, 0} (the wire rows of the fused send)
@@ -923,6 +1066,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       }));
   m.def("local_forward", &local_forward_op);
   m.def("local_backward", &local_backward_op);
+  m.def("local_moe_forward", &local_moe_forward_op);
+  m.def("local_moe_backward", &local_moe_backward_op);
+  m.attr("gate_max_experts") = kProjMaxE;
   m.def("importance_order", &importance_order_op);
   m.def("remap_slot_map", &remap_slot_map_op);
   m.def("gate_backward", &gate_backward_op);

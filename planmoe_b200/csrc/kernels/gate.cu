@@ -54,16 +54,18 @@ gate_stats_kernel(const T* __restrict__ logits, int S, int E, int K, int nblk,
                   int* __restrict__ rank_in_blk,  // [K][S]
                   int* __restrict__ blk_count,    // [K][E][nblk]
                   float* __restrict__ blk_score,  // [E][nblk]  sum of softmax scores
-                  int* __restrict__ slot_map, long long slots)
+                  int* __restrict__ slot_map, long long slots,
+                  const int* __restrict__ perm)   // token at each position of the slot order, or null: token order
 {
   __shared__ int warp_cnt[kGateWarps][kMaxK][kMaxE];
   __shared__ float score_sum[kGateWarps][kMaxE];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int t = blockIdx.x * kGateThreads + tid;
-  const bool live = t < S;
+  const int pos = blockIdx.x * kGateThreads + tid;
+  const bool live = pos < S;
+  const int t = live && perm != nullptr ? perm[pos] : pos;
 
   for (int i = tid; i < kGateWarps * kMaxK * kMaxE; i += kGateThreads) (&warp_cnt[0][0][0])[i] = 0;
-  for (long long i = t; i < slots; i += (long long)gridDim.x * kGateThreads) slot_map[i] = -1;
+  for (long long i = pos; i < slots; i += (long long)gridDim.x * kGateThreads) slot_map[i] = -1;
   __syncthreads();
 
   float p[ME];
@@ -135,7 +137,9 @@ gate_assign_kernel(int S, int E, int K, int C, int normalize, float eps,
                    int* __restrict__ loc, GatePtrs gates, int* __restrict__ slot_map,
                    int* __restrict__ top1_count,  // [E] tokens whose first pick is e
                    int* __restrict__ used,        // [E] slots of expert e that hold a token, or null
-                   float* __restrict__ l_aux)     // [1]
+                   float* __restrict__ l_aux,     // [1]
+                   __nv_bfloat16* __restrict__ l_aux_bf16,   // [1] or null
+                   const int* __restrict__ perm)
 {
   __shared__ int base[kMaxK][kMaxE];
   __shared__ float red[kMaxE];
@@ -156,8 +160,9 @@ gate_assign_kernel(int S, int E, int K, int C, int normalize, float eps,
   }
   __syncthreads();
 
-  const int t = b * kGateThreads + tid;
-  if (t < S) {
+  const int pos = b * kGateThreads + tid;
+  if (pos < S) {
+    const int t = perm != nullptr ? perm[pos] : pos;
     float g[kMaxK];
     float denom = 0.f;
     for (int k = 0; k < K; ++k) { g[k] = raw_gate[(size_t)k * S + t]; denom += g[k]; }
@@ -168,7 +173,7 @@ gate_assign_kernel(int S, int E, int K, int C, int normalize, float eps,
       const int l = base[k][e] + rank_in_blk[(size_t)k * S + t];
       loc[(size_t)k * S + t] = l;
       gates.p[k][t] = norm ? g[k] / denom : g[k];
-      if (l < C) slot_map[(size_t)e * C + l] = t * K + k;
+      if (slot_map != nullptr && l < C) slot_map[(size_t)e * C + l] = t * K + k;
     }
   }
 
@@ -200,7 +205,9 @@ gate_assign_kernel(int S, int E, int K, int C, int normalize, float eps,
     if (tid == 0) {
       float acc = 0.f;
       for (int e = 0; e < E; ++e) acc += red[e];
-      l_aux[0] = acc * (float)E / ((float)S * (float)S);
+      acc = acc * (float)E / ((float)S * (float)S);
+      l_aux[0] = acc;
+      if (l_aux_bf16 != nullptr) l_aux_bf16[0] = __float2bfloat16_rn(acc);
     }
   }
 }
@@ -210,6 +217,7 @@ __global__ void __launch_bounds__(kGateThreads)
 gate_bwd_kernel(const T* __restrict__ logits, int S, int E, int K, int normalize, float eps,
                 const int* __restrict__ idx, GatePtrs dgates,                     // K rows of S, null = zeros
                 const float* __restrict__ dl_aux,                                 // [1] or null
+                const __nv_bfloat16* __restrict__ dl_aux_bf16,                    // [1] or null
                 const int* __restrict__ top1_count, T* __restrict__ dlogits) {
   const int t = blockIdx.x * kGateThreads + threadIdx.x;
   if (t >= S) return;
@@ -218,7 +226,8 @@ gate_bwd_kernel(const T* __restrict__ logits, int S, int E, int K, int normalize
   if constexpr (!SCORES) softmax_row<ME>(p, E);
 
   // d(score): loss part for every expert, gate part for the picked ones
-  const float lw = dl_aux ? dl_aux[0] * (float)E / ((float)S * (float)S) : 0.f;
+  const float dl = dl_aux ? dl_aux[0] : dl_aux_bf16 ? __bfloat162float(dl_aux_bf16[0]) : 0.f;
+  const float lw = dl * (float)E / ((float)S * (float)S);
   int pk[kMaxK];
   float ds_pick[kMaxK];
   float denom = 0.f, dot = 0.f;
@@ -266,25 +275,27 @@ template <class T, bool SCORES>
 void launch_gate_forward(const T* logits, int S, int E, int K, int C, bool normalize, float eps,
                          int* idx, int* loc, GatePtrs gates, float* raw_gate, int* slot_map,
                          int* top1_count, int* used, float* l_aux, int* ws_rank, int* ws_blk_count,
-                         float* ws_blk_score, cudaStream_t stream) {
+                         float* ws_blk_score, cudaStream_t stream, const int* perm, void* l_aux_bf16) {
   const int nblk = (S + kGateThreads - 1) / kGateThreads;
   auto stats = E <= 8 ? gate_stats_kernel<T, 8, SCORES> : E <= 16 ? gate_stats_kernel<T, 16, SCORES>
              : E <= 32 ? gate_stats_kernel<T, 32, SCORES> : gate_stats_kernel<T, 64, SCORES>;
   stats<<<nblk, kGateThreads, 0, stream>>>(logits, S, E, K, nblk, idx, raw_gate, ws_rank, ws_blk_count, ws_blk_score,
-                                           slot_map, (long long)E * C);
+                                           slot_map, slot_map != nullptr ? (long long)E * C : 0, perm);
   gate_assign_kernel<<<nblk, kGateThreads, 0, stream>>>(S, E, K, C, normalize ? 1 : 0, eps, idx,
                                                       raw_gate, ws_rank, ws_blk_count, ws_blk_score,
-                                                      nblk, loc, gates, slot_map, top1_count, used, l_aux);
+                                                      nblk, loc, gates, slot_map, top1_count, used, l_aux,
+                                                      reinterpret_cast<__nv_bfloat16*>(l_aux_bf16), perm);
 }
 
 template <class T, bool SCORES>
 void launch_gate_backward(const T* logits, int S, int E, int K, bool normalize, float eps,
                           const int* idx, GatePtrs dgates, const float* dl_aux,
-                          const int* top1_count, T* dlogits, cudaStream_t stream) {
+                          const int* top1_count, T* dlogits, cudaStream_t stream, const void* dl_aux_bf16) {
   const int nblk = (S + kGateThreads - 1) / kGateThreads;
   auto bwd = E <= 8 ? gate_bwd_kernel<T, 8, SCORES> : E <= 16 ? gate_bwd_kernel<T, 16, SCORES>
            : E <= 32 ? gate_bwd_kernel<T, 32, SCORES> : gate_bwd_kernel<T, 64, SCORES>;
-  bwd<<<nblk, kGateThreads, 0, stream>>>(logits, S, E, K, normalize ? 1 : 0, eps, idx, dgates, dl_aux, top1_count, dlogits);
+  bwd<<<nblk, kGateThreads, 0, stream>>>(logits, S, E, K, normalize ? 1 : 0, eps, idx, dgates, dl_aux,
+                                         reinterpret_cast<const __nv_bfloat16*>(dl_aux_bf16), top1_count, dlogits);
 }
 
 int gate_workspace_blocks(int S) { return (S + kGateThreads - 1) / kGateThreads; }
@@ -309,22 +320,38 @@ importance_key_kernel(const T* __restrict__ logits, int S, int E, float* __restr
 }
 
 // 32 tokens per CTA, eight threads per token: each thread counts over an eighth of every key tile, the eight
-// counts are added by shuffles.  S / 32 CTAs keep the whole machine busy for a few thousand tokens.
+// counts are added by shuffles.  S / 32 CTAs keep the whole machine busy for a few thousand tokens.  Ties need the index
+// only in the tile that holds the token: every key of an earlier tile goes before it from equality on, every key of a
+// later one only when it is larger, so that a comparison is one test and one add on four keys per load (16384 tokens:
+// 115 us with the full test on single keys).
+constexpr int kRankTile = 1024;
 __global__ void __launch_bounds__(256)
 importance_rank_kernel(const float* __restrict__ key, int S, int* __restrict__ rank, int* __restrict__ perm) {
-  __shared__ float tile[1024];
+  __shared__ __align__(16) float tile[kRankTile];
   const int part = threadIdx.x & 7;
-  const int t = blockIdx.x * 32 + (threadIdx.x >> 3);
+  const int t0 = blockIdx.x * 32, t = t0 + (threadIdx.x >> 3);   // a CTA's tokens lie in one tile
   const float mine = t < S ? key[t] : 0.f;
   int before = 0;
-  for (int base = 0; base < S; base += 1024) {
+  for (int base = 0; base < S; base += kRankTile) {
     __syncthreads();
-    for (int i = threadIdx.x; i < 1024; i += blockDim.x) tile[i] = base + i < S ? key[base + i] : -INFINITY;
+    for (int i = threadIdx.x; i < kRankTile; i += blockDim.x) tile[i] = base + i < S ? key[base + i] : -INFINITY;
     __syncthreads();
-    const int n = min(1024, S - base);
-    for (int i = part; i < n; i += 8) {
-      const float other = tile[i];
-      before += (other > mine || (other == mine && base + i < t)) ? 1 : 0;
+    const int own = t0 - base;
+    if (own >= 0 && own < kRankTile) {
+      const int n = min(kRankTile, S - base);
+      for (int i = part; i < n; i += 8) before += (tile[i] > mine || (tile[i] == mine && base + i < t)) ? 1 : 0;
+    } else if (own > 0) {
+#pragma unroll 4
+      for (int i = part * 4; i < kRankTile; i += 32) {           // an earlier tile is full
+        const float4 k = *reinterpret_cast<const float4*>(tile + i);
+        before += (k.x >= mine) + (k.y >= mine) + (k.z >= mine) + (k.w >= mine);
+      }
+    } else {
+#pragma unroll 4
+      for (int i = part * 4; i < kRankTile; i += 32) {           // keys are positive: the padding never counts
+        const float4 k = *reinterpret_cast<const float4*>(tile + i);
+        before += (k.x > mine) + (k.y > mine) + (k.z > mine) + (k.w > mine);
+      }
     }
   }
   before += __shfl_xor_sync(0xffffffffu, before, 1);
@@ -357,9 +384,9 @@ void launch_remap_slot_map(int* slot_map, long long n, const int* perm, int K, c
 #define INSTANTIATE(T, SCORES)                                                                    \
   template void launch_gate_forward<T, SCORES>(const T*, int, int, int, int, bool, float, int*, int*,     \
                                                GatePtrs, float*, int*, int*, int*, float*, int*, int*, float*, \
-                                               cudaStream_t);                                             \
+                                               cudaStream_t, const int*, void*);                          \
   template void launch_gate_backward<T, SCORES>(const T*, int, int, int, bool, float, const int*, GatePtrs, \
-                                                const float*, const int*, T*, cudaStream_t);
+                                                const float*, const int*, T*, cudaStream_t, const void*);
 INSTANTIATE(float, false)
 INSTANTIATE(__nv_bfloat16, false)
 INSTANTIATE(__half, false)

@@ -1,0 +1,349 @@
+// The linear gate's projection and its gradients (sm_100a), on bf16 tokens as they are.
+//
+//   gate_project   logits[t][e] = <x[t], w[e]>
+//   gate_wgrad     dw[e][m] = sum_t dlogits[t][e] * x[t][m], as partial sums over chunks of tokens
+//   gather_gate    dx[t] = sum_k (gate *) slot row of pick k + sum_e dlogits[t][e] * w[e]: the two parts of a token's
+//                  gradient in one pass, rounded once
+//
+// The composition that they take the place of (x.float(), an fp32 library GEMM, its two gradient GEMMs, a cast and an
+// add) read and wrote the [tokens, model_dim] matrix nine times, six of them in fp32: 728 us of a training step of 16384
+// tokens of 4096 with 8 experts.  Every one of these kernels reads it once.
+//
+// All products and sums are at fp32 precision: tokens are exact in bf16, and fp32 weights enter the tensor cores as the sum
+// of three bf16 terms of eight bits each, which is exact.
+
+#include "planmoe.h"
+#include "kernels/common.cuh"
+
+#include <type_traits>
+
+namespace planmoe {
+
+namespace {
+
+constexpr int kProjWarps = 8;
+
+__device__ __forceinline__ void mma_16816(float* c, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// upper halves of two fp32 words = their leading eight significant bits as bf16 (towards zero)
+__device__ __forceinline__ uint32_t upper_halves(float a, float b) {
+  return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
+}
+__device__ __forceinline__ float below_upper(float a) { return a - __uint_as_float(__float_as_uint(a) & 0xffff0000u); }
+
+// One block per 16 * MT tokens; its warps share the contraction, 32 columns at a time (chunk w, w + 8, ...), and their
+// sums are added in warp order.  A lane's 16-byte pieces of two token rows and of one weight row are the fragments of two
+// m16n8k16 steps: which column a fragment register stands for is free as long as both operands agree.  Bound by the token
+// rows (DRAM) and, with many experts, by the weights that every block reads again from L2; 32 tokens a block halve the
+// latter once there are blocks enough without (kProjWide).
+constexpr int kProjWide = 4096;                   // tokens from which on a block takes 32
+
+template <int NT, int MT, bool W_BF16>
+__global__ void __launch_bounds__(kProjWarps * 32)
+gate_project_kernel(const __nv_bfloat16* __restrict__ x, const void* __restrict__ w_, float* __restrict__ logits, int S, int E,
+                    int M, int round_bf16) {
+  __shared__ float part[kProjWarps][16 * MT][NT * 8 + 1];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3;
+  const int t0 = blockIdx.x * 16 * MT;
+  const uint4* xr[MT][2];
+#pragma unroll
+  for (int m = 0; m < MT; ++m)
+#pragma unroll
+    for (int h = 0; h < 2; ++h)                   // rows past the end repeat the last one (not stored)
+      xr[m][h] = reinterpret_cast<const uint4*>(x + (long long)min(t0 + m * 16 + h * 8 + g, S - 1) * M) + c;
+  float acc[MT][NT][4];
+#pragma unroll
+  for (int m = 0; m < MT; ++m)
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) acc[m][n][i] = 0.f;
+  const int chunks = M / 32;
+#pragma unroll 2
+  for (int ch = warp; ch < chunks; ch += kProjWarps) {
+    uint4 a[MT][2];
+#pragma unroll
+    for (int m = 0; m < MT; ++m) {
+      a[m][0] = __ldg(xr[m][0] + ch * 4);
+      a[m][1] = __ldg(xr[m][1] + ch * 4);
+    }
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+      const long long at = (long long)min(n * 8 + g, E - 1) * M + ch * 32 + c * 8;
+      uint4 b[W_BF16 ? 1 : 3];
+      if constexpr (W_BF16) {
+        b[0] = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(w_) + at));
+      } else {
+        const float4 lo = __ldg(reinterpret_cast<const float4*>(reinterpret_cast<const float*>(w_) + at));
+        const float4 hi = __ldg(reinterpret_cast<const float4*>(reinterpret_cast<const float*>(w_) + at) + 1);
+        float f[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+#pragma unroll
+        for (int s = 0; s < 3; ++s) {
+          b[s] = make_uint4(upper_halves(f[0], f[1]), upper_halves(f[2], f[3]), upper_halves(f[4], f[5]), upper_halves(f[6], f[7]));
+          if (s < 2) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) f[i] = below_upper(f[i]);
+          }
+        }
+      }
+#pragma unroll
+      for (int s = (W_BF16 ? 1 : 3) - 1; s >= 0; --s) {          // the small terms first
+#pragma unroll
+        for (int m = 0; m < MT; ++m) {
+          mma_16816(acc[m][n], a[m][0].x, a[m][1].x, a[m][0].y, a[m][1].y, b[s].x, b[s].y);
+          mma_16816(acc[m][n], a[m][0].z, a[m][1].z, a[m][0].w, a[m][1].w, b[s].z, b[s].w);
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int m = 0; m < MT; ++m)
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+      part[warp][m * 16 + g][n * 8 + 2 * c] = acc[m][n][0];
+      part[warp][m * 16 + g][n * 8 + 2 * c + 1] = acc[m][n][1];
+      part[warp][m * 16 + g + 8][n * 8 + 2 * c] = acc[m][n][2];
+      part[warp][m * 16 + g + 8][n * 8 + 2 * c + 1] = acc[m][n][3];
+    }
+  __syncthreads();
+  for (int i = threadIdx.x; i < 16 * MT * E; i += kProjWarps * 32) {
+    const int r = i / E, e = i - r * E;
+    if (t0 + r >= S) break;
+    float s = 0.f;
+#pragma unroll
+    for (int w = 0; w < kProjWarps; ++w) s += part[w][r][e];
+    logits[(long long)(t0 + r) * E + e] = round_bf16 ? __bfloat162float(__float2bfloat16_rn(s)) : s;
+  }
+}
+
+// ---- packed fp32 pairs: two fused multiply-adds per instruction on sm_100 ----
+__device__ __forceinline__ unsigned long long pair_of(float a, float b) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 unpair(unsigned long long v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ unsigned long long fma_pair(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ void bf16_pairs(const uint4& raw, unsigned long long* p) {
+  const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) p[i] = pair_of(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xffff0000u));
+}
+
+// Block (column slab of 256, chunk of tokens): a lane holds 8 columns of EB experts, the 8 warps take the chunk's tokens in
+// turn; their sums are added in warp order through shared memory, one expert after the other.  The gradients of the logits
+// wait in shared memory as pairs {d, d}.
+constexpr int kWgradTokens = 64;                  // tokens whose logit gradients are staged at a time
+
+template <int EB>
+__global__ void __launch_bounds__(256)
+gate_wgrad_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ dl, float* __restrict__ partial, int S, int E,
+                  int M, int chunk_tokens) {
+  __shared__ float2 d_s[kWgradTokens][EB];
+  __shared__ float red[8][256];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int col = blockIdx.x * 256 + lane * 8;
+  const bool in = col < M;                        // M is a multiple of 8
+  const int c0 = blockIdx.y * chunk_tokens, c1 = min(S, c0 + chunk_tokens);
+  unsigned long long acc[EB][4];
+#pragma unroll
+  for (int e = 0; e < EB; ++e)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) acc[e][i] = 0ull;
+  for (int b0 = c0; b0 < c1; b0 += kWgradTokens) {
+    const int n = min(kWgradTokens, c1 - b0);
+    __syncthreads();
+    for (int i = threadIdx.x; i < n * EB; i += 256) {
+      const int t = i / EB, e = i - t * EB;
+      const float v = e < E ? dl[(long long)(b0 + t) * E + e] : 0.f;
+      d_s[t][e] = make_float2(v, v);
+    }
+    __syncthreads();
+#pragma unroll 4
+    for (int t = warp; t < n; t += 8) {
+      uint4 raw = make_uint4(0, 0, 0, 0);
+      if (in) raw = __ldg(reinterpret_cast<const uint4*>(x + (long long)(b0 + t) * M + col));
+      unsigned long long p[4];
+      bf16_pairs(raw, p);
+#pragma unroll
+      for (int e = 0; e < EB; ++e) {
+        const unsigned long long d = *reinterpret_cast<const unsigned long long*>(&d_s[t][e]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[e][i] = fma_pair(p[i], d, acc[e][i]);
+      }
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < EB; ++e) {
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 f = unpair(acc[e][i]);
+      red[warp][lane * 8 + 2 * i] = f.x;
+      red[warp][lane * 8 + 2 * i + 1] = f.y;
+    }
+    __syncthreads();
+    const int m = blockIdx.x * 256 + threadIdx.x;
+    if (e < E && m < M) {
+      float s = 0.f;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) s += red[w][threadIdx.x];
+      partial[((long long)blockIdx.y * E + e) * M + m] = s;
+    }
+  }
+}
+
+// One warp per (8 tokens, 256 columns): the weights of a column are read once for the eight tokens.
+constexpr int kGatherTokens = 8;
+
+template <int MAXK, bool W_BF16, bool GATED>
+__global__ void __launch_bounds__(256, MAXK <= 2 ? 2 : 1)
+gather_gate_kernel(const __nv_bfloat16* __restrict__ slots, const int* __restrict__ idx, const int* __restrict__ loc,
+                   const float* __restrict__ gates, const float* __restrict__ dl, const void* __restrict__ w_,
+                   __nv_bfloat16* __restrict__ dx, int K, int S, int M, int E, int C) {
+  extern __shared__ float2 dl_s[];                // [warp][8 tokens][E]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int slabs = (M + 255) / 256;
+  const long long item = (long long)blockIdx.x * 8 + warp;
+  const int t0 = (int)(item / slabs) * kGatherTokens, col = (int)(item % slabs) * 256 + lane * 8;
+  if (t0 >= S) return;
+  float2* mine = dl_s + warp * kGatherTokens * E;
+  for (int i = lane; i < kGatherTokens * E; i += 32) {
+    const int t = min(t0 + i / E, S - 1);
+    const float v = dl[(long long)t * E + i % E];
+    mine[i] = make_float2(v, v);
+  }
+  __syncwarp();
+  if (col >= M) return;
+  uint4 raw[kGatherTokens][MAXK];
+  float gw[kGatherTokens][GATED ? MAXK : 1];
+#pragma unroll
+  for (int t = 0; t < kGatherTokens; ++t) {
+#pragma unroll
+    for (int k = 0; k < MAXK; ++k) {
+      raw[t][k] = make_uint4(0, 0, 0, 0);
+      if constexpr (GATED) gw[t][k] = 0.f;
+      const int tok = t0 + t;
+      if (k < K && tok < S) {
+        const int e = idx[(size_t)k * S + tok], l = loc[(size_t)k * S + tok];
+        if (l >= 0 && l < C && e >= 0) {
+          raw[t][k] = __ldg(reinterpret_cast<const uint4*>(slots + ((long long)e * C + l) * M + col));
+          if constexpr (GATED) gw[t][k] = gates[(size_t)k * S + tok];
+        }
+      }
+    }
+  }
+  unsigned long long acc[kGatherTokens][4];
+#pragma unroll
+  for (int t = 0; t < kGatherTokens; ++t) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) acc[t][i] = 0ull;
+#pragma unroll
+    for (int k = 0; k < MAXK; ++k) {
+      unsigned long long p[4];
+      bf16_pairs(raw[t][k], p);
+      const float gk = GATED ? gw[t][GATED ? k : 0] : 1.f;
+      const unsigned long long gp = pair_of(gk, gk);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) acc[t][i] = fma_pair(p[i], gp, acc[t][i]);
+    }
+  }
+  for (int e = 0; e < E; ++e) {
+    unsigned long long w[4];
+    if constexpr (W_BF16) {
+      bf16_pairs(__ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(w_) + (long long)e * M + col)), w);
+    } else {
+      const float4* wp = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(w_) + (long long)e * M + col);
+      const float4 lo = __ldg(wp), hi = __ldg(wp + 1);
+      w[0] = pair_of(lo.x, lo.y); w[1] = pair_of(lo.z, lo.w); w[2] = pair_of(hi.x, hi.y); w[3] = pair_of(hi.z, hi.w);
+    }
+#pragma unroll
+    for (int t = 0; t < kGatherTokens; ++t) {
+      const unsigned long long d = *reinterpret_cast<const unsigned long long*>(&mine[t * E + e]);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) acc[t][i] = fma_pair(w[i], d, acc[t][i]);
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < kGatherTokens; ++t) {
+    if (t0 + t >= S) break;
+    uint32_t o[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 f = unpair(acc[t][i]);
+      const __nv_bfloat162 h = __floats2bfloat162_rn(f.x, f.y);
+      o[i] = *reinterpret_cast<const uint32_t*>(&h);
+    }
+    *reinterpret_cast<uint4*>(dx + (long long)(t0 + t) * M + col) = make_uint4(o[0], o[1], o[2], o[3]);
+  }
+}
+
+template <int NT, bool W_BF16>
+void project_nt(const void* x, const void* w, float* logits, int S, int E, int M, bool round_bf16, cudaStream_t stream) {
+  const __nv_bfloat16* xb = reinterpret_cast<const __nv_bfloat16*>(x);
+  if (S >= kProjWide)
+    gate_project_kernel<NT, 2, W_BF16><<<(S + 31) / 32, kProjWarps * 32, 0, stream>>>(xb, w, logits, S, E, M, round_bf16);
+  else
+    gate_project_kernel<NT, 1, W_BF16><<<(S + 15) / 16, kProjWarps * 32, 0, stream>>>(xb, w, logits, S, E, M, round_bf16);
+}
+
+}  // namespace
+
+void launch_gate_project(const void* x, const void* w, bool w_bf16, float* logits, int S, int E, int M, bool round_bf16,
+                         cudaStream_t stream) {
+  if (E <= 8) {
+    if (w_bf16) project_nt<1, true>(x, w, logits, S, E, M, round_bf16, stream);
+    else project_nt<1, false>(x, w, logits, S, E, M, round_bf16, stream);
+  } else {
+    if (w_bf16) project_nt<2, true>(x, w, logits, S, E, M, round_bf16, stream);
+    else project_nt<2, false>(x, w, logits, S, E, M, round_bf16, stream);
+  }
+}
+
+// Chunks of tokens: about four blocks per SM over all column slabs, at least 32 tokens each.
+int gate_wgrad_chunks(int S, int M) {
+  const int slabs = (M + 255) / 256;
+  int n = 4 * 148 / slabs;
+  if (n > S / 32) n = S / 32;
+  return n < 1 ? 1 : n;
+}
+
+void launch_gate_wgrad(const void* x, const float* dl, float* partial, int S, int E, int M, cudaStream_t stream) {
+  const int n = gate_wgrad_chunks(S, M), tokens = (S + n - 1) / n;
+  const dim3 grid((M + 255) / 256, n);
+  const __nv_bfloat16* xb = reinterpret_cast<const __nv_bfloat16*>(x);
+  if (E <= 2) gate_wgrad_kernel<2><<<grid, 256, 0, stream>>>(xb, dl, partial, S, E, M, tokens);
+  else if (E <= 4) gate_wgrad_kernel<4><<<grid, 256, 0, stream>>>(xb, dl, partial, S, E, M, tokens);
+  else if (E <= 8) gate_wgrad_kernel<8><<<grid, 256, 0, stream>>>(xb, dl, partial, S, E, M, tokens);
+  else gate_wgrad_kernel<16><<<grid, 256, 0, stream>>>(xb, dl, partial, S, E, M, tokens);
+}
+
+void launch_gather_gate(const void* slots, const int* idx, const int* loc, const float* gates, const float* dl, const void* w,
+                        bool w_bf16, void* dx, int K, int S, int M, int E, int C, cudaStream_t stream) {
+  const long long items = (long long)((S + kGatherTokens - 1) / kGatherTokens) * ((M + 255) / 256);
+  const unsigned grid = (unsigned)((items + 7) / 8);
+  const int smem = 8 * kGatherTokens * E * (int)sizeof(float2);
+  const __nv_bfloat16* sb = reinterpret_cast<const __nv_bfloat16*>(slots);
+  __nv_bfloat16* db = reinterpret_cast<__nv_bfloat16*>(dx);
+  auto pick = [&](auto gated) {
+    constexpr bool G = decltype(gated)::value;
+    return K <= 1 ? (w_bf16 ? gather_gate_kernel<1, true, G> : gather_gate_kernel<1, false, G>)
+         : K <= 2 ? (w_bf16 ? gather_gate_kernel<2, true, G> : gather_gate_kernel<2, false, G>)
+                  : (w_bf16 ? gather_gate_kernel<4, true, G> : gather_gate_kernel<4, false, G>);
+  };
+  auto kern = gates != nullptr ? pick(std::true_type{}) : pick(std::false_type{});
+  kern<<<grid, 256, smem, stream>>>(sb, idx, loc, gates, dl, w, db, K, S, M, E, C);
+}
+
+}  // namespace planmoe

@@ -74,22 +74,37 @@ void launch_slots_gate_grad(const void* disp, const void* dy, const int* idx, co
                             const int* used, float* dgates, void* ddisp, int K, int S, int M, int E, int C,
                             cudaStream_t stream);
 
+// ---- kernels/gate_proj.cu: the linear gate on bf16 tokens [S, M], M % 32 == 0, at most kProjMaxE experts ----
+// `w`: [E, M], fp32 or bf16.  logits fp32, rounded to bf16 values if asked for.
+constexpr int kProjMaxE = 16;
+void launch_gate_project(const void* x, const void* w, bool w_bf16, float* logits, int S, int E, int M, bool round_bf16,
+                         cudaStream_t stream);
+// partial: gate_wgrad_chunks(S, M) rows of [E, M] fp32, to be added up (launch_colsum_jobs)
+int gate_wgrad_chunks(int S, int M);
+void launch_gate_wgrad(const void* x, const float* dl, float* partial, int S, int E, int M, cudaStream_t stream);
+// dx[t] = sum_k (gates[k][t] *) slots[slot_k(t)] + sum_e dl[t][e] * w[e]
+void launch_gather_gate(const void* slots, const int* idx, const int* loc, const float* gates, const float* dl, const void* w,
+                        bool w_bf16, void* dx, int K, int S, int M, int E, int C, cudaStream_t stream);
+
 // ---- kernels/gate.cu -------------------------------------------------------------------------
 int gate_workspace_blocks(int S);
 // One fp32 row of S values per pick (gates, or their gradients; null = zeros).
 struct GatePtrs { float* p[4]; };
 // SCORES: the input is a [S, E] matrix of scores to pick from as they are; otherwise logits, softmax first.
 // slot_map: [E * C], written completely.  used (optional): [E] slots of every expert that hold a token; an expert's
-// slots are handed out from 0 on, so these are its first ones.
+// slots are handed out from 0 on, so these are its first ones.  perm (optional): the order in which tokens claim slots.
+// slot_map may be null (no map).  l_aux_bf16 / dl_aux_bf16 (optional): the loss and its gradient in bf16.
 template <class T, bool SCORES>
 void launch_gate_forward(const T* logits, int S, int E, int K, int C, bool normalize, float eps,
                          int* idx, int* loc, GatePtrs gates, float* raw_gate, int* slot_map,
                          int* top1_count, int* used, float* l_aux, int* ws_rank, int* ws_blk_count,
-                         float* ws_blk_score, cudaStream_t stream);
+                         float* ws_blk_score, cudaStream_t stream, const int* perm = nullptr,
+                         void* l_aux_bf16 = nullptr);
 template <class T, bool SCORES>
 void launch_gate_backward(const T* logits, int S, int E, int K, bool normalize, float eps,
                           const int* idx, GatePtrs dgates, const float* dl_aux,
-                          const int* top1_count, T* dlogits, cudaStream_t stream);
+                          const int* top1_count, T* dlogits, cudaStream_t stream,
+                          const void* dl_aux_bf16 = nullptr);
 // order of tokens for batch-prioritised routing: rank[t] = position of token t (best top score first, ties by index),
 // perm[position] = token; `key` is an fp32 [S] workspace
 template <class T>
@@ -239,8 +254,9 @@ int colsum_slabs(long long rows);
 void launch_colsum_bf16(const void* x, float* out, int groups, long long rows, int N,
                         long long row_stride, long long group_stride, int fold, void* out_bf16,
                         cudaStream_t stream);
-// One or two column-sum jobs in the same two launches (see launch_colsum_bf16 for the meaning of the fields).
+// Up to three column-sum jobs in the same two launches (see launch_colsum_bf16 for the meaning of the fields).
 // `partial`: groups * colsum_slabs(rows) * N floats; `counters` is reserved (the two-stage form does not use it).
+// A job without x brings its partial sums along (rows = 128 * their number) and takes part in the second launch only.
 struct ColsumJob {
   const void* x; float* out; void* out_bf16; float* partial; unsigned* counters;
   long long rows, row_stride, group_stride;

@@ -277,6 +277,7 @@ class _FusedGate(torch.autograd.Function):
     @staticmethod
     def forward(ctx, logits, top_k, capacity, normalize):
         lib = native.lib()
+        ctx.set_materialize_grads(False)
         logits = logits.contiguous()
         idx, loc, gates, slot_map, top1, l_aux, used = lib.gate_forward_used(logits, top_k, capacity, normalize)
         ctx.save_for_backward(logits, idx, top1)
@@ -485,7 +486,7 @@ class _LocalExperts(torch.autograd.Function):
         x, gates, w1, w2, xs, dact, h, ys, idx, loc, slot_map, used = ctx.saved_tensors
         route = _local_route(gates, dict(ctx.meta, idx=idx, loc=loc, slot_map=slot_map, used=used))
         dx, dgates, dw1, db1, dw2, db2 = native.lib().local_backward(
-            _aligned(dy), x, route, w1, w2, xs, dact, h, ys, list(ctx.needs_input_grad[2:6]), _stages())
+            _aligned(dy), x, route, w1, w2, xs, dact, h, ys, list(ctx.needs_input_grad[:6]), _stages())
         return dx, dgates, dw1, db1, dw2, db2, None
 
 
@@ -506,6 +507,81 @@ def _local_experts(x, gates, w1, b1, w2, b2, meta):
     return _local_forward(x, gates, w1, b1, w2, b2, meta, False)[0]
 
 
+class _LocalLayer(torch.autograd.Function):
+    """The same with the linear gate in it: tokens and the gate's weight in, output and balance loss out."""
+
+    @staticmethod
+    def forward(ctx, x, wg, w1, b1, w2, b2, m):
+        ctx.set_materialize_grads(False)
+        (y, l_aux, *saved), m['capacity'] = _local_layer_forward(x, wg, w1, b1, w2, b2, m, True)
+        m['routing'] = saved[4], saved[5]
+        ctx.save_for_backward(x, wg, w1, w2, *saved)
+        ctx.m = {k: m[k] for k in ('capacity', 'act', 'postscore', 'normalize', 'bf16_logits', 'budget_ms', 'status')}
+        return y, l_aux
+
+    @staticmethod
+    def backward(ctx, dy, dl_aux):
+        x, wg, w1, w2, logits, top1, slot_map, used, idx, loc, gates, xs, dact, h, ys = ctx.saved_tensors
+        m = ctx.m
+        if dy is None:
+            dy = torch.zeros((x.size(0), w2.size(2)), dtype=x.dtype, device=x.device)
+        route = _local_route(gates, dict(m, C=m['capacity'], idx=idx, loc=loc, slot_map=slot_map, used=used))
+        return (*native.lib().local_moe_backward(_aligned(dy), dl_aux, x, wg, route, w1, w2, logits, top1, xs, dact, h, ys,
+                                                 m['normalize'], m['bf16_logits'], list(ctx.needs_input_grad[:6]), _stages()),
+                None)
+
+
+def _local_layer_forward(x, wg, w1, b1, w2, b2, m, want_grad):
+    return native.lib().local_moe_forward(x, wg, w1, b1, w2, b2, m['K'], m['capacity'], m['round_up'], m['normalize'],
+                                          m['bf16_logits'], m['prio'], m['act'], m['postscore'], m['budget_ms'],
+                                          m['status'].device_ptr(), want_grad, _stages())
+
+
+def _unhooked(module, cls):
+    """A plain ``cls`` whose call is its forward and nothing else."""
+    return (type(module) is cls and 'forward' not in module.__dict__ and not module._forward_hooks
+            and not module._forward_pre_hooks and not module._backward_hooks and not module._backward_pre_hooks)
+
+
+def _linear_gate(layer, gctx, x):
+    """Whether the gate is a plain linear one that the gate kernels take in one pass with the experts: its weight is used as
+    it is, by nobody else's hook, without noise, with the GShard loss."""
+    from torch.nn.modules import module as nnm
+    from ..gates.top import LinearTopKGate
+    if not _unhooked(gctx, LinearTopKGate) or not _unhooked(gctx.wg, torch.nn.Linear) or not layer.is_gshard_loss:
+        return False
+    if nnm._global_forward_hooks or nnm._global_forward_pre_hooks or nnm._global_backward_hooks or nnm._global_backward_pre_hooks:
+        return False
+    w = gctx.wg.weight
+    return (type(w) is torch.nn.Parameter and not (layer.training and gctx.gate_noise > 0) and gctx.wg.bias is None
+            and 1 <= w.size(0) <= native.lib().gate_max_experts and w.device == x.device
+            and w.dtype in ((torch.float32, torch.bfloat16) if gctx.fp32_gate else (torch.bfloat16,))
+            and w.is_contiguous() and w.data_ptr() % 16 == 0 and x.size(0) > 0 and x.size(1) % 32 == 0)
+
+
+def _local_layer(layer, st, x, gctx, top_k, capacity, align):
+    ex, w = layer.experts, gctx.wg.weight
+    m = dict(K=top_k, capacity=capacity, round_up=lambda peak: _capacity_step(peak, align), normalize=layer.normalize_gate,
+             bf16_logits=not gctx.fp32_gate, prio=layer.batch_prioritized_routing, act=ACT_CODES[ex.act_name],
+             postscore=layer.is_postscore, budget_ms=st.tr.budget_ms, status=st.tr.status)
+    args = (_aligned(x), w, ex.batched_fc1_w, ex.batched_fc1_bias, ex.batched_fc2_w, ex.batched_fc2_bias)
+    if torch.is_grad_enabled() and any(t.requires_grad for t in args):
+        y, l_aux = _LocalLayer.apply(*args, m)
+    else:
+        (y, l_aux, *saved), m['capacity'] = _local_layer_forward(*args, m, False)
+        m['routing'] = saved[4], saved[5]
+    return y, l_aux, m['capacity'], m['routing']
+
+
+def _capacity_step(cap, align):
+    """``cap`` rounded up to the next of a coarse ladder (steps of about 12 %)."""
+    step = max(align, 64)
+    ladder = step
+    while ladder < cap:
+        ladder = max(ladder + step, (int(ladder * 1.125) + step - 1) // step * step)
+    return ladder
+
+
 def _dynamic_capacity(lib, logits, top_k, normalize, group, align):
     """Capacity for ``capacity_factor == 0``: the largest slot any expert hands out, over all ranks, plus one
     (reference: PlanMoE/impls/fast_dispatch.py:183-184, including its one host read of the all-reduced value).
@@ -518,11 +594,7 @@ def _dynamic_capacity(lib, logits, top_k, normalize, group, align):
         if dist.is_available() and dist.is_initialized() and dist.get_world_size(group) > 1:
             dist.all_reduce(peak, op=dist.ReduceOp.MAX, group=group)
         cap = int(peak.item()) + 1
-    step = max(align, 64)
-    ladder = step
-    while ladder < cap:
-        ladder = max(ladder + step, (int(ladder * 1.125) + step - 1) // step * step)
-    return ladder
+    return _capacity_step(cap, align)
 
 
 def check_routing_bounds(idx, loc, slot_map, S, E, capacity, top_k):
@@ -563,23 +635,31 @@ def forward(layer, x, gctx, top_k, capacity_factor, degree):
     top_k = min(int(top_k), E)
     assert degree <= MAX_CHUNKS and top_k <= MAX_TOP_K, "plan outside the fused kernels' limits"
 
+    align = 4 * layer.sharded_count * degree
+    per_expert = (S + E - 1) // E
+    capacity = -1                                 # sized to the busiest expert
+    if capacity_factor > 0:
+        capacity = top_k * int(capacity_factor * per_expert)
+    elif capacity_factor < 0:
+        capacity = top_k * int(-capacity_factor * per_expert)
+    if capacity_factor != 0:
+        capacity = max(capacity, 1)
+        capacity += -capacity % align
+    q8 = layer.compress_name == 'int8'
+    if _local_path(st.tr, q8) and _linear_gate(layer, gctx, x):
+        y, l_aux, capacity, (idx, loc) = _local_layer(layer, st, x, gctx, top_k, capacity, align)
+        _note_stats(layer, st, q8, idx, loc, E, capacity, degree, x)
+        return y, l_aux
+
     with torch.autocast('cuda', enabled=False), stage('fwd.gate_linear'):
         clean = gctx(x)
         logits = clean
         if layer.training and gctx.gate_noise > 0:
             logits = clean + gctx.gate_noise * torch.randn_like(clean) / E
         logits = logits.contiguous()
-    align = 4 * layer.sharded_count * degree
-    per_expert = (S + E - 1) // E
-    if capacity_factor > 0:
-        capacity = top_k * int(capacity_factor * per_expert)
-    elif capacity_factor < 0:
-        capacity = top_k * int(-capacity_factor * per_expert)
-    else:
+    if capacity_factor == 0:
         capacity = _dynamic_capacity(lib, logits, top_k, layer.normalize_gate, layer.group, align)
-    capacity = max(capacity, 1)
-    if capacity % align:
-        capacity += align - capacity % align
+        capacity += -capacity % align
 
     with stage('fwd.gate_topk_scan'):
         if layer.batch_prioritized_routing:
@@ -599,7 +679,6 @@ def forward(layer, x, gctx, top_k, capacity_factor, degree):
     if T.debug_guards():
         check_routing_bounds(idx, loc, slot_map, S, E, capacity, top_k)
     ex = layer.experts
-    q8 = layer.compress_name == 'int8'
     args = (gates, ex.batched_fc1_w, ex.batched_fc1_bias, ex.batched_fc2_w, ex.batched_fc2_bias)
     if _local_path(st.tr, q8):
         y = _local_experts(x, *args, dict(idx=idx, loc=loc, slot_map=slot_map, used=used, C=capacity,
@@ -609,12 +688,16 @@ def forward(layer, x, gctx, top_k, capacity_factor, degree):
         meta = dict(state=st, idx=idx, loc=loc, slot_map=slot_map, E=E, C=capacity, degree=degree, K=top_k,
                     act=ACT_CODES[ex.act_name], postscore=layer.is_postscore, q8=q8)
         y = _FusedExperts.apply(x.contiguous(), *args, meta)
+    _note_stats(layer, st, q8, idx, loc, E, capacity, degree, x)
+    return y, l_aux.to(logits.dtype)
+
+
+def _note_stats(layer, st, q8, idx, loc, E, capacity, degree, x):
     # both 'naive' and 'pipe' run as the flat push of the copy role / push epilogue: say so instead of echoing the name
     layer.last_stats = dict(capacity=capacity, degree=degree, path='fused', comm='flat-push',
                             wire=('int8' if q8 else 'bf16'))
     if getattr(layer, 'collect_stats', False):
         from ..utils import metrics
         layer.last_stats.update(metrics.routing_stats(idx, loc, E, capacity))
-        layer.last_stats.update(metrics.wire_stats(E, capacity, M, x.element_size(), st.tr.world, layer.compress_name,
+        layer.last_stats.update(metrics.wire_stats(E, capacity, x.size(1), x.element_size(), st.tr.world, layer.compress_name,
                                                    layer.comm_name, degree))
-    return y, l_aux.to(logits.dtype)

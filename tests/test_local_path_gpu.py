@@ -9,13 +9,17 @@ pytestmark = pytest.mark.gpu
 TOL = 2.0 ** -7          # one bf16 rounding of an intermediate, on either side
 
 
-def _layer(E, M, H, k, cf, act='gelu', **kw):
+def _layer(E, M, H, k, cf, act='gelu', fp32_gate=True, **kw):
     from planmoe_b200 import moe
-    layer = moe.moe_layer(gate_type={'type': 'top', 'k': k, 'capacity_factor': cf, 'fp32_gate': True}, model_dim=M,
+    layer = moe.moe_layer(gate_type={'type': 'top', 'k': k, 'capacity_factor': cf, 'fp32_gate': fp32_gate}, model_dim=M,
                           experts={'type': 'ffn', 'count_per_node': E, 'hidden_size_per_expert': H, 'activation_fn': act},
                           seeds=(1, 2, 3), **kw)
-    layer = layer.cuda().to(torch.bfloat16)
-    layer.gates.float()
+    layer = layer.cuda()
+    gate = layer.gates[0].wg.weight.detach().clone()
+    layer = layer.to(torch.bfloat16)
+    if fp32_gate:
+        layer.gates.float()
+        layer.gates[0].wg.weight.data.copy_(gate)         # all 24 bits of it
     return layer
 
 
@@ -43,7 +47,7 @@ def _close(a, b):
 
 
 @pytest.mark.parametrize('S,E,k,cf', [(1, 1, 1, 1.0), (16, 8, 2, 2.0), (130, 3, 3, 1.0), (700, 5, 1, 0.0), (1000, 2, 2, 1.0),
-                                      (2048, 4, 4, 0.3), (3001, 6, 2, 1.25), (600, 64, 2, 1.0)])
+                                      (2048, 4, 4, 0.3), (3001, 6, 2, 1.25), (600, 64, 2, 1.0), (4100, 16, 2, 1.0), (5000, 9, 2, 0.0)])
 @pytest.mark.parametrize('postscore', [True, False])
 def test_matches_the_exchange(S, E, k, cf, postscore, monkeypatch):
     layer = _layer(E, 192, 320, k, cf, is_postscore=postscore)
@@ -91,3 +95,48 @@ def test_unused_rows_are_never_read():
     again = _pass(layer, x, dy)
     for u, v in zip(first, again):
         assert torch.equal(u, v) and torch.isfinite(u).all()
+
+
+@pytest.mark.parametrize('fp32_gate,S', [(False, 33), (False, 4097), (True, 515)])
+def test_gate_forms(fp32_gate, S, monkeypatch):
+    """A bf16 gate (logits and balance loss in bf16), a bf16 weight under an fp32 gate, and a gate that somebody listens to."""
+    layer = _layer(2, 320, 128, 2, 1.0, fp32_gate=fp32_gate)
+    layer.gates[0].to(torch.bfloat16)
+    torch.manual_seed(2)
+    x = torch.randn(S, 320, device='cuda').bfloat16()
+    dy = torch.randn(S, 320, device='cuda').bfloat16()
+    here = _pass(layer, x, dy)
+    with torch.no_grad():
+        layer(x)
+    assert layer.l_aux.dtype == (torch.float32 if fp32_gate else torch.bfloat16)
+    seen = []
+    handle = layer.gates[0].wg.register_forward_hook(lambda mod, args, out: seen.append(out.shape))
+    if not fp32_gate:                                     # an fp32 gate uses the weight without calling the linear module
+        hooked = _pass(layer, x, dy)
+        assert seen == [(S, 2)]
+        _close(here, hooked)
+    handle.remove()
+    monkeypatch.setenv('PLANMOE_LOCAL', '0')
+    _close(here, _pass(layer, x, dy))
+
+
+@pytest.mark.parametrize('S,E,M', [(1, 1, 64), (37, 3, 96), (4096, 8, 2048), (4113, 16, 1056)])
+def test_projection_is_at_fp32_precision(S, E, M):
+    """Logits and the weight's gradient against 64 bits, no further off than an fp32 GEMM is."""
+    from planmoe_b200.ops import native
+    torch.manual_seed(0)
+    layer = _layer(E, M, 64, 1, 1.0)
+    x = torch.randn(S, M, device='cuda').bfloat16()
+    w = layer.gates[0].wg.weight
+    ex = layer.experts
+    from planmoe_b200.parallel import transport
+    tr = transport.get_transport(layer.group)
+    out, _cap = native.lib().local_moe_forward(x, w, ex.batched_fc1_w, ex.batched_fc1_bias, ex.batched_fc2_w, ex.batched_fc2_bias,
+                                               1, 4 * S, None, True, False, False, 1, True, tr.budget_ms,
+                                               tr.status.device_ptr(), True, None)
+    logits = out[2].double()
+    ref = x.double() @ w.detach().double().t()
+    lib = (x.float() @ w.detach().float().t()).double()
+    # 2^-22 of the largest sum of magnitudes: two roundings, whatever order the library added in
+    slack = 2.0 ** -22 * float((x.double().abs() @ w.detach().double().abs().t()).max())
+    assert float((logits - ref).abs().max()) <= max(float((lib - ref).abs().max()), slack)
