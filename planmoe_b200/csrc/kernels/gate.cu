@@ -212,14 +212,16 @@ gate_assign_kernel(int S, int E, int K, int C, int normalize, float eps,
   }
 }
 
+// No histograms here: small blocks spread 8192 tokens over all SMs (11 us with 128 threads and 16 experts).
+constexpr int kGateBwdThreads = 32;
 template <class T, int ME, bool SCORES>
-__global__ void __launch_bounds__(kGateThreads)
+__global__ void __launch_bounds__(kGateBwdThreads)
 gate_bwd_kernel(const T* __restrict__ logits, int S, int E, int K, int normalize, float eps,
                 const int* __restrict__ idx, GatePtrs dgates,                     // K rows of S, null = zeros
                 const float* __restrict__ dl_aux,                                 // [1] or null
                 const __nv_bfloat16* __restrict__ dl_aux_bf16,                    // [1] or null
                 const int* __restrict__ top1_count, T* __restrict__ dlogits) {
-  const int t = blockIdx.x * kGateThreads + threadIdx.x;
+  const int t = blockIdx.x * kGateBwdThreads + threadIdx.x;
   if (t >= S) return;
   float p[ME];
   load_row<T, ME>(logits + (size_t)t * E, E, p);
@@ -291,10 +293,10 @@ template <class T, bool SCORES>
 void launch_gate_backward(const T* logits, int S, int E, int K, bool normalize, float eps,
                           const int* idx, GatePtrs dgates, const float* dl_aux,
                           const int* top1_count, T* dlogits, cudaStream_t stream, const void* dl_aux_bf16) {
-  const int nblk = (S + kGateThreads - 1) / kGateThreads;
+  const int nblk = (S + kGateBwdThreads - 1) / kGateBwdThreads;
   auto bwd = E <= 8 ? gate_bwd_kernel<T, 8, SCORES> : E <= 16 ? gate_bwd_kernel<T, 16, SCORES>
            : E <= 32 ? gate_bwd_kernel<T, 32, SCORES> : gate_bwd_kernel<T, 64, SCORES>;
-  bwd<<<nblk, kGateThreads, 0, stream>>>(logits, S, E, K, normalize ? 1 : 0, eps, idx, dgates, dl_aux,
+  bwd<<<nblk, kGateBwdThreads, 0, stream>>>(logits, S, E, K, normalize ? 1 : 0, eps, idx, dgates, dl_aux,
                                          reinterpret_cast<const __nv_bfloat16*>(dl_aux_bf16), top1_count, dlogits);
 }
 
@@ -316,55 +318,79 @@ importance_key_kernel(const T* __restrict__ logits, int S, int E, float* __restr
   for (int e = 0; e < E; ++e) mx = fmaxf(mx, to_f32(row[e]));
   float sum = 0.f;
   for (int e = 0; e < E; ++e) sum += expf(to_f32(row[e]) - mx);
-  key[t] = 1.f / sum;
+  const float k = 1.f / sum;
+  key[t] = k > 0.f ? k : 0.f;                     // NaN scores go last: ranks stay a permutation
 }
 
-// 32 tokens per CTA, eight threads per token: each thread counts over an eighth of every key tile, the eight
-// counts are added by shuffles.  S / 32 CTAs keep the whole machine busy for a few thousand tokens.  Ties need the index
-// only in the tile that holds the token: every key of an earlier tile goes before it from equality on, every key of a
-// later one only when it is larger, so that a comparison is one test and one add on four keys per load (16384 tokens:
-// 115 us with the full test on single keys).
-constexpr int kRankTile = 1024;
+// 32 tokens per CTA and pass, eight threads per token: each thread counts over an eighth of every key tile, the eight
+// counts are added by shuffles.  Ties need the index only in the tile that holds the token: every key of an earlier tile
+// goes before it from equality on, every key of a later one only when it is larger, so that a comparison is one test and
+// one add, on four keys per load.  Two tokens a thread share the loads once there are tokens enough for all SMs, and
+// a tile of 4096 keys leaves few barriers.  (16384 tokens: 115 us with the full test on single keys, 55 us with one token a
+// thread and tiles of 1024.)
+constexpr int kRankTile = 4096;
+template <int TOK>
 __global__ void __launch_bounds__(256)
 importance_rank_kernel(const float* __restrict__ key, int S, int* __restrict__ rank, int* __restrict__ perm) {
   __shared__ __align__(16) float tile[kRankTile];
   const int part = threadIdx.x & 7;
-  const int t0 = blockIdx.x * 32, t = t0 + (threadIdx.x >> 3);   // a CTA's tokens lie in one tile
-  const float mine = t < S ? key[t] : 0.f;
-  int before = 0;
+  const int t0 = blockIdx.x * 32 * TOK;           // a CTA's tokens lie in one tile
+  float mine[TOK];
+  int before[TOK];
+#pragma unroll
+  for (int j = 0; j < TOK; ++j) {
+    const int t = t0 + j * 32 + (threadIdx.x >> 3);
+    mine[j] = t < S ? key[t] : 0.f;
+    before[j] = 0;
+  }
   for (int base = 0; base < S; base += kRankTile) {
     __syncthreads();
     for (int i = threadIdx.x; i < kRankTile; i += blockDim.x) tile[i] = base + i < S ? key[base + i] : -INFINITY;
     __syncthreads();
     const int own = t0 - base;
+    const int n = min(kRankTile, S - base);       // keys are positive: the padding behind the last one never counts
     if (own >= 0 && own < kRankTile) {
-      const int n = min(kRankTile, S - base);
-      for (int i = part; i < n; i += 8) before += (tile[i] > mine || (tile[i] == mine && base + i < t)) ? 1 : 0;
+      for (int i = part; i < n; i += 8) {
+#pragma unroll
+        for (int j = 0; j < TOK; ++j) {
+          const int t = t0 + j * 32 + (threadIdx.x >> 3);
+          before[j] += (tile[i] > mine[j] || (tile[i] == mine[j] && base + i < t)) ? 1 : 0;
+        }
+      }
     } else if (own > 0) {
 #pragma unroll 4
-      for (int i = part * 4; i < kRankTile; i += 32) {           // an earlier tile is full
+      for (int i = part * 4; i < n; i += 32) {    // an earlier tile is full
         const float4 k = *reinterpret_cast<const float4*>(tile + i);
-        before += (k.x >= mine) + (k.y >= mine) + (k.z >= mine) + (k.w >= mine);
+#pragma unroll
+        for (int j = 0; j < TOK; ++j)
+          before[j] += (k.x >= mine[j]) + (k.y >= mine[j]) + (k.z >= mine[j]) + (k.w >= mine[j]);
       }
     } else {
 #pragma unroll 4
-      for (int i = part * 4; i < kRankTile; i += 32) {           // keys are positive: the padding never counts
+      for (int i = part * 4; i < n; i += 32) {
         const float4 k = *reinterpret_cast<const float4*>(tile + i);
-        before += (k.x > mine) + (k.y > mine) + (k.z > mine) + (k.w > mine);
+#pragma unroll
+        for (int j = 0; j < TOK; ++j)
+          before[j] += (k.x > mine[j]) + (k.y > mine[j]) + (k.z > mine[j]) + (k.w > mine[j]);
       }
     }
   }
-  before += __shfl_xor_sync(0xffffffffu, before, 1);
-  before += __shfl_xor_sync(0xffffffffu, before, 2);
-  before += __shfl_xor_sync(0xffffffffu, before, 4);
-  if (part == 0 && t < S) { rank[t] = before; perm[before] = t; }
+#pragma unroll
+  for (int j = 0; j < TOK; ++j) {
+    before[j] += __shfl_xor_sync(0xffffffffu, before[j], 1);
+    before[j] += __shfl_xor_sync(0xffffffffu, before[j], 2);
+    before[j] += __shfl_xor_sync(0xffffffffu, before[j], 4);
+    const int t = t0 + j * 32 + (threadIdx.x >> 3);
+    if (part == 0 && t < S) { rank[t] = before[j]; perm[before[j]] = t; }
+  }
 }
 
 template <class T>
 void launch_importance_order(const T* logits, int S, int E, float* key, int* rank, int* perm, cudaStream_t stream) {
   if (S <= 0) return;
   importance_key_kernel<T><<<(S + 255) / 256, 256, 0, stream>>>(logits, S, E, key);
-  importance_rank_kernel<<<(S + 31) / 32, 256, 0, stream>>>(key, S, rank, perm);
+  if (S >= 64 * 148) importance_rank_kernel<2><<<(S + 63) / 64, 256, 0, stream>>>(key, S, rank, perm);
+  else importance_rank_kernel<1><<<(S + 31) / 32, 256, 0, stream>>>(key, S, rank, perm);
 }
 template void launch_importance_order<float>(const float*, int, int, float*, int*, int*, cudaStream_t);
 template void launch_importance_order<__nv_bfloat16>(const __nv_bfloat16*, int, int, float*, int*, int*, cudaStream_t);

@@ -61,25 +61,35 @@ gate_project_kernel(const __nv_bfloat16* __restrict__ x, const void* __restrict_
     for (int n = 0; n < NT; ++n)
 #pragma unroll
       for (int i = 0; i < 4; ++i) acc[m][n][i] = 0.f;
+  // The rows and weights of a warp's next chunk are on their way while it works on this one: without that the kernel took
+  // 48 us for 16384 x 4096, 20 of them for the bytes.
   const int chunks = M / 32;
-#pragma unroll 2
-  for (int ch = warp; ch < chunks; ch += kProjWarps) {
-    uint4 a[MT][2];
+  uint4 a[2][MT][2], wr[2][NT][W_BF16 ? 1 : 2];
+  auto fetch = [&](int buf, int ch) {
 #pragma unroll
     for (int m = 0; m < MT; ++m) {
-      a[m][0] = __ldg(xr[m][0] + ch * 4);
-      a[m][1] = __ldg(xr[m][1] + ch * 4);
+      a[buf][m][0] = __ldg(xr[m][0] + ch * 4);
+      a[buf][m][1] = __ldg(xr[m][1] + ch * 4);
     }
 #pragma unroll
     for (int n = 0; n < NT; ++n) {
       const long long at = (long long)min(n * 8 + g, E - 1) * M + ch * 32 + c * 8;
+      const uint4* src = W_BF16 ? reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(w_) + at)
+                                : reinterpret_cast<const uint4*>(reinterpret_cast<const float*>(w_) + at);
+#pragma unroll
+      for (int i = 0; i < (W_BF16 ? 1 : 2); ++i) wr[buf][n][i] = __ldg(src + i);
+    }
+  };
+  auto multiply = [&](int buf) {
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
       uint4 b[W_BF16 ? 1 : 3];
       if constexpr (W_BF16) {
-        b[0] = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(w_) + at));
+        b[0] = wr[buf][n][0];
       } else {
-        const float4 lo = __ldg(reinterpret_cast<const float4*>(reinterpret_cast<const float*>(w_) + at));
-        const float4 hi = __ldg(reinterpret_cast<const float4*>(reinterpret_cast<const float*>(w_) + at) + 1);
-        float f[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+        const uint4 lo = wr[buf][n][0], hi = wr[buf][n][W_BF16 ? 0 : 1];
+        float f[8] = {__uint_as_float(lo.x), __uint_as_float(lo.y), __uint_as_float(lo.z), __uint_as_float(lo.w),
+                      __uint_as_float(hi.x), __uint_as_float(hi.y), __uint_as_float(hi.z), __uint_as_float(hi.w)};
 #pragma unroll
         for (int s = 0; s < 3; ++s) {
           b[s] = make_uint4(upper_halves(f[0], f[1]), upper_halves(f[2], f[3]), upper_halves(f[4], f[5]), upper_halves(f[6], f[7]));
@@ -93,11 +103,19 @@ gate_project_kernel(const __nv_bfloat16* __restrict__ x, const void* __restrict_
       for (int s = (W_BF16 ? 1 : 3) - 1; s >= 0; --s) {          // the small terms first
 #pragma unroll
         for (int m = 0; m < MT; ++m) {
-          mma_16816(acc[m][n], a[m][0].x, a[m][1].x, a[m][0].y, a[m][1].y, b[s].x, b[s].y);
-          mma_16816(acc[m][n], a[m][0].z, a[m][1].z, a[m][0].w, a[m][1].w, b[s].z, b[s].w);
+          mma_16816(acc[m][n], a[buf][m][0].x, a[buf][m][1].x, a[buf][m][0].y, a[buf][m][1].y, b[s].x, b[s].y);
+          mma_16816(acc[m][n], a[buf][m][0].z, a[buf][m][1].z, a[buf][m][0].w, a[buf][m][1].w, b[s].z, b[s].w);
         }
       }
     }
+  };
+  if (warp < chunks) fetch(0, warp);
+  for (int ch = warp; ch < chunks; ch += 2 * kProjWarps) {
+    const int c1 = ch + kProjWarps, c2 = c1 + kProjWarps;
+    if (c1 < chunks) fetch(1, c1);
+    multiply(0);
+    if (c2 < chunks) fetch(0, c2);
+    if (c1 < chunks) multiply(1);
   }
 #pragma unroll
   for (int m = 0; m < MT; ++m)
@@ -127,7 +145,8 @@ __device__ __forceinline__ void bf16_pairs(const uint4& raw, unsigned long long*
 
 // Block (column slab of 256, chunk of tokens): a lane holds 8 columns of EB experts, the 8 warps take the chunk's tokens in
 // turn; their sums are added in warp order through shared memory, one expert after the other.  The gradients of the logits
-// wait in shared memory as pairs {d, d}.
+// wait in shared memory as pairs {d, d}; a warp's eight rows of a stage are requested together, before the barriers around
+// those (one row at a time: 104 us for 16384 x 4096, 20 of them for the bytes).
 constexpr int kWgradTokens = 64;                  // tokens whose logit gradients are staged at a time
 
 template <int EB>
@@ -145,24 +164,30 @@ gate_wgrad_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__
   for (int e = 0; e < EB; ++e)
 #pragma unroll
     for (int i = 0; i < 4; ++i) acc[e][i] = 0ull;
+  constexpr int kRows = kWgradTokens / 8;
   for (int b0 = c0; b0 < c1; b0 += kWgradTokens) {
     const int n = min(kWgradTokens, c1 - b0);
+    uint4 raw[kRows];
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) {
+      const int t = warp + 8 * r;
+      raw[r] = make_uint4(0, 0, 0, 0);
+      if (in && t < n) raw[r] = __ldg(reinterpret_cast<const uint4*>(x + (long long)(b0 + t) * M + col));
+    }
     __syncthreads();
-    for (int i = threadIdx.x; i < n * EB; i += 256) {
+    for (int i = threadIdx.x; i < kWgradTokens * EB; i += 256) {
       const int t = i / EB, e = i - t * EB;
-      const float v = e < E ? dl[(long long)(b0 + t) * E + e] : 0.f;
+      const float v = t < n && e < E ? dl[(long long)(b0 + t) * E + e] : 0.f;
       d_s[t][e] = make_float2(v, v);
     }
     __syncthreads();
-#pragma unroll 4
-    for (int t = warp; t < n; t += 8) {
-      uint4 raw = make_uint4(0, 0, 0, 0);
-      if (in) raw = __ldg(reinterpret_cast<const uint4*>(x + (long long)(b0 + t) * M + col));
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) {
       unsigned long long p[4];
-      bf16_pairs(raw, p);
+      bf16_pairs(raw[r], p);
 #pragma unroll
       for (int e = 0; e < EB; ++e) {
-        const unsigned long long d = *reinterpret_cast<const unsigned long long*>(&d_s[t][e]);
+        const unsigned long long d = *reinterpret_cast<const unsigned long long*>(&d_s[warp + 8 * r][e]);
 #pragma unroll
         for (int i = 0; i < 4; ++i) acc[e][i] = fma_pair(p[i], d, acc[e][i]);
       }
@@ -188,46 +213,59 @@ gate_wgrad_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__
   }
 }
 
-// One warp per (8 tokens, 256 columns): the weights of a column are read once for the eight tokens.
-constexpr int kGatherTokens = 8;
+// One block per (32 tokens, 256 columns), 4 tokens a warp.  The slab of the weights is staged once per block, and a warp's
+// slots are looked up by one load per lane, so that all its rows are requested together.  (With the weights read by every
+// warp and the slots looked up token by token: 128 us for 16384 x 4096, top-2, 8 experts; 61 of them for the bytes.)
+constexpr int kGatherTokens = 4;                    // 8: 110 us, two blocks per SM
 
 template <int MAXK, bool W_BF16, bool GATED>
-__global__ void __launch_bounds__(256, MAXK <= 2 ? 2 : 1)
+__global__ void __launch_bounds__(256, MAXK <= 2 ? 4 : 2)
 gather_gate_kernel(const __nv_bfloat16* __restrict__ slots, const int* __restrict__ idx, const int* __restrict__ loc,
                    const float* __restrict__ gates, const float* __restrict__ dl, const void* __restrict__ w_,
                    __nv_bfloat16* __restrict__ dx, int K, int S, int M, int E, int C) {
-  extern __shared__ float2 dl_s[];                // [warp][8 tokens][E]
+  extern __shared__ __align__(16) float gather_smem[];
+  float* w_s = gather_smem;                                                       // [E][256]
+  float2* dl_s = reinterpret_cast<float2*>(gather_smem + E * 256);                // [32 tokens][E], pairs {d, d}
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int slabs = (M + 255) / 256;
-  const long long item = (long long)blockIdx.x * 8 + warp;
-  const int t0 = (int)(item / slabs) * kGatherTokens, col = (int)(item % slabs) * 256 + lane * 8;
-  if (t0 >= S) return;
-  float2* mine = dl_s + warp * kGatherTokens * E;
-  for (int i = lane; i < kGatherTokens * E; i += 32) {
-    const int t = min(t0 + i / E, S - 1);
-    const float v = dl[(long long)t * E + i % E];
-    mine[i] = make_float2(v, v);
-  }
-  __syncwarp();
-  if (col >= M) return;
-  uint4 raw[kGatherTokens][MAXK];
-  float gw[kGatherTokens][GATED ? MAXK : 1];
-#pragma unroll
-  for (int t = 0; t < kGatherTokens; ++t) {
-#pragma unroll
-    for (int k = 0; k < MAXK; ++k) {
-      raw[t][k] = make_uint4(0, 0, 0, 0);
-      if constexpr (GATED) gw[t][k] = 0.f;
-      const int tok = t0 + t;
-      if (k < K && tok < S) {
-        const int e = idx[(size_t)k * S + tok], l = loc[(size_t)k * S + tok];
-        if (l >= 0 && l < C && e >= 0) {
-          raw[t][k] = __ldg(reinterpret_cast<const uint4*>(slots + ((long long)e * C + l) * M + col));
-          if constexpr (GATED) gw[t][k] = gates[(size_t)k * S + tok];
-        }
-      }
+  const int slabs = (M + 255) / 256;              // neighbouring blocks take neighbouring columns of the same tokens
+  const int tb = (int)(blockIdx.x / slabs) * 8 * kGatherTokens, c0 = (int)(blockIdx.x % slabs) * 256;
+  const int col = c0 + lane * 8, t0 = tb + warp * kGatherTokens;
+  // lane (token, pick): its slot, -1 without one
+  static_assert(kGatherTokens * MAXK <= 32, "one lane per token and pick");
+  long long at = -1;
+  float gv = 0.f;
+  {
+    const int tok = t0 + lane / MAXK, k = lane % MAXK;
+    if (lane < kGatherTokens * MAXK && k < K && tok < S) {
+      const int e = idx[(size_t)k * S + tok], l = loc[(size_t)k * S + tok];
+      if (e >= 0 && l >= 0 && l < C) at = (long long)e * C + l;
+      if constexpr (GATED) gv = gates[(size_t)k * S + tok];
     }
   }
+  uint4 raw[kGatherTokens][MAXK];
+#pragma unroll
+  for (int t = 0; t < kGatherTokens; ++t)
+#pragma unroll
+    for (int k = 0; k < MAXK; ++k) {
+      const long long row = __shfl_sync(0xffffffffu, at, t * MAXK + k);
+      raw[t][k] = make_uint4(0, 0, 0, 0);
+      if (row >= 0 && col < M) raw[t][k] = __ldg(reinterpret_cast<const uint4*>(slots + row * M + col));
+    }
+  for (int i = threadIdx.x; i < E * 256; i += 256) {
+    const int m = c0 + (i & 255);
+    float v = 0.f;
+    if (m < M) {
+      const long long o = (long long)(i >> 8) * M + m;
+      v = W_BF16 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(w_)[o]) : reinterpret_cast<const float*>(w_)[o];
+    }
+    w_s[i] = v;
+  }
+  for (int i = threadIdx.x; i < 8 * kGatherTokens * E; i += 256) {
+    const int t = tb + i / E;
+    const float v = t < S ? dl[(long long)tb * E + i] : 0.f;
+    dl_s[i] = make_float2(v, v);
+  }
+  __syncthreads();
   unsigned long long acc[kGatherTokens][4];
 #pragma unroll
   for (int t = 0; t < kGatherTokens; ++t) {
@@ -237,21 +275,18 @@ gather_gate_kernel(const __nv_bfloat16* __restrict__ slots, const int* __restric
     for (int k = 0; k < MAXK; ++k) {
       unsigned long long p[4];
       bf16_pairs(raw[t][k], p);
-      const float gk = GATED ? gw[t][GATED ? k : 0] : 1.f;
+      const float gk = GATED ? __shfl_sync(0xffffffffu, gv, t * MAXK + k) : 1.f;
       const unsigned long long gp = pair_of(gk, gk);
 #pragma unroll
       for (int i = 0; i < 4; ++i) acc[t][i] = fma_pair(p[i], gp, acc[t][i]);
     }
   }
+  const float2* mine = dl_s + warp * kGatherTokens * E;
+#pragma unroll 2
   for (int e = 0; e < E; ++e) {
-    unsigned long long w[4];
-    if constexpr (W_BF16) {
-      bf16_pairs(__ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(w_) + (long long)e * M + col)), w);
-    } else {
-      const float4* wp = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(w_) + (long long)e * M + col);
-      const float4 lo = __ldg(wp), hi = __ldg(wp + 1);
-      w[0] = pair_of(lo.x, lo.y); w[1] = pair_of(lo.z, lo.w); w[2] = pair_of(hi.x, hi.y); w[3] = pair_of(hi.z, hi.w);
-    }
+    const ulonglong2 lo = *reinterpret_cast<const ulonglong2*>(w_s + e * 256 + lane * 8);
+    const ulonglong2 hi = *reinterpret_cast<const ulonglong2*>(w_s + e * 256 + lane * 8 + 4);
+    const unsigned long long w[4] = {lo.x, lo.y, hi.x, hi.y};
 #pragma unroll
     for (int t = 0; t < kGatherTokens; ++t) {
       const unsigned long long d = *reinterpret_cast<const unsigned long long*>(&mine[t * E + e]);
@@ -259,6 +294,7 @@ gather_gate_kernel(const __nv_bfloat16* __restrict__ slots, const int* __restric
       for (int i = 0; i < 4; ++i) acc[t][i] = fma_pair(w[i], d, acc[t][i]);
     }
   }
+  if (col >= M) return;
 #pragma unroll
   for (int t = 0; t < kGatherTokens; ++t) {
     if (t0 + t >= S) break;
@@ -315,9 +351,8 @@ void launch_gate_wgrad(const void* x, const float* dl, float* partial, int S, in
 
 void launch_gather_gate(const void* slots, const int* idx, const int* loc, const float* gates, const float* dl, const void* w,
                         bool w_bf16, void* dx, int K, int S, int M, int E, int C, cudaStream_t stream) {
-  const long long items = (long long)((S + kGatherTokens - 1) / kGatherTokens) * ((M + 255) / 256);
-  const unsigned grid = (unsigned)((items + 7) / 8);
-  const int smem = 8 * kGatherTokens * E * (int)sizeof(float2);
+  const unsigned grid = (unsigned)((S + 8 * kGatherTokens - 1) / (8 * kGatherTokens)) * (unsigned)((M + 255) / 256);
+  const int smem = E * 256 * (int)sizeof(float) + 8 * kGatherTokens * E * (int)sizeof(float2);      // at most 24 KiB
   const __nv_bfloat16* sb = reinterpret_cast<const __nv_bfloat16*>(slots);
   __nv_bfloat16* db = reinterpret_cast<__nv_bfloat16*>(dx);
   auto pick = [&](auto gated) {

@@ -140,3 +140,20 @@ def test_projection_is_at_fp32_precision(S, E, M):
     # 2^-22 of the largest sum of magnitudes: two roundings, whatever order the library added in
     slack = 2.0 ** -22 * float((x.double().abs() @ w.detach().double().abs().t()).max())
     assert float((logits - ref).abs().max()) <= max(float((lib - ref).abs().max()), slack)
+
+
+def test_priority_order_is_a_permutation_whatever_the_scores():
+    """Ties, NaN rows, more than one key tile, a token count that no tile divides: ranks and order stay inverse to each other."""
+    from planmoe_b200.ops import native
+    torch.manual_seed(0)
+    for S in (1, 63, 4097, 9473, 20000):
+        logits = torch.randn(S, 8, device='cuda')
+        logits[S // 2] = float('nan')
+        logits[: S // 3] = logits[0]
+        rank, perm = native.lib().importance_order(logits)
+        assert torch.equal(rank[perm.long()], torch.arange(S, device='cuda', dtype=torch.int32))
+        key = torch.softmax(logits, 1).max(1).values.nan_to_num(0.0)
+        ordered = key[perm.long()]
+        assert bool((ordered[:-1] >= ordered[1:] - 2e-7).all())
+        tied = rank[: S // 3]
+        assert bool((tied[1:] > tied[:-1]).all())          # equal keys: token order
