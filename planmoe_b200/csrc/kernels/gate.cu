@@ -88,7 +88,9 @@ gate_stats_kernel(const T* __restrict__ logits, int S, int E, int K, int nblk,
   }
 
   unsigned long long taken = 0ull;
-  for (int k = 0; k < K; ++k) {
+#pragma unroll
+  for (int k = 0; k < kMaxK; ++k) {
+    if (k >= K) break;                           // unrolled: the picks stay in registers
     int best = -1;                               // K <= E: one expert is always left
     float bv = 0.f;
 #pragma unroll
@@ -109,7 +111,9 @@ gate_stats_kernel(const T* __restrict__ logits, int S, int E, int K, int nblk,
   }
   __syncthreads();
 
-  for (int k = 0; k < K; ++k) {
+#pragma unroll
+  for (int k = 0; k < kMaxK; ++k) {
+    if (k >= K) break;                           // unrolled: the picks stay in registers
     if (!live) break;
     const int e = pick[k] & 0xff, r = pick[k] >> 8;
     int before = 0;
@@ -145,6 +149,18 @@ gate_assign_kernel(int S, int E, int K, int C, int normalize, float eps,
   __shared__ float red[kMaxE];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int b = blockIdx.x;
+  // the token's own values are on their way while the histograms are summed
+  const int pos = b * kGateThreads + tid;
+  const int t = pos < S ? (perm != nullptr ? perm[pos] : pos) : 0;
+  int pick[kMaxK], rank[kMaxK];
+  float g[kMaxK];
+#pragma unroll
+  for (int k = 0; k < kMaxK; ++k) {
+    if (k >= K || pos >= S) break;
+    pick[k] = idx[(size_t)k * S + t];
+    rank[k] = rank_in_blk[(size_t)k * S + t];
+    g[k] = raw_gate[(size_t)k * S + t];
+  }
   // base[k][e] = picks of expert e that rank before this block's k-th picks: every block's picks of a lower k,
   // then the k-th picks of the blocks before this one.  One warp per (k, e), lanes strided over that list.
   for (int i = warp; i < K * E; i += kGateWarps) {
@@ -160,20 +176,19 @@ gate_assign_kernel(int S, int E, int K, int C, int normalize, float eps,
   }
   __syncthreads();
 
-  const int pos = b * kGateThreads + tid;
   if (pos < S) {
-    const int t = perm != nullptr ? perm[pos] : pos;
-    float g[kMaxK];
-    float denom = 0.f;
-    for (int k = 0; k < K; ++k) { g[k] = raw_gate[(size_t)k * S + t]; denom += g[k]; }
     const bool norm = normalize && K > 1;
+    float denom = 0.f;
+#pragma unroll
+    for (int k = 0; k < kMaxK; ++k) denom += k < K ? g[k] : 0.f;
     denom = fmaxf(denom, eps);
-    for (int k = 0; k < K; ++k) {
-      const int e = idx[(size_t)k * S + t];
-      const int l = base[k][e] + rank_in_blk[(size_t)k * S + t];
+#pragma unroll
+    for (int k = 0; k < kMaxK; ++k) {
+      if (k >= K) break;
+      const int l = base[k][pick[k]] + rank[k];
       loc[(size_t)k * S + t] = l;
       gates.p[k][t] = norm ? g[k] / denom : g[k];
-      if (slot_map != nullptr && l < C) slot_map[(size_t)e * C + l] = t * K + k;
+      if (slot_map != nullptr && l < C) slot_map[(size_t)pick[k] * C + l] = t * K + k;
     }
   }
 
@@ -233,7 +248,9 @@ gate_bwd_kernel(const T* __restrict__ logits, int S, int E, int K, int normalize
   int pk[kMaxK];
   float ds_pick[kMaxK];
   float denom = 0.f, dot = 0.f;
-  for (int k = 0; k < K; ++k) {
+#pragma unroll
+  for (int k = 0; k < kMaxK; ++k) {
+    if (k >= K) break;                           // unrolled: the picks stay in registers
     pk[k] = idx[(size_t)k * S + t];
     float s = 0.f;
 #pragma unroll
@@ -242,11 +259,15 @@ gate_bwd_kernel(const T* __restrict__ logits, int S, int E, int K, int normalize
     denom += s;
   }
   const bool norm = normalize && K > 1;
-  for (int k = 0; k < K; ++k) {
+#pragma unroll
+  for (int k = 0; k < kMaxK; ++k) {
+    if (k >= K) break;                           // unrolled: the picks stay in registers
     const float dg = dgates.p[k] ? dgates.p[k][t] : 0.f;
     dot += dg * ds_pick[k];
   }
-  for (int k = 0; k < K; ++k) {
+#pragma unroll
+  for (int k = 0; k < kMaxK; ++k) {
+    if (k >= K) break;                           // unrolled: the picks stay in registers
     const float dg = dgates.p[k] ? dgates.p[k][t] : 0.f;
     if (norm) {
       if (denom > eps) ds_pick[k] = dg / denom - dot / (denom * denom);
@@ -262,7 +283,8 @@ gate_bwd_kernel(const T* __restrict__ logits, int S, int E, int K, int normalize
     float d = 0.f;
     if (e < E) {
       d = lw * (float)top1_count[e];
-      for (int k = 0; k < K; ++k) d += (pk[k] == e) ? ds_pick[k] : 0.f;
+#pragma unroll
+      for (int k = 0; k < kMaxK; ++k) d += (k < K && pk[k] == e) ? ds_pick[k] : 0.f;
     }
     ds[e] = d;
     inner += d * p[e];
