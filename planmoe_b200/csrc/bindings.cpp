@@ -1069,6 +1069,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("local_moe_forward", &local_moe_forward_op);
   m.def("local_moe_backward", &local_moe_backward_op);
   m.attr("gate_max_experts") = kProjMaxE;
+  // whether the environment leaves a single rank to the direct path (read at every call, like all of these switches)
+  m.def("local_by_env", [] {
+    auto is = [](const char* v, char c) { return v != nullptr && v[0] == c && v[1] == 0; };
+    return !is(getenv("PLANMOE_LOCAL"), '0') && getenv("PLANMOE_FUSE_SEND") == nullptr &&
+           !is(getenv("PLANMOE_DEBUG_GUARDS"), '1') && !is(getenv("PLANMOE_GEMM_TRACE"), '1');
+  });
   m.def("importance_order", &importance_order_op);
   m.def("remap_slot_map", &remap_slot_map_op);
   m.def("gate_backward", &gate_backward_op);

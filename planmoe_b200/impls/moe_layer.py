@@ -348,9 +348,11 @@ class MOELayer(torch.nn.Module):
         assert len(original_shape) >= 2, \
             "Input data must be at least 2D tensor: (s)amples, .., (m)odel_dim"
         x = input.reshape(-1, original_shape[-reserve_dims:].numel())
-        for p in self.experts.parameters():
-            x = x.to(p.dtype)
-            break
+        first = self.experts._parameters.get('batched_fc1_w')       # the FFN experts' first parameter
+        if first is None:
+            first = next(iter(self.experts.parameters()), None)
+        if first is not None and x.dtype != first.dtype:
+            x = x.to(first.dtype)
         gctx = self.gates[gate_index]
         degree = self.a2a_ffn_overlap_degree if a2a_ffn_overlap_degree is None \
             else a2a_ffn_overlap_degree
@@ -362,8 +364,11 @@ class MOELayer(torch.nn.Module):
             self.save_count += 1
         y, l_aux = self._forward_core(x, gctx, top_k, cf, int(degree), reserve_shape, comm_name)
 
-        y = y.view(list(original_shape)).to(original_dtype)
-        self.l_aux = y.l_aux = l_aux
+        y = y.view(list(original_shape))
+        if y.dtype != original_dtype:
+            y = y.to(original_dtype)
+        y.l_aux = l_aux
+        object.__setattr__(self, 'l_aux', l_aux)                    # a plain attribute: no parameter or buffer of that name
         return self.result_func(y) if self.result_func is not None else y
 
     def _forward_core(self, x, gctx, top_k, cf, degree, reserve_shape, comm_name=None):

@@ -455,9 +455,7 @@ class _FusedExperts(torch.autograd.Function):
 def _local_path(tr, q8):
     """Whether a layer's experts run without the exchange: one rank and bf16 rows.  PLANMOE_LOCAL=0, a choice of the send's
     form (PLANMOE_FUSE_SEND), the debug guards and the role trace keep the exchange, which is what they are about."""
-    return (tr.world == 1 and not tr.emulated and not q8 and os.environ.get('PLANMOE_LOCAL', '1') != '0'
-            and 'PLANMOE_FUSE_SEND' not in os.environ and not T.debug_guards()
-            and os.environ.get('PLANMOE_GEMM_TRACE', '0') != '1')
+    return tr.world == 1 and not tr.emulated and not q8 and native.lib().local_by_env()
 
 
 def _aligned(t):

@@ -276,5 +276,6 @@ def get_comm(name, group=None):
     return factory(group)
 
 
-for _cls in (NaiveComm, NcclComm, PipeComm, DdComm, HeTuComm):
+BUILTIN = (NaiveComm, NcclComm, PipeComm, DdComm, HeTuComm)
+for _cls in BUILTIN:
     register_comm(_cls.name, _cls)
