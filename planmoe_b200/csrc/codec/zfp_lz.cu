@@ -262,7 +262,8 @@ __host__ __device__ inline void lz_decode_one(const uint8_t* packed, uint8_t* ra
 
 // Warp-parallel block coder.  One warp codes one 2 KiB block, 32 positions ("a row") at a time, and produces exactly
 // the bytes of the serial coder lz_encode_block (the CPU twin, which the tests compare against).  A row's symbols are
-// held bit-sliced: B[b] is the ballot of bit b over the row.
+// held bit-sliced: B[b] is bit b of all 32 symbols, from a bit transpose over the warp (of two rows at once with 16-bit
+// symbols), read back from shared memory by every lane.
 //   1. lane d compares the row with the symbols d + 1 positions back: all 32 positions at once, by and-ing, over the
 //      symbol's bits, B[b] with itself shifted across the row boundary.  A 32 x 32 bit transpose over the warp turns
 //      that into one mask of candidate distances per position (bit d set: in[p] == in[p - d - 1]).
@@ -274,8 +275,9 @@ __host__ __device__ inline void lz_decode_one(const uint8_t* packed, uint8_t* ra
 //      over the row, the set of starts a walk from it visits and where that walk enters the next row; the row's own
 //      entry picks one of them.
 //   4. the row's tokens are written at their ordinals; their flags are compressed by one or-reduction.
-// Bound by issue: the former coder compared through shared memory, 32 loads a position, then walked its tokens
-// serially per lane (13.7 k warp instructions a block; 537 us for 8192 x 4096 bf16).
+// Bound by the integer pipe.  8192 x 4096 bf16: 537 us when candidates were compared through shared memory and tokens
+// walked serially per lane; 432 us with a ballot per bit and the match length counted symbol by symbol (10.4 k warp
+// instructions a block).
 //
 // scratch layout: [slices][nb] slots of kLzScratchSlot bytes {token data, flag words, token count}, then int sizes
 // [slices][nb] (bytes of the block's code)
@@ -300,57 +302,75 @@ __device__ __forceinline__ uint32_t warp_transpose32(uint32_t x, int lane) {
 
 template <class Sym>
 __device__ __forceinline__ void lz_encode_block_warp(const Sym* __restrict__ in, int nsym, uint8_t* __restrict__ slot,
-                                                     int* __restrict__ out_size, uint32_t* eqs, int lane) {
+                                                     int* __restrict__ out_size, uint32_t* sm, int lane) {
   constexpr int kBits = 8 * (int)sizeof(Sym);
+  constexpr int kRowsAtOnce = 32 / kBits;         // rows whose symbols fill one word per lane
   constexpr int min_match = sizeof(Sym) == 2 ? 2 : 1;
   const uint32_t lt = (1u << lane) - 1u;
+  uint32_t* masks = sm;                           // candidate masks of the row in work and of the next one
+  uint32_t* bits = sm + 64;                       // B of the newest kRowsAtOnce rows
   uint16_t* data = reinterpret_cast<uint16_t*>(slot);
   uint32_t* flag_words = reinterpret_cast<uint32_t*>(slot + kLzScratchFlags);
-  uint32_t prev[kBits];                           // the row before, bit-sliced
+  uint32_t prev[kBits];                           // B of the row before
 #pragma unroll
   for (int b = 0; b < kBits; ++b) prev[b] = 0u;
   const int rows = (nsym + 31) >> 5;
-  auto row_mask = [&](int k) { const int left = nsym - k * 32; return left >= 32 ? 0xffffffffu : (1u << left) - 1u; };
+  auto row_mask = [&](int k) { const int left = nsym - k * 32; return left >= 32 ? 0xffffffffu : left <= 0 ? 0u : (1u << left) - 1u; };
   auto load = [&](int k) { const int p = k * 32 + lane; return p < nsym ? in[p] : (Sym)0; };
-  auto candidates = [&](Sym v, int k) {
+  // B of rows k .. k + kRowsAtOnce - 1, symbols v (and u): lane b gets the word of bit b
+  auto slice = [&](Sym v, Sym u) {
+    const uint32_t w = warp_transpose32(kBits == 32 ? (uint32_t)v : (uint32_t)v | ((uint32_t)u << (kBits & 31)), lane);
+    __syncwarp();                                 // the last readers of `bits` are done
+    bits[lane] = w;
+    __syncwarp();
+  };
+  auto candidates = [&](int k) {
     uint32_t acc = row_mask(k);
     if (k == 0) acc &= ~((2u << lane) - 1u);      // nothing lies before position 0
+    const uint4* words = reinterpret_cast<const uint4*>(bits + (k % kRowsAtOnce) * kBits);
 #pragma unroll
-    for (int b = 0; b < kBits; ++b) {
-      const uint32_t cur = __ballot_sync(0xffffffffu, (v >> b) & 1u);
-      acc &= ~(cur ^ __funnelshift_lc(prev[b], cur, lane + 1));
-      prev[b] = cur;
+    for (int b4 = 0; b4 < kBits / 4; ++b4) {
+      const uint4 q = words[b4];
+      const uint32_t cur[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        acc &= ~(cur[j] ^ __funnelshift_lc(prev[b4 * 4 + j], cur[j], lane + 1));
+        prev[b4 * 4 + j] = cur[j];
+      }
     }
     return warp_transpose32(acc, lane);
   };
 
-  Sym v = load(0);
-  uint32_t eq = candidates(v, 0);                 // this lane's mask of row k
-  eqs[lane] = eq;
+  // symbols are loaded kRowsAtOnce rows ahead of their slicing
+  Sym v = load(0), v_next = load(1), a0 = load(2), a1 = load(3);
+  slice(v, v_next);
+  uint32_t eq = candidates(0);                    // this lane's mask of row k
   int entry = 0, ntok = 0, dbytes = 0;
   uint64_t facc = 0;                              // flags not yet written, first token lowest
   int fbits = 0;
-  Sym v_ahead = rows > 1 ? load(1) : (Sym)0;
   for (int k = 0; k < rows; ++k) {
-    const Sym v_next = v_ahead;
     uint32_t eq_next = 0u;
-    if (k + 1 < rows) eq_next = candidates(v_next, k + 1);
-    if (k + 2 < rows) v_ahead = load(k + 2);
-    eqs[((k + 1) & 1) * 32 + lane] = eq_next;
+    if (k + 1 < rows) {
+      if ((k + 1) % kRowsAtOnce == 0) slice(v_next, a0);
+      eq_next = candidates(k + 1);
+    }
+    masks[lane] = eq;
+    masks[32 + lane] = eq_next;
     __syncwarp();
 
-    // 2. longest match (the first four symbols without a branch)
-    const int at = (k & 1) * 32 + lane;           // masks of positions p .. p + 31 lie at (at + i) & 63
-    const uint32_t m1 = eq & eqs[(at + 1) & 63];
-    const uint32_t m2 = m1 & eqs[(at + 2) & 63];
-    const uint32_t m3 = m2 & eqs[(at + 3) & 63];
-    int best = (eq != 0u) + (m1 != 0u) + (m2 != 0u) + (m3 != 0u);
-    uint32_t m = m1 ? m1 : eq;
-    m = m2 ? m2 : m;
-    if (m3) {
-      m = m3;
+    // 2. longest match: up to seven symbols without a branch.  m_i: distances that match i + 1 symbols.
+    const uint32_t* at = masks + lane;
+    const uint32_t m1 = eq & at[1], m2 = m1 & at[2], m3 = m2 & at[3], m4 = m3 & at[4], m5 = m4 & at[5], m6 = m5 & at[6];
+    const bool four = m3 != 0u;
+    uint32_t m = four ? m3 : eq;
+    int best = four ? 4 : eq != 0u ? 1 : 0;
+    const uint32_t two = four ? m5 : m1;          // two (four: six) symbols
+    if (two != 0u) { m = two; best = four ? 6 : 2; }
+    const uint32_t odd = four ? (two != 0u ? m6 : m4) : (two != 0u ? m2 : 0u);
+    if (odd != 0u) { m = odd; ++best; }
+    if (m6 != 0u) {
       while (best < kLzMaxMatch) {
-        const uint32_t t = m & eqs[(at + best) & 63];
+        const uint32_t t = m & at[best];
         if (t == 0u) break;
         m = t;
         ++best;
@@ -398,6 +418,9 @@ __device__ __forceinline__ void lz_encode_block_warp(const Sym* __restrict__ in,
       fbits -= 32;
     }
     v = v_next;
+    v_next = a0;
+    a0 = a1;
+    a1 = load(k + 4);
     eq = eq_next;
   }
   if (lane == 0) {
@@ -411,7 +434,7 @@ template <class Sym>
 __global__ void __launch_bounds__(kLzWarps * 32)
 lz_encode_blocks_kernel(const uint8_t* __restrict__ raw, uint8_t* __restrict__ slots, int* __restrict__ blk_sizes,
                         long long slices, long long raw_bytes) {
-  __shared__ uint32_t eqs[kLzWarps][64];
+  __shared__ __align__(16) uint32_t sm[kLzWarps][96];     // see lz_encode_block_warp
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long long nb = lz_blocks(raw_bytes);
   const long long i = (long long)blockIdx.x * kLzWarps + warp;
@@ -420,7 +443,7 @@ lz_encode_blocks_kernel(const uint8_t* __restrict__ raw, uint8_t* __restrict__ s
   const long long off = b * kLzBlockBytes;
   const int bytes = (int)(raw_bytes - off < kLzBlockBytes ? raw_bytes - off : kLzBlockBytes);
   lz_encode_block_warp<Sym>(reinterpret_cast<const Sym*>(raw + s * raw_bytes + off), bytes / (int)sizeof(Sym),
-                            slots + i * kLzScratchSlot, blk_sizes + i, eqs[warp], lane);
+                            slots + i * kLzScratchSlot, blk_sizes + i, sm[warp], lane);
 }
 
 // One CTA per slice: exclusive scan of the block sizes -> header of the slice payload.  Four sizes a thread, so that a
