@@ -577,7 +577,7 @@ struct Stage {
 struct LocalRoute {
   Tensor idx, loc, slot_map, used, gates;
   int64_t C, act;
-  bool postscore;
+  bool postscore, int8;                           // int8: rows as int8 transfers deliver them, both ways
   int64_t budget_ms, status_ptr;
 };
 
@@ -595,6 +595,29 @@ static void local_check(const Tensor& x, const LocalRoute& r, const Tensor& w1) 
   rows16(x);
   TORCH_CHECK(i32(r.idx, K * S) && i32(r.loc, K * S) && i32(r.slot_map, E * r.C) && i32(r.used, E) && K <= 4 && E <= 64);
   TORCH_CHECK(r.gates.is_cuda() && r.gates.scalar_type() == at::kFloat && r.gates.is_contiguous() && r.gates.numel() == K * S);
+  TORCH_CHECK(!r.int8 || (r.postscore && r.C % 32 == 0 && x.size(1) % 128 == 0), "int8 rows: post-score, 128-column groups, whole slices");
+}
+
+// The expert GEMM whose epilogue writes int8 rows ([E * C, N] bytes and a (scale, low) pair per 128 columns and row) for one
+// rank: the push epilogue with this rank's own memory as the destination, addressed from a base of zero, and a flag that
+// nobody waits for.
+struct Int8Out { Tensor rows, scales; };
+static Int8Out local_gemm_int8(const Tensor& a, const Tensor& w, bool w_mn, const c10::optional<Tensor>& bias, const LocalRoute& r) {
+  const int64_t E = a.size(0), N = w_mn ? w.size(2) : w.size(1);
+  TORCH_CHECK(N % 128 == 0, "int8 rows: 128-column groups");
+  Int8Out out{torch::empty({E * r.C, N}, a.options().dtype(at::kByte)),
+              torch::empty({N / 128, E * r.C, 2}, a.options().dtype(at::kFloat))};
+  Tensor base = torch::zeros({2}, a.options().dtype(at::kLong));     // the base address, the flag
+  GemmOpts o;
+  o.epilogue = kEpiPush; o.budget_ms = r.budget_ms; o.status_ptr = r.status_ptr; o.bias = bias;
+  o.heap_bases_ptr = reinterpret_cast<int64_t>(base.data_ptr());
+  o.heap_bases_host = {0};
+  o.push_flag_off = o.heap_bases_ptr + 8;
+  o.push_data_off = reinterpret_cast<int64_t>(out.rows.data_ptr());
+  o.push_scale_off = reinterpret_cast<int64_t>(out.scales.data_ptr());
+  o.push_q8 = 1; o.push_rows = o.push_C = r.C; o.chunk_groups = E;
+  grouped_gemm_op(a, false, w, w_mn, o);
+  return out;
 }
 
 static GemmOpts local_opts(const LocalRoute& r, int64_t epilogue) {
@@ -604,8 +627,8 @@ static GemmOpts local_opts(const LocalRoute& r, int64_t epilogue) {
   return o;
 }
 
-// {y [S, O], xs [E, C, M], dact [E, C, H], h [E, C, H], ys [E, C, O]}; without `want_grad` no derivative is saved (dact
-// is empty)
+// {y [S, O], xs [E, C, M], dact [E, C, H], h [E, C, H], ys [E, C, O], scales}; without `want_grad` no derivative is saved
+// (dact is empty); with int8 rows ys is [E * C, O] bytes and has scales
 std::vector<Tensor> local_forward_op(const Tensor& x, const LocalRoute& r, const Tensor& w1, const Tensor& b1, const Tensor& w2,
                                      const Tensor& b2, bool want_grad, const py::object& stages) {
   local_check(x, r, w1);
@@ -616,8 +639,9 @@ std::vector<Tensor> local_forward_op(const Tensor& x, const LocalRoute& r, const
     Stage st(stages, "fwd.slots");
     count_launch(1);
     launch_slots_fill(x.data_ptr(), r.slot_map.data_ptr<int>(), r.postscore ? nullptr : r.gates.data_ptr<float>(),
-                      r.used.data_ptr<int>(), xs.data_ptr(), K, S, M, E, C, cur_stream());
+                      r.used.data_ptr<int>(), xs.data_ptr(), K, S, M, E, C, r.int8, cur_stream());
   }
+  Tensor scales;
   {
     Stage st(stages, "fwd.gemm1");
     GemmOpts o = local_opts(r, kEpiBiasAct);
@@ -627,18 +651,24 @@ std::vector<Tensor> local_forward_op(const Tensor& x, const LocalRoute& r, const
   }
   {
     Stage st(stages, "fwd.gemm2");
-    GemmOpts o = local_opts(r, kEpiStore);
-    o.bias = b2;
-    ys = grouped_gemm_op(h, false, w2, true, o);
+    if (r.int8) {
+      const Int8Out q = local_gemm_int8(h, w2, true, b2, r);
+      ys = q.rows; scales = q.scales;
+    } else {
+      GemmOpts o = local_opts(r, kEpiStore);
+      o.bias = b2;
+      ys = grouped_gemm_op(h, false, w2, true, o);
+    }
   }
   {
     Stage st(stages, "fwd.combine");
     count_launch(1);
-    launch_gather_rows<__nv_bfloat16>(ys.data_ptr(), nullptr, r.idx.data_ptr<int>(), r.loc.data_ptr<int>(),
-                                      r.postscore ? r.gates.data_ptr<float>() : nullptr,
-                                      reinterpret_cast<__nv_bfloat16*>(y.data_ptr()), K, S, O, C, nullptr, cur_stream());
+    launch_gather_rows<__nv_bfloat16>(ys.data_ptr(), r.int8 ? scales.data_ptr<float>() : nullptr, r.idx.data_ptr<int>(),
+                                      r.loc.data_ptr<int>(), r.postscore ? r.gates.data_ptr<float>() : nullptr,
+                                      reinterpret_cast<__nv_bfloat16*>(y.data_ptr()), K, S, O, C, nullptr, cur_stream(),
+                                      r.int8 ? E * C : 0);
   }
-  return {y, xs, dact, h, ys};
+  return {y, xs, dact, h, ys, scales};
 }
 
 // The linear gate of a pass: logits fp32 [S, E] and what its backward needs.
@@ -671,7 +701,8 @@ static Tensor local_gate_backward(const LocalGate& g, const LocalRoute& r, const
 // gate's part in it, without it the gradient of the gates.  `need`: which of x, (gates or wg), w1, b1, w2, b2 are asked for.
 static std::vector<Tensor> local_backward(const Tensor& dy, const Tensor& x, const LocalRoute& r, const Tensor& w1,
                                           const Tensor& w2, const Tensor& xs, const Tensor& dact, const Tensor& h,
-                                          const Tensor& ys, const std::vector<bool>& need, const LocalGate* gate,
+                                          const Tensor& ys, const c10::optional<Tensor>& scales,
+                                          const std::vector<bool>& need, const LocalGate* gate,
                                           const c10::optional<Tensor>& dl_aux, const py::object& stages) {
   local_check(x, r, w1);
   c10::cuda::CUDAGuard guard(x.device());
@@ -681,15 +712,18 @@ static std::vector<Tensor> local_backward(const Tensor& dy, const Tensor& x, con
   const int *idx = r.idx.data_ptr<int>(), *loc = r.loc.data_ptr<int>(), *used = r.used.data_ptr<int>();
   const float* gates = r.gates.data_ptr<float>();
   Tensor dgates = torch::empty({K, S}, r.gates.options()), dys = torch::empty({E, C, O}, x.options());
-  Tensor dx, dh, dxs, dl, dwg, dw1, dw2, db1, db2;
+  Tensor dx, dh, dxs, dx_scales, dl, dwg, dw1, dw2, db1, db2;
   {
     Stage st(stages, "bwd.gate_grad");
     count_launch(1);
-    if (r.postscore)
+    if (r.int8)
+      launch_slots_gate_grad_q8(ys.data_ptr(), scales->data_ptr<float>(), dyp, idx, loc, gates, used, dgates.data_ptr<float>(),
+                                dys.data_ptr(), K, S, O, E, C, cur_stream());
+    else if (r.postscore)
       launch_slots_gate_grad(ys.data_ptr(), dyp, idx, loc, gates, used, dgates.data_ptr<float>(), dys.data_ptr(), K, S, O, E, C,
                              cur_stream());
     else
-      launch_slots_fill(dyp, r.slot_map.data_ptr<int>(), nullptr, used, dys.data_ptr(), K, S, O, E, C, cur_stream());
+      launch_slots_fill(dyp, r.slot_map.data_ptr<int>(), nullptr, used, dys.data_ptr(), K, S, O, E, C, false, cur_stream());
     if (gate != nullptr && r.postscore) dl = local_gate_backward(*gate, r, dgates, dl_aux);
   }
   {
@@ -701,7 +735,12 @@ static std::vector<Tensor> local_backward(const Tensor& dy, const Tensor& x, con
   const bool gate_from_dx = !r.postscore && (need[1] || gate != nullptr);
   if (need[0] || gate_from_dx) {
     Stage st(stages, "bwd.dgrad1");               // dX slots = dH . W1^T
-    dxs = grouped_gemm_op(dh, false, w1, false, local_opts(r, kEpiStore));
+    if (r.int8) {
+      const Int8Out q = local_gemm_int8(dh, w1, false, c10::nullopt, r);
+      dxs = q.rows; dx_scales = q.scales;
+    } else {
+      dxs = grouped_gemm_op(dh, false, w1, false, local_opts(r, kEpiStore));
+    }
   }
   {
     Stage st(stages, "bwd.dispatch");
@@ -716,11 +755,12 @@ static std::vector<Tensor> local_backward(const Tensor& dy, const Tensor& x, con
       dx = torch::empty_like(x);
       count_launch(1);
       if (gate != nullptr)
-        launch_gather_gate(dxs.data_ptr(), idx, loc, r.postscore ? nullptr : gates, dl.data_ptr<float>(), gate->w.data_ptr(),
+        launch_gather_gate(dxs.data_ptr(), r.int8 ? dx_scales.data_ptr<float>() : nullptr, idx, loc, r.postscore ? nullptr : gates, dl.data_ptr<float>(), gate->w.data_ptr(),
                            gate->w.scalar_type() == at::kBFloat16, dx.data_ptr(), K, S, M, E, C, cur_stream());
       else
-        launch_gather_rows<__nv_bfloat16>(dxs.data_ptr(), nullptr, idx, loc, r.postscore ? nullptr : gates,
-                                          reinterpret_cast<__nv_bfloat16*>(dx.data_ptr()), K, S, M, C, nullptr, cur_stream());
+        launch_gather_rows<__nv_bfloat16>(dxs.data_ptr(), r.int8 ? dx_scales.data_ptr<float>() : nullptr, idx, loc,
+                                          r.postscore ? nullptr : gates, reinterpret_cast<__nv_bfloat16*>(dx.data_ptr()), K, S,
+                                          M, C, nullptr, cur_stream(), r.int8 ? E * C : 0);
     }
   }
   if (need[4]) {
@@ -763,16 +803,17 @@ static std::vector<Tensor> local_backward(const Tensor& dy, const Tensor& x, con
 
 std::vector<Tensor> local_backward_op(const Tensor& dy, const Tensor& x, const LocalRoute& r, const Tensor& w1, const Tensor& w2,
                                       const Tensor& xs, const Tensor& dact, const Tensor& h, const Tensor& ys,
-                                      const std::vector<bool>& need, const py::object& stages) {
-  return local_backward(dy, x, r, w1, w2, xs, dact, h, ys, need, nullptr, c10::nullopt, stages);
+                                      const c10::optional<Tensor>& scales, const std::vector<bool>& need,
+                                      const py::object& stages) {
+  return local_backward(dy, x, r, w1, w2, xs, dact, h, ys, scales, need, nullptr, c10::nullopt, stages);
 }
 
 // The whole layer with a linear gate `wg` [E, M].  capacity < 0: as many slots as the busiest expert needs, rounded up by
-// `round_up` (one host read).  Returns {y, l_aux, logits, top1, slot_map, used, idx, loc, gates, xs, dact, h, ys} and the
-// capacity.
+// `round_up` (one host read).  Returns {y, l_aux, logits, top1, slot_map, used, idx, loc, gates, xs, dact, h, ys, scales} and
+// the capacity.
 std::tuple<std::vector<Tensor>, int64_t> local_moe_forward_op(
     const Tensor& x, const Tensor& wg, const Tensor& w1, const Tensor& b1, const Tensor& w2, const Tensor& b2, int64_t K,
-    int64_t capacity, const py::object& round_up, bool normalize, bool bf16_logits, bool prio, int64_t act, bool postscore,
+    int64_t capacity, const py::object& round_up, bool normalize, bool bf16_logits, bool prio, int64_t act, bool postscore, bool int8,
     int64_t budget_ms, int64_t status_ptr, bool want_grad, const py::object& stages) {
   TORCH_CHECK(x.is_cuda() && x.dim() == 2 && x.scalar_type() == at::kBFloat16);
   const int64_t S = x.size(0), M = x.size(1), E = w1.size(0);
@@ -785,7 +826,7 @@ std::tuple<std::vector<Tensor>, int64_t> local_moe_forward_op(
   auto fopt = x.options().dtype(at::kFloat);
   const int64_t nblk = gate_workspace_blocks(S);
   LocalRoute r{torch::empty({K, S}, iopt), torch::empty({K, S}, iopt), {}, {}, torch::empty({K, S}, fopt), capacity, act,
-               postscore, budget_ms, status_ptr};
+               postscore, int8, budget_ms, status_ptr};
   Tensor logits = torch::empty({S, E}, fopt), counts = torch::empty({2, E}, iopt);
   Tensor laux = torch::empty({}, fopt), laux_bf16;
   if (bf16_logits) laux_bf16 = torch::empty({}, x.options());
@@ -832,16 +873,16 @@ std::tuple<std::vector<Tensor>, int64_t> local_moe_forward_op(
   r.used = counts[1];
   std::vector<Tensor> e = local_forward_op(x, r, w1, b1, w2, b2, want_grad, stages);
   return {{e[0], bf16_logits ? laux_bf16 : laux, logits, counts[0], r.slot_map, r.used, r.idx, r.loc, r.gates, e[1], e[2], e[3],
-           e[4]}, r.C};
+           e[4], e[5]}, r.C};
 }
 
 std::vector<Tensor> local_moe_backward_op(const Tensor& dy, const c10::optional<Tensor>& dl_aux, const Tensor& x, const Tensor& wg,
                                           const LocalRoute& r, const Tensor& w1, const Tensor& w2, const Tensor& logits,
                                           const Tensor& top1, const Tensor& xs, const Tensor& dact, const Tensor& h,
-                                          const Tensor& ys, bool normalize, bool bf16_logits, const std::vector<bool>& need,
-                                          const py::object& stages) {
+                                          const Tensor& ys, const c10::optional<Tensor>& scales, bool normalize,
+                                          bool bf16_logits, const std::vector<bool>& need, const py::object& stages) {
   const LocalGate g{wg, logits, top1, normalize, bf16_logits};
-  return local_backward(dy, x, r, w1, w2, xs, dact, h, ys, need, &g, dl_aux, stages);
+  return local_backward(dy, x, r, w1, w2, xs, dact, h, ys, scales, need, &g, dl_aux, stages);
 }
 
 // rows [R, M] -> uint8 [R, M + 16]: M quantised bytes + {scale, low, 0, 0} (the wire rows of the fused send)
@@ -1061,8 +1102,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gate_forward_used", &gate_forward_used_op);
   py::class_<LocalRoute>(m, "LocalRoute")
       .def(py::init([](Tensor idx, Tensor loc, Tensor slot_map, Tensor used, Tensor gates, int64_t C, int64_t act, bool postscore,
-                       int64_t budget_ms, int64_t status_ptr) {
-        return LocalRoute{idx, loc, slot_map, used, gates, C, act, postscore, budget_ms, status_ptr};
+                       bool int8, int64_t budget_ms, int64_t status_ptr) {
+        return LocalRoute{idx, loc, slot_map, used, gates, C, act, postscore, int8, budget_ms, status_ptr};
       }));
   m.def("local_forward", &local_forward_op);
   m.def("local_backward", &local_backward_op);

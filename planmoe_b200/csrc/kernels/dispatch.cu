@@ -455,8 +455,28 @@ __device__ __forceinline__ int slots_end(int used, int C) {
 }
 constexpr int kRowUnroll = 4;                      // 16-byte loads a lane has in flight per row
 
+// What a row is after it has travelled as int8: 255 steps between its lowest and its highest value (the wire rows of
+// int8_rows_encode and their expansion in front of the GEMM, with the same roundings).
+struct Int8Row {
+  float lo, inv, scale;
+  __device__ Int8Row(const uint4* row, int nvec, int lane) {
+    float l = INFINITY, h = -INFINITY;
+    for (int v = lane; v < nvec; v += 32) {
+      const uint4 raw = __ldg(row + v);
+      const Pack<__nv_bfloat16> p = *reinterpret_cast<const Pack<__nv_bfloat16>*>(&raw);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) { const float f = __bfloat162float(p.v[i]); l = fminf(l, f); h = fmaxf(h, f); }
+    }
+    lo = warp_min(l);
+    const float range = warp_max(h) - lo;
+    inv = range > 0.f ? 255.f / range : 0.f;
+    scale = range;
+  }
+  __device__ float step(float f) const { return fminf(fmaxf(rintf((f - lo) * inv), 0.f), 255.f); }
+};
+
 // One warp per slot.  Bound by memory: 34 MB read and 67 MB written for 8192 tokens of 2048, top-2.
-template <bool SCALE>
+template <bool SCALE, bool Q8>
 __global__ void __launch_bounds__(kRowThreads)
 slots_fill_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ slot_map, const float* __restrict__ gates,
                   const int* __restrict__ used, __nv_bfloat16* __restrict__ out, int K, int S, int M, int E, int C) {
@@ -476,6 +496,18 @@ slots_fill_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ s
     const int t = owner / K;
     const uint4* src = reinterpret_cast<const uint4*>(x + (long long)t * M);
     const float gw = SCALE ? gates[(size_t)(owner - t * K) * S + t] : 1.f;
+    if constexpr (Q8) {
+      const Int8Row row(src, nvec, lane);
+      const float scale = row.scale * (1.f / 255.f);
+      for (int v = lane; v < nvec; v += 32) {
+        uint4 raw = __ldg(src + v);
+        Pack<__nv_bfloat16> q = *reinterpret_cast<Pack<__nv_bfloat16>*>(&raw);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) q.v[j] = __float2bfloat16_rn(fmaf(row.step(__bfloat162float(q.v[j])), scale, row.lo));
+        dst[v] = *reinterpret_cast<uint4*>(&q);
+      }
+      continue;
+    }
     for (int v0 = lane; v0 < nvec; v0 += 32 * kRowUnroll) {
       uint4 raw[kRowUnroll];
 #pragma unroll
@@ -570,6 +602,61 @@ slots_gate_grad_kernel(const __nv_bfloat16* __restrict__ disp, const __nv_bfloat
   }
 }
 
+// The same for int8 transfers: expert outputs as uint8 rows with a (scale, low) pair per 128 columns and row ([M / 128][E *
+// C] pairs), the weighted dy rows as int8 would deliver them.  Gates are not negative, so gate * dy takes the same steps as
+// dy, with range and low scaled.
+__global__ void __launch_bounds__(kRowThreads)
+slots_gate_grad_q8_kernel(const unsigned char* __restrict__ disp, const float2* __restrict__ disp_scales,
+                          const __nv_bfloat16* __restrict__ dy, const int* __restrict__ idx, const int* __restrict__ loc,
+                          const float* __restrict__ gates, const int* __restrict__ used, float* __restrict__ dgates,
+                          __nv_bfloat16* __restrict__ ddisp, int K, int S, int M, int E, int C) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nvec = M / 8;
+  const long long items = (long long)S + (long long)E * kSlotBlock, slots = (long long)E * C;
+  for (long long it = (long long)blockIdx.x * kRowWarps + warp; it < items; it += (long long)gridDim.x * kRowWarps) {
+    if (it >= S) {
+      const int q = (int)(it - S), e = q / kSlotBlock;
+      const int n = used[e], c = n + (q - e * kSlotBlock);
+      if (c >= slots_end(n, C)) continue;
+      uint4* dst = reinterpret_cast<uint4*>(ddisp + ((long long)e * C + c) * M);
+      for (int v = lane; v < nvec; v += 32) dst[v] = make_uint4(0, 0, 0, 0);
+      continue;
+    }
+    const int t = (int)it;
+    const uint4* b = reinterpret_cast<const uint4*>(dy + (long long)t * M);
+    const Int8Row row(b, nvec, lane);
+    for (int k = 0; k < K; ++k) {
+      const int e = idx[(size_t)k * S + t], l = loc[(size_t)k * S + t];
+      float acc = 0.f;
+      if (e >= 0 && l >= 0 && l < C) {
+        const long long slot = (long long)e * C + l;
+        const float gw = gates[(size_t)k * S + t];
+        const float scale = gw * row.scale * (1.f / 255.f), low = gw * row.lo;
+        const uint2* a = reinterpret_cast<const uint2*>(disp + slot * M);
+        uint4* dst = reinterpret_cast<uint4*>(ddisp + slot * M);
+#pragma unroll 2
+        for (int v = lane; v < nvec; v += 32) {
+          const uint4 raw = __ldg(b + v);
+          const uint2 q = __ldg(a + v);
+          const float2 sl = __ldg(disp_scales + (size_t)(v >> 4) * slots + slot);
+          const Pack<__nv_bfloat16> pb = *reinterpret_cast<const Pack<__nv_bfloat16>*>(&raw);
+          Pack<__nv_bfloat16> o;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const float fb = __bfloat162float(pb.v[j]);
+            const float fa = (float)(((j < 4 ? q.x : q.y) >> (8 * (j & 3))) & 0xffu);
+            acc += fmaf(sl.x, fa, sl.y) * fb;
+            o.v[j] = __float2bfloat16_rn(fmaf(row.step(fb), scale, low));
+          }
+          dst[v] = *reinterpret_cast<const uint4*>(&o);
+        }
+      }
+      acc = warp_sum(acc);
+      if (lane == 0) dgates[(size_t)k * S + t] = acc;
+    }
+  }
+}
+
 unsigned row_grid(long long rows) {
   const long long ctas = (rows + kRowWarps - 1) / kRowWarps;
   return (unsigned)(ctas < 1 ? 1 : ctas > 148 * 8 ? 148 * 8 : ctas);
@@ -578,10 +665,19 @@ unsigned row_grid(long long rows) {
 }  // namespace
 
 void launch_slots_fill(const void* x, const int* slot_map, const float* gates, const int* used, void* out, int K, int S,
-                       int M, int E, int C, cudaStream_t stream) {
-  auto kern = gates != nullptr ? slots_fill_kernel<true> : slots_fill_kernel<false>;
+                       int M, int E, int C, bool int8, cudaStream_t stream) {
+  auto kern = int8 ? slots_fill_kernel<false, true> : gates != nullptr ? slots_fill_kernel<true, false> : slots_fill_kernel<false, false>;
   kern<<<row_grid((long long)E * C), kRowThreads, 0, stream>>>(reinterpret_cast<const __nv_bfloat16*>(x), slot_map, gates,
                                                                used, reinterpret_cast<__nv_bfloat16*>(out), K, S, M, E, C);
+}
+
+void launch_slots_gate_grad_q8(const void* disp, const float* disp_scales, const void* dy, const int* idx, const int* loc,
+                               const float* gates, const int* used, float* dgates, void* ddisp, int K, int S, int M, int E,
+                               int C, cudaStream_t stream) {
+  slots_gate_grad_q8_kernel<<<row_grid((long long)S + (long long)E * kSlotBlock), kRowThreads, 0, stream>>>(
+      reinterpret_cast<const unsigned char*>(disp), reinterpret_cast<const float2*>(disp_scales),
+      reinterpret_cast<const __nv_bfloat16*>(dy), idx, loc, gates, used, dgates, reinterpret_cast<__nv_bfloat16*>(ddisp), K, S, M,
+      E, C);
 }
 
 void launch_slots_gate_grad(const void* disp, const void* dy, const int* idx, const int* loc, const float* gates,

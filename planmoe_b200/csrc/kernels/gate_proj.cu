@@ -218,11 +218,14 @@ gate_wgrad_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__
 // warp and the slots looked up token by token: 128 us for 16384 x 4096, top-2, 8 experts; 61 of them for the bytes.)
 constexpr int kGatherTokens = 4;                    // 8: 110 us, two blocks per SM
 
-template <int MAXK, bool W_BF16, bool GATED>
+enum GatherForm { kGatherPlain, kGatherGated, kGatherInt8 };
+
+template <int MAXK, bool W_BF16, int FORM>
 __global__ void __launch_bounds__(256, MAXK <= 2 ? 4 : 2)
-gather_gate_kernel(const __nv_bfloat16* __restrict__ slots, const int* __restrict__ idx, const int* __restrict__ loc,
+gather_gate_kernel(const void* __restrict__ slots_, const float2* __restrict__ scales, const int* __restrict__ idx, const int* __restrict__ loc,
                    const float* __restrict__ gates, const float* __restrict__ dl, const void* __restrict__ w_,
                    __nv_bfloat16* __restrict__ dx, int K, int S, int M, int E, int C) {
+  constexpr bool GATED = FORM == kGatherGated, Q8 = FORM == kGatherInt8;
   extern __shared__ __align__(16) float gather_smem[];
   float* w_s = gather_smem;                                                       // [E][256]
   float2* dl_s = reinterpret_cast<float2*>(gather_smem + E * 256);                // [32 tokens][E], pairs {d, d}
@@ -242,14 +245,22 @@ gather_gate_kernel(const __nv_bfloat16* __restrict__ slots, const int* __restric
       if constexpr (GATED) gv = gates[(size_t)k * S + tok];
     }
   }
-  uint4 raw[kGatherTokens][MAXK];
+  uint4 raw[kGatherTokens][MAXK];                 // int8: eight bytes and the pair
 #pragma unroll
   for (int t = 0; t < kGatherTokens; ++t)
 #pragma unroll
     for (int k = 0; k < MAXK; ++k) {
       const long long row = __shfl_sync(0xffffffffu, at, t * MAXK + k);
       raw[t][k] = make_uint4(0, 0, 0, 0);
-      if (row >= 0 && col < M) raw[t][k] = __ldg(reinterpret_cast<const uint4*>(slots + row * M + col));
+      if (row >= 0 && col < M) {
+        if constexpr (Q8) {
+          const uint2 q = __ldg(reinterpret_cast<const uint2*>(reinterpret_cast<const unsigned char*>(slots_) + row * M + col));
+          const float2 sl = __ldg(scales + (size_t)(col >> 7) * ((size_t)E * C) + row);
+          raw[t][k] = make_uint4(q.x, q.y, __float_as_uint(sl.x), __float_as_uint(sl.y));
+        } else {
+          raw[t][k] = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(slots_) + row * M + col));
+        }
+      }
     }
   for (int i = threadIdx.x; i < E * 256; i += 256) {
     const int m = c0 + (i & 255);
@@ -274,7 +285,16 @@ gather_gate_kernel(const __nv_bfloat16* __restrict__ slots, const int* __restric
 #pragma unroll
     for (int k = 0; k < MAXK; ++k) {
       unsigned long long p[4];
-      bf16_pairs(raw[t][k], p);
+      if constexpr (Q8) {                         // a pick without a slot has scale and low zero
+        const unsigned long long sc = pair_const(__uint_as_float(raw[t][k].z)), low = pair_const(__uint_as_float(raw[t][k].w));
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const uint32_t w = (i < 2 ? raw[t][k].x : raw[t][k].y) >> (16 * (i & 1));
+          p[i] = fma_pair(pair_of((float)(w & 0xffu), (float)((w >> 8) & 0xffu)), sc, low);
+        }
+      } else {
+        bf16_pairs(raw[t][k], p);
+      }
       const float gk = GATED ? __shfl_sync(0xffffffffu, gv, t * MAXK + k) : 1.f;
       const unsigned long long gp = pair_of(gk, gk);
 #pragma unroll
@@ -349,20 +369,22 @@ void launch_gate_wgrad(const void* x, const float* dl, float* partial, int S, in
   else gate_wgrad_kernel<16><<<grid, 256, 0, stream>>>(xb, dl, partial, S, E, M, tokens);
 }
 
-void launch_gather_gate(const void* slots, const int* idx, const int* loc, const float* gates, const float* dl, const void* w,
-                        bool w_bf16, void* dx, int K, int S, int M, int E, int C, cudaStream_t stream) {
+void launch_gather_gate(const void* slots, const float* scales, const int* idx, const int* loc, const float* gates,
+                        const float* dl, const void* w, bool w_bf16, void* dx, int K, int S, int M, int E, int C,
+                        cudaStream_t stream) {
   const unsigned grid = (unsigned)((S + 8 * kGatherTokens - 1) / (8 * kGatherTokens)) * (unsigned)((M + 255) / 256);
-  const int smem = E * 256 * (int)sizeof(float) + 8 * kGatherTokens * E * (int)sizeof(float2);      // at most 24 KiB
-  const __nv_bfloat16* sb = reinterpret_cast<const __nv_bfloat16*>(slots);
+  const int smem = E * 256 * (int)sizeof(float) + 8 * kGatherTokens * E * (int)sizeof(float2);      // at most 20 KiB
   __nv_bfloat16* db = reinterpret_cast<__nv_bfloat16*>(dx);
-  auto pick = [&](auto gated) {
-    constexpr bool G = decltype(gated)::value;
-    return K <= 1 ? (w_bf16 ? gather_gate_kernel<1, true, G> : gather_gate_kernel<1, false, G>)
-         : K <= 2 ? (w_bf16 ? gather_gate_kernel<2, true, G> : gather_gate_kernel<2, false, G>)
-                  : (w_bf16 ? gather_gate_kernel<4, true, G> : gather_gate_kernel<4, false, G>);
+  auto pick = [&](auto form) {
+    constexpr int F = decltype(form)::value;
+    return K <= 1 ? (w_bf16 ? gather_gate_kernel<1, true, F> : gather_gate_kernel<1, false, F>)
+         : K <= 2 ? (w_bf16 ? gather_gate_kernel<2, true, F> : gather_gate_kernel<2, false, F>)
+                  : (w_bf16 ? gather_gate_kernel<4, true, F> : gather_gate_kernel<4, false, F>);
   };
-  auto kern = gates != nullptr ? pick(std::true_type{}) : pick(std::false_type{});
-  kern<<<grid, 256, smem, stream>>>(sb, idx, loc, gates, dl, w, db, K, S, M, E, C);
+  auto kern = scales != nullptr ? pick(std::integral_constant<int, kGatherInt8>{})
+            : gates != nullptr  ? pick(std::integral_constant<int, kGatherGated>{})
+                                : pick(std::integral_constant<int, kGatherPlain>{});
+  kern<<<grid, 256, smem, stream>>>(slots, reinterpret_cast<const float2*>(scales), idx, loc, gates, dl, w, db, K, S, M, E, C);
 }
 
 }  // namespace planmoe

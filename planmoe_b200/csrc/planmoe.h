@@ -66,13 +66,19 @@ void launch_gate_grad(const T* disp, const T* dy, const int* idx, const int* loc
 // Of an expert's C slots only the first used[e] hold tokens.  What computes on slots does so in blocks of at most
 // kSlotBlock rows and stops behind the block with the last token; the rows of that block behind it are zeros.
 constexpr int kSlotBlock = 256;
-// out[e * C + c] = (gate *) row of the token that holds the slot
+// out[e * C + c] = (gate *) row of the token that holds the slot; int8 (without gates): the row as an int8 transfer
+// delivers it
 void launch_slots_fill(const void* x, const int* slot_map, const float* gates, const int* used, void* out, int K, int S,
-                       int M, int E, int C, cudaStream_t stream);
+                       int M, int E, int C, bool int8, cudaStream_t stream);
 // dgates[k][t] = <disp[slot_k(t)], dy[t]>, ddisp[slot_k(t)] = gates[k][t] * dy[t]
 void launch_slots_gate_grad(const void* disp, const void* dy, const int* idx, const int* loc, const float* gates,
                             const int* used, float* dgates, void* ddisp, int K, int S, int M, int E, int C,
                             cudaStream_t stream);
+
+// the same with int8 transfers: disp uint8 rows, disp_scales fp32 [M / 128][E * C][2]
+void launch_slots_gate_grad_q8(const void* disp, const float* disp_scales, const void* dy, const int* idx, const int* loc,
+                               const float* gates, const int* used, float* dgates, void* ddisp, int K, int S, int M, int E,
+                               int C, cudaStream_t stream);
 
 // ---- kernels/gate_proj.cu: the linear gate on bf16 tokens [S, M], M % 32 == 0, at most kProjMaxE experts ----
 // `w`: [E, M], fp32 or bf16.  logits fp32, rounded to bf16 values if asked for.
@@ -82,8 +88,9 @@ void launch_gate_project(const void* x, const void* w, bool w_bf16, float* logit
 // partial: gate_wgrad_chunks(S, M) rows of [E, M] fp32, to be added up (launch_colsum_jobs)
 int gate_wgrad_chunks(int S, int M);
 void launch_gate_wgrad(const void* x, const float* dl, float* partial, int S, int E, int M, cudaStream_t stream);
-// dx[t] = sum_k (gates[k][t] *) slots[slot_k(t)] + sum_e dl[t][e] * w[e]
-void launch_gather_gate(const void* slots, const int* idx, const int* loc, const float* gates, const float* dl, const void* w,
+// dx[t] = sum_k (gates[k][t] *) slots[slot_k(t)] + sum_e dl[t][e] * w[e]; with `scales` the slots are uint8 rows with a
+// (scale, low) pair per 128 columns and row, [M / 128][E * C] pairs (without gates)
+void launch_gather_gate(const void* slots, const float* scales, const int* idx, const int* loc, const float* gates, const float* dl, const void* w,
                         bool w_bf16, void* dx, int K, int S, int M, int E, int C, cudaStream_t stream);
 
 // ---- kernels/gate.cu -------------------------------------------------------------------------

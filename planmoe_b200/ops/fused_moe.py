@@ -452,10 +452,11 @@ class _FusedExperts(torch.autograd.Function):
         return dx, dgates, dw1, db1, dw2, db2, None
 
 
-def _local_path(tr, q8):
-    """Whether a layer's experts run without the exchange: one rank and bf16 rows.  PLANMOE_LOCAL=0, a choice of the send's
-    form (PLANMOE_FUSE_SEND), the debug guards and the role trace keep the exchange, which is what they are about."""
-    return tr.world == 1 and not tr.emulated and not q8 and native.lib().local_by_env()
+def _local_path(tr, q8, capacity):
+    """Whether a layer's experts run without the exchange: one rank.  The GEMM epilogue that writes int8 rows does so in
+    slices of 32 (a capacity that is sized to the busiest expert, -1, is a multiple of 64).  PLANMOE_LOCAL=0, a choice of the
+    send's form (PLANMOE_FUSE_SEND), the debug guards and the role trace keep the exchange, which is what they are about."""
+    return tr.world == 1 and not tr.emulated and not (q8 and capacity > 0 and capacity % 32) and native.lib().local_by_env()
 
 
 def _aligned(t):
@@ -474,23 +475,23 @@ class _LocalExperts(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, gates, w1, b1, w2, b2, meta):
-        y, xs, dact, h, ys = _local_forward(x, gates, w1, b1, w2, b2, meta, True)
-        ctx.save_for_backward(x, gates, w1, w2, xs, dact, h, ys, meta['idx'], meta['loc'], meta['slot_map'], meta['used'])
-        ctx.meta = {k: meta[k] for k in ('C', 'act', 'postscore', 'budget_ms', 'status')}
+        y, xs, dact, h, ys, scales = _local_forward(x, gates, w1, b1, w2, b2, meta, True)
+        ctx.save_for_backward(x, gates, w1, w2, xs, dact, h, ys, scales, meta['idx'], meta['loc'], meta['slot_map'], meta['used'])
+        ctx.meta = {k: meta[k] for k in ('C', 'act', 'postscore', 'int8', 'budget_ms', 'status')}
         return y
 
     @staticmethod
     def backward(ctx, dy):
-        x, gates, w1, w2, xs, dact, h, ys, idx, loc, slot_map, used = ctx.saved_tensors
+        x, gates, w1, w2, xs, dact, h, ys, scales, idx, loc, slot_map, used = ctx.saved_tensors
         route = _local_route(gates, dict(ctx.meta, idx=idx, loc=loc, slot_map=slot_map, used=used))
         dx, dgates, dw1, db1, dw2, db2 = native.lib().local_backward(
-            _aligned(dy), x, route, w1, w2, xs, dact, h, ys, list(ctx.needs_input_grad[:6]), _stages())
+            _aligned(dy), x, route, w1, w2, xs, dact, h, ys, scales, list(ctx.needs_input_grad[:6]), _stages())
         return dx, dgates, dw1, db1, dw2, db2, None
 
 
 def _local_route(gates, m):
     return native.lib().LocalRoute(m['idx'], m['loc'], m['slot_map'], m['used'], gates, m['C'], m['act'], m['postscore'],
-                                   m['budget_ms'], m['status'].device_ptr())
+                                   m['int8'], m['budget_ms'], m['status'].device_ptr())
 
 
 def _local_forward(x, gates, w1, b1, w2, b2, meta, want_grad):
@@ -514,25 +515,25 @@ class _LocalLayer(torch.autograd.Function):
         (y, l_aux, *saved), m['capacity'] = _local_layer_forward(x, wg, w1, b1, w2, b2, m, True)
         m['routing'] = saved[4], saved[5]
         ctx.save_for_backward(x, wg, w1, w2, *saved)
-        ctx.m = {k: m[k] for k in ('capacity', 'act', 'postscore', 'normalize', 'bf16_logits', 'budget_ms', 'status')}
+        ctx.m = {k: m[k] for k in ('capacity', 'act', 'postscore', 'int8', 'normalize', 'bf16_logits', 'budget_ms', 'status')}
         return y, l_aux
 
     @staticmethod
     def backward(ctx, dy, dl_aux):
-        x, wg, w1, w2, logits, top1, slot_map, used, idx, loc, gates, xs, dact, h, ys = ctx.saved_tensors
+        x, wg, w1, w2, logits, top1, slot_map, used, idx, loc, gates, xs, dact, h, ys, scales = ctx.saved_tensors
         m = ctx.m
         if dy is None:
             dy = torch.zeros((x.size(0), w2.size(2)), dtype=x.dtype, device=x.device)
         route = _local_route(gates, dict(m, C=m['capacity'], idx=idx, loc=loc, slot_map=slot_map, used=used))
         return (*native.lib().local_moe_backward(_aligned(dy), dl_aux, x, wg, route, w1, w2, logits, top1, xs, dact, h, ys,
-                                                 m['normalize'], m['bf16_logits'], list(ctx.needs_input_grad[:6]), _stages()),
+                                                 scales, m['normalize'], m['bf16_logits'], list(ctx.needs_input_grad[:6]), _stages()),
                 None)
 
 
 def _local_layer_forward(x, wg, w1, b1, w2, b2, m, want_grad):
     return native.lib().local_moe_forward(x, wg, w1, b1, w2, b2, m['K'], m['capacity'], m['round_up'], m['normalize'],
-                                          m['bf16_logits'], m['prio'], m['act'], m['postscore'], m['budget_ms'],
-                                          m['status'].device_ptr(), want_grad, _stages())
+                                          m['bf16_logits'], m['prio'], m['act'], m['postscore'], m['int8'],
+                                          m['budget_ms'], m['status'].device_ptr(), want_grad, _stages())
 
 
 def _unhooked(module, cls):
@@ -561,7 +562,8 @@ def _local_layer(layer, st, x, gctx, top_k, capacity, align):
     ex, w = layer.experts, gctx.wg.weight
     m = dict(K=top_k, capacity=capacity, round_up=lambda peak: _capacity_step(peak, align), normalize=layer.normalize_gate,
              bf16_logits=not gctx.fp32_gate, prio=layer.batch_prioritized_routing, act=ACT_CODES[ex.act_name],
-             postscore=layer.is_postscore, budget_ms=st.tr.budget_ms, status=st.tr.status)
+             postscore=layer.is_postscore, int8=layer.compress_name == 'int8', budget_ms=st.tr.budget_ms,
+             status=st.tr.status)
     args = (_aligned(x), w, ex.batched_fc1_w, ex.batched_fc1_bias, ex.batched_fc2_w, ex.batched_fc2_bias)
     if torch.is_grad_enabled() and any(t.requires_grad for t in args):
         y, l_aux = _LocalLayer.apply(*args, m)
@@ -644,7 +646,7 @@ def forward(layer, x, gctx, top_k, capacity_factor, degree):
         capacity = max(capacity, 1)
         capacity += -capacity % align
     q8 = layer.compress_name == 'int8'
-    if _local_path(st.tr, q8) and _linear_gate(layer, gctx, x):
+    if _local_path(st.tr, q8, capacity) and _linear_gate(layer, gctx, x):
         y, l_aux, capacity, (idx, loc) = _local_layer(layer, st, x, gctx, top_k, capacity, align)
         _note_stats(layer, st, q8, idx, loc, E, capacity, degree, x)
         return y, l_aux
@@ -678,9 +680,9 @@ def forward(layer, x, gctx, top_k, capacity_factor, degree):
         check_routing_bounds(idx, loc, slot_map, S, E, capacity, top_k)
     ex = layer.experts
     args = (gates, ex.batched_fc1_w, ex.batched_fc1_bias, ex.batched_fc2_w, ex.batched_fc2_bias)
-    if _local_path(st.tr, q8):
+    if _local_path(st.tr, q8, capacity):
         y = _local_experts(x, *args, dict(idx=idx, loc=loc, slot_map=slot_map, used=used, C=capacity,
-                                          act=ACT_CODES[ex.act_name], postscore=layer.is_postscore,
+                                          act=ACT_CODES[ex.act_name], postscore=layer.is_postscore, int8=q8,
                                           budget_ms=st.tr.budget_ms, status=st.tr.status))
     else:
         meta = dict(state=st, idx=idx, loc=loc, slot_map=slot_map, E=E, C=capacity, degree=degree, K=top_k,

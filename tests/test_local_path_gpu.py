@@ -132,7 +132,7 @@ def test_projection_is_at_fp32_precision(S, E, M):
     from planmoe_b200.parallel import transport
     tr = transport.get_transport(layer.group)
     out, _cap = native.lib().local_moe_forward(x, w, ex.batched_fc1_w, ex.batched_fc1_bias, ex.batched_fc2_w, ex.batched_fc2_bias,
-                                               1, 4 * S, None, True, False, False, 1, True, tr.budget_ms,
+                                               1, 4 * S, None, True, False, False, 1, True, False, tr.budget_ms,
                                                tr.status.device_ptr(), True, None)
     logits = out[2].double()
     ref = x.double() @ w.detach().double().t()
@@ -157,3 +157,18 @@ def test_priority_order_is_a_permutation_whatever_the_scores():
         assert bool((ordered[:-1] >= ordered[1:] - 2e-7).all())
         tied = rank[: S // 3]
         assert bool((tied[1:] > tied[:-1]).all())          # equal keys: token order
+
+
+@pytest.mark.parametrize('S,E,k,cf', [(32, 1, 1, 1.0), (768, 3, 2, 1.0), (1000, 5, 2, 0.0), (2048, 32, 2, 1.0)])
+def test_int8_rows_match_the_exchange(S, E, k, cf, monkeypatch):
+    """Rows quantised and expanded where the slots are filled against wire rows, landing buffer and de-quantiser role."""
+    layer = _layer(E, 256, 384, k, cf, compress_name='int8')
+    torch.manual_seed(9)
+    x = torch.randn(S, 256, device='cuda').bfloat16()
+    x[S // 3] = 0.5                                       # a constant row has no range
+    dy = torch.randn(S, 256, device='cuda').bfloat16()
+    here = _pass(layer, x, dy)
+    assert layer.last_stats['wire'] == 'int8'
+    if layer.last_stats['capacity'] % 32 == 0:
+        monkeypatch.setenv('PLANMOE_LOCAL', '0')
+        _close(here, _pass(layer, x, dy))
