@@ -115,7 +115,7 @@ Tensor build_slot_map_op(const Tensor& idx, const Tensor& loc, int64_t E, int64_
 }
 
 Tensor dispatch_scatter_op(const Tensor& x, const Tensor& slot_map, const c10::optional<Tensor>& gates, int64_t K,
-                           int64_t n_slots) {
+                           int64_t n_slots, bool round_gates) {
   count_launch(1);
   TORCH_CHECK(x.is_cuda() && x.dim() == 2 && x.is_contiguous(), "x must be contiguous [S, M] on CUDA");
   const int S = x.size(0), M = x.size(1);
@@ -125,13 +125,13 @@ Tensor dispatch_scatter_op(const Tensor& x, const Tensor& slot_map, const c10::o
   DISPATCH_FLOAT(x, "dispatch_scatter", [&] {
     launch_scatter_rows<scalar_t>(reinterpret_cast<const scalar_t*>(x.data_ptr()), slot_map.data_ptr<int>(),
                                   opt_f32(gates), reinterpret_cast<scalar_t*>(out.data_ptr()), K, S, M, 1, n_slots,
-                                  nullptr, false, cur_stream());
+                                  nullptr, false, cur_stream(), round_gates);
   });
   return out;
 }
 
 Tensor dispatch_gather_op(const Tensor& disp, const Tensor& idx, const Tensor& loc, const c10::optional<Tensor>& gates,
-                          int64_t C) {
+                          int64_t C, bool round_gates) {
   count_launch(1);
   TORCH_CHECK(disp.is_cuda() && disp.dim() == 2 && disp.is_contiguous());
   const int K = idx.size(0), S = idx.size(1), M = disp.size(1);
@@ -141,7 +141,7 @@ Tensor dispatch_gather_op(const Tensor& disp, const Tensor& idx, const Tensor& l
   Tensor out = torch::empty({S, M}, disp.options());
   DISPATCH_FLOAT(disp, "dispatch_gather", [&] {
     launch_gather_rows<scalar_t>(disp.data_ptr(), nullptr, idx.data_ptr<int>(), loc.data_ptr<int>(), opt_f32(gates),
-                                 reinterpret_cast<scalar_t*>(out.data_ptr()), K, S, M, C, nullptr, cur_stream());
+                                 reinterpret_cast<scalar_t*>(out.data_ptr()), K, S, M, C, nullptr, cur_stream(), 0, round_gates);
   });
   return out;
 }
@@ -299,9 +299,13 @@ std::vector<Tensor> route_scores_op(const Tensor& scores, int64_t K, int64_t C, 
   Tensor ws = torch::empty({2 * K * S + (K + 1) * nblk * E}, iopt);
   int* w = ws.data_ptr<int>();
   std::vector<Tensor> out{idx, loc, smap, top1, loss};
+  // the picks' gates are tensors of their own (no views of one another) on consecutive rows of one storage, so that who
+  // wants them stacked need not copy
   GatePtrs gp{};
+  const Tensor rows = torch::empty({K, S}, scores.options());
   for (int k = 0; k < K; ++k) {
-    out.push_back(torch::empty({S}, scores.options()));
+    out.push_back(torch::empty({0}, scores.options()));
+    out.back().set_(rows.storage(), k * S, {S}, {1});
     gp.p[k] = out.back().data_ptr<float>();
   }
   launch_gate_forward<float, true>(scores.data_ptr<float>(), S, E, K, C, normalize, kFloatEps, idx.data_ptr<int>(),
@@ -1093,8 +1097,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("cpu_gather", &cpu_gather_op);
   m.def("cpu_gate_grad", &cpu_gate_grad_op);
   m.def("build_slot_map", &build_slot_map_op);
-  m.def("dispatch_scatter", &dispatch_scatter_op);
-  m.def("dispatch_gather", &dispatch_gather_op);
+  m.def("dispatch_scatter", &dispatch_scatter_op, py::arg("x"), py::arg("slot_map"), py::arg("gates"), py::arg("K"),
+        py::arg("n_slots"), py::arg("round_gates") = false);
+  m.def("dispatch_gather", &dispatch_gather_op, py::arg("disp"), py::arg("idx"), py::arg("loc"), py::arg("gates"), py::arg("C"),
+        py::arg("round_gates") = false);
   m.def("dispatch_gate_grad", &dispatch_gate_grad_op);
   m.def("dispatch_gate_grad_scaled", &dispatch_gate_grad_scaled_op);
   m.def("dispatch_gate_grad_q8", &dispatch_gate_grad_q8_op);

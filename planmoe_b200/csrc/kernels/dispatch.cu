@@ -56,7 +56,7 @@ template <class T, bool QUANT>
 __global__ void __launch_bounds__(kRowThreads, 6)
 scatter_rows_kernel(const T* __restrict__ x, const int* __restrict__ slot_map,
                     const float* __restrict__ gates, T* __restrict__ local_out, int K, int S,
-                    int M, PushGeom g) {
+                    int M, PushGeom g, bool round_gates) {
   // 1-D persistent grid.  Chunks are served in order (chunk 0 leaves first for every destination),
   // destinations start at my right-hand neighbour so that ranks do not all hit the same peer at once.
   // After a chunk has been stored for all destinations the CTA fences once and adds one arrival to the
@@ -102,7 +102,8 @@ scatter_rows_kernel(const T* __restrict__ x, const int* __restrict__ slot_map,
         if (gates == nullptr) {
           for (int v = lane; v < nvec; v += 32) st16(dst + v * V, ld16(src + v * V));
         } else {
-          const float gw = gates[(size_t)k * S + t];
+          float gw = gates[(size_t)k * S + t];
+          if (round_gates) gw = to_f32(from_f32<T>(gw));
           for (int v = lane; v < nvec; v += 32) {
             Pack<T> p = ld16(src + v * V);
 #pragma unroll
@@ -170,7 +171,7 @@ scatter_rows_kernel(const T* __restrict__ x, const int* __restrict__ slot_map,
 template <class T>
 void launch_scatter_rows(const T* x, const int* slot_map, const float* gates, T* local_out, int K,
                          int S, int M, int E, int C, const PushArgs* push, bool quant,
-                         cudaStream_t stream) {
+                         cudaStream_t stream, bool round_gates) {
   PushGeom g{};
   int ctas;
   if (push == nullptr) {
@@ -187,9 +188,9 @@ void launch_scatter_rows(const T* x, const int* slot_map, const float* gates, T*
   }
   if (ctas < 1) ctas = 1;
   if (quant)
-    scatter_rows_kernel<T, true><<<ctas, kRowThreads, 0, stream>>>(x, slot_map, gates, local_out, K, S, M, g);
+    scatter_rows_kernel<T, true><<<ctas, kRowThreads, 0, stream>>>(x, slot_map, gates, local_out, K, S, M, g, round_gates);
   else
-    scatter_rows_kernel<T, false><<<ctas, kRowThreads, 0, stream>>>(x, slot_map, gates, local_out, K, S, M, g);
+    scatter_rows_kernel<T, false><<<ctas, kRowThreads, 0, stream>>>(x, slot_map, gates, local_out, K, S, M, g, round_gates);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -211,7 +212,7 @@ __global__ void __launch_bounds__(kRowThreads, MAXK <= 2 ? 8 : 4)
 gather_rows_kernel(const void* __restrict__ disp_, const float* __restrict__ scale_bias,
                    const int* __restrict__ idx, const int* __restrict__ loc,
                    const float* __restrict__ gates, T* __restrict__ out, int K, int S, int M,
-                   int C, WaitGeom w, long long group_rows) {
+                   int C, WaitGeom w, long long group_rows, bool round_gates) {
   __shared__ int ok_s;
   if (w.flags != nullptr) {
     if (threadIdx.x == 0) ok_s = 1;
@@ -237,6 +238,7 @@ gather_rows_kernel(const void* __restrict__ disp_, const float* __restrict__ sca
         if (e >= 0 && l >= 0 && l < C) {
           slot[k] = (long long)e * C + l;
           gw[k] = gates ? gates[(size_t)k * S + t] : 1.f;
+          if (round_gates) gw[k] = to_f32(from_f32<T>(gw[k]));
         }
       }
     }
@@ -326,7 +328,7 @@ gather_rows_kernel(const void* __restrict__ disp_, const float* __restrict__ sca
 template <class T>
 void launch_gather_rows(const void* disp, const float* scale_bias, const int* idx, const int* loc,
                         const float* gates, T* out, int K, int S, int M, int C,
-                        const WaitArgs* wait, cudaStream_t stream, long long group_rows) {
+                        const WaitArgs* wait, cudaStream_t stream, long long group_rows, bool round_gates) {
   WaitGeom w{};
   if (wait != nullptr) {
     w.flags = wait->flags; w.n_flags = wait->n_flags; w.want = wait->want; w.want_ptr = wait->want_ptr;
@@ -336,13 +338,13 @@ void launch_gather_rows(const void* disp, const float* scale_bias, const int* id
   if (ctas > 148 * 8) ctas = 148 * 8;
   if (ctas < 1) ctas = 1;
   if (scale_bias != nullptr && group_rows > 0)
-    gather_rows_kernel<T, 2, 8><<<ctas, kRowThreads, 0, stream>>>(disp, scale_bias, idx, loc, gates, out, K, S, M, C, w, group_rows);
+    gather_rows_kernel<T, 2, 8><<<ctas, kRowThreads, 0, stream>>>(disp, scale_bias, idx, loc, gates, out, K, S, M, C, w, group_rows, round_gates);
   else if (scale_bias != nullptr)
-    gather_rows_kernel<T, 1, 8><<<ctas, kRowThreads, 0, stream>>>(disp, scale_bias, idx, loc, gates, out, K, S, M, C, w, 0);
+    gather_rows_kernel<T, 1, 8><<<ctas, kRowThreads, 0, stream>>>(disp, scale_bias, idx, loc, gates, out, K, S, M, C, w, 0, round_gates);
   else if (K <= 2)
-    gather_rows_kernel<T, 0, 2><<<ctas, kRowThreads, 0, stream>>>(disp, scale_bias, idx, loc, gates, out, K, S, M, C, w, 0);
+    gather_rows_kernel<T, 0, 2><<<ctas, kRowThreads, 0, stream>>>(disp, scale_bias, idx, loc, gates, out, K, S, M, C, w, 0, round_gates);
   else
-    gather_rows_kernel<T, 0, 8><<<ctas, kRowThreads, 0, stream>>>(disp, scale_bias, idx, loc, gates, out, K, S, M, C, w, 0);
+    gather_rows_kernel<T, 0, 8><<<ctas, kRowThreads, 0, stream>>>(disp, scale_bias, idx, loc, gates, out, K, S, M, C, w, 0, round_gates);
 }
 
 // dgates[k][t] = <disp[slot_k(t)], dy[t]>.  With `scaled` != null the same pass also writes the
@@ -691,10 +693,10 @@ void launch_slots_gate_grad(const void* disp, const void* dy, const int* idx, co
 
 #define INSTANTIATE(T)                                                                             \
   template void launch_scatter_rows<T>(const T*, const int*, const float*, T*, int, int, int, int, \
-                                       int, const PushArgs*, bool, cudaStream_t);                  \
+                                       int, const PushArgs*, bool, cudaStream_t, bool);            \
   template void launch_gather_rows<T>(const void*, const float*, const int*, const int*,           \
                                       const float*, T*, int, int, int, int, const WaitArgs*,       \
-                                      cudaStream_t, long long);                                    \
+                                      cudaStream_t, long long, bool);                              \
   template void launch_gate_grad<T>(const T*, const T*, const int*, const int*, float*, const float*, \
                                     T*, int, int, int, int, cudaStream_t, const float*, long long, unsigned char*);
 INSTANTIATE(float)

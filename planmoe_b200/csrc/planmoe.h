@@ -46,14 +46,15 @@ void launch_build_slot_map(const int* idx, const int* loc, int* slot_map, int K,
 template <class T>
 void launch_scatter_rows(const T* x, const int* slot_map, const float* gates, T* local_out, int K,
                          int S, int M, int E, int C, const PushArgs* push, bool quant,
-                         cudaStream_t stream);
+                         cudaStream_t stream, bool round_gates = false);
+// round_gates: the fp32 gates count as values of T
 // scale_bias: null (rows of T), or fp32 (range, low) per row with uint8 rows (int8 codec), or -- with
 // group_rows > 0 -- fp32 (scale, low) per (128-column group, row), laid out [M / 128][group_rows], with uint8 rows
 // (what the int8 push epilogue of the grouped GEMM writes)
 template <class T>
 void launch_gather_rows(const void* disp, const float* scale_bias, const int* idx, const int* loc,
                         const float* gates, T* out, int K, int S, int M, int C, const WaitArgs* wait,
-                        cudaStream_t stream, long long group_rows = 0);
+                        cudaStream_t stream, long long group_rows = 0, bool round_gates = false);
 // `gates` / `scaled` optional: also write scaled[t * K + k] = gates[k][t] * dy[t]
 // disp_scales != null: disp holds uint8 rows with fp32 (scale, low) per (128-column group, row), [M / 128][E * C];
 // scaled_q (int8 mode only): the gate-weighted dy rows as int8 wire rows [S * K][M + 16] instead of `scaled`

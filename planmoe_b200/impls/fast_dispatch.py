@@ -119,7 +119,7 @@ class _RouteLoss(torch.autograd.Function):
     @staticmethod
     def forward(ctx, scores, value, top1, idx):
         ctx.save_for_backward(scores, idx, top1)
-        return value.clone()
+        return value.detach()                   # its own tensor on the value's memory
 
     @staticmethod
     def backward(ctx, dloss):
@@ -243,6 +243,8 @@ fast_dispatcher = TutelMoeFastDispatcher
 def fast_encode(data, critial_data, is_postscore=True):
     """[S, M] tokens -> [E, C, M] expert slots (gate-weighted iff ``not is_postscore``)."""
     plan = _as_plan(critial_data)
+    if not is_postscore and D.picks_ok(data, plan.slots, plan[3]):
+        return D.scatter_picks(data, plan.slots, plan[3]).view(plan[0], -1, data.size(-1))
     gates = None if is_postscore else plan.stacked_gates().to(data.dtype)
     return D.scatter(data, plan.slots, gates).view(plan[0], -1, data.size(-1))
 
@@ -250,5 +252,7 @@ def fast_encode(data, critial_data, is_postscore=True):
 def fast_decode(data, critial_data, is_postscore=True):
     """[E, C, M] expert slots -> [S, M] tokens (gate-weighted iff ``is_postscore``)."""
     plan = _as_plan(critial_data)
+    if is_postscore and D.picks_ok(data, plan.slots, plan[3]):
+        return D.gather_picks(data.reshape(-1, data.size(-1)), plan.slots, plan[3])
     gates = plan.stacked_gates().to(data.dtype) if is_postscore else None
     return D.gather(data.reshape(-1, data.size(-1)), plan.slots, gates)

@@ -91,3 +91,35 @@ def test_changed_lists_and_other_forms_take_the_composition(monkeypatch):
     monkeypatch.setattr(gating, 'use_fast_cumsum', False)             # the cumsum kernel knows no function transforms
     grad = torch.func.grad(lambda s: FD.extract_critical(s, 2)[1])(scores)
     assert torch.isfinite(grad).all()
+
+
+@pytest.mark.parametrize('dtype', [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize('postscore', [True, False])
+@pytest.mark.parametrize('S,E,k', [(1, 2, 2), (257, 5, 1), (300, 8, 3)])
+def test_encode_and_decode_by_pick(dtype, postscore, S, E, k):
+    """Gates handed over pick by pick (on one storage, and as tensors of their own) against the stacked, rounded ones."""
+    from planmoe_b200.impls import fast_dispatch as FD
+    from planmoe_b200.ops import dispatch as D
+    torch.manual_seed(S)
+    x = torch.randn(S, 64, device='cuda').to(dtype)
+    dy = torch.randn(S, 64, device='cuda').to(dtype)
+    scores = torch.softmax(torch.randn(S, E, device='cuda'), dim=1)
+    out = []
+    for form in ('made', 'separate', 'stacked'):
+        xl, sl = x.clone().requires_grad_(), scores.clone().requires_grad_()
+        plan, _ = FD.extract_critical(sl, k, capacity_factor=0.8)
+        gates = [g * 1 for g in plan[3]] if form == 'separate' else plan[3]
+        plan = FD.RoutingPlan(plan[0], plan[1], plan[2], gates, plan[4], plan.slots)
+        if form == 'stacked':
+            g = plan.stacked_gates().to(dtype)
+            slots = D.scatter(xl, plan.slots, None if postscore else g)
+            y = D.gather(slots, plan.slots, g if postscore else None)
+        else:
+            y = FD.fast_decode(FD.fast_encode(xl, plan, postscore), plan, postscore)
+        y.backward(dy)
+        out.append((y.detach(), xl.grad, sl.grad))
+    for got in out[:2]:
+        assert torch.equal(got[0], out[2][0]) and torch.equal(got[1], out[2][1])
+        # the stacked form rounds the gates' gradient to the data's type
+        eps = torch.finfo(dtype).eps
+        assert float((got[2] - out[2][2]).abs().max()) <= 4 * eps * float(out[2][2].abs().max()) + 1e-6
