@@ -204,8 +204,11 @@ PM_HD void zfp_decode_block(const uint32_t* words, float* f, int maxbits) {
 // ---- the same block coder, bit planes at a time -------------------------------------------------
 // Writes and reads exactly the stream of zfp_encode_block / zfp_decode_block (the serial form, which the CPU twin runs
 // and the tests compare with).  What the serial form spends its instructions on is collecting one bit of each of the 16
-// coefficients per plane and moving the code bit by bit; here all planes come from one 16 x 32 bit-matrix transpose,
-// and a group test with the run of zeros and the one that follow it is one append (or one look at the next 17 bits).
+// coefficients per plane and moving the code bit by bit; here all planes come from one 16 x 32 bit-matrix transpose.
+// The encoder then writes a plane as one append: behind the group test's 1, a zero bit is a 0 and a one bit is a 1 and the
+// next group test, 1 while there is more; so the plane's tests and bits are its bits with every one doubled, up to the
+// last one, whose second bit is 0 - or which is left out altogether, second bit and all, in the sixteenth place.  The
+// decoder takes a group test with the run of zeros and the one that follow it as one look at the next 17 bits.
 // `planes` is room for 16 words and `words` for the block's code words, both `stride` words apart, so that a
 // thread block can keep one column per thread in shared memory.
 
@@ -238,7 +241,40 @@ PM_HD int low_zeros(uint32_t x) {            // number of zero bits below the lo
 #endif
 }
 
-PM_HD void zfp_encode_block_planes(const float* f, uint32_t* planes, uint32_t* words, int stride, int maxbits) {
+PM_HD int high_zeros(uint32_t x) {           // number of zero bits above the highest one; x != 0
+#if defined(__CUDA_ARCH__)
+  return __clz((int)x);
+#else
+  return __builtin_clz(x);
+#endif
+}
+PM_HD int count_ones(uint32_t x) {
+#if defined(__CUDA_ARCH__)
+  return __popc(x);
+#else
+  return __builtin_popcount(x);
+#endif
+}
+
+// A byte with every one bit doubled, lowest first: 0 -> 0, 1 -> 11.
+struct DoubledOnes {
+  uint16_t v[256];
+  constexpr DoubledOnes() : v() {
+    for (int b = 0; b < 256; ++b) {
+      unsigned out = 0;
+      int at = 0;
+      for (int i = 0; i < 8; ++i) {
+        if ((b >> i) & 1) { out |= 3u << at; at += 2; }
+        else ++at;
+      }
+      v[b] = (uint16_t)out;
+    }
+  }
+};
+
+// `doubled`: the table of DoubledOnes.
+PM_HD void zfp_encode_block_planes(const float* f, uint32_t* planes, uint32_t* words, const uint16_t* doubled, int stride,
+                                   int maxbits) {
   const int nwords = maxbits / 32;
   float amax = 0.f;
   for (int i = 0; i < 16; ++i) { const float a = f[i] < 0 ? -f[i] : f[i]; if (a > amax) amax = a; }
@@ -254,48 +290,36 @@ PM_HD void zfp_encode_block_planes(const float* f, uint32_t* planes, uint32_t* w
     bit_transpose16(u);
     for (int i = 0; i < 16; ++i) planes[i * stride] = u[i];   // plane k: bits (k & 16) .. +15 of word k & 15
     uint64_t acc = (2u * (uint32_t)(emax + 127) + 1u) & 0x1ffu;   // pending code bits, LSB first; below 32 between rounds
-    int nacc = 9, bits = maxbits - 9, n = 0, k = 31;
-    uint32_t x = planes[15 * stride] >> 16;
-    bool fresh = true;                                        // x is a plane whose first n bits are not written yet
-    while (true) {
-      uint32_t val = 0;
-      int len = 0;
-      if (fresh) {
-        len = n < bits ? n : bits;
-        val = x & ((1u << len) - 1u);
-        x >>= n;
-        bits -= len;
-      }
-      bool next = true;
-      if (n < 16 && bits > 0) {
-        if (x == 0u) {                                        // group test: nothing more in this plane
+    int nacc = 9, bits = maxbits - 9, n = 0;
+    for (int k = 31; k >= 0 && bits > 0; --k) {
+      const uint32_t plane = (planes[(k & 15) * stride] >> (k & 16)) & 0xffffu;
+      const uint32_t x = plane >> n;
+      uint32_t val = plane & ((1u << n) - 1u);                // the coefficients that are under way already
+      int len = n;
+      if (n < 16) {
+        if (x == 0u) {                                        // group test: nothing new in this plane
           ++len;
-          --bits;
-        } else {                                              // group test, z zeros and, unless it is the last place, a one
-          const int z = low_zeros(x);
-          int l = z + 2 - (n + z == 15 ? 1 : 0);
-          l = l < bits ? l : bits;
-          val |= ((1u | (2u << z)) & ((1u << l) - 1u)) << len;
-          len += l;
-          bits -= l;
-          x >>= z + 1;
-          n += z + 1;
-          next = n >= 16;
+        } else {
+          const int top = 31 - high_zeros(x), low_ones = count_ones(x & 0xffu);
+          const uint32_t twice = (uint32_t)doubled[x & 0xffu] | ((uint32_t)doubled[x >> 8] << (8 + low_ones));
+          const bool last = n + top == 15;
+          const int used = top + 2 + low_ones + count_ones(x >> 8) - (last ? 2 : 0);      // at most 31 bits
+          const uint32_t keep = (1u << (last ? used : used - 1)) - 1u;                    // the last test is a 0
+          val |= ((1u | (twice << 1)) & keep) << n;
+          len += used;                                        // at most 32 bits with the n before
+          n += top + 1;
         }
       }
-      acc |= (uint64_t)val << nacc;                           // at most 17 bits a round
+      if (len > bits) len = bits;
+      val &= 0xffffffffu >> (32 - len);
+      bits -= len;
+      acc |= (uint64_t)val << nacc;
       nacc += len;
       if (nacc >= 32) {
         words[widx * stride] = (uint32_t)acc;
         ++widx;
         acc >>= 32;
         nacc -= 32;
-      }
-      if (bits == 0) break;
-      fresh = next;
-      if (next) {
-        if (--k < 0) break;
-        x = (planes[(k & 15) * stride] >> (k & 16)) & 0xffffu;
       }
     }
     if (nacc > 0) { words[widx * stride] = (uint32_t)acc; ++widx; }

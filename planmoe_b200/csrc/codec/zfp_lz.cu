@@ -78,10 +78,11 @@ inline void zfp_block_io(bool encode, const void* x_in, void* x_out, int elem, u
 
 // One thread per block, the bit planes of its 16 coefficients and its code words in its own column of shared memory.
 // Bound by integer issue: the serial bit-plane coder took 4685 warp instructions per 32 blocks (318 us to encode 8192 x
-// 4096 bf16, 84 % of the issue slots); see zfp_encode_block_planes for what replaced it.  VEC: rows of a block are
+// 4096 bf16, 84 % of the issue slots), its group tests one by one 2070 (140 us); see zfp_encode_block_planes.  VEC: rows of a block are
 // moved as one 4-element vector, which needs the tensor's base to lie on such a vector (rows are multiples of four
 // elements); other bases take the element loop.
 constexpr int kZfpThreads = 128;
+__device__ const DoubledOnes kDoubledOnes;          // half a KiB: it stays in L1
 
 template <int ELEM> struct ZfpElem { using type = float; };
 template <> struct ZfpElem<1> { using type = __nv_bfloat16; };
@@ -155,7 +156,7 @@ zfp_encode_kernel(const void* __restrict__ x, uint8_t* __restrict__ stream, long
     }
   }
   uint32_t* w = words + threadIdx.x;
-  zfp_encode_block_planes(f, planes + threadIdx.x, w, kZfpThreads, 16 * rate);
+  zfp_encode_block_planes(f, planes + threadIdx.x, w, kDoubledOnes.v, kZfpThreads, 16 * rate);
   uint8_t* dst = stream + b * (2 * rate);         // the stream is a fresh allocation: 8-byte stores are aligned
   for (int i = 0; i < rate / 2; i += 2)
     *reinterpret_cast<uint2*>(dst + 4 * i) = make_uint2(w[i * kZfpThreads], w[(i + 1) * kZfpThreads]);
