@@ -398,6 +398,7 @@ struct GemmOpts {
   int64_t dq_ptr = 0, dq_arrival_ptr = 0, dq_ready_ptr = 0;
   int64_t trace_ptr = 0;                     // optional u64 [grid][8] role trace (see GemmArgs::trace)
   c10::optional<Tensor> rows_used;           // optional int32 [groups] (see GemmArgs::rows_used)
+  c10::optional<Tensor> colsum;              // optional fp32 [groups, (M + 31) / 32, N] (see GemmArgs::colsum)
 };
 
 GemmOperand operand_of(const Tensor& t, bool mn_major) {
@@ -474,6 +475,12 @@ Tensor grouped_gemm_op(const Tensor& A, bool a_mn, const Tensor& B, bool b_mn, c
     const Tensor& u = *o.rows_used;
     TORCH_CHECK(u.is_cuda() && u.scalar_type() == at::kInt && u.is_contiguous() && u.numel() == groups, "rows_used: int32 [groups]");
     g.rows_used = u.data_ptr<int>();
+  }
+  if (o.colsum.has_value() && o.colsum->defined()) {
+    const Tensor& c = *o.colsum;
+    TORCH_CHECK(c.is_cuda() && c.scalar_type() == at::kFloat && c.is_contiguous() &&
+                c.numel() == (int64_t)groups * ((g.M + 31) / 32) * g.N, "colsum: fp32 [groups, (M + 31) / 32, N]");
+    g.colsum = c.data_ptr<float>();
   }
   g.max_ctas = o.max_ctas;
   g.cta_group = o.cta_group;
@@ -716,7 +723,7 @@ static std::vector<Tensor> local_backward(const Tensor& dy, const Tensor& x, con
   const int *idx = r.idx.data_ptr<int>(), *loc = r.loc.data_ptr<int>(), *used = r.used.data_ptr<int>();
   const float* gates = r.gates.data_ptr<float>();
   Tensor dgates = torch::empty({K, S}, r.gates.options()), dys = torch::empty({E, C, O}, x.options());
-  Tensor dx, dh, dxs, dx_scales, dl, dwg, dw1, dw2, db1, db2;
+  Tensor dx, dh, dxs, dx_scales, dh_sums, dl, dwg, dw1, dw2, db1, db2;
   {
     Stage st(stages, "bwd.gate_grad");
     count_launch(1);
@@ -734,6 +741,7 @@ static std::vector<Tensor> local_backward(const Tensor& dy, const Tensor& x, con
     Stage st(stages, "bwd.dgrad2");               // dH = (dY . W2^T) * act'
     GemmOpts o = local_opts(r, kEpiDAct);
     o.aux = dact;
+    if (need[3]) o.colsum = dh_sums = torch::empty({E, (C + 31) / 32, w2.size(1)}, r.gates.options());
     dh = grouped_gemm_op(dys, false, w2, false, o);
   }
   const bool gate_from_dx = !r.postscore && (need[1] || gate != nullptr);
@@ -781,8 +789,15 @@ static std::vector<Tensor> local_backward(const Tensor& dy, const Tensor& x, con
     Tensor keep[3];
     int n = 0;
     if (need[5]) { keep[n] = colsum_job(dys, 1, true, j[n], db2, used); ++n; }
-    if (need[3]) { keep[n] = colsum_job(dh, 1, true, j[n], db1, used); ++n; }
     if (n > 0) count_launch(1);
+    if (need[3]) {                                // the slices' sums came with dH
+      const int64_t H = w2.size(1);
+      db1 = torch::empty({E, H}, x.options());
+      keep[n] = torch::empty({E, H}, r.gates.options());
+      j[n].partial = dh_sums.data_ptr<float>(); j[n].out = keep[n].data_ptr<float>(); j[n].out_bf16 = db1.data_ptr();
+      j[n].rows = C; j[n].slab_rows = 32; j[n].N = (int)H; j[n].groups = (int)E; j[n].fold = 1; j[n].rows_used = used;
+      ++n;
+    }
     if (gate != nullptr && need[1]) {
       const int chunks = gate_wgrad_chunks(S, M);
       keep[n] = torch::empty({(int64_t)chunks + 1, E * M}, r.gates.options());

@@ -37,9 +37,11 @@ __device__ __forceinline__ float below_upper(float a) { return a - __uint_as_flo
 // One block per 16 * MT tokens; its warps share the contraction, 32 columns at a time (chunk w, w + 8, ...), and their
 // sums are added in warp order.  A lane's 16-byte pieces of two token rows and of one weight row are the fragments of two
 // m16n8k16 steps: which column a fragment register stands for is free as long as both operands agree.  Bound by the token
-// rows (DRAM) and, with many experts, by the weights that every block reads again from L2; 32 tokens a block halve the
-// latter once there are blocks enough without (kProjWide).
-constexpr int kProjWide = 4096;                   // tokens from which on a block takes 32
+// rows (DRAM) and, with many experts, by the weights that every block reads again from L2: with more than eight experts,
+// 32 tokens a block halve the latter once there are blocks enough (8192 x 4096, 16 experts: 24 us against 34 with 16
+// tokens; 4096 tokens: the same).  With fewer experts 16 tokens a block are better at every size (16384 x 4096, 8 experts:
+// 34 us against 42).
+constexpr int kProjWide = 4096;                   // tokens from which on a block takes 32, with more than eight experts
 
 template <int NT, int MT, bool W_BF16>
 __global__ void __launch_bounds__(kProjWarps * 32)
@@ -281,8 +283,6 @@ gather_gate_kernel(const void* __restrict__ slots_, const float2* __restrict__ s
 #pragma unroll
   for (int t = 0; t < kGatherTokens; ++t) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) acc[t][i] = 0ull;
-#pragma unroll
     for (int k = 0; k < MAXK; ++k) {
       unsigned long long p[4];
       if constexpr (Q8) {                         // a pick without a slot has scale and low zero
@@ -295,10 +295,14 @@ gather_gate_kernel(const void* __restrict__ slots_, const float2* __restrict__ s
       } else {
         bf16_pairs(raw[t][k], p);
       }
-      const float gk = GATED ? __shfl_sync(0xffffffffu, gv, t * MAXK + k) : 1.f;
-      const unsigned long long gp = pair_of(gk, gk);
+      if constexpr (GATED) {
+        const unsigned long long gp = pair_const(__shfl_sync(0xffffffffu, gv, t * MAXK + k));
 #pragma unroll
-      for (int i = 0; i < 4; ++i) acc[t][i] = fma_pair(p[i], gp, acc[t][i]);
+        for (int i = 0; i < 4; ++i) acc[t][i] = k == 0 ? mul_pair(p[i], gp) : fma_pair(p[i], gp, acc[t][i]);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[t][i] = k == 0 ? p[i] : add_pair(acc[t][i], p[i]);
+      }
     }
   }
   const float2* mine = dl_s + warp * kGatherTokens * E;
@@ -332,10 +336,13 @@ gather_gate_kernel(const void* __restrict__ slots_, const float2* __restrict__ s
 template <int NT, bool W_BF16>
 void project_nt(const void* x, const void* w, float* logits, int S, int E, int M, bool round_bf16, cudaStream_t stream) {
   const __nv_bfloat16* xb = reinterpret_cast<const __nv_bfloat16*>(x);
-  if (S >= kProjWide)
-    gate_project_kernel<NT, 2, W_BF16><<<(S + 31) / 32, kProjWarps * 32, 0, stream>>>(xb, w, logits, S, E, M, round_bf16);
-  else
-    gate_project_kernel<NT, 1, W_BF16><<<(S + 15) / 16, kProjWarps * 32, 0, stream>>>(xb, w, logits, S, E, M, round_bf16);
+  if constexpr (NT > 1) {
+    if (S >= kProjWide) {
+      gate_project_kernel<NT, 2, W_BF16><<<(S + 31) / 32, kProjWarps * 32, 0, stream>>>(xb, w, logits, S, E, M, round_bf16);
+      return;
+    }
+  }
+  gate_project_kernel<NT, 1, W_BF16><<<(S + 15) / 16, kProjWarps * 32, 0, stream>>>(xb, w, logits, S, E, M, round_bf16);
 }
 
 }  // namespace
@@ -351,10 +358,11 @@ void launch_gate_project(const void* x, const void* w, bool w_bf16, float* logit
   }
 }
 
-// Chunks of tokens: about four blocks per SM over all column slabs, at least 32 tokens each.
+// Chunks of tokens: two blocks per SM over all column slabs (what is resident with eight experts), at least 32 tokens each.
+// Twice as many chunks were a second, half empty wave and twice the partial sums to add up.
 int gate_wgrad_chunks(int S, int M) {
   const int slabs = (M + 255) / 256;
-  int n = 4 * 148 / slabs;
+  int n = 2 * 148 / slabs;
   if (n > S / 32) n = S / 32;
   return n < 1 ? 1 : n;
 }

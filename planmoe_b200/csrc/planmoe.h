@@ -212,6 +212,9 @@ struct GemmArgs {
   // at least one is computed, so rows up to the end of the last block (kSlotBlock) have to be finite, and zero in
   // one operand of a weight gradient.  At most 64 groups, one chunk, no flag gate, no push, no copy role.
   const int* rows_used;
+  // Optional (activation backward without a copy role): column sums of every 32-row slice of D as stored, fp32 [groups][M /
+  // 32, rounded up][N]; slices behind the last computed row block are left unwritten.
+  float* colsum;
   unsigned long long budget_ns; int* status;
   // Optional role trace, device u64 [grid][32] (ns of %globaltimer): [0] kernel entry, [1] / [2] copy role begin / end,
   // [3] time the TMA producer spent waiting on gate flags, [4] kernel exit, [5] de-quantiser role end; in SM clocks,
@@ -264,12 +267,14 @@ void launch_colsum_bf16(const void* x, float* out, int groups, long long rows, i
                         cudaStream_t stream);
 // Up to three column-sum jobs in the same two launches (see launch_colsum_bf16 for the meaning of the fields).
 // `partial`: groups * colsum_slabs(rows) * N floats; `counters` is reserved (the two-stage form does not use it).
-// A job without x brings its partial sums along (rows = 128 * their number) and takes part in the second launch only.
+// A job without x brings its partial sums along ([groups][rows / slab_rows, rounded up][N]) and takes part in the second
+// launch only.
 struct ColsumJob {
   const void* x; float* out; void* out_bf16; float* partial; unsigned* counters;
   long long rows, row_stride, group_stride;
   int N, groups, fold;
   const int* rows_used;            // optional device [groups]: rows behind the first rows_used[g] are left out
+  int slab_rows;                   // rows behind one partial sum of a job without x (0: 128)
 };
 int colsum_colblocks(int N);
 void launch_colsum_jobs(const ColsumJob* jobs, int n, cudaStream_t stream);
