@@ -229,7 +229,7 @@ gather_gate_kernel(const void* __restrict__ slots_, const float2* __restrict__ s
                    __nv_bfloat16* __restrict__ dx, int K, int S, int M, int E, int C) {
   constexpr bool GATED = FORM == kGatherGated, Q8 = FORM == kGatherInt8;
   extern __shared__ __align__(16) float gather_smem[];
-  float* w_s = gather_smem;                                                       // [E][256]
+  float* w_s = gather_smem;        // [E][first four, last four of eight columns][32 lanes][4]: no bank conflicts
   float2* dl_s = reinterpret_cast<float2*>(gather_smem + E * 256);                // [32 tokens][E], pairs {d, d}
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int slabs = (M + 255) / 256;              // neighbouring blocks take neighbouring columns of the same tokens
@@ -271,7 +271,7 @@ gather_gate_kernel(const void* __restrict__ slots_, const float2* __restrict__ s
       const long long o = (long long)(i >> 8) * M + m;
       v = W_BF16 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(w_)[o]) : reinterpret_cast<const float*>(w_)[o];
     }
-    w_s[i] = v;
+    w_s[(i & ~255) + ((i & 4) ? 128 : 0) + ((i & 255) >> 3) * 4 + (i & 3)] = v;
   }
   for (int i = threadIdx.x; i < 8 * kGatherTokens * E; i += 256) {
     const int t = tb + i / E;
@@ -308,8 +308,8 @@ gather_gate_kernel(const void* __restrict__ slots_, const float2* __restrict__ s
   const float2* mine = dl_s + warp * kGatherTokens * E;
 #pragma unroll 2
   for (int e = 0; e < E; ++e) {
-    const ulonglong2 lo = *reinterpret_cast<const ulonglong2*>(w_s + e * 256 + lane * 8);
-    const ulonglong2 hi = *reinterpret_cast<const ulonglong2*>(w_s + e * 256 + lane * 8 + 4);
+    const ulonglong2 lo = *reinterpret_cast<const ulonglong2*>(w_s + e * 256 + lane * 4);
+    const ulonglong2 hi = *reinterpret_cast<const ulonglong2*>(w_s + e * 256 + 128 + lane * 4);
     const unsigned long long w[4] = {lo.x, lo.y, hi.x, hi.y};
 #pragma unroll
     for (int t = 0; t < kGatherTokens; ++t) {
