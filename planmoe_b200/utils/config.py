@@ -44,7 +44,8 @@ ENV = {
     'PLANMOE_GEMM_CTA_GROUP': ('auto', '1 or 2: force one-CTA (128 x 256) or two-CTA (256 x 256) tiles'),
     'PLANMOE_GEMM_TMA_STORE': ('1', '0: epilogues write with 16-byte stores instead of bulk tensor stores'),
     'PLANMOE_GEMM_COPY_VARIANT': ('0', '1: plain launches use the kernel variant that carries the dispatch send (one ring '
-                                  'stage less); for measuring that variant alone'),
+                                  'stage less), for measuring that variant alone; launches with column sums or used-row '
+                                  'counts, which it does not have, keep theirs'),
     'PLANMOE_LOCAL_FIRST': ('0', '0: the dispatch send interleaves all destinations from the first row and the tile loop '
                             'visits sources round-robin; 1: own rows are sent and consumed first (measured slower)'),
     'PLANMOE_GEMM_TRACE': ('0', '1: fused launches record per-CTA role timestamps; fused_moe.last_trace() summarises them'),

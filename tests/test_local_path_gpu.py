@@ -1,6 +1,10 @@
 """One rank without the exchange against the exchange of one rank (PLANMOE_LOCAL=0), over the forms both take: capacities
 that are no multiple of a row block, experts without a token, dropped tokens, every number of picks."""
 
+import os
+import subprocess
+import sys
+
 import pytest
 import torch
 
@@ -172,3 +176,26 @@ def test_int8_rows_match_the_exchange(S, E, k, cf, monkeypatch):
     if layer.last_stats['capacity'] % 32 == 0:
         monkeypatch.setenv('PLANMOE_LOCAL', '0')
         _close(here, _pass(layer, x, dy))
+
+
+_VARIANT_CHILD = """
+import os, torch
+from tests.test_local_path_gpu import _close, _layer, _pass
+torch.use_deterministic_algorithms(True, warn_only=True)      # new tensors start as NaN
+layer = _layer(4, 128, 256, 2, 2.0)
+x = torch.randn(700, 128, device='cuda').bfloat16()
+dy = torch.randn_like(x)
+here = _pass(layer, x, dy)
+os.environ['PLANMOE_LOCAL'] = '0'
+_close(here, _pass(layer, x, dy))
+print('same')
+"""
+
+
+def test_measuring_switch_of_the_send_variant_changes_no_result():
+    """PLANMOE_GEMM_COPY_VARIANT=1 selects a kernel without column sums and used-row counts: launches that need them keep
+    theirs.  The switch is read once per process."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    child = subprocess.run([sys.executable, '-c', _VARIANT_CHILD], cwd=root, capture_output=True, text=True, timeout=300,
+                           env=dict(os.environ, PLANMOE_GEMM_COPY_VARIANT='1', PYTHONPATH=root))
+    assert child.returncode == 0 and 'same' in child.stdout, child.stderr[-2000:]
