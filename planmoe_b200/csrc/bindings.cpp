@@ -588,7 +588,7 @@ struct Stage {
 struct LocalRoute {
   Tensor idx, loc, slot_map, used, gates;
   int64_t C, act;
-  bool postscore, int8;                           // int8: rows as int8 transfers deliver them, both ways
+  bool postscore, int8;                           // int8: rows as int8 transfers deliver them, both ways (C % 32 == 0)
   int64_t budget_ms, status_ptr;
 };
 
@@ -828,7 +828,9 @@ std::vector<Tensor> local_backward_op(const Tensor& dy, const Tensor& x, const L
 }
 
 // The whole layer with a linear gate `wg` [E, M].  capacity < 0: as many slots as the busiest expert needs, rounded up by
-// `round_up` (one host read).  Returns {y, l_aux, logits, top1, slot_map, used, idx, loc, gates, xs, dact, h, ys, scales} and
+// `round_up` (one host read).  Returns {y, l_aux, logits, top1, slot_map, used, idx, loc, gates, xs, dact, h, ys, scales, loc as
+// routed} and the capacity.  int8 rows are stored in slices of 32: the experts' slots are then laid out C = capacity rounded
+// up to that apart (xs.size(1)), and the first `loc` has a dropped pick behind all of them; what is dropped stays a matter of
 // the capacity.
 std::tuple<std::vector<Tensor>, int64_t> local_moe_forward_op(
     const Tensor& x, const Tensor& wg, const Tensor& w1, const Tensor& b1, const Tensor& w2, const Tensor& b2, int64_t K,
@@ -846,6 +848,7 @@ std::tuple<std::vector<Tensor>, int64_t> local_moe_forward_op(
   const int64_t nblk = gate_workspace_blocks(S);
   LocalRoute r{torch::empty({K, S}, iopt), torch::empty({K, S}, iopt), {}, {}, torch::empty({K, S}, fopt), capacity, act,
                postscore, int8, budget_ms, status_ptr};
+  const Tensor loc = r.loc;
   Tensor logits = torch::empty({S, E}, fopt), counts = torch::empty({2, E}, iopt);
   Tensor laux = torch::empty({}, fopt), laux_bf16;
   if (bf16_logits) laux_bf16 = torch::empty({}, x.options());
@@ -866,15 +869,15 @@ std::tuple<std::vector<Tensor>, int64_t> local_moe_forward_op(
       launch_importance_order<float>(logits.data_ptr<float>(), S, E, reinterpret_cast<float*>(o), o + S, o + 2 * S, cur_stream());
       perm = o + 2 * S;
     }
-    const bool dynamic = capacity < 0;
-    if (!dynamic) r.slot_map = torch::empty({E * capacity}, iopt);
+    const bool dynamic = capacity < 0, map_later = dynamic || (int8 && capacity % 32 != 0);
+    if (!map_later) r.slot_map = torch::empty({E * capacity}, iopt);
     GatePtrs gp{};
     for (int k = 0; k < K; ++k) gp.p[k] = r.gates.data_ptr<float>() + (int64_t)k * S;
     int* w = ws.data_ptr<int>();
     count_launch(2);
     launch_gate_forward<float, false>(logits.data_ptr<float>(), S, E, K, dynamic ? INT_MAX : (int)capacity, normalize,
                                       bf16_logits ? 7.8125e-03f : kFloatEps, r.idx.data_ptr<int>(), r.loc.data_ptr<int>(), gp,
-                                      reinterpret_cast<float*>(w), dynamic ? nullptr : r.slot_map.data_ptr<int>(),
+                                      reinterpret_cast<float*>(w), map_later ? nullptr : r.slot_map.data_ptr<int>(),
                                       counts.data_ptr<int>(), counts.data_ptr<int>() + E, laux.data_ptr<float>(), w + K * S,
                                       w + 2 * K * S, reinterpret_cast<float*>(w + 2 * K * S + K * nblk * E), cur_stream(), perm,
                                       bf16_logits ? laux_bf16.data_ptr() : nullptr);
@@ -882,8 +885,13 @@ std::tuple<std::vector<Tensor>, int64_t> local_moe_forward_op(
       const Tensor host = counts[1].cpu();
       int peak = 0;
       for (int64_t e = 0; e < E; ++e) peak = std::max(peak, host.data_ptr<int>()[e]);
-      r.C = round_up(peak).cast<int64_t>();
-      TORCH_CHECK(r.C >= peak);
+      capacity = round_up(peak).cast<int64_t>();
+      TORCH_CHECK(capacity >= peak);
+    } else if (map_later) {
+      r.loc = loc.masked_fill(loc.ge(capacity), INT_MAX);
+    }
+    if (map_later) {
+      r.C = int8 ? (capacity + 31) / 32 * 32 : capacity;
       r.slot_map = torch::empty({E * r.C}, iopt);
       count_launch(1);
       launch_build_slot_map(r.idx.data_ptr<int>(), r.loc.data_ptr<int>(), r.slot_map.data_ptr<int>(), K, S, E, r.C, cur_stream());
@@ -892,7 +900,7 @@ std::tuple<std::vector<Tensor>, int64_t> local_moe_forward_op(
   r.used = counts[1];
   std::vector<Tensor> e = local_forward_op(x, r, w1, b1, w2, b2, want_grad, stages);
   return {{e[0], bf16_logits ? laux_bf16 : laux, logits, counts[0], r.slot_map, r.used, r.idx, r.loc, r.gates, e[1], e[2], e[3],
-           e[4], e[5]}, r.C};
+           e[4], e[5], loc}, capacity};
 }
 
 std::vector<Tensor> local_moe_backward_op(const Tensor& dy, const c10::optional<Tensor>& dl_aux, const Tensor& x, const Tensor& wg,

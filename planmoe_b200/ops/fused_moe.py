@@ -452,11 +452,20 @@ class _FusedExperts(torch.autograd.Function):
         return dx, dgates, dw1, db1, dw2, db2, None
 
 
-def _local_path(tr, q8, capacity):
-    """Whether a layer's experts run without the exchange: one rank.  The GEMM epilogue that writes int8 rows does so in
-    slices of 32 (a capacity that is sized to the busiest expert, -1, is a multiple of 64).  PLANMOE_LOCAL=0, a choice of the
-    send's form (PLANMOE_FUSE_SEND), the debug guards and the role trace keep the exchange, which is what they are about."""
-    return tr.world == 1 and not tr.emulated and not (q8 and capacity > 0 and capacity % 32) and native.lib().local_by_env()
+def _local_path(tr):
+    """Whether a layer's experts run without the exchange: one rank.  PLANMOE_LOCAL=0, a choice of the send's form
+    (PLANMOE_FUSE_SEND), the debug guards and the role trace keep the exchange, which is what they are about."""
+    return tr.world == 1 and not tr.emulated and native.lib().local_by_env()
+
+
+def _whole_slices(m):
+    """``m`` with the slots of int8 rows laid out in whole slices of 32, which is how the GEMM epilogue stores them.  What is
+    dropped stays a matter of the capacity: such a pick gets a slot behind all others."""
+    C = m['C']
+    if not m['int8'] or C % 32 == 0:
+        return m
+    loc, slots = m['loc'].masked_fill(m['loc'] >= C, 2 ** 31 - 1), C + -C % 32
+    return dict(m, loc=loc, C=slots, slot_map=native.lib().build_slot_map(m['idx'], loc, m['used'].numel(), slots))
 
 
 def _aligned(t):
@@ -500,7 +509,7 @@ def _local_forward(x, gates, w1, b1, w2, b2, meta, want_grad):
 
 
 def _local_experts(x, gates, w1, b1, w2, b2, meta):
-    x, gates = _aligned(x), gates.contiguous()
+    x, gates, meta = _aligned(x), gates.contiguous(), _whole_slices(meta)
     if torch.is_grad_enabled() and any(t.requires_grad for t in (x, gates, w1, b1, w2, b2)):
         return _LocalExperts.apply(x, gates, w1, b1, w2, b2, meta)
     return _local_forward(x, gates, w1, b1, w2, b2, meta, False)[0]
@@ -512,10 +521,10 @@ class _LocalLayer(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, wg, w1, b1, w2, b2, m):
         ctx.set_materialize_grads(False)
-        (y, l_aux, *saved), m['capacity'] = _local_layer_forward(x, wg, w1, b1, w2, b2, m, True)
-        m['routing'] = saved[4], saved[5]
+        (y, l_aux, *saved, loc), m['capacity'] = _local_layer_forward(x, wg, w1, b1, w2, b2, m, True)
+        m['routing'] = saved[4], loc
         ctx.save_for_backward(x, wg, w1, w2, *saved)
-        ctx.m = {k: m[k] for k in ('capacity', 'act', 'postscore', 'int8', 'normalize', 'bf16_logits', 'budget_ms', 'status')}
+        ctx.m = {k: m[k] for k in ('act', 'postscore', 'int8', 'normalize', 'bf16_logits', 'budget_ms', 'status')}
         return y, l_aux
 
     @staticmethod
@@ -524,7 +533,7 @@ class _LocalLayer(torch.autograd.Function):
         m = ctx.m
         if dy is None:
             dy = torch.zeros((x.size(0), w2.size(2)), dtype=x.dtype, device=x.device)
-        route = _local_route(gates, dict(m, C=m['capacity'], idx=idx, loc=loc, slot_map=slot_map, used=used))
+        route = _local_route(gates, dict(m, C=xs.size(1), idx=idx, loc=loc, slot_map=slot_map, used=used))
         return (*native.lib().local_moe_backward(_aligned(dy), dl_aux, x, wg, route, w1, w2, logits, top1, xs, dact, h, ys,
                                                  scales, m['normalize'], m['bf16_logits'], list(ctx.needs_input_grad[:6]), _stages()),
                 None)
@@ -568,8 +577,8 @@ def _local_layer(layer, st, x, gctx, top_k, capacity, align):
     if torch.is_grad_enabled() and any(t.requires_grad for t in args):
         y, l_aux = _LocalLayer.apply(*args, m)
     else:
-        (y, l_aux, *saved), m['capacity'] = _local_layer_forward(*args, m, False)
-        m['routing'] = saved[4], saved[5]
+        (y, l_aux, *saved, loc), m['capacity'] = _local_layer_forward(*args, m, False)
+        m['routing'] = saved[4], loc
     return y, l_aux, m['capacity'], m['routing']
 
 
@@ -646,7 +655,7 @@ def forward(layer, x, gctx, top_k, capacity_factor, degree):
         capacity = max(capacity, 1)
         capacity += -capacity % align
     q8 = layer.compress_name == 'int8'
-    if _local_path(st.tr, q8, capacity) and _linear_gate(layer, gctx, x):
+    if _local_path(st.tr) and _linear_gate(layer, gctx, x):
         y, l_aux, capacity, (idx, loc) = _local_layer(layer, st, x, gctx, top_k, capacity, align)
         _note_stats(layer, st, q8, idx, loc, E, capacity, degree, x)
         return y, l_aux
@@ -680,7 +689,7 @@ def forward(layer, x, gctx, top_k, capacity_factor, degree):
         check_routing_bounds(idx, loc, slot_map, S, E, capacity, top_k)
     ex = layer.experts
     args = (gates, ex.batched_fc1_w, ex.batched_fc1_bias, ex.batched_fc2_w, ex.batched_fc2_bias)
-    if _local_path(st.tr, q8, capacity):
+    if _local_path(st.tr):
         y = _local_experts(x, *args, dict(idx=idx, loc=loc, slot_map=slot_map, used=used, C=capacity,
                                           act=ACT_CODES[ex.act_name], postscore=layer.is_postscore, int8=q8,
                                           budget_ms=st.tr.budget_ms, status=st.tr.status))
