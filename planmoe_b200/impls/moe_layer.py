@@ -318,11 +318,12 @@ class MOELayer(torch.nn.Module):
             return False
         if self.compress_name == 'int8':
             # int8 rows: quantised per token before the send (so no gate scaling on the way: post-score layers),
-            # 128-column groups in the push epilogue, the fused send as the carrier
+            # 128-column groups and whole slices of rows in the push epilogue, the fused send as the carrier
             from ..ops import fused_moe as _fm
             out_dim = self.experts.batched_fc2_w.size(2)
             if not self.is_postscore or x.size(-1) % 128 or out_dim % 128 or not _fm._fuse_send(self.world_size) \
-                    or (max(x.size(-1), out_dim) + 16) > _fm.MAX_ROW_BYTES:
+                    or (max(x.size(-1), out_dim) + 16) > _fm.MAX_ROW_BYTES \
+                    or not _fm.int8_capacity_ok(self, x.size(0), top_k, cf, int(degree)):
                 return False
         # on one NVSwitch domain the flat push is Pipe-A2A's equal (every peer is one hop away at full rate);
         # the hierarchical algorithms exist on the generic path

@@ -48,6 +48,7 @@ from ..utils.stage_timer import stage
 MAX_CHUNKS = 32      # largest pipeline degree (flag slots per phase are sized for it)
 MAX_TOP_K = 4        # the fused gate kernel keeps at most four picks per token
 GATE_BLOCK = 128     # rows per arrival flag of a dispatched GEMM operand
+SLICE_ROWS = 32      # rows that a warp of the GEMM epilogue stores at once
 MAX_ROW_BYTES = 16384  # longest bf16 row the fused send moves (one bulk-copy slot)
 FUSED_CODECS = ('no', 'int8')  # wire formats of the fused kernels
 # flag regions of a buffer set: the four exchanges, then the "de-quantised and ready" flags of the two
@@ -459,12 +460,12 @@ def _local_path(tr):
 
 
 def _whole_slices(m):
-    """``m`` with the slots of int8 rows laid out in whole slices of 32, which is how the GEMM epilogue stores them.  What is
+    """``m`` with the slots of int8 rows laid out in whole slices, which is how the GEMM epilogue stores them.  What is
     dropped stays a matter of the capacity: such a pick gets a slot behind all others."""
     C = m['C']
-    if not m['int8'] or C % 32 == 0:
+    if not m['int8'] or C % SLICE_ROWS == 0:
         return m
-    loc, slots = m['loc'].masked_fill(m['loc'] >= C, 2 ** 31 - 1), C + -C % 32
+    loc, slots = m['loc'].masked_fill(m['loc'] >= C, 2 ** 31 - 1), C + -C % SLICE_ROWS
     return dict(m, loc=loc, C=slots, slot_map=native.lib().build_slot_map(m['idx'], loc, m['used'].numel(), slots))
 
 
@@ -582,6 +583,21 @@ def _local_layer(layer, st, x, gctx, top_k, capacity, align):
     return y, l_aux, m['capacity'], m['routing']
 
 
+def _static_capacity(S, E, top_k, capacity_factor, align):
+    """Slots per expert for a capacity factor other than zero (its size alone counts)."""
+    capacity = max(top_k * int(abs(capacity_factor) * ((S + E - 1) // E)), 1)
+    return capacity + -capacity % align
+
+
+def int8_capacity_ok(layer, S, top_k, capacity_factor, degree):
+    """Whether int8 rows of this call fit the exchange: the push epilogue stores a source rank's rows of a chunk in slices of
+    ``SLICE_ROWS``.  A dynamic capacity is sized for that, and a single rank lays its slots out by itself (``_local_path``)."""
+    if capacity_factor == 0 or (layer.world_size == 1 and native.lib().local_by_env()):
+        return True
+    E = layer.num_global_experts
+    return _static_capacity(S, E, min(int(top_k), E), capacity_factor, 4 * degree) % (SLICE_ROWS * degree) == 0
+
+
 def _capacity_step(cap, align):
     """``cap`` rounded up to the next of a coarse ladder (steps of about 12 %)."""
     step = max(align, 64)
@@ -645,17 +661,10 @@ def forward(layer, x, gctx, top_k, capacity_factor, degree):
     assert degree <= MAX_CHUNKS and top_k <= MAX_TOP_K, "plan outside the fused kernels' limits"
 
     align = 4 * layer.sharded_count * degree
-    per_expert = (S + E - 1) // E
-    capacity = -1                                 # sized to the busiest expert
-    if capacity_factor > 0:
-        capacity = top_k * int(capacity_factor * per_expert)
-    elif capacity_factor < 0:
-        capacity = top_k * int(-capacity_factor * per_expert)
-    if capacity_factor != 0:
-        capacity = max(capacity, 1)
-        capacity += -capacity % align
+    capacity = _static_capacity(S, E, top_k, capacity_factor, align) if capacity_factor != 0 else -1
     q8 = layer.compress_name == 'int8'
-    if _local_path(st.tr) and _linear_gate(layer, gctx, x):
+    local = _local_path(st.tr)
+    if local and _linear_gate(layer, gctx, x):
         y, l_aux, capacity, (idx, loc) = _local_layer(layer, st, x, gctx, top_k, capacity, align)
         _note_stats(layer, st, q8, idx, loc, E, capacity, degree, x)
         return y, l_aux
@@ -667,6 +676,8 @@ def forward(layer, x, gctx, top_k, capacity_factor, degree):
             logits = clean + gctx.gate_noise * torch.randn_like(clean) / E
         logits = logits.contiguous()
     if capacity_factor == 0:
+        if q8 and not local:
+            align = SLICE_ROWS * degree
         capacity = _dynamic_capacity(lib, logits, top_k, layer.normalize_gate, layer.group, align)
         capacity += -capacity % align
 
@@ -689,7 +700,7 @@ def forward(layer, x, gctx, top_k, capacity_factor, degree):
         check_routing_bounds(idx, loc, slot_map, S, E, capacity, top_k)
     ex = layer.experts
     args = (gates, ex.batched_fc1_w, ex.batched_fc1_bias, ex.batched_fc2_w, ex.batched_fc2_bias)
-    if _local_path(st.tr):
+    if local:
         y = _local_experts(x, *args, dict(idx=idx, loc=loc, slot_map=slot_map, used=used, C=capacity,
                                           act=ACT_CODES[ex.act_name], postscore=layer.is_postscore, int8=q8,
                                           budget_ms=st.tr.budget_ms, status=st.tr.status))

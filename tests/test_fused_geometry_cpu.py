@@ -241,3 +241,29 @@ def test_routing_bounds_check_accepts_consistent_and_rejects_corrupt():
     bad = slot_map.clone(); bad[1] = 3; bad[2] = 2                       # two picks swapped: they no longer own their slots
     with pytest.raises(AssertionError):
         check_routing_bounds(idx, loc, bad, S, E, C, K)
+
+
+@pytest.mark.parametrize('world', [1, 2, 8])
+@pytest.mark.parametrize('degree', [1, 2, 3, 8])
+def test_int8_exchange_gets_whole_slices(world, degree, monkeypatch):
+    """Every capacity that the dispatch rule lets into the int8 exchange is a whole number of 32-row slices per chunk (the
+    GEMM launcher refuses others), and one rank, which lays its slots out by itself, is not restricted."""
+    from types import SimpleNamespace
+    from planmoe_b200.ops import fused_moe
+    monkeypatch.delenv('PLANMOE_FUSE_SEND', raising=False)
+    layer = SimpleNamespace(world_size=world, num_global_experts=8)
+    taken = 0
+    for local in ('1', '0'):
+        monkeypatch.setenv('PLANMOE_LOCAL', local)
+        for S in range(1, 1200, 7):
+            for cf in (1.0, 1.25, -0.7):
+                ok = fused_moe.int8_capacity_ok(layer, S, 2, cf, degree)
+                C = fused_moe._static_capacity(S, 8, 2, cf, 4 * degree)
+                assert C > 0 and C % (4 * degree) == 0
+                if world == 1 and local == '1':
+                    assert ok
+                else:
+                    assert ok == (C % degree == 0 and C // degree % fused_moe.SLICE_ROWS == 0)
+                    taken += ok
+        assert fused_moe.int8_capacity_ok(layer, 77, 2, 0.0, degree)
+    assert taken

@@ -227,6 +227,24 @@ def test_int8_dynamic_capacity_of_a_deep_pipeline():
         assert torch.equal(u, v)
 
 
+@pytest.mark.parametrize('S,cf,degree,path', [(1000, 1.01, 1, 'generic'), (1024, 1.0, 1, 'fused'), (1024, 1.0, 3, 'generic'),
+                                              (1000, 0.0, 1, 'fused'), (1000, 0.0, 3, 'fused'), (1000, 0.0, 20, 'fused')])
+def test_int8_exchange_takes_whole_slices_only(S, cf, degree, path, monkeypatch):
+    """Static capacities that are no whole slices per chunk take the generic path, dynamic ones are sized to fit."""
+    layer = _layer(8, 256, 384, 2, cf, compress_name='int8')
+    torch.manual_seed(13)
+    x = torch.randn(S, 256, device='cuda').bfloat16()
+    dy = torch.randn(S, 256, device='cuda').bfloat16()
+    here = _pass(layer, x, dy, degree=degree)
+    assert layer.last_stats['path'] == 'fused'
+    monkeypatch.setenv('PLANMOE_LOCAL', '0')
+    there = _pass(layer, x, dy, degree=degree)
+    assert layer.last_stats['path'] == path
+    if cf == 0:
+        assert layer.last_stats['capacity'] % (32 * degree) == 0
+    _int8_close(here, there)
+
+
 _VARIANT_CHILD = """
 import os, torch
 from tests.test_local_path_gpu import _close, _layer, _pass
