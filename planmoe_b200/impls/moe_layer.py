@@ -349,7 +349,8 @@ class MOELayer(torch.nn.Module):
         assert len(original_shape) >= 2, \
             "Input data must be at least 2D tensor: (s)amples, .., (m)odel_dim"
         x = input.reshape(-1, original_shape[-reserve_dims:].numel())
-        first = self.experts._parameters.get('batched_fc1_w')       # the FFN experts' first parameter
+        # tokens take the type of the experts' first parameter; the FFN experts' is known without a walk over all of them
+        first = getattr(self.experts, 'batched_fc1_w', None) if self.experts_type == 'ffn' else None
         if first is None:
             first = next(iter(self.experts.parameters()), None)
         if first is not None and x.dtype != first.dtype:

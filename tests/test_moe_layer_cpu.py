@@ -169,3 +169,48 @@ def test_all_tokens_to_one_expert_and_an_idle_expert():
     params = [layer.gates[0].wg.weight, ex.batched_fc1_w, ex.batched_fc1_bias, ex.batched_fc2_w, ex.batched_fc2_bias]
     yr, _ = dense_moe_reference(x.detach(), *[p.detach() for p in params], top_k=1, capacity_factor=1.0, alignment=4)
     assert torch.allclose(y, yr, atol=2e-5, rtol=1e-4)
+
+
+class _TwoTypes(torch.nn.Module):
+    """A custom expert with a parameter that shares its name with one of the FFN experts', but is not the first."""
+
+    def __init__(self):
+        super().__init__()
+        self.scale = torch.nn.Parameter(torch.full((), 2.0, dtype=torch.float64))
+        self.batched_fc1_w = torch.nn.Parameter(torch.ones(()))
+
+    def update(self, ctx):
+        pass
+
+    def forward(self, x, ctx):
+        return x * self.scale
+
+
+class _NoModule:
+    """The same duties without torch.nn.Module."""
+
+    def update(self, ctx):
+        pass
+
+    def named_parameters(self):
+        return []
+
+    def parameters(self):
+        return iter([])
+
+    def __call__(self, x, ctx):
+        return x * 2
+
+
+@pytest.mark.parametrize('expert,dtype', [(_TwoTypes, torch.float64), (_NoModule, torch.float32)])
+def test_tokens_take_the_type_of_a_custom_experts_first_parameter(expert, dtype):
+    layer = moe.moe_layer(gate_type={'type': 'top', 'k': 1, 'capacity_factor': 4.0}, model_dim=8,
+                          experts={'type': 'custom', 'count_per_node': 2, 'module': expert()}, seeds=(1, 2, 3))
+    layer.gates.to(dtype)
+    seen = []
+    layer.gates[0].register_forward_pre_hook(lambda mod, args: seen.append(args[0].dtype))
+    x = torch.randn(32, 8)
+    y = layer(x)
+    assert seen == [dtype] and y.dtype == x.dtype
+    scores = F.softmax(F.linear(x.to(dtype), layer.gates[0].wg.weight), dim=1).max(1, keepdim=True).values
+    torch.testing.assert_close(y, (2 * scores * x.to(dtype)).float(), rtol=1e-5, atol=1e-6)      # one pick: its score weighs it
