@@ -689,12 +689,14 @@ struct LocalGate {
   float eps() const { return bf16_logits ? 7.8125e-03f : kFloatEps; }
 };
 
+// `dgates` undefined: the loss alone has a gradient.
 static Tensor local_gate_backward(const LocalGate& g, const LocalRoute& r, const Tensor& dgates,
                                   const c10::optional<Tensor>& dl_aux) {
   const int S = g.logits.size(0), E = g.logits.size(1), K = r.idx.size(0);
   Tensor dl = torch::empty_like(g.logits);
   GatePtrs gp{};
-  for (int k = 0; k < K; ++k) gp.p[k] = dgates.data_ptr<float>() + (int64_t)k * S;
+  if (dgates.defined())
+    for (int k = 0; k < K; ++k) gp.p[k] = dgates.data_ptr<float>() + (int64_t)k * S;
   const float* f = nullptr;
   const void* h = nullptr;
   if (dl_aux.has_value() && dl_aux->defined()) {
@@ -706,6 +708,50 @@ static Tensor local_gate_backward(const LocalGate& g, const LocalRoute& r, const
   launch_gate_backward<float, false>(g.logits.data_ptr<float>(), S, E, K, g.normalize, g.eps(), r.idx.data_ptr<int>(), gp, f,
                                      g.top1.data_ptr<int>(), dl.data_ptr<float>(), cur_stream(), h);
   return dl;
+}
+
+// The gradient of the gate's weight from that of the logits, as partial sums and the job that adds them up into `dwg`;
+// returns the partial sums' memory.
+static Tensor gate_wgrad_job(const LocalGate& g, const Tensor& x, const Tensor& dl, ColsumJob& j, Tensor& dwg) {
+  const int64_t S = x.size(0), M = x.size(1), E = g.w.size(0);
+  const int chunks = gate_wgrad_chunks(S, M);
+  Tensor keep = torch::empty({(int64_t)chunks + 1, E * M}, dl.options());
+  const bool bf16 = g.w.scalar_type() == at::kBFloat16;
+  dwg = torch::empty_like(g.w);
+  float* partial = keep.data_ptr<float>();
+  count_launch(1);
+  launch_gate_wgrad(x.data_ptr(), dl.data_ptr<float>(), partial, S, E, M, cur_stream());
+  j.partial = partial;
+  j.out = bf16 ? partial + (int64_t)chunks * E * M : dwg.data_ptr<float>();
+  j.out_bf16 = bf16 ? dwg.data_ptr() : nullptr;
+  j.rows = (long long)chunks * 128; j.N = (int)(E * M); j.groups = j.fold = 1;
+  return keep;
+}
+
+// A backward that only the balance loss takes part in: the experts have no gradient then, the tokens and the gate's weight
+// theirs through the logits.
+static std::vector<Tensor> local_loss_backward(const Tensor& x, const LocalRoute& r, const LocalGate& gate,
+                                               const c10::optional<Tensor>& dl_aux, const std::vector<bool>& need,
+                                               const py::object& stages) {
+  c10::cuda::CUDAGuard guard(x.device());
+  const int64_t S = x.size(0), M = x.size(1), E = gate.w.size(0);
+  Tensor dx, dwg;
+  Stage st(stages, "bwd.gate_grad");
+  const Tensor dl = local_gate_backward(gate, r, Tensor(), dl_aux);
+  if (need[0]) {
+    const Tensor none = torch::full({1, S}, -1, r.idx.options());     // no pick has a slot: no row is read
+    dx = torch::empty_like(x);
+    count_launch(1);
+    launch_gather_gate(nullptr, nullptr, none.data_ptr<int>(), none.data_ptr<int>(), nullptr, dl.data_ptr<float>(),
+                       gate.w.data_ptr(), gate.w.scalar_type() == at::kBFloat16, dx.data_ptr(), 1, S, M, E, 0, cur_stream());
+  }
+  if (need[1]) {
+    ColsumJob j{};
+    const Tensor keep = gate_wgrad_job(gate, x, dl, j, dwg);
+    count_launch(1);
+    launch_colsum_jobs(&j, 1, cur_stream());
+  }
+  return {dx, dwg, {}, {}, {}, {}};
 }
 
 // {dx, dgates or dwg, dw1, db1, dw2, db2}: with `gate` the second is the gradient of the gate's weight and dx has the
@@ -799,17 +845,7 @@ static std::vector<Tensor> local_backward(const Tensor& dy, const Tensor& x, con
       ++n;
     }
     if (gate != nullptr && need[1]) {
-      const int chunks = gate_wgrad_chunks(S, M);
-      keep[n] = torch::empty({(int64_t)chunks + 1, E * M}, r.gates.options());
-      const bool bf16 = gate->w.scalar_type() == at::kBFloat16;
-      dwg = torch::empty_like(gate->w);
-      float* partial = keep[n].data_ptr<float>();
-      count_launch(1);
-      launch_gate_wgrad(x.data_ptr(), dl.data_ptr<float>(), partial, S, E, M, cur_stream());
-      j[n].partial = partial;
-      j[n].out = bf16 ? partial + (int64_t)chunks * E * M : dwg.data_ptr<float>();
-      j[n].out_bf16 = bf16 ? dwg.data_ptr() : nullptr;
-      j[n].rows = (long long)chunks * 128; j[n].N = (int)(E * M); j[n].groups = j[n].fold = 1;
+      keep[n] = gate_wgrad_job(*gate, x, dl, j[n], dwg);
       ++n;
     }
     if (n > 0) {
@@ -903,13 +939,15 @@ std::tuple<std::vector<Tensor>, int64_t> local_moe_forward_op(
            e[4], e[5], loc}, capacity};
 }
 
-std::vector<Tensor> local_moe_backward_op(const Tensor& dy, const c10::optional<Tensor>& dl_aux, const Tensor& x, const Tensor& wg,
+// `dy` undefined: see local_loss_backward
+std::vector<Tensor> local_moe_backward_op(const c10::optional<Tensor>& dy, const c10::optional<Tensor>& dl_aux, const Tensor& x, const Tensor& wg,
                                           const LocalRoute& r, const Tensor& w1, const Tensor& w2, const Tensor& logits,
                                           const Tensor& top1, const Tensor& xs, const Tensor& dact, const Tensor& h,
                                           const Tensor& ys, const c10::optional<Tensor>& scales, bool normalize,
                                           bool bf16_logits, const std::vector<bool>& need, const py::object& stages) {
   const LocalGate g{wg, logits, top1, normalize, bf16_logits};
-  return local_backward(dy, x, r, w1, w2, xs, dact, h, ys, scales, need, &g, dl_aux, stages);
+  if (!dy.has_value() || !dy->defined()) return local_loss_backward(x, r, g, dl_aux, need, stages);
+  return local_backward(*dy, x, r, w1, w2, xs, dact, h, ys, scales, need, &g, dl_aux, stages);
 }
 
 // rows [R, M] -> uint8 [R, M + 16]: M quantised bytes + {scale, low, 0, 0} (the wire rows of the fused send)

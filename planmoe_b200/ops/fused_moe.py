@@ -532,11 +532,12 @@ class _LocalLayer(torch.autograd.Function):
     def backward(ctx, dy, dl_aux):
         x, wg, w1, w2, logits, top1, slot_map, used, idx, loc, gates, xs, dact, h, ys, scales = ctx.saved_tensors
         m = ctx.m
-        if dy is None:
-            dy = torch.zeros((x.size(0), w2.size(2)), dtype=x.dtype, device=x.device)
+        if dy is None and dl_aux is None:
+            return (None,) * 7
         route = _local_route(gates, dict(m, C=xs.size(1), idx=idx, loc=loc, slot_map=slot_map, used=used))
-        return (*native.lib().local_moe_backward(_aligned(dy), dl_aux, x, wg, route, w1, w2, logits, top1, xs, dact, h, ys,
-                                                 scales, m['normalize'], m['bf16_logits'], list(ctx.needs_input_grad[:6]), _stages()),
+        return (*native.lib().local_moe_backward(_aligned(dy) if dy is not None else None, dl_aux, x, wg, route, w1, w2, logits,
+                                                 top1, xs, dact, h, ys, scales, m['normalize'], m['bf16_logits'],
+                                                 list(ctx.needs_input_grad[:6]), _stages()),
                 None)
 
 

@@ -245,6 +245,25 @@ def test_int8_exchange_takes_whole_slices_only(S, cf, degree, path, monkeypatch)
     _int8_close(here, there)
 
 
+@pytest.mark.parametrize('fp32_gate', [True, False])
+@pytest.mark.parametrize('S,M,E,k', [(500, 128, 4, 2), (33, 320, 9, 1)])
+def test_backward_of_the_balance_loss_alone(S, M, E, k, fp32_gate, monkeypatch):
+    """The experts take no part in it: no gradient, rather than one of zeros that an optimizer would act on."""
+    layer = _layer(E, M, 256, k, 1.0, fp32_gate=fp32_gate)
+    torch.manual_seed(14)
+    x0 = torch.randn(S, M, device='cuda').bfloat16()
+    out = []
+    for local in ('1', '0'):
+        monkeypatch.setenv('PLANMOE_LOCAL', local)
+        x = x0.clone().requires_grad_()
+        layer.zero_grad(set_to_none=True)
+        layer(x).l_aux.backward()
+        out.append([x.grad] + [p.grad for p in layer.parameters()])
+        layer.l_aux = None
+    assert sum(g is not None for g in out[0]) == 2
+    _close(*out)
+
+
 _VARIANT_CHILD = """
 import os, torch
 from tests.test_local_path_gpu import _close, _layer, _pass
