@@ -509,9 +509,16 @@ def _local_forward(x, gates, w1, b1, w2, b2, meta, want_grad):
     return native.lib().local_forward(x, route, w1, b1, w2, b2, want_grad, _stages())
 
 
+def _needs_node(tensors):
+    """Whether a call goes through its autograd function.  Forward-mode tangents and function transforms do not depend on
+    the gradient mode: the function refuses them, where the kernels would drop them without a word."""
+    return (torch.autograd.forward_ad._current_level >= 0 or torch._C._are_functorch_transforms_active()
+            or (torch.is_grad_enabled() and any(t.requires_grad for t in tensors)))
+
+
 def _local_experts(x, gates, w1, b1, w2, b2, meta):
     x, gates, meta = _aligned(x), gates.contiguous(), _whole_slices(meta)
-    if torch.is_grad_enabled() and any(t.requires_grad for t in (x, gates, w1, b1, w2, b2)):
+    if _needs_node((x, gates, w1, b1, w2, b2)):
         return _LocalExperts.apply(x, gates, w1, b1, w2, b2, meta)
     return _local_forward(x, gates, w1, b1, w2, b2, meta, False)[0]
 
@@ -576,7 +583,7 @@ def _local_layer(layer, st, x, gctx, top_k, capacity, align):
              postscore=layer.is_postscore, int8=layer.compress_name == 'int8', budget_ms=st.tr.budget_ms,
              status=st.tr.status)
     args = (_aligned(x), w, ex.batched_fc1_w, ex.batched_fc1_bias, ex.batched_fc2_w, ex.batched_fc2_bias)
-    if torch.is_grad_enabled() and any(t.requires_grad for t in args):
+    if _needs_node(args):
         y, l_aux = _LocalLayer.apply(*args, m)
     else:
         (y, l_aux, *saved, loc), m['capacity'] = _local_layer_forward(*args, m, False)

@@ -264,6 +264,25 @@ def test_backward_of_the_balance_loss_alone(S, M, E, k, fp32_gate, monkeypatch):
     _close(*out)
 
 
+@pytest.mark.parametrize('local', ['0', '1'])
+@pytest.mark.parametrize('plain_gate', [True, False])
+def test_forward_mode_is_refused_without_gradients_too(local, plain_gate, monkeypatch):
+    """No tangent is dropped: the kernels have no forward-mode rule, with or without the exchange."""
+    import torch.autograd.forward_ad as fwAD
+    monkeypatch.setenv('PLANMOE_LOCAL', local)
+    layer = _layer(4, 128, 256, 2, 1.0)
+    if not plain_gate:
+        layer.gates[0].register_forward_hook(lambda mod, args, out: out.detach())
+    x = torch.randn(64, 128, device='cuda').bfloat16()
+    with torch.no_grad():
+        with fwAD.dual_level():
+            with pytest.raises(NotImplementedError, match='jvp'):
+                layer(fwAD.make_dual(x, torch.ones_like(x)))
+        with pytest.raises(Exception):
+            torch.func.vmap(layer)(x.view(2, 32, 128))
+        assert torch.isfinite(layer(x)).all()
+
+
 _VARIANT_CHILD = """
 import os, torch
 from tests.test_local_path_gpu import _close, _layer, _pass
