@@ -918,7 +918,11 @@ std::tuple<std::vector<Tensor>, int64_t> local_moe_forward_op(
                                       w + 2 * K * S, reinterpret_cast<float*>(w + 2 * K * S + K * nblk * E), cur_stream(), perm,
                                       bf16_logits ? laux_bf16.data_ptr() : nullptr);
     if (dynamic) {
-      const Tensor host = counts[1].cpu();
+      Tensor host;
+      {
+        py::gil_scoped_release others;            // the wait for the stream keeps no other Python thread waiting
+        host = counts[1].cpu();
+      }
       int peak = 0;
       for (int64_t e = 0; e < E; ++e) peak = std::max(peak, host.data_ptr<int>()[e]);
       capacity = round_up(peak).cast<int64_t>();

@@ -4,6 +4,8 @@ that are no multiple of a row block, experts without a token, dropped tokens, ev
 import os
 import subprocess
 import sys
+import threading
+import time
 
 import pytest
 import torch
@@ -281,6 +283,32 @@ def test_forward_mode_is_refused_without_gradients_too(local, plain_gate, monkey
         with pytest.raises(Exception):
             torch.func.vmap(layer)(x.view(2, 32, 128))
         assert torch.isfinite(layer(x)).all()
+
+
+def test_other_threads_run_while_the_capacity_is_awaited():
+    layer = _layer(4, 128, 256, 2, 0.0)
+    x = torch.randn(512, 128, device='cuda').bfloat16()
+    beats, done = [], threading.Event()
+
+    def beat():
+        while not done.wait(0.005):
+            beats.append(time.perf_counter())
+
+    with torch.no_grad():
+        layer(x)
+        torch.cuda.synchronize()
+        other = threading.Thread(target=beat)
+        other.start()
+        try:
+            torch.cuda._sleep(900_000_000)                # about half a second of device time in front of the layer
+            start = time.perf_counter()
+            layer(x)
+            end = time.perf_counter()
+        finally:
+            done.set()
+            other.join()
+    assert end - start > 0.1
+    assert sum(start < t < end for t in beats) > 5
 
 
 _VARIANT_CHILD = """
