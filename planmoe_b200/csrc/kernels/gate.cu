@@ -181,7 +181,7 @@ gate_assign_kernel(int S, int E, int K, int C, int normalize, float eps,
     float denom = 0.f;
 #pragma unroll
     for (int k = 0; k < kMaxK; ++k) denom += k < K ? g[k] : 0.f;
-    denom = fmaxf(denom, eps);
+    denom = denom < eps ? eps : denom;             // like torch.clamp: a NaN stays one
 #pragma unroll
     for (int k = 0; k < kMaxK; ++k) {
       if (k >= K) break;
@@ -270,8 +270,8 @@ gate_bwd_kernel(const T* __restrict__ logits, int S, int E, int K, int normalize
     if (k >= K) break;                           // unrolled: the picks stay in registers
     const float dg = dgates.p[k] ? dgates.p[k][t] : 0.f;
     if (norm) {
-      if (denom > eps) ds_pick[k] = dg / denom - dot / (denom * denom);
-      else ds_pick[k] = dg / eps;
+      if (denom < eps) ds_pick[k] = dg / eps;
+      else ds_pick[k] = dg / denom - dot / (denom * denom);
     } else {
       ds_pick[k] = dg;
     }

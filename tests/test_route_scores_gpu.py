@@ -77,6 +77,27 @@ def test_unusual_scores(monkeypatch):
         assert sorted(loc[idx == e].tolist()) == list(range(int((idx == e).sum())))
 
 
+def test_gates_of_unusual_scores(monkeypatch):
+    """A NaN pick makes all gates of its token NaN, as the clamp of the composition does; infinities, negative and vanishing
+    sums likewise agree, with their gradients."""
+    scores = torch.rand(200, 6, generator=torch.Generator().manual_seed(4)).cuda()
+    scores[1, 3] = float('nan')
+    scores[2, 0], scores[2, 5] = float('nan'), float('inf')
+    scores[3, 1] = float('inf')
+    scores[4] = -scores[4]                                # sums below the clamp's bound
+    scores[5] *= 1e-9
+    scores[6, 2], scores[6, 4] = 3.0, -float('inf')
+    weights = torch.rand(2, 200, device='cuda')
+    got = []
+    for leaf, p, _ in _both(scores, monkeypatch, top_k=2):
+        grad, = torch.autograd.grad([p[3][0], p[3][1]], leaf, list(weights))
+        got.append((torch.stack(p[1]), torch.stack([g.detach() for g in p[3]]), grad))
+    (ia, ga, da), (ib, gb, db) = got
+    assert torch.equal(ia, ib) and bool(ga[:, 1].isnan().all())
+    torch.testing.assert_close(ga, gb, rtol=4e-7, atol=0, equal_nan=True)       # a sum of two scores and a division
+    torch.testing.assert_close(da, db, rtol=1e-5, atol=1e-5, equal_nan=True)
+
+
 def test_changed_lists_and_other_forms_take_the_composition(monkeypatch):
     from planmoe_b200.impls import fast_dispatch as FD, losses
     scores = torch.softmax(torch.randn(64, 4, device='cuda'), dim=1)
