@@ -284,7 +284,8 @@ Tensor gate_backward_op(const Tensor& logits, const Tensor& idx, const c10::opti
   return out;
 }
 
-// Routing from a [S, E] fp32 score matrix (extract_critical): {idx, loc, slot_map, top1, loss, gate of pick 0, 1, ...}.
+// Routing from a [S, E] fp32 score matrix (extract_critical): {idx, loc, slot_map, top1, loss, picks, gate of pick 0, 1, ...}.
+// picks: idx once more, for the gradient, which nobody else gets to write to.
 std::vector<Tensor> route_scores_op(const Tensor& scores, int64_t K, int64_t C, bool normalize) {
   count_launch(2);
   TORCH_CHECK(scores.is_cuda() && scores.dim() == 2 && scores.is_contiguous() && scores.scalar_type() == at::kFloat);
@@ -296,9 +297,10 @@ std::vector<Tensor> route_scores_op(const Tensor& scores, int64_t K, int64_t C, 
   const int64_t nblk = gate_workspace_blocks(S);
   Tensor idx = torch::empty({K, S}, iopt), loc = torch::empty({K, S}, iopt), smap = torch::empty({E * C}, iopt);
   Tensor top1 = torch::empty({E}, iopt), loss = torch::empty({}, scores.options());
+  Tensor picks = torch::empty({K, S}, iopt);
   Tensor ws = torch::empty({2 * K * S + (K + 1) * nblk * E}, iopt);
   int* w = ws.data_ptr<int>();
-  std::vector<Tensor> out{idx, loc, smap, top1, loss};
+  std::vector<Tensor> out{idx, loc, smap, top1, loss, picks};
   // the picks' gates are tensors of their own (no views of one another) on consecutive rows of one storage, so that who
   // wants them stacked need not copy
   GatePtrs gp{};
@@ -311,17 +313,22 @@ std::vector<Tensor> route_scores_op(const Tensor& scores, int64_t K, int64_t C, 
   launch_gate_forward<float, true>(scores.data_ptr<float>(), S, E, K, C, normalize, kFloatEps, idx.data_ptr<int>(),
                                    loc.data_ptr<int>(), gp, reinterpret_cast<float*>(w), smap.data_ptr<int>(),
                                    top1.data_ptr<int>(), nullptr, loss.data_ptr<float>(), w + K * S, w + 2 * K * S,
-                                   reinterpret_cast<float*>(w + 2 * K * S + K * nblk * E), cur_stream());
+                                   reinterpret_cast<float*>(w + 2 * K * S + K * nblk * E), cur_stream(), nullptr, nullptr,
+                                   picks.data_ptr<int>());
   return out;
 }
 
-Tensor route_scores_backward_op(const Tensor& scores, const Tensor& idx, const std::vector<c10::optional<Tensor>>& dgates,
-                                const c10::optional<Tensor>& dloss, const Tensor& top1, bool normalize) {
+// Gradient [S, E] of the scores from that of the gates (scores and picks as above) or, without picks, of the loss.
+Tensor route_scores_backward_op(const c10::optional<Tensor>& scores, const c10::optional<Tensor>& picks,
+                                const std::vector<c10::optional<Tensor>>& dgates, const c10::optional<Tensor>& dloss,
+                                const Tensor& top1, int64_t S, bool normalize) {
   count_launch(1);
-  const int S = scores.size(0), E = scores.size(1), K = idx.size(0);
-  c10::cuda::CUDAGuard guard(scores.device());
-  TORCH_CHECK((int)dgates.size() == K);
-  Tensor out = torch::empty_like(scores);
+  const int64_t E = top1.numel(), K = dgates.size();
+  c10::cuda::CUDAGuard guard(top1.device());
+  TORCH_CHECK(K == 0 || (scores.has_value() && scores->is_contiguous() && scores->numel() == S * E &&
+                         scores->scalar_type() == at::kFloat && picks.has_value() && picks->is_contiguous() &&
+                         picks->numel() == K * S));
+  Tensor out = torch::empty({S, E}, top1.options().dtype(at::kFloat));
   std::vector<Tensor> keep;
   GatePtrs gp{};
   for (int k = 0; k < K; ++k) {
@@ -332,7 +339,8 @@ Tensor route_scores_backward_op(const Tensor& scores, const Tensor& idx, const s
   }
   Tensor dl;
   if (dloss.has_value() && dloss->defined()) dl = dloss->to(at::kFloat).contiguous();
-  launch_gate_backward<float, true>(scores.data_ptr<float>(), S, E, K, normalize, kFloatEps, idx.data_ptr<int>(), gp,
+  launch_gate_backward<float, true>(K > 0 ? scores->data_ptr<float>() : nullptr, S, E, K, normalize, kFloatEps,
+                                    K > 0 ? picks->data_ptr<int>() : nullptr, gp,
                                     dl.defined() ? dl.data_ptr<float>() : nullptr, top1.data_ptr<int>(),
                                     out.data_ptr<float>(), cur_stream());
   return out;

@@ -143,7 +143,8 @@ gate_assign_kernel(int S, int E, int K, int C, int normalize, float eps,
                    int* __restrict__ used,        // [E] slots of expert e that hold a token, or null
                    float* __restrict__ l_aux,     // [1]
                    __nv_bfloat16* __restrict__ l_aux_bf16,   // [1] or null
-                   const int* __restrict__ perm)
+                   const int* __restrict__ perm,
+                   int* __restrict__ idx_copy)    // [K][S] or null
 {
   __shared__ int base[kMaxK][kMaxE];
   __shared__ float red[kMaxE];
@@ -188,6 +189,7 @@ gate_assign_kernel(int S, int E, int K, int C, int normalize, float eps,
       const int l = base[k][pick[k]] + rank[k];
       loc[(size_t)k * S + t] = l;
       gates.p[k][t] = norm ? g[k] / denom : g[k];
+      if (idx_copy != nullptr) idx_copy[(size_t)k * S + t] = pick[k];
       if (slot_map != nullptr && l < C) slot_map[(size_t)pick[k] * C + l] = t * K + k;
     }
   }
@@ -239,8 +241,13 @@ gate_bwd_kernel(const T* __restrict__ logits, int S, int E, int K, int normalize
   const int t = blockIdx.x * kGateBwdThreads + threadIdx.x;
   if (t >= S) return;
   float p[ME];
-  load_row<T, ME>(logits + (size_t)t * E, E, p);
-  if constexpr (!SCORES) softmax_row<ME>(p, E);
+  if (SCORES && K == 0) {                         // the loss alone: its gradient does not depend on the scores
+#pragma unroll
+    for (int e = 0; e < ME; ++e) p[e] = 0.f;
+  } else {
+    load_row<T, ME>(logits + (size_t)t * E, E, p);
+    if constexpr (!SCORES) softmax_row<ME>(p, E);
+  }
 
   // d(score): loss part for every expert, gate part for the picked ones
   const float dl = dl_aux ? dl_aux[0] : dl_aux_bf16 ? __bfloat162float(dl_aux_bf16[0]) : 0.f;
@@ -299,7 +306,7 @@ template <class T, bool SCORES>
 void launch_gate_forward(const T* logits, int S, int E, int K, int C, bool normalize, float eps,
                          int* idx, int* loc, GatePtrs gates, float* raw_gate, int* slot_map,
                          int* top1_count, int* used, float* l_aux, int* ws_rank, int* ws_blk_count,
-                         float* ws_blk_score, cudaStream_t stream, const int* perm, void* l_aux_bf16) {
+                         float* ws_blk_score, cudaStream_t stream, const int* perm, void* l_aux_bf16, int* idx_copy) {
   const int nblk = (S + kGateThreads - 1) / kGateThreads;
   auto stats = E <= 8 ? gate_stats_kernel<T, 8, SCORES> : E <= 16 ? gate_stats_kernel<T, 16, SCORES>
              : E <= 32 ? gate_stats_kernel<T, 32, SCORES> : gate_stats_kernel<T, 64, SCORES>;
@@ -308,7 +315,7 @@ void launch_gate_forward(const T* logits, int S, int E, int K, int C, bool norma
   gate_assign_kernel<<<nblk, kGateThreads, 0, stream>>>(S, E, K, C, normalize ? 1 : 0, eps, idx,
                                                       raw_gate, ws_rank, ws_blk_count, ws_blk_score,
                                                       nblk, loc, gates, slot_map, top1_count, used, l_aux,
-                                                      reinterpret_cast<__nv_bfloat16*>(l_aux_bf16), perm);
+                                                      reinterpret_cast<__nv_bfloat16*>(l_aux_bf16), perm, idx_copy);
 }
 
 template <class T, bool SCORES>
@@ -432,7 +439,7 @@ void launch_remap_slot_map(int* slot_map, long long n, const int* perm, int K, c
 #define INSTANTIATE(T, SCORES)                                                                    \
   template void launch_gate_forward<T, SCORES>(const T*, int, int, int, int, bool, float, int*, int*,     \
                                                GatePtrs, float*, int*, int*, int*, float*, int*, int*, float*, \
-                                               cudaStream_t, const int*, void*);                          \
+                                               cudaStream_t, const int*, void*, int*);                    \
   template void launch_gate_backward<T, SCORES>(const T*, int, int, int, bool, float, const int*, GatePtrs, \
                                                 const float*, const int*, T*, cudaStream_t, const void*);
 INSTANTIATE(float, false)

@@ -88,46 +88,49 @@ def _gates_of(gates_all, normalize_gate):
 
 class _RouteScores(torch.autograd.Function):
     """Top-k, gates, locations, slot map and the value of the GShard loss of fp32 scores in two launches; the gates'
-    gradient in one."""
+    gradient in one.  The picks that it uses are its own: the caller may change the lists of a plan in place."""
 
     @staticmethod
     def forward(ctx, scores, top_k, capacity, normalize):
         ctx.set_materialize_grads(False)
-        idx, loc, slot_map, top1, loss, *gates = native.lib().route_scores(scores, top_k, capacity, normalize)
-        ctx.save_for_backward(scores, idx, top1)
+        idx, loc, slot_map, top1, loss, picks, *gates = native.lib().route_scores(scores, top_k, capacity, normalize)
+        ctx.save_for_backward(scores, picks, top1)
         ctx.normalize = normalize
         ctx.mark_non_differentiable(loss, top1, idx, loc, slot_map)
         return (loss, top1, idx, loc, slot_map, *gates)
 
     @staticmethod
     def backward(ctx, _loss, _top1, _idx, _loc, _map, *dgates):
-        scores, idx, top1 = ctx.saved_tensors
         if all(d is None for d in dgates):
             return None, None, None, None
+        scores, picks, top1 = ctx.saved_tensors
         if torch.is_grad_enabled():             # create_graph: the same gradient as differentiable operations
-            pairs = [(g, d) for g, d in zip(_gates_of(scores.gather(1, idx.t().long()), ctx.normalize), dgates)
+            pairs = [(g, d) for g, d in zip(_gates_of(scores.gather(1, picks.t().long()), ctx.normalize), dgates)
                      if d is not None]
             return torch.autograd.grad([g for g, _ in pairs], scores, [d for _, d in pairs], create_graph=True)[0], \
                 None, None, None
-        return native.lib().route_scores_backward(scores, idx, list(dgates), None, top1, ctx.normalize), None, None, None
+        return native.lib().route_scores_backward(scores, picks, list(dgates), None, top1, scores.size(0), ctx.normalize), \
+            None, None, None
 
 
 class _RouteLoss(torch.autograd.Function):
     """The GShard loss that ``_RouteScores`` computed, as a node of its own: its backward can run before, after or without
-    the gates'."""
+    the gates'.  It is linear in the scores, sum_t sum_e scores[t, e] * top1[e] * E / S^2: their values may change before
+    the backward."""
 
     @staticmethod
-    def forward(ctx, scores, value, top1, idx):
-        ctx.save_for_backward(scores, idx, top1)
+    def forward(ctx, scores, value, top1):
+        ctx.save_for_backward(top1)
+        ctx.shape = scores.shape
         return value.detach()                   # its own tensor on the value's memory
 
     @staticmethod
     def backward(ctx, dloss):
-        scores, idx, top1 = ctx.saved_tensors
+        top1, = ctx.saved_tensors
+        S, E = ctx.shape
         if torch.is_grad_enabled():
-            return torch.autograd.grad(losses.gshard_loss(scores, idx.t()), scores, dloss, create_graph=True)[0], \
-                None, None, None
-        return native.lib().route_scores_backward(scores, idx, [None] * idx.size(0), dloss, top1, False), None, None, None
+            return (dloss * (E / (S * S)) * top1.to(dloss.dtype)).expand(S, E), None, None
+        return native.lib().route_scores_backward(None, None, [], dloss, top1, S, False), None, None
 
 
 def _route_on_kernels(scores, top_k, loss_fn):
@@ -157,7 +160,7 @@ def extract_critical(scores, top_k, loss_fn=losses.gshard_loss, capacity_factor=
         capacity = _align(top_k * int(capacity_factor * per_expert), alignment) if capacity_factor > 0 else 0
         scores = scores.contiguous()
         l_loss, top1, idx, loc, slot_map, *gates_s = _RouteScores.apply(scores, top_k, capacity, bool(normalize_gate))
-        l_loss = _RouteLoss.apply(scores, l_loss, top1, idx) if loss_fn is not None else None
+        l_loss = _RouteLoss.apply(scores, l_loss, top1) if loss_fn is not None else None
         if capacity_factor <= 0:
             peak = simple_all_reduce(loc.max(), group=group, op=torch.distributed.ReduceOp.MAX)
             capacity = int(peak) + 1

@@ -98,6 +98,31 @@ def test_gates_of_unusual_scores(monkeypatch):
     torch.testing.assert_close(da, db, rtol=1e-5, atol=1e-5, equal_nan=True)
 
 
+def test_what_may_change_in_place_before_the_backward(monkeypatch):
+    """As with the composition: the plan's lists may, the scores may for the loss, but not for the gates."""
+    from planmoe_b200.impls import fast_dispatch as FD
+    from planmoe_b200.jit_kernels import gating
+    scores = torch.softmax(torch.randn(300, 8, device='cuda'), dim=1)
+    weight = torch.rand(300, device='cuda')
+    got = []
+    for fast in (True, False):
+        monkeypatch.setattr(gating, 'use_fast_cumsum', fast)
+        leaf = scores.clone().requires_grad_()
+        plan, loss = FD.extract_critical(leaf, 2)
+        plan[1][0][::3] = -1                              # the caller drops some picks
+        plan[2][1].add_(5)
+        both, = torch.autograd.grad((plan[3][0] * weight).sum() + loss, leaf)
+        held = leaf * 1
+        plan, loss = FD.extract_critical(held, 2)
+        held.mul_(3)
+        alone, = torch.autograd.grad(loss, leaf, retain_graph=True)
+        with pytest.raises(RuntimeError, match='inplace'):
+            torch.autograd.grad(plan[3][0].sum(), leaf)
+        got.append((both, alone))
+    for u, v in zip(*got):
+        torch.testing.assert_close(u, v, rtol=1e-5, atol=1e-6)
+
+
 def test_changed_lists_and_other_forms_take_the_composition(monkeypatch):
     from planmoe_b200.impls import fast_dispatch as FD, losses
     scores = torch.softmax(torch.randn(64, 4, device='cuda'), dim=1)
