@@ -284,8 +284,8 @@ Tensor gate_backward_op(const Tensor& logits, const Tensor& idx, const c10::opti
   return out;
 }
 
-// Routing from a [S, E] fp32 score matrix (extract_critical): {idx, loc, slot_map, top1, loss, picks, gate of pick 0, 1, ...}.
-// picks: idx once more, for the gradient, which nobody else gets to write to.
+// Routing from a [S, E] fp32 score matrix (extract_critical): {idx, loc, slot_map, top1, loss, own, gate of pick 0, 1, ...}.
+// own [2, K, S]: idx and loc once more, for the gradient and the slots, which no caller gets to write to.
 std::vector<Tensor> route_scores_op(const Tensor& scores, int64_t K, int64_t C, bool normalize) {
   count_launch(2);
   TORCH_CHECK(scores.is_cuda() && scores.dim() == 2 && scores.is_contiguous() && scores.scalar_type() == at::kFloat);
@@ -297,10 +297,10 @@ std::vector<Tensor> route_scores_op(const Tensor& scores, int64_t K, int64_t C, 
   const int64_t nblk = gate_workspace_blocks(S);
   Tensor idx = torch::empty({K, S}, iopt), loc = torch::empty({K, S}, iopt), smap = torch::empty({E * C}, iopt);
   Tensor top1 = torch::empty({E}, iopt), loss = torch::empty({}, scores.options());
-  Tensor picks = torch::empty({K, S}, iopt);
+  Tensor own = torch::empty({2, K, S}, iopt);
   Tensor ws = torch::empty({2 * K * S + (K + 1) * nblk * E}, iopt);
   int* w = ws.data_ptr<int>();
-  std::vector<Tensor> out{idx, loc, smap, top1, loss, picks};
+  std::vector<Tensor> out{idx, loc, smap, top1, loss, own};
   // the picks' gates are tensors of their own (no views of one another) on consecutive rows of one storage, so that who
   // wants them stacked need not copy
   GatePtrs gp{};
@@ -314,11 +314,11 @@ std::vector<Tensor> route_scores_op(const Tensor& scores, int64_t K, int64_t C, 
                                    loc.data_ptr<int>(), gp, reinterpret_cast<float*>(w), smap.data_ptr<int>(),
                                    top1.data_ptr<int>(), nullptr, loss.data_ptr<float>(), w + K * S, w + 2 * K * S,
                                    reinterpret_cast<float*>(w + 2 * K * S + K * nblk * E), cur_stream(), nullptr, nullptr,
-                                   picks.data_ptr<int>());
+                                   own.data_ptr<int>());
   return out;
 }
 
-// Gradient [S, E] of the scores from that of the gates (scores and picks as above) or, without picks, of the loss.
+// Gradient [S, E] of the scores from that of the gates (picks: own[0]) or, without picks, of the loss.
 Tensor route_scores_backward_op(const c10::optional<Tensor>& scores, const c10::optional<Tensor>& picks,
                                 const std::vector<c10::optional<Tensor>>& dgates, const c10::optional<Tensor>& dloss,
                                 const Tensor& top1, int64_t S, bool normalize) {

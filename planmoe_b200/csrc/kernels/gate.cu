@@ -144,7 +144,7 @@ gate_assign_kernel(int S, int E, int K, int C, int normalize, float eps,
                    float* __restrict__ l_aux,     // [1]
                    __nv_bfloat16* __restrict__ l_aux_bf16,   // [1] or null
                    const int* __restrict__ perm,
-                   int* __restrict__ idx_copy)    // [K][S] or null
+                   int* __restrict__ copies)      // [2][K][S]: idx and loc once more, or null
 {
   __shared__ int base[kMaxK][kMaxE];
   __shared__ float red[kMaxE];
@@ -189,7 +189,10 @@ gate_assign_kernel(int S, int E, int K, int C, int normalize, float eps,
       const int l = base[k][pick[k]] + rank[k];
       loc[(size_t)k * S + t] = l;
       gates.p[k][t] = norm ? g[k] / denom : g[k];
-      if (idx_copy != nullptr) idx_copy[(size_t)k * S + t] = pick[k];
+      if (copies != nullptr) {
+        copies[(size_t)k * S + t] = pick[k];
+        copies[(size_t)(K + k) * S + t] = l;
+      }
       if (slot_map != nullptr && l < C) slot_map[(size_t)pick[k] * C + l] = t * K + k;
     }
   }
@@ -306,7 +309,7 @@ template <class T, bool SCORES>
 void launch_gate_forward(const T* logits, int S, int E, int K, int C, bool normalize, float eps,
                          int* idx, int* loc, GatePtrs gates, float* raw_gate, int* slot_map,
                          int* top1_count, int* used, float* l_aux, int* ws_rank, int* ws_blk_count,
-                         float* ws_blk_score, cudaStream_t stream, const int* perm, void* l_aux_bf16, int* idx_copy) {
+                         float* ws_blk_score, cudaStream_t stream, const int* perm, void* l_aux_bf16, int* copies) {
   const int nblk = (S + kGateThreads - 1) / kGateThreads;
   auto stats = E <= 8 ? gate_stats_kernel<T, 8, SCORES> : E <= 16 ? gate_stats_kernel<T, 16, SCORES>
              : E <= 32 ? gate_stats_kernel<T, 32, SCORES> : gate_stats_kernel<T, 64, SCORES>;
@@ -315,7 +318,7 @@ void launch_gate_forward(const T* logits, int S, int E, int K, int C, bool norma
   gate_assign_kernel<<<nblk, kGateThreads, 0, stream>>>(S, E, K, C, normalize ? 1 : 0, eps, idx,
                                                       raw_gate, ws_rank, ws_blk_count, ws_blk_score,
                                                       nblk, loc, gates, slot_map, top1_count, used, l_aux,
-                                                      reinterpret_cast<__nv_bfloat16*>(l_aux_bf16), perm, idx_copy);
+                                                      reinterpret_cast<__nv_bfloat16*>(l_aux_bf16), perm, copies);
 }
 
 template <class T, bool SCORES>

@@ -101,14 +101,14 @@ struct GatePtrs { float* p[4]; };
 // SCORES: the input is a [S, E] matrix of scores to pick from as they are; otherwise logits, softmax first.
 // slot_map: [E * C], written completely.  used (optional): [E] slots of every expert that hold a token; an expert's
 // slots are handed out from 0 on, so these are its first ones.  perm (optional): the order in which tokens claim slots.
-// slot_map may be null (no map).  l_aux_bf16 / dl_aux_bf16 (optional): the loss and its gradient in bf16.  idx_copy
-// (optional): idx a second time.
+// slot_map may be null (no map).  l_aux_bf16 / dl_aux_bf16 (optional): the loss and its gradient in bf16.  copies
+// (optional): [2][K][S], idx and loc a second time.
 template <class T, bool SCORES>
 void launch_gate_forward(const T* logits, int S, int E, int K, int C, bool normalize, float eps,
                          int* idx, int* loc, GatePtrs gates, float* raw_gate, int* slot_map,
                          int* top1_count, int* used, float* l_aux, int* ws_rank, int* ws_blk_count,
                          float* ws_blk_score, cudaStream_t stream, const int* perm = nullptr,
-                         void* l_aux_bf16 = nullptr, int* idx_copy = nullptr);
+                         void* l_aux_bf16 = nullptr, int* copies = nullptr);
 // With SCORES, K = 0 and null logits and idx: the gradient of the loss alone.
 template <class T, bool SCORES>
 void launch_gate_backward(const T* logits, int S, int E, int K, bool normalize, float eps,

@@ -35,8 +35,9 @@ class RoutingPlan(tuple):
     def __new__(cls, num_experts, indices_s, locations_s, gates_s, capacity, slots=None):
         self = super().__new__(cls, (num_experts, indices_s, locations_s, gates_s, capacity))
         self._slots = self._made = None
-        if slots is not None and not slots.idx.is_inference():
-            self._made = (slots, tuple(indices_s), tuple(locations_s), slots.idx._version, slots.loc._version)
+        lists = (*indices_s, *locations_s) if slots is not None else ()
+        if lists and not any(t.is_inference() for t in lists):
+            self._made = slots, [(t, t._version) for t in lists]
         return self
 
     @property
@@ -44,11 +45,9 @@ class RoutingPlan(tuple):
         if self._slots is None:
             if self._made is not None:
                 # the routing kernels' own stacked tensors, unless the lists were changed since
-                slots, indices, locations, vi, vl = self._made
-                if len(self[1]) == len(indices) and len(self[2]) == len(locations) \
-                        and all(a is b for a, b in zip(self[1], indices)) \
-                        and all(a is b for a, b in zip(self[2], locations)) \
-                        and slots.idx._version == vi and slots.loc._version == vl:
+                slots, made = self._made
+                lists = (*self[1], *self[2])
+                if len(lists) == len(made) and all(t is m and t._version == v for t, (m, v) in zip(lists, made)):
                     self._slots = slots
                     return slots
             idx = torch.stack([x.to(torch.int32).view(-1) for x in self[1]])
@@ -88,22 +87,24 @@ def _gates_of(gates_all, normalize_gate):
 
 class _RouteScores(torch.autograd.Function):
     """Top-k, gates, locations, slot map and the value of the GShard loss of fp32 scores in two launches; the gates'
-    gradient in one.  The picks that it uses are its own: the caller may change the lists of a plan in place."""
+    gradient in one.  The gradient and the slots use the last output, a second copy of picks and locations: the caller may
+    change the lists of a plan in place."""
 
     @staticmethod
     def forward(ctx, scores, top_k, capacity, normalize):
         ctx.set_materialize_grads(False)
-        idx, loc, slot_map, top1, loss, picks, *gates = native.lib().route_scores(scores, top_k, capacity, normalize)
-        ctx.save_for_backward(scores, picks, top1)
+        idx, loc, slot_map, top1, loss, own, *gates = native.lib().route_scores(scores, top_k, capacity, normalize)
+        ctx.save_for_backward(scores, own, top1)
         ctx.normalize = normalize
-        ctx.mark_non_differentiable(loss, top1, idx, loc, slot_map)
-        return (loss, top1, idx, loc, slot_map, *gates)
+        ctx.mark_non_differentiable(loss, top1, idx, loc, slot_map, own)
+        return (loss, top1, idx, loc, slot_map, own, *gates)
 
     @staticmethod
-    def backward(ctx, _loss, _top1, _idx, _loc, _map, *dgates):
+    def backward(ctx, _loss, _top1, _idx, _loc, _map, _own, *dgates):
         if all(d is None for d in dgates):
             return None, None, None, None
-        scores, picks, top1 = ctx.saved_tensors
+        scores, own, top1 = ctx.saved_tensors
+        picks = own[0]
         if torch.is_grad_enabled():             # create_graph: the same gradient as differentiable operations
             pairs = [(g, d) for g, d in zip(_gates_of(scores.gather(1, picks.t().long()), ctx.normalize), dgates)
                      if d is not None]
@@ -159,7 +160,7 @@ def extract_critical(scores, top_k, loss_fn=losses.gshard_loss, capacity_factor=
     if not batch_prioritized_routing and _route_on_kernels(scores, top_k, loss_fn):
         capacity = _align(top_k * int(capacity_factor * per_expert), alignment) if capacity_factor > 0 else 0
         scores = scores.contiguous()
-        l_loss, top1, idx, loc, slot_map, *gates_s = _RouteScores.apply(scores, top_k, capacity, bool(normalize_gate))
+        l_loss, top1, idx, loc, slot_map, own, *gates_s = _RouteScores.apply(scores, top_k, capacity, bool(normalize_gate))
         l_loss = _RouteLoss.apply(scores, l_loss, top1) if loss_fn is not None else None
         if capacity_factor <= 0:
             peak = simple_all_reduce(loc.max(), group=group, op=torch.distributed.ReduceOp.MAX)
@@ -168,7 +169,7 @@ def extract_critical(scores, top_k, loss_fn=losses.gshard_loss, capacity_factor=
                 capacity = min(capacity, top_k * int(-capacity_factor * per_expert))
             capacity, slot_map = _align(capacity, alignment), None
         plan = RoutingPlan(E, list(idx.unbind(0)), list(loc.unbind(0)), gates_s, capacity,
-                           D.SlotPlan(idx, loc, E, capacity, slot_map))
+                           D.SlotPlan(own[0], own[1], E, capacity, slot_map))
         return plan, l_loss
     topk_indices = torch.topk(scores, top_k, dim=1).indices
     gates_all = scores.gather(1, topk_indices)                      # [S, k], differentiable

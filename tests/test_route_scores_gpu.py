@@ -123,6 +123,30 @@ def test_what_may_change_in_place_before_the_backward(monkeypatch):
         torch.testing.assert_close(u, v, rtol=1e-5, atol=1e-6)
 
 
+@pytest.mark.parametrize('cf', [1.0, 0.0])
+def test_lists_changed_after_the_first_use_of_a_plan(cf, monkeypatch):
+    """The slots of a plan are laid down by its first use: neither decode nor the gradients see later changes of the lists."""
+    from planmoe_b200.impls import fast_dispatch as FD
+    from planmoe_b200.jit_kernels import gating
+    scores = torch.softmax(torch.randn(300, 8, device='cuda'), dim=1)
+    x = torch.randn(300, 64, device='cuda')
+    dy = torch.randn(300, 64, device='cuda')
+    got = []
+    for fast in (True, False):
+        monkeypatch.setattr(gating, 'use_fast_cumsum', fast)
+        leaf, xl = scores.clone().requires_grad_(), x.clone().requires_grad_()
+        plan, _ = FD.extract_critical(leaf, 2, capacity_factor=cf)
+        slots = FD.fast_encode(xl, plan)
+        plan[1][0].add_(1).remainder_(8)
+        plan[2][1].add_(3)
+        y = FD.fast_decode(slots, plan)
+        plan[2][0].add_(3)
+        y.backward(dy)
+        got.append((slots.detach(), y.detach(), xl.grad, leaf.grad))
+    for u, v in zip(*got):
+        torch.testing.assert_close(u, v, rtol=1e-5, atol=1e-5)
+
+
 def test_changed_lists_and_other_forms_take_the_composition(monkeypatch):
     from planmoe_b200.impls import fast_dispatch as FD, losses
     scores = torch.softmax(torch.randn(64, 4, device='cuda'), dim=1)
