@@ -285,7 +285,7 @@ Tensor gate_backward_op(const Tensor& logits, const Tensor& idx, const c10::opti
 }
 
 // Routing from a [S, E] fp32 score matrix (extract_critical): {idx, loc, slot_map, top1, loss, own, gate of pick 0, 1, ...}.
-// own [2, K, S]: idx and loc once more, for the gradient and the slots, which no caller gets to write to.
+// own [3, K, S]: idx, loc and gates (fp32) once more, for the gradients and the slots, which no caller gets to write to.
 std::vector<Tensor> route_scores_op(const Tensor& scores, int64_t K, int64_t C, bool normalize) {
   count_launch(2);
   TORCH_CHECK(scores.is_cuda() && scores.dim() == 2 && scores.is_contiguous() && scores.scalar_type() == at::kFloat);
@@ -297,17 +297,13 @@ std::vector<Tensor> route_scores_op(const Tensor& scores, int64_t K, int64_t C, 
   const int64_t nblk = gate_workspace_blocks(S);
   Tensor idx = torch::empty({K, S}, iopt), loc = torch::empty({K, S}, iopt), smap = torch::empty({E * C}, iopt);
   Tensor top1 = torch::empty({E}, iopt), loss = torch::empty({}, scores.options());
-  Tensor own = torch::empty({2, K, S}, iopt);
+  Tensor own = torch::empty({3, K, S}, iopt);
   Tensor ws = torch::empty({2 * K * S + (K + 1) * nblk * E}, iopt);
   int* w = ws.data_ptr<int>();
   std::vector<Tensor> out{idx, loc, smap, top1, loss, own};
-  // the picks' gates are tensors of their own (no views of one another) on consecutive rows of one storage, so that who
-  // wants them stacked need not copy
   GatePtrs gp{};
-  const Tensor rows = torch::empty({K, S}, scores.options());
-  for (int k = 0; k < K; ++k) {
-    out.push_back(torch::empty({0}, scores.options()));
-    out.back().set_(rows.storage(), k * S, {S}, {1});
+  for (int k = 0; k < K; ++k) {                   // tensors of their own, no views of one another
+    out.push_back(torch::empty({S}, scores.options()));
     gp.p[k] = out.back().data_ptr<float>();
   }
   launch_gate_forward<float, true>(scores.data_ptr<float>(), S, E, K, C, normalize, kFloatEps, idx.data_ptr<int>(),

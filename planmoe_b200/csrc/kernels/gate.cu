@@ -144,7 +144,7 @@ gate_assign_kernel(int S, int E, int K, int C, int normalize, float eps,
                    float* __restrict__ l_aux,     // [1]
                    __nv_bfloat16* __restrict__ l_aux_bf16,   // [1] or null
                    const int* __restrict__ perm,
-                   int* __restrict__ copies)      // [2][K][S]: idx and loc once more, or null
+                   int* __restrict__ copies)      // [3][K][S]: idx, loc and gates (fp32) once more, or null
 {
   __shared__ int base[kMaxK][kMaxE];
   __shared__ float red[kMaxE];
@@ -188,10 +188,12 @@ gate_assign_kernel(int S, int E, int K, int C, int normalize, float eps,
       if (k >= K) break;
       const int l = base[k][pick[k]] + rank[k];
       loc[(size_t)k * S + t] = l;
-      gates.p[k][t] = norm ? g[k] / denom : g[k];
+      const float gate = norm ? g[k] / denom : g[k];
+      gates.p[k][t] = gate;
       if (copies != nullptr) {
         copies[(size_t)k * S + t] = pick[k];
         copies[(size_t)(K + k) * S + t] = l;
+        copies[(size_t)(2 * K + k) * S + t] = __float_as_int(gate);
       }
       if (slot_map != nullptr && l < C) slot_map[(size_t)pick[k] * C + l] = t * K + k;
     }

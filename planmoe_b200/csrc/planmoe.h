@@ -102,7 +102,7 @@ struct GatePtrs { float* p[4]; };
 // slot_map: [E * C], written completely.  used (optional): [E] slots of every expert that hold a token; an expert's
 // slots are handed out from 0 on, so these are its first ones.  perm (optional): the order in which tokens claim slots.
 // slot_map may be null (no map).  l_aux_bf16 / dl_aux_bf16 (optional): the loss and its gradient in bf16.  copies
-// (optional): [2][K][S], idx and loc a second time.
+// (optional): [3][K][S], idx, loc and gates (fp32) a second time.
 template <class T, bool SCORES>
 void launch_gate_forward(const T* logits, int S, int E, int K, int C, bool normalize, float eps,
                          int* idx, int* loc, GatePtrs gates, float* raw_gate, int* slot_map,

@@ -28,28 +28,34 @@ from ..ops import dispatch as D
 from ..ops import native
 
 
+def _versions(tensors):
+    """What ``_unchanged`` compares with, None where versions are not counted (inference tensors)."""
+    return None if any(t.is_inference() for t in tensors) else [(t, t._version) for t in tensors]
+
+
+def _unchanged(tensors, made):
+    return made is not None and len(tensors) == len(made) and all(t is m and t._version == v for t, (m, v) in zip(tensors, made))
+
+
 class RoutingPlan(tuple):
     """The 5-tuple ``(E, indices_s, locations_s, gates_s, capacity)`` plus cached stacked
-    tensors for the kernels (``.slots`` is an ``ops.dispatch.SlotPlan``)."""
+    tensors for the kernels (``.slots`` is an ``ops.dispatch.SlotPlan``).  ``slots`` and ``rows`` (fp32 gates ``[K, S]``) are
+    what the lists say in memory of their own; each is used as long as its lists are what they were."""
 
-    def __new__(cls, num_experts, indices_s, locations_s, gates_s, capacity, slots=None):
+    def __new__(cls, num_experts, indices_s, locations_s, gates_s, capacity, slots=None, rows=None):
         self = super().__new__(cls, (num_experts, indices_s, locations_s, gates_s, capacity))
-        self._slots = self._made = None
-        lists = (*indices_s, *locations_s) if slots is not None else ()
-        if lists and not any(t.is_inference() for t in lists):
-            self._made = slots, [(t, t._version) for t in lists]
+        self._slots = None
+        self._made = slots, _versions((*indices_s, *locations_s)) if slots is not None else None
+        self._rows = rows, _versions(gates_s) if rows is not None else None
         return self
 
     @property
     def slots(self):
         if self._slots is None:
-            if self._made is not None:
-                # the routing kernels' own stacked tensors, unless the lists were changed since
-                slots, made = self._made
-                lists = (*self[1], *self[2])
-                if len(lists) == len(made) and all(t is m and t._version == v for t, (m, v) in zip(lists, made)):
-                    self._slots = slots
-                    return slots
+            slots, made = self._made
+            if _unchanged((*self[1], *self[2]), made):
+                self._slots = slots
+                return slots
             idx = torch.stack([x.to(torch.int32).view(-1) for x in self[1]])
             loc = torch.stack([x.to(torch.int32).view(-1) for x in self[2]])
             self._slots = D.SlotPlan(idx, loc, self[0], self[4])
@@ -57,6 +63,11 @@ class RoutingPlan(tuple):
 
     def stacked_gates(self):
         return torch.stack(list(self[3]))
+
+    def gate_rows(self):
+        """The gates as they are now, detached, in memory that the lists' owner does not write to."""
+        rows, made = self._rows
+        return rows if _unchanged(self[3], made) else torch.stack([g.detach() for g in self[3]])
 
 
 def _as_plan(crit):
@@ -87,8 +98,8 @@ def _gates_of(gates_all, normalize_gate):
 
 class _RouteScores(torch.autograd.Function):
     """Top-k, gates, locations, slot map and the value of the GShard loss of fp32 scores in two launches; the gates'
-    gradient in one.  The gradient and the slots use the last output, a second copy of picks and locations: the caller may
-    change the lists of a plan in place."""
+    gradient in one.  Gradients and slots use ``own``, a second copy of picks, locations and gates: the caller may change the
+    lists of a plan in place."""
 
     @staticmethod
     def forward(ctx, scores, top_k, capacity, normalize):
@@ -169,7 +180,7 @@ def extract_critical(scores, top_k, loss_fn=losses.gshard_loss, capacity_factor=
                 capacity = min(capacity, top_k * int(-capacity_factor * per_expert))
             capacity, slot_map = _align(capacity, alignment), None
         plan = RoutingPlan(E, list(idx.unbind(0)), list(loc.unbind(0)), gates_s, capacity,
-                           D.SlotPlan(own[0], own[1], E, capacity, slot_map))
+                           D.SlotPlan(own[0], own[1], E, capacity, slot_map), own[2].view(torch.float32))
         return plan, l_loss
     topk_indices = torch.topk(scores, top_k, dim=1).indices
     gates_all = scores.gather(1, topk_indices)                      # [S, k], differentiable
@@ -248,7 +259,7 @@ def fast_encode(data, critial_data, is_postscore=True):
     """[S, M] tokens -> [E, C, M] expert slots (gate-weighted iff ``not is_postscore``)."""
     plan = _as_plan(critial_data)
     if not is_postscore and D.picks_ok(data, plan.slots, plan[3]):
-        return D.scatter_picks(data, plan.slots, plan[3]).view(plan[0], -1, data.size(-1))
+        return D.scatter_picks(data, plan.slots, plan.gate_rows(), plan[3]).view(plan[0], -1, data.size(-1))
     gates = None if is_postscore else plan.stacked_gates().to(data.dtype)
     return D.scatter(data, plan.slots, gates).view(plan[0], -1, data.size(-1))
 
@@ -257,6 +268,6 @@ def fast_decode(data, critial_data, is_postscore=True):
     """[E, C, M] expert slots -> [S, M] tokens (gate-weighted iff ``is_postscore``)."""
     plan = _as_plan(critial_data)
     if is_postscore and D.picks_ok(data, plan.slots, plan[3]):
-        return D.gather_picks(data.reshape(-1, data.size(-1)), plan.slots, plan[3])
+        return D.gather_picks(data.reshape(-1, data.size(-1)), plan.slots, plan.gate_rows(), plan[3])
     gates = plan.stacked_gates().to(data.dtype) if is_postscore else None
     return D.gather(data.reshape(-1, data.size(-1)), plan.slots, gates)

@@ -174,64 +174,53 @@ class _Gather(torch.autograd.Function):
         return ddisp, dg, None
 
 
-def _rows_of(gates):
-    """The fp32 gates of every pick as one ``[K, S]``: a look at their memory where they lie on consecutive rows of one
-    storage (the routing kernels' do), a copy otherwise."""
-    first = gates[0].detach()
-    n, at = first.numel(), first.storage_offset()
-    base = first.untyped_storage().data_ptr()
-    if all(g.is_contiguous() and g.storage_offset() == at + k * n and g.untyped_storage().data_ptr() == base
-           for k, g in enumerate(gates)):
-        return first.as_strided((len(gates), n), (n, 1))
-    return torch.stack([g.detach() for g in gates])
-
-
 class _ScatterPicks(torch.autograd.Function):
-    """``_Scatter`` with the gates as one fp32 tensor per pick, rounded to the data's type by the kernels."""
+    """``_Scatter`` with the gates as fp32 ``rows [K, S]``, rounded to the data's type by the kernels; their gradient goes to
+    the picks' own tensors."""
 
     @staticmethod
-    def forward(ctx, x, plan, *gates):
+    def forward(ctx, x, plan, rows, *gates):
         ctx.plan, ctx.round = plan, x.dtype != torch.float32
         ctx.set_materialize_grads(False)
-        ctx.save_for_backward(x, *gates)
-        return native.lib().dispatch_scatter(x.contiguous(), plan.slot_map, _rows_of(gates), plan.K, plan.E * plan.C, ctx.round)
+        ctx.save_for_backward(x, rows)
+        return native.lib().dispatch_scatter(x.contiguous(), plan.slot_map, rows, plan.K, plan.E * plan.C, ctx.round)
 
     @staticmethod
     def backward(ctx, ddisp):
-        x, *gates = ctx.saved_tensors
+        x, rows = ctx.saved_tensors
         plan = ctx.plan
         if ddisp is None:
-            return (None,) * (2 + len(gates))
+            return (None,) * (3 + plan.K)
         ddisp = ddisp.contiguous()
-        dx = native.lib().dispatch_gather(ddisp, plan.idx, plan.loc, _rows_of(gates), plan.C, ctx.round)
-        dg = [None] * len(gates)
-        if any(ctx.needs_input_grad[2:]):
+        dx = native.lib().dispatch_gather(ddisp, plan.idx, plan.loc, rows, plan.C, ctx.round)
+        dg = [None] * plan.K
+        if any(ctx.needs_input_grad[3:]):
             dg = _gate_grad(ddisp, x, plan).unbind(0)
-        return (dx, None, *dg)
+        return (dx, None, None, *dg)
 
 
 class _GatherPicks(torch.autograd.Function):
-    """``_Gather`` with the gates as one fp32 tensor per pick."""
+    """``_Gather`` with the gates as fp32 ``rows [K, S]``."""
 
     @staticmethod
-    def forward(ctx, disp, plan, *gates):
+    def forward(ctx, disp, plan, rows, *gates):
         ctx.plan, ctx.round = plan, disp.dtype != torch.float32
         ctx.set_materialize_grads(False)
-        ctx.save_for_backward(disp, *gates)
-        return native.lib().dispatch_gather(disp.contiguous(), plan.idx, plan.loc, _rows_of(gates), plan.C, ctx.round)
+        ctx.save_for_backward(disp, rows)
+        return native.lib().dispatch_gather(disp.contiguous(), plan.idx, plan.loc, rows, plan.C, ctx.round)
 
     @staticmethod
     def backward(ctx, dy):
-        disp, *gates = ctx.saved_tensors
+        disp, rows = ctx.saved_tensors
         plan = ctx.plan
         if dy is None:
-            return (None,) * (2 + len(gates))
+            return (None,) * (3 + plan.K)
         dy = dy.contiguous()
-        ddisp = native.lib().dispatch_scatter(dy, plan.slot_map, _rows_of(gates), plan.K, plan.E * plan.C, ctx.round)
-        dg = [None] * len(gates)
-        if any(ctx.needs_input_grad[2:]):
+        ddisp = native.lib().dispatch_scatter(dy, plan.slot_map, rows, plan.K, plan.E * plan.C, ctx.round)
+        dg = [None] * plan.K
+        if any(ctx.needs_input_grad[3:]):
             dg = _gate_grad(disp, dy, plan).unbind(0)
-        return (ddisp, None, *dg)
+        return (ddisp, None, None, *dg)
 
 
 def picks_ok(x, plan, gates):
@@ -240,12 +229,12 @@ def picks_ok(x, plan, gates):
             and all(g.dtype == torch.float32 and g.device == x.device and g.shape == (plan.S,) for g in gates))
 
 
-def scatter_picks(x, plan, gates):
-    return _ScatterPicks.apply(x, plan, *gates)
+def scatter_picks(x, plan, rows, gates):
+    return _ScatterPicks.apply(x, plan, rows, *gates)
 
 
-def gather_picks(disp, plan, gates):
-    return _GatherPicks.apply(disp, plan, *gates)
+def gather_picks(disp, plan, rows, gates):
+    return _GatherPicks.apply(disp, plan, rows, *gates)
 
 
 def scatter(x, plan, gates=None):

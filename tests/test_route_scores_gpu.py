@@ -147,6 +147,34 @@ def test_lists_changed_after_the_first_use_of_a_plan(cf, monkeypatch):
         torch.testing.assert_close(u, v, rtol=1e-5, atol=1e-5)
 
 
+@pytest.mark.parametrize('dtype', [torch.float32, torch.float16])
+@pytest.mark.parametrize('postscore', [True, False])
+@pytest.mark.parametrize('before', [True, False])
+def test_gates_changed_around_the_uses_of_a_plan(dtype, postscore, before, monkeypatch):
+    """Encode and decode each take the gates as they are at the call, and keep them for their gradients."""
+    from planmoe_b200.impls import fast_dispatch as FD
+    from planmoe_b200.jit_kernels import gating
+    scores = torch.softmax(torch.randn(300, 8, device='cuda'), dim=1)
+    x = torch.randn(300, 64, device='cuda').to(dtype)
+    dy = torch.randn(300, 64, device='cuda').to(dtype)
+    got = []
+    for fast in (True, False):
+        monkeypatch.setattr(gating, 'use_fast_cumsum', fast)
+        leaf, xl = scores.clone().requires_grad_(), x.clone().requires_grad_()
+        plan, _ = FD.extract_critical(leaf, 2)
+        if before:
+            plan[3][1].mul_(0.5)
+        slots = FD.fast_encode(xl, plan, postscore)
+        y = FD.fast_decode(slots, plan, postscore)
+        with torch.no_grad():
+            plan[3][0].mul_(7.0)                          # the caller's own use of the list, afterwards
+        y.backward(dy)
+        got.append((slots.detach(), y.detach(), xl.grad, leaf.grad))
+    eps = torch.finfo(dtype).eps
+    for u, v in zip(*got):                                # the composition rounds the gates' gradient to the data's type
+        assert float((u.float() - v.float()).abs().max()) <= 4 * eps * float(v.float().abs().max()) + 1e-6
+
+
 def test_changed_lists_and_other_forms_take_the_composition(monkeypatch):
     from planmoe_b200.impls import fast_dispatch as FD, losses
     scores = torch.softmax(torch.randn(64, 4, device='cuda'), dim=1)
@@ -179,7 +207,8 @@ def test_encode_and_decode_by_pick(dtype, postscore, S, E, k):
         xl, sl = x.clone().requires_grad_(), scores.clone().requires_grad_()
         plan, _ = FD.extract_critical(sl, k, capacity_factor=0.8)
         gates = [g * 1 for g in plan[3]] if form == 'separate' else plan[3]
-        plan = FD.RoutingPlan(plan[0], plan[1], plan[2], gates, plan[4], plan.slots)
+        if form != 'made':
+            plan = FD.RoutingPlan(plan[0], plan[1], plan[2], gates, plan[4], plan.slots)
         if form == 'stacked':
             g = plan.stacked_gates().to(dtype)
             slots = D.scatter(xl, plan.slots, None if postscore else g)
