@@ -1,6 +1,7 @@
 """One rank without the exchange against the exchange of one rank (PLANMOE_LOCAL=0), over the forms both take: capacities
 that are no multiple of a row block, experts without a token, dropped tokens, every number of picks."""
 
+import contextlib
 import os
 import subprocess
 import sys
@@ -91,16 +92,46 @@ def test_rows_off_the_vector_boundary():
         assert torch.equal(layer(off), layer(off.clone()))
 
 
-def test_unused_rows_are_never_read():
-    """Memory that an earlier tensor left behind as NaN shows up nowhere, whatever the blocks behind the used rows hold."""
-    layer = _layer(4, 128, 256, 2, 4.0)
-    x = torch.randn(500, 128, device='cuda').bfloat16()
+@contextlib.contextmanager
+def _poisoned():
+    """New floating-point tensors start as NaN."""
+    before = torch.are_deterministic_algorithms_enabled(), torch.is_deterministic_algorithms_warn_only_enabled()
+    fill = torch.utils.deterministic.fill_uninitialized_memory
+    torch.use_deterministic_algorithms(True, warn_only=True)
+    torch.utils.deterministic.fill_uninitialized_memory = True
+    try:
+        yield
+    finally:
+        torch.use_deterministic_algorithms(before[0], warn_only=before[1])
+        torch.utils.deterministic.fill_uninitialized_memory = fill
+
+
+@pytest.mark.parametrize('wire', ['no', 'int8'])
+def test_unused_rows_are_never_read(wire):
+    """Rows behind an expert's last used block are not written (they keep the NaN that every tensor starts with here), and
+    show up in no result; two experts have no token at all."""
+    from planmoe_b200.ops import native
+    from planmoe_b200.parallel import transport
+    layer = _layer(4, 128, 256, 2, 4.0, compress_name=wire)
+    with torch.no_grad():
+        layer.gates[0].wg.weight[2:].mul_(0).sub_(0.05)   # tokens with a positive sum never reach experts 2 and 3
+    torch.manual_seed(6)
+    x = torch.rand(500, 128, device='cuda').bfloat16()
     dy = torch.randn(500, 128, device='cuda').bfloat16()
     first = _pass(layer, x, dy)
-    torch.full((64 << 20,), float('nan'), device='cuda')              # freed at once: the next pass may be given it
-    again = _pass(layer, x, dy)
+    ex, tr = layer.experts, transport.get_transport(layer.group)
+    with _poisoned():
+        again = _pass(layer, x, dy)
+        out, capacity = native.lib().local_moe_forward(
+            x, layer.gates[0].wg.weight, ex.batched_fc1_w, ex.batched_fc1_bias, ex.batched_fc2_w, ex.batched_fc2_bias, 2, 1000,
+            None, True, False, False, 1, True, wire == 'int8', tr.budget_ms, tr.status.device_ptr(), True, None)
     for u, v in zip(first, again):
         assert torch.equal(u, v) and torch.isfinite(u).all()
+    used, rows, h = out[5].tolist(), out[9], out[11]
+    assert used == [500, 500, 0, 0] and rows.size(1) >= capacity
+    for slots in (rows, h):
+        assert slots[:2, 512:].isnan().all() and slots[2:, 256:].isnan().all()
+        assert torch.isfinite(slots[:2, :512]).all() and torch.isfinite(slots[2:, :256]).all()
 
 
 @pytest.mark.parametrize('fp32_gate,S', [(False, 33), (False, 4097), (True, 515)])
@@ -314,7 +345,8 @@ def test_other_threads_run_while_the_capacity_is_awaited():
 _VARIANT_CHILD = """
 import os, torch
 from tests.test_local_path_gpu import _close, _layer, _pass
-torch.use_deterministic_algorithms(True, warn_only=True)      # new tensors start as NaN
+torch.use_deterministic_algorithms(True, warn_only=True)
+torch.utils.deterministic.fill_uninitialized_memory = True    # new tensors start as NaN
 layer = _layer(4, 128, 256, 2, 2.0)
 x = torch.randn(700, 128, device='cuda').bfloat16()
 dy = torch.randn_like(x)
