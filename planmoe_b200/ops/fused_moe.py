@@ -607,12 +607,12 @@ def int8_capacity_ok(layer, S, top_k, capacity_factor, degree):
 
 
 def _capacity_step(cap, align):
-    """``cap`` rounded up to the next of a coarse ladder (steps of about 12 %)."""
+    """``cap`` rounded up to the next of a coarse ladder (steps of about 12 %), and that to a multiple of ``align``."""
     step = max(align, 64)
     ladder = step
     while ladder < cap:
         ladder = max(ladder + step, (int(ladder * 1.125) + step - 1) // step * step)
-    return ladder
+    return ladder + -ladder % align
 
 
 def _dynamic_capacity(lib, logits, top_k, normalize, group, align):
@@ -674,7 +674,7 @@ def forward(layer, x, gctx, top_k, capacity_factor, degree):
     local = _local_path(st.tr)
     if local and _linear_gate(layer, gctx, x):
         y, l_aux, capacity, (idx, loc) = _local_layer(layer, st, x, gctx, top_k, capacity, align)
-        _note_stats(layer, st, q8, idx, loc, E, capacity, degree, x)
+        _note_stats(layer, st, q8, idx, loc, E, capacity, degree, x, local)
         return y, l_aux
 
     with torch.autocast('cuda', enabled=False), stage('fwd.gate_linear'):
@@ -687,7 +687,6 @@ def forward(layer, x, gctx, top_k, capacity_factor, degree):
         if q8 and not local:
             align = SLICE_ROWS * degree
         capacity = _dynamic_capacity(lib, logits, top_k, layer.normalize_gate, layer.group, align)
-        capacity += -capacity % align
 
     with stage('fwd.gate_topk_scan'):
         if layer.batch_prioritized_routing:
@@ -716,13 +715,14 @@ def forward(layer, x, gctx, top_k, capacity_factor, degree):
         meta = dict(state=st, idx=idx, loc=loc, slot_map=slot_map, E=E, C=capacity, degree=degree, K=top_k,
                     act=ACT_CODES[ex.act_name], postscore=layer.is_postscore, q8=q8)
         y = _FusedExperts.apply(x.contiguous(), *args, meta)
-    _note_stats(layer, st, q8, idx, loc, E, capacity, degree, x)
+    _note_stats(layer, st, q8, idx, loc, E, capacity, degree, x, local)
     return y, l_aux.to(logits.dtype)
 
 
-def _note_stats(layer, st, q8, idx, loc, E, capacity, degree, x):
-    # both 'naive' and 'pipe' run as the flat push of the copy role / push epilogue: say so instead of echoing the name
-    layer.last_stats = dict(capacity=capacity, degree=degree, path='fused', comm='flat-push',
+def _note_stats(layer, st, q8, idx, loc, E, capacity, degree, x, local):
+    # 'naive' and 'pipe' both run as the flat push of the copy role / push epilogue, and on one rank as no exchange at all:
+    # say so instead of echoing the name
+    layer.last_stats = dict(capacity=capacity, degree=degree, path='fused', comm='none' if local else 'flat-push',
                             wire=('int8' if q8 else 'bf16'))
     if getattr(layer, 'collect_stats', False):
         from ..utils import metrics

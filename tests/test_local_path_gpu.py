@@ -342,6 +342,22 @@ def test_other_threads_run_while_the_capacity_is_awaited():
     assert sum(start < t < end for t in beats) > 5
 
 
+@pytest.mark.parametrize('degree', [1, 3, 20])
+def test_stats_say_what_ran(degree, monkeypatch):
+    """A dynamic capacity is a multiple of 4 * degree whichever way the layer runs, and no exchange is called none."""
+    layer = _layer(4, 128, 256, 2, 0.0)
+    torch.manual_seed(15)
+    x = torch.randn(300, 128, device='cuda').bfloat16()
+    seen = []
+    for local in ('1', '0'):
+        monkeypatch.setenv('PLANMOE_LOCAL', local)
+        with torch.no_grad():
+            layer(x, a2a_ffn_overlap_degree=degree)
+        seen.append(layer.last_stats)
+    assert seen[0]['capacity'] == seen[1]['capacity'] and seen[0]['capacity'] % (4 * degree) == 0
+    assert [s['comm'] for s in seen] == ['none', 'flat-push']
+
+
 _VARIANT_CHILD = """
 import os, torch
 from tests.test_local_path_gpu import _close, _layer, _pass
