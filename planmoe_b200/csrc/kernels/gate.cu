@@ -234,7 +234,9 @@ gate_assign_kernel(int S, int E, int K, int C, int normalize, float eps,
   }
 }
 
-// No histograms here: small blocks spread 8192 tokens over all SMs (11 us with 128 threads and 16 experts).
+// No histograms here, so that blocks may be small, which spreads few tokens with many experts over more SMs: 128 threads take
+// 4.6, 6.0 and 20.9 us for 8192 tokens with 8, 16 and 64 experts (top-2, 2, 4), 32 threads 4.5, 5.6 and 17.1; from 16384 tokens
+// on the two differ by less than 4 % either way.
 constexpr int kGateBwdThreads = 32;
 template <class T, int ME, bool SCORES>
 __global__ void __launch_bounds__(kGateBwdThreads)

@@ -65,7 +65,9 @@ void launch_gate_grad(const T* disp, const T* dy, const int* idx, const int* loc
 
 // ---- one rank: tokens straight into the experts' slots ----
 // Of an expert's C slots only the first used[e] hold tokens.  What computes on slots does so in blocks of at most
-// kSlotBlock rows and stops behind the block with the last token; the rows of that block behind it are zeros.
+// kSlotBlock rows and stops behind the block with the last token; the rows of that block behind it are zeros.  The exception
+// is the GEMM that writes int8 rows: its push epilogue covers all slots, and what it makes of rows that hold nothing is never
+// gathered.
 constexpr int kSlotBlock = 256;
 // out[e * C + c] = (gate *) row of the token that holds the slot; int8 (without gates): the row as an int8 transfer
 // delivers it
@@ -82,6 +84,8 @@ void launch_slots_gate_grad_q8(const void* disp, const float* disp_scales, const
                                int C, cudaStream_t stream);
 
 // ---- kernels/gate_proj.cu: the linear gate on bf16 tokens [S, M], M % 32 == 0, at most kProjMaxE experts ----
+// Sixteen: the weight gradient holds eight columns of every expert in fp32, 128 of its 198 registers at 16, and the
+// projection's accumulators and weight fragments grow the same way; with more experts both would read the tokens again.
 // `w`: [E, M], fp32 or bf16.  logits fp32, rounded to bf16 values if asked for.
 constexpr int kProjMaxE = 16;
 void launch_gate_project(const void* x, const void* w, bool w_bf16, float* logits, int S, int E, int M, bool round_bf16,

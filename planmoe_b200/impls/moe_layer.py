@@ -270,14 +270,14 @@ class MOELayer(torch.nn.Module):
 
     def _codec_verdict(self, x, top_k, cf):
         """For a configured codec: whether, by the model, its encode + decode time is paid back by the bytes it
-        takes off NVLink (kernels at their measured rates; recorded in the scheduler's report)."""
+        takes off NVLink (kernels at their rates on [8192, 4096] bf16; recorded in the scheduler's report)."""
         if self.compress_name in ('no', None):
             return None
         from ..parallel import scheduler
         W, E = self.world_size, self.num_global_experts
         C = top_k * int(max(cf, 1.0) * ((x.size(0) + E - 1) // E))
         raw = E * C * x.size(-1) * x.element_size()
-        rates = {'int8': (1800e9, 2300e9, 2.0), 'zfp': (190e9, 160e9, 2.0), 'lz': (20e9, 230e9, 1.2)}
+        rates = {'int8': (1800e9, 2400e9, 2.0), 'zfp': (640e9, 400e9, 2.0), 'lz': (160e9, 480e9, 1.2)}
         enc, dec, ratio = rates.get(self.compress_name, (1e12, 1e12, 1.0))
         t_raw = raw * (W - 1) / max(W, 1) / 770e9
         pays = scheduler.codec_pays_off(raw / enc, raw / dec, t_raw, ratio)
