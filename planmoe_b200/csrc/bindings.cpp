@@ -58,6 +58,13 @@ const float* opt_f32(const c10::optional<Tensor>& t) {
   return t->data_ptr<float>();
 }
 
+// What kernels that move rows as 16-byte vectors read: a contiguous view may start anywhere in its storage, and a vector
+// access off its boundary is a fault.
+const void* rows16(const Tensor& t) {
+  TORCH_CHECK(t.is_contiguous() && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0, "rows must be contiguous and 16-byte aligned");
+  return t.data_ptr();
+}
+
 // ---- CPU sparse ops -------------------------------------------------------------------------
 template <class T>
 const T* opt_ptr(const c10::optional<Tensor>& t) {
@@ -123,7 +130,7 @@ Tensor dispatch_scatter_op(const Tensor& x, const Tensor& slot_map, const c10::o
   c10::cuda::CUDAGuard guard(x.device());
   Tensor out = torch::empty({n_slots, M}, x.options());
   DISPATCH_FLOAT(x, "dispatch_scatter", [&] {
-    launch_scatter_rows<scalar_t>(reinterpret_cast<const scalar_t*>(x.data_ptr()), slot_map.data_ptr<int>(),
+    launch_scatter_rows<scalar_t>(reinterpret_cast<const scalar_t*>(rows16(x)), slot_map.data_ptr<int>(),
                                   opt_f32(gates), reinterpret_cast<scalar_t*>(out.data_ptr()), K, S, M, 1, n_slots,
                                   nullptr, false, cur_stream(), round_gates);
   });
@@ -140,7 +147,7 @@ Tensor dispatch_gather_op(const Tensor& disp, const Tensor& idx, const Tensor& l
   c10::cuda::CUDAGuard guard(disp.device());
   Tensor out = torch::empty({S, M}, disp.options());
   DISPATCH_FLOAT(disp, "dispatch_gather", [&] {
-    launch_gather_rows<scalar_t>(disp.data_ptr(), nullptr, idx.data_ptr<int>(), loc.data_ptr<int>(), opt_f32(gates),
+    launch_gather_rows<scalar_t>(rows16(disp), nullptr, idx.data_ptr<int>(), loc.data_ptr<int>(), opt_f32(gates),
                                  reinterpret_cast<scalar_t*>(out.data_ptr()), K, S, M, C, nullptr, cur_stream(), 0, round_gates);
   });
   return out;
@@ -149,12 +156,13 @@ Tensor dispatch_gather_op(const Tensor& disp, const Tensor& idx, const Tensor& l
 Tensor dispatch_gate_grad_op(const Tensor& disp, const Tensor& dy, const Tensor& idx, const Tensor& loc, int64_t C) {
   count_launch(1);
   TORCH_CHECK(disp.is_cuda() && disp.is_contiguous() && dy.is_contiguous() && disp.scalar_type() == dy.scalar_type());
+  TORCH_CHECK((disp.size(1) * disp.element_size()) % 16 == 0, "row bytes must be a multiple of 16");
   const int K = idx.size(0), S = idx.size(1), M = disp.size(1);
   c10::cuda::CUDAGuard guard(disp.device());
   Tensor out = torch::empty({K, S}, disp.options().dtype(at::kFloat));
   DISPATCH_FLOAT(disp, "dispatch_gate_grad", [&] {
-    launch_gate_grad<scalar_t>(reinterpret_cast<const scalar_t*>(disp.data_ptr()),
-                               reinterpret_cast<const scalar_t*>(dy.data_ptr()), idx.data_ptr<int>(),
+    launch_gate_grad<scalar_t>(reinterpret_cast<const scalar_t*>(rows16(disp)),
+                               reinterpret_cast<const scalar_t*>(rows16(dy)), idx.data_ptr<int>(),
                                loc.data_ptr<int>(), out.data_ptr<float>(), nullptr, nullptr, K, S, M, C, cur_stream());
   });
   return out;
@@ -166,6 +174,7 @@ std::vector<Tensor> dispatch_gate_grad_scaled_op(const Tensor& disp, const Tenso
                                                  const Tensor& loc, const Tensor& gates, int64_t C) {
   count_launch(1);
   TORCH_CHECK(disp.is_cuda() && disp.is_contiguous() && dy.is_contiguous() && disp.scalar_type() == dy.scalar_type());
+  TORCH_CHECK((disp.size(1) * disp.element_size()) % 16 == 0, "row bytes must be a multiple of 16");
   TORCH_CHECK(gates.is_cuda() && gates.scalar_type() == at::kFloat && gates.is_contiguous());
   const int K = idx.size(0), S = idx.size(1), M = disp.size(1);
   TORCH_CHECK(gates.numel() == (int64_t)K * S && dy.size(0) == S && dy.size(1) == M);
@@ -173,8 +182,8 @@ std::vector<Tensor> dispatch_gate_grad_scaled_op(const Tensor& disp, const Tenso
   Tensor out = torch::empty({K, S}, disp.options().dtype(at::kFloat));
   Tensor scaled = torch::empty({(int64_t)S * K, (int64_t)M}, dy.options());
   DISPATCH_FLOAT(disp, "dispatch_gate_grad_scaled", [&] {
-    launch_gate_grad<scalar_t>(reinterpret_cast<const scalar_t*>(disp.data_ptr()),
-                               reinterpret_cast<const scalar_t*>(dy.data_ptr()), idx.data_ptr<int>(),
+    launch_gate_grad<scalar_t>(reinterpret_cast<const scalar_t*>(rows16(disp)),
+                               reinterpret_cast<const scalar_t*>(rows16(dy)), idx.data_ptr<int>(),
                                loc.data_ptr<int>(), out.data_ptr<float>(), gates.data_ptr<float>(),
                                reinterpret_cast<scalar_t*>(scaled.data_ptr()), K, S, M, C, cur_stream());
   });
@@ -199,7 +208,7 @@ std::vector<Tensor> dispatch_gate_grad_q8_op(int64_t disp_ptr, int64_t scales_pt
     scaled = torch::empty({(int64_t)S * K, (int64_t)M + 16}, dy.options().dtype(at::kByte));
   }
   DISPATCH_FLOAT(dy, "dispatch_gate_grad_q8", [&] {
-    launch_gate_grad<scalar_t>(reinterpret_cast<const scalar_t*>(disp_ptr), reinterpret_cast<const scalar_t*>(dy.data_ptr()),
+    launch_gate_grad<scalar_t>(reinterpret_cast<const scalar_t*>(disp_ptr), reinterpret_cast<const scalar_t*>(rows16(dy)),
                                idx.data_ptr<int>(), loc.data_ptr<int>(), out.data_ptr<float>(), opt_f32(gates),
                                nullptr, K, S, M, C, cur_stream(), reinterpret_cast<const float*>(scales_ptr), group_rows,
                                want_scaled ? scaled.data_ptr<uint8_t>() : nullptr);
@@ -362,7 +371,7 @@ std::vector<Tensor> int8_encode_op(const Tensor& rows) {
   Tensor q = torch::empty({R, M}, rows.options().dtype(at::kByte));
   Tensor scale = torch::empty({R}, rows.options().dtype(at::kFloat)), bias = torch::empty_like(scale);
   DISPATCH_FLOAT(rows, "int8_encode", [&] {
-    launch_int8_encode<scalar_t>(reinterpret_cast<const scalar_t*>(rows.data_ptr()), q.data_ptr<uint8_t>(),
+    launch_int8_encode<scalar_t>(reinterpret_cast<const scalar_t*>(rows16(rows)), q.data_ptr<uint8_t>(),
                                  scale.data_ptr<float>(), bias.data_ptr<float>(), R, M, cur_stream());
   });
   return {q, scale, bias};
@@ -374,7 +383,7 @@ Tensor int8_decode_op(const Tensor& q, const Tensor& scale, const Tensor& bias, 
   const int R = q.size(0), M = q.size(1);
   Tensor out = torch::empty({R, M}, q.options().dtype(dtype));
   DISPATCH_FLOAT(out, "int8_decode", [&] {
-    launch_int8_decode<scalar_t>(q.data_ptr<uint8_t>(), scale.data_ptr<float>(), bias.data_ptr<float>(),
+    launch_int8_decode<scalar_t>(static_cast<const uint8_t*>(rows16(q)), scale.data_ptr<float>(), bias.data_ptr<float>(),
                                  reinterpret_cast<scalar_t*>(out.data_ptr()), R, M, cur_stream());
   });
   return out;
@@ -526,7 +535,8 @@ Tensor grouped_gemm_op(const Tensor& A, bool a_mn, const Tensor& B, bool b_mn, c
 static void colsum_check(const Tensor& x, int64_t fold) {
   TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.dim() == 3 && x.stride(2) == 1);
   TORCH_CHECK(fold >= 1 && x.size(0) % fold == 0, "colsum: groups must be a multiple of fold");
-  TORCH_CHECK(x.size(2) % 8 == 0 && x.stride(1) % 8 == 0 && x.stride(0) % 8 == 0, "colsum needs 16-byte aligned rows");
+  TORCH_CHECK(x.size(2) % 8 == 0 && x.stride(1) % 8 == 0 && x.stride(0) % 8 == 0 &&
+              reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0, "colsum needs 16-byte aligned rows");
 }
 
 // scratch of one job: [out][partials][counters]; fills `j`, returns the buffer
@@ -595,11 +605,6 @@ struct LocalRoute {
   bool postscore, int8;                           // int8: rows as int8 transfers deliver them, both ways (C % 32 == 0)
   int64_t budget_ms, status_ptr;
 };
-
-static const void* rows16(const Tensor& t) {      // a row tensor the vector kernels may read
-  TORCH_CHECK(t.is_contiguous() && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0, "rows must be 16-byte aligned");
-  return t.data_ptr();
-}
 
 static void local_check(const Tensor& x, const LocalRoute& r, const Tensor& w1) {
   const int64_t K = r.idx.size(0), S = r.idx.size(1), E = w1.size(0);
@@ -967,7 +972,7 @@ Tensor int8_rows_encode_op(const Tensor& x) {
   const int R = x.size(0), M = x.size(1);
   Tensor out = torch::empty({(int64_t)R, (int64_t)M + 16}, x.options().dtype(at::kByte));
   DISPATCH_FLOAT(x, "int8_rows_encode", [&] {
-    launch_int8_rows_encode<scalar_t>(reinterpret_cast<const scalar_t*>(x.data_ptr()), out.data_ptr<uint8_t>(), R, M,
+    launch_int8_rows_encode<scalar_t>(reinterpret_cast<const scalar_t*>(rows16(x)), out.data_ptr<uint8_t>(), R, M,
                                       cur_stream());
   });
   return out;
@@ -988,7 +993,7 @@ void scatter_push_op(const Tensor& x, const Tensor& slot_map, const c10::optiona
   TORCH_CHECK(E % W == 0 && C % chunks == 0);
   const int S = x.size(0), M = x.size(1);
   DISPATCH_FLOAT(x, "scatter_push", [&] {
-    launch_scatter_rows<scalar_t>(reinterpret_cast<const scalar_t*>(x.data_ptr()), slot_map.data_ptr<int>(),
+    launch_scatter_rows<scalar_t>(reinterpret_cast<const scalar_t*>(rows16(x)), slot_map.data_ptr<int>(),
                                   opt_f32(gates), nullptr, K, S, M, E, C, &pa, false, cur_stream());
   });
 }
@@ -1043,6 +1048,7 @@ Tensor zfp_encode_op(const Tensor& x, int64_t rate) {
 Tensor zfp_decode_op(const Tensor& stream, int64_t lead, int64_t rows, int64_t M, int64_t rate, at::ScalarType dtype) {
   TORCH_CHECK(stream.is_contiguous() && stream.scalar_type() == at::kByte);
   TORCH_CHECK(stream.numel() == lead * (int64_t)zfp_stream_bytes(rows, M, rate), "zfp stream size mismatch");
+  TORCH_CHECK(reinterpret_cast<uintptr_t>(stream.data_ptr()) % 4 == 0, "zfp stream must be 4-byte aligned");
   Tensor out = torch::empty({lead, rows, M}, stream.options().dtype(dtype));
   if (stream.is_cuda()) {
     count_launch(1);
@@ -1058,6 +1064,7 @@ std::vector<Tensor> lz_encode_op(const Tensor& raw, int64_t sym) {
   TORCH_CHECK(raw.dim() == 2 && raw.is_contiguous() && raw.scalar_type() == at::kByte);
   TORCH_CHECK((sym == 2 || sym == 4) && raw.size(1) % sym == 0 && raw.size(1) % 16 == 0,
               "lz codec: slice bytes must be a multiple of 16 and of the symbol size");
+  TORCH_CHECK(reinterpret_cast<uintptr_t>(raw.data_ptr()) % sym == 0, "lz codec: symbols must be aligned");
   const int64_t slices = raw.size(0), raw_bytes = raw.size(1);
   const int64_t cap = (int64_t)lz_payload_capacity(raw_bytes);
   Tensor payload = torch::empty({slices, cap}, raw.options());
@@ -1076,6 +1083,9 @@ std::vector<Tensor> lz_encode_op(const Tensor& raw, int64_t sym) {
 
 Tensor lz_decode_op(const Tensor& payload, const Tensor& sizes, int64_t raw_bytes, int64_t sym) {
   TORCH_CHECK(payload.dim() == 2 && payload.is_contiguous() && payload.scalar_type() == at::kByte);
+  TORCH_CHECK((sym == 2 || sym == 4) && raw_bytes >= 0 && raw_bytes % sym == 0, "lz codec: slice bytes must be a multiple of the symbol size");
+  TORCH_CHECK(payload.size(1) % 4 == 0 && reinterpret_cast<uintptr_t>(payload.data_ptr()) % 4 == 0,
+              "lz codec: slices must be 4-byte aligned");
   const int64_t slices = payload.size(0);
   Tensor raw = torch::empty({slices, raw_bytes}, payload.options());
   if (payload.is_cuda()) {

@@ -104,22 +104,26 @@ def _native_ok(x):
             and not native.force_python_fallback())
 
 
+def _rows(x):
+    return native.aligned(x) if x.is_cuda else x.contiguous()
+
+
 def _scatter(x, plan, gates):
-    x = x.contiguous()
+    x = _rows(x)
     if x.is_cuda:
         return native.lib().dispatch_scatter(x, plan.slot_map, gates, plan.K, plan.E * plan.C)
     return native.lib().cpu_scatter(x, plan.idx, plan.loc, gates, plan.E, plan.C)
 
 
 def _gather(disp, plan, gates):
-    disp = disp.contiguous()
+    disp = _rows(disp)
     if disp.is_cuda:
         return native.lib().dispatch_gather(disp, plan.idx, plan.loc, gates, plan.C)
     return native.lib().cpu_gather(disp, plan.idx, plan.loc, gates, plan.C)
 
 
 def _gate_grad(disp, dy, plan):
-    disp, dy = disp.contiguous(), dy.contiguous()
+    disp, dy = _rows(disp), _rows(dy)
     if disp.is_cuda:
         return native.lib().dispatch_gate_grad(disp, dy, plan.idx, plan.loc, plan.C)
     return native.lib().cpu_gate_grad(disp, dy, plan.idx, plan.loc, plan.C)
@@ -145,7 +149,7 @@ class _Scatter(torch.autograd.Function):
     def backward(ctx, ddisp):
         x, g = ctx.saved_tensors
         plan = ctx.plan
-        ddisp = ddisp.contiguous()
+        ddisp = _rows(ddisp)
         dx = _gather(ddisp, plan, g)
         dg = None
         if g is not None and ctx.needs_input_grad[1]:
@@ -166,7 +170,7 @@ class _Gather(torch.autograd.Function):
     def backward(ctx, dy):
         disp, g = ctx.saved_tensors
         plan = ctx.plan
-        dy = dy.contiguous()
+        dy = _rows(dy)
         ddisp = _scatter(dy, plan, g)
         dg = None
         if g is not None and ctx.needs_input_grad[1]:
@@ -183,7 +187,7 @@ class _ScatterPicks(torch.autograd.Function):
         ctx.plan, ctx.round = plan, x.dtype != torch.float32
         ctx.set_materialize_grads(False)
         ctx.save_for_backward(x, rows)
-        return native.lib().dispatch_scatter(x.contiguous(), plan.slot_map, rows, plan.K, plan.E * plan.C, ctx.round)
+        return native.lib().dispatch_scatter(_rows(x), plan.slot_map, rows, plan.K, plan.E * plan.C, ctx.round)
 
     @staticmethod
     def backward(ctx, ddisp):
@@ -191,7 +195,7 @@ class _ScatterPicks(torch.autograd.Function):
         plan = ctx.plan
         if ddisp is None:
             return (None,) * (3 + plan.K)
-        ddisp = ddisp.contiguous()
+        ddisp = _rows(ddisp)
         dx = native.lib().dispatch_gather(ddisp, plan.idx, plan.loc, rows, plan.C, ctx.round)
         dg = [None] * plan.K
         if any(ctx.needs_input_grad[3:]):
@@ -207,7 +211,7 @@ class _GatherPicks(torch.autograd.Function):
         ctx.plan, ctx.round = plan, disp.dtype != torch.float32
         ctx.set_materialize_grads(False)
         ctx.save_for_backward(disp, rows)
-        return native.lib().dispatch_gather(disp.contiguous(), plan.idx, plan.loc, rows, plan.C, ctx.round)
+        return native.lib().dispatch_gather(_rows(disp), plan.idx, plan.loc, rows, plan.C, ctx.round)
 
     @staticmethod
     def backward(ctx, dy):
@@ -215,7 +219,7 @@ class _GatherPicks(torch.autograd.Function):
         plan = ctx.plan
         if dy is None:
             return (None,) * (3 + plan.K)
-        dy = dy.contiguous()
+        dy = _rows(dy)
         ddisp = native.lib().dispatch_scatter(dy, plan.slot_map, rows, plan.K, plan.E * plan.C, ctx.round)
         dg = [None] * plan.K
         if any(ctx.needs_input_grad[3:]):

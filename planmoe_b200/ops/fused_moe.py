@@ -386,7 +386,7 @@ class _FusedExperts(torch.autograd.Function):
         act, postscore = meta['act'], meta['postscore']
         bases = bs.block.bases_ptr
         budget, status = tr.budget_ms, tr.status_ptr
-        dout = dout.contiguous()
+        dout = native.aligned(dout)
 
         q8 = bs.q8
         rows_y = E * C
@@ -469,12 +469,6 @@ def _whole_slices(m):
     return dict(m, loc=loc, C=slots, slot_map=native.lib().build_slot_map(m['idx'], loc, m['used'].numel(), slots))
 
 
-def _aligned(t):
-    """``t`` contiguous, its first element on a 16-byte boundary (the kernels move rows as 16-byte vectors)."""
-    t = t.contiguous()
-    return t if t.data_ptr() % 16 == 0 else t.clone()
-
-
 def _stages():
     return stage if stage_timer.enabled() else None
 
@@ -495,7 +489,7 @@ class _LocalExperts(torch.autograd.Function):
         x, gates, w1, w2, xs, dact, h, ys, scales, idx, loc, slot_map, used = ctx.saved_tensors
         route = _local_route(gates, dict(ctx.meta, idx=idx, loc=loc, slot_map=slot_map, used=used))
         dx, dgates, dw1, db1, dw2, db2 = native.lib().local_backward(
-            _aligned(dy), x, route, w1, w2, xs, dact, h, ys, scales, list(ctx.needs_input_grad[:6]), _stages())
+            native.aligned(dy), x, route, w1, w2, xs, dact, h, ys, scales, list(ctx.needs_input_grad[:6]), _stages())
         return dx, dgates, dw1, db1, dw2, db2, None
 
 
@@ -517,7 +511,7 @@ def _needs_node(tensors):
 
 
 def _local_experts(x, gates, w1, b1, w2, b2, meta):
-    x, gates, meta = _aligned(x), gates.contiguous(), _whole_slices(meta)
+    x, gates, meta = native.aligned(x), gates.contiguous(), _whole_slices(meta)
     if _needs_node((x, gates, w1, b1, w2, b2)):
         return _LocalExperts.apply(x, gates, w1, b1, w2, b2, meta)
     return _local_forward(x, gates, w1, b1, w2, b2, meta, False)[0]
@@ -542,7 +536,7 @@ class _LocalLayer(torch.autograd.Function):
         if dy is None and dl_aux is None:
             return (None,) * 7
         route = _local_route(gates, dict(m, C=xs.size(1), idx=idx, loc=loc, slot_map=slot_map, used=used))
-        return (*native.lib().local_moe_backward(_aligned(dy) if dy is not None else None, dl_aux, x, wg, route, w1, w2, logits,
+        return (*native.lib().local_moe_backward(native.aligned(dy) if dy is not None else None, dl_aux, x, wg, route, w1, w2, logits,
                                                  top1, xs, dact, h, ys, scales, m['normalize'], m['bf16_logits'],
                                                  list(ctx.needs_input_grad[:6]), _stages()),
                 None)
@@ -582,7 +576,7 @@ def _local_layer(layer, st, x, gctx, top_k, capacity, align):
              bf16_logits=not gctx.fp32_gate, prio=layer.batch_prioritized_routing, act=ACT_CODES[ex.act_name],
              postscore=layer.is_postscore, int8=layer.compress_name == 'int8', budget_ms=st.tr.budget_ms,
              status=st.tr.status)
-    args = (_aligned(x), w, ex.batched_fc1_w, ex.batched_fc1_bias, ex.batched_fc2_w, ex.batched_fc2_bias)
+    args = (native.aligned(x), w, ex.batched_fc1_w, ex.batched_fc1_bias, ex.batched_fc2_w, ex.batched_fc2_bias)
     if _needs_node(args):
         y, l_aux = _LocalLayer.apply(*args, m)
     else:
@@ -714,7 +708,7 @@ def forward(layer, x, gctx, top_k, capacity_factor, degree):
     else:
         meta = dict(state=st, idx=idx, loc=loc, slot_map=slot_map, E=E, C=capacity, degree=degree, K=top_k,
                     act=ACT_CODES[ex.act_name], postscore=layer.is_postscore, q8=q8)
-        y = _FusedExperts.apply(x.contiguous(), *args, meta)
+        y = _FusedExperts.apply(native.aligned(x), *args, meta)
     _note_stats(layer, st, q8, idx, loc, E, capacity, degree, x, local)
     return y, l_aux.to(logits.dtype)
 

@@ -47,6 +47,13 @@ def maybe_lib():
     return _LIB
 
 
+def aligned(t):
+    """``t`` contiguous with its first element on a 16-byte boundary: what kernels that move rows as 16-byte vectors take.  A
+    contiguous view may start anywhere in its storage."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 def force_python_fallback():
     """True when env PLANMOE_NO_NATIVE=1 asks CPU paths to avoid the extension."""
     return os.environ.get("PLANMOE_NO_NATIVE", "0") == "1"

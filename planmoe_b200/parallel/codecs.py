@@ -75,7 +75,7 @@ class Int8Compressor(AbstractCompressor):
         t = t.contiguous()
         rows = t.reshape(-1, t.size(-1))
         if t.is_cuda:
-            q, scale, bias = native.lib().int8_encode(rows)
+            q, scale, bias = native.lib().int8_encode(native.aligned(rows))
         else:
             f = rows.float()
             lo, hi = f.min(dim=1).values, f.max(dim=1).values
@@ -91,7 +91,7 @@ class Int8Compressor(AbstractCompressor):
         (dtype,) = packed.meta
         rows = q.reshape(-1, q.size(-1))
         if q.is_cuda:
-            out = native.lib().int8_decode(rows, scale.reshape(-1).contiguous(),
+            out = native.lib().int8_decode(native.aligned(rows), scale.reshape(-1).contiguous(),
                                            bias.reshape(-1).contiguous(), dtype)
         else:
             out = (rows.float() * (scale.reshape(-1, 1) / 255.0) + bias.reshape(-1, 1)).to(dtype)

@@ -79,3 +79,22 @@ def test_lz_forms_match_the_serial_coder(sym, nbytes, kind):
         assert torch.equal(p_gpu[s, :used].cpu(), p_cpu[s, :used])
     assert torch.equal(lib.lz_decode(p_gpu, n_gpu, raw.size(1), sym).cpu(), raw)
     assert torch.equal(lib.lz_decode(p_cpu.cuda(), n_cpu.cuda(), raw.size(1), sym).cpu(), raw)
+
+
+@pytest.mark.parametrize('dtype', [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize('name', ['int8', 'zfp', 'lz'])
+def test_codecs_take_tensors_off_the_vector_boundary(name, dtype):
+    from planmoe_b200.parallel import codecs
+    codec = codecs.get_compressor(name)
+    x = torch.relu(torch.randn(4 * 24 * 64 + 1, device='cuda')).to(dtype)
+    off = x[1:].view(4, 24, 64)
+    assert off.is_contiguous() and off.data_ptr() % 16
+    a, b = codec.compress(off, 4), codec.compress(off.clone(), 4)
+    assert torch.equal(codec.decompress(a), codec.decompress(b))
+    if name != 'lz':                             # behind a slice's code an lz wire holds anything
+        for u, v in zip(a.wires, b.wires):
+            assert torch.equal(u, v)
+    if name == 'int8':                           # so may the wire
+        room = torch.empty(a.wires[0].numel() + 1, dtype=torch.uint8, device='cuda')
+        moved = codecs.Packed([room[1:].view_as(a.wires[0]).copy_(a.wires[0])] + a.wires[1:], a.meta)
+        assert torch.equal(codec.decompress(moved), codec.decompress(b))

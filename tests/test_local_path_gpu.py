@@ -83,13 +83,25 @@ def test_experts_without_tokens_and_frozen_weights(act, monkeypatch):
     _close(here, _pass(layer, x, dy, degree=2))
 
 
-def test_rows_off_the_vector_boundary():
-    layer = _layer(2, 128, 256, 2, 1.0)
-    x = torch.randn(300 * 128 + 1, device='cuda').bfloat16()
-    off = x[1:].view(300, 128)
-    assert off.data_ptr() % 16
+@pytest.mark.parametrize('local', ['1', '0'])
+@pytest.mark.parametrize('wire', ['no', 'int8'])
+def test_rows_off_the_vector_boundary(local, wire, monkeypatch):
+    monkeypatch.setenv('PLANMOE_LOCAL', local)
+    layer = _layer(2, 128, 256, 2, 1.0, compress_name=wire)
+    off = [torch.randn(320 * 128 + 1, device='cuda').bfloat16()[1:].view(320, 128) for _ in range(2)]
+    assert all(t.data_ptr() % 16 for t in off)
     with torch.no_grad():
-        assert torch.equal(layer(off), layer(off.clone()))
+        assert torch.equal(layer(off[0]), layer(off[0].clone()))
+    from planmoe_b200.parallel import transport
+    got = []
+    for place in (lambda t: t, torch.clone):
+        x = place(off[0].detach()).requires_grad_()
+        layer.zero_grad(set_to_none=True)
+        layer(x).backward(place(off[1]))
+        got.append([x.grad] + [p.grad for p in layer.parameters()])
+    transport.get_transport(layer.group).check()
+    for u, v in zip(*got):
+        assert torch.equal(u, v)
 
 
 @contextlib.contextmanager

@@ -222,3 +222,57 @@ def test_encode_and_decode_by_pick(dtype, postscore, S, E, k):
         # the stacked form rounds the gates' gradient to the data's type
         eps = torch.finfo(dtype).eps
         assert float((got[2] - out[2][2]).abs().max()) <= 4 * eps * float(out[2][2].abs().max()) + 1e-6
+
+
+def _off(t, by=1):
+    """The same values as a contiguous view that starts ``by`` elements into its storage."""
+    room = torch.empty(t.numel() + by, dtype=t.dtype, device=t.device)
+    view = room[by:].view(t.shape).copy_(t)
+    assert view.is_contiguous() and view.data_ptr() % 16
+    return view
+
+
+@pytest.mark.parametrize('dtype', [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize('postscore', [True, False])
+@pytest.mark.parametrize('gates32', [True, False])
+def test_rows_off_the_vector_boundary(dtype, postscore, gates32):
+    """Tokens, slots and gradients may start anywhere in their storage: the kernels get aligned copies."""
+    from planmoe_b200.impls import fast_dispatch as FD
+    torch.manual_seed(3)
+    x = torch.randn(70, 64, device='cuda').to(dtype)
+    dy = torch.randn(70, 64, device='cuda').to(dtype)
+    scores = torch.softmax(torch.randn(70, 4, device='cuda'), dim=1)
+    if not gates32:
+        scores = scores.half()
+    out = []
+    for place in (lambda t: t, _off):
+        xl, sl = place(x.clone()).requires_grad_(), scores.clone().requires_grad_()
+        plan, _ = FD.extract_critical(sl, 2)
+        slots = FD.fast_encode(xl, plan, postscore)
+        held = place(slots.detach()).requires_grad_()
+        y = FD.fast_decode(held, plan, postscore)
+        y.backward(place(dy), retain_graph=True)
+        slots.backward(place(held.grad))
+        out.append((slots.detach(), y.detach(), held.grad, xl.grad, sl.grad))
+    for u, v in zip(*out):
+        assert torch.equal(u, v)
+
+
+def test_kernels_refuse_rows_off_the_vector_boundary():
+    """The bindings turn a misaligned base into an error on the host."""
+    from planmoe_b200.ops import native
+    lib = native.lib()
+    x = _off(torch.randn(16, 64, device='cuda').bfloat16())
+    good = x.clone()
+    idx = torch.zeros(1, 16, dtype=torch.int32, device='cuda')
+    loc = torch.arange(16, dtype=torch.int32, device='cuda').view(1, 16)
+    smap = lib.build_slot_map(idx, loc, 1, 16)
+    calls = [lambda: lib.dispatch_scatter(x, smap, None, 1, 16), lambda: lib.dispatch_gather(x, idx, loc, None, 16),
+             lambda: lib.dispatch_gate_grad(x, good, idx, loc, 16), lambda: lib.dispatch_gate_grad(good, x, idx, loc, 16),
+             lambda: lib.int8_encode(x), lambda: lib.int8_rows_encode(x), lambda: lib.colsum(x.view(1, 16, 64), 1, True),
+             lambda: lib.int8_decode(_off(torch.zeros(16, 64, dtype=torch.uint8, device='cuda')), torch.ones(16, device='cuda'),
+                                     torch.ones(16, device='cuda'), torch.bfloat16)]
+    for call in calls:
+        with pytest.raises(RuntimeError, match='aligned'):
+            call()
+    torch.cuda.synchronize()
