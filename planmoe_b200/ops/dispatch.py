@@ -108,8 +108,15 @@ def _rows(x):
     return native.aligned(x) if x.is_cuda else x.contiguous()
 
 
+def _vector_rows(x):
+    """Whether rows are whole 16-byte vectors, which is what the CUDA kernels move; others take the composite."""
+    return x.size(-1) * x.element_size() % 16 == 0
+
+
 def _scatter(x, plan, gates):
     x = _rows(x)
+    if x.is_cuda and not _vector_rows(x):
+        return scatter_torch(x, plan, gates)
     if x.is_cuda:
         return native.lib().dispatch_scatter(x, plan.slot_map, gates, plan.K, plan.E * plan.C)
     return native.lib().cpu_scatter(x, plan.idx, plan.loc, gates, plan.E, plan.C)
@@ -117,6 +124,8 @@ def _scatter(x, plan, gates):
 
 def _gather(disp, plan, gates):
     disp = _rows(disp)
+    if disp.is_cuda and not _vector_rows(disp):
+        return gather_torch(disp.float(), plan, gates).to(disp.dtype)     # added up in fp32, as the kernel does
     if disp.is_cuda:
         return native.lib().dispatch_gather(disp, plan.idx, plan.loc, gates, plan.C)
     return native.lib().cpu_gather(disp, plan.idx, plan.loc, gates, plan.C)
@@ -124,6 +133,8 @@ def _gather(disp, plan, gates):
 
 def _gate_grad(disp, dy, plan):
     disp, dy = _rows(disp), _rows(dy)
+    if disp.is_cuda and not _vector_rows(disp):
+        return gate_grad_torch(disp, dy, plan)
     if disp.is_cuda:
         return native.lib().dispatch_gate_grad(disp, dy, plan.idx, plan.loc, plan.C)
     return native.lib().cpu_gate_grad(disp, dy, plan.idx, plan.loc, plan.C)
@@ -229,7 +240,7 @@ class _GatherPicks(torch.autograd.Function):
 
 def picks_ok(x, plan, gates):
     """Whether gates go to the kernels pick by pick: fp32 gates of every token for data of the CUDA kernels."""
-    return (x.is_cuda and _native_ok(x) and len(gates) == plan.K
+    return (x.is_cuda and _native_ok(x) and _vector_rows(x) and len(gates) == plan.K
             and all(g.dtype == torch.float32 and g.device == x.device and g.shape == (plan.S,) for g in gates))
 
 

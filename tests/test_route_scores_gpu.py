@@ -276,3 +276,30 @@ def test_kernels_refuse_rows_off_the_vector_boundary():
         with pytest.raises(RuntimeError, match='aligned'):
             call()
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize('dtype,dim', [(torch.float32, 66), (torch.float32, 1), (torch.float16, 36), (torch.bfloat16, 7)])
+@pytest.mark.parametrize('postscore', [True, False])
+def test_rows_that_are_no_whole_vectors(dtype, dim, postscore):
+    """Model dims whose rows the 16-byte kernels cannot move, against the same rows padded to whole vectors."""
+    from planmoe_b200.impls import fast_dispatch as FD
+    torch.manual_seed(dim)
+    pad = torch.nn.functional.pad
+    wide = (dim + 7) // 8 * 8
+    x = torch.randn(70, dim, device='cuda').to(dtype)
+    dy = torch.randn(70, dim, device='cuda').to(dtype)
+    scores = torch.softmax(torch.randn(70, 4, device='cuda'), dim=1)
+    out = []
+    for padded in (False, True):
+        xl = (pad(x, (0, wide - dim)) if padded else x.clone()).requires_grad_()
+        sl = scores.clone().requires_grad_()
+        plan, _ = FD.extract_critical(sl, 2, capacity_factor=0.8)
+        slots = FD.fast_encode(xl, plan, postscore)
+        y = FD.fast_decode(slots, plan, postscore)
+        y.backward(pad(dy, (0, wide - dim)) if padded else dy)
+        out.append((slots.detach()[..., :dim], y.detach()[..., :dim], xl.grad[..., :dim], sl.grad))
+    for u, v in zip(out[0][:3], out[1][:3]):
+        torch.testing.assert_close(u, v, rtol=2 * torch.finfo(dtype).eps, atol=1e-6)      # two products, added and rounded
+    # the gates' gradient: `dim` products in another order, rounded to the data's type by the composite
+    top = float(out[1][3].abs().max())
+    assert float((out[0][3] - out[1][3]).abs().max()) <= (4 * torch.finfo(dtype).eps + 1e-5) * top
