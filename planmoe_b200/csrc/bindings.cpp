@@ -1086,6 +1086,9 @@ Tensor lz_decode_op(const Tensor& payload, const Tensor& sizes, int64_t raw_byte
   TORCH_CHECK((sym == 2 || sym == 4) && raw_bytes >= 0 && raw_bytes % sym == 0, "lz codec: slice bytes must be a multiple of the symbol size");
   TORCH_CHECK(payload.size(1) % 4 == 0 && reinterpret_cast<uintptr_t>(payload.data_ptr()) % 4 == 0,
               "lz codec: slices must be 4-byte aligned");
+  long long len_off = 0, header = 0;
+  lz_slice_layout(raw_bytes, &len_off, &header);
+  TORCH_CHECK(payload.size(1) >= header, "lz codec: slices are shorter than their header");
   const int64_t slices = payload.size(0);
   Tensor raw = torch::empty({slices, raw_bytes}, payload.options());
   if (payload.is_cuda()) {

@@ -248,6 +248,12 @@ namespace {
 __host__ __device__ inline long long lz_blocks(long long raw_bytes) { return (raw_bytes + kLzBlockBytes - 1) / kLzBlockBytes; }
 __host__ __device__ inline long long lz_header_bytes(long long nb) { return ((4 + 4 * (nb + 1)) + 15) / 16 * 16; }
 
+// Bytes of block b's code by its slice's header, 0 if they cannot be a code or do not lie inside the slice.
+__host__ __device__ inline int lz_code_bytes(const uint32_t* hdr, long long b, long long nb, long long slice_bytes) {
+  const long long from = hdr[1 + b], to = hdr[2 + b];
+  return to - from < 2 || to - from > kLzSlotBytes || lz_header_bytes(nb) + to > slice_bytes ? 0 : (int)(to - from);
+}
+
 __host__ __device__ inline int lz_encode_one(const uint8_t* raw, long long raw_bytes, long long blk, int sym, uint8_t* slot) {
   const long long off = blk * kLzBlockBytes;
   const int bytes = (int)(raw_bytes - off < kLzBlockBytes ? raw_bytes - off : kLzBlockBytes);
@@ -635,9 +641,10 @@ lz_decode_blocks_kernel(const uint8_t* __restrict__ payload, uint8_t* __restrict
   const uint32_t* hdr = reinterpret_cast<const uint32_t*>(base);
   const long long off = b * kLzBlockBytes;
   const int bytes = (int)(raw_bytes - off < kLzBlockBytes ? raw_bytes - off : kLzBlockBytes);
-  const int code_bytes = (int)(hdr[2 + b] - hdr[1 + b]);
-  if (code_bytes < 2 || code_bytes > kLzSlotBytes) return;       // corrupt header: leave the block untouched
-  lz_decode_block_warp<Sym>(base + lz_header_bytes(nb) + hdr[1 + b], code_bytes,
+  const long long code_at = lz_header_bytes(nb) + (long long)hdr[1 + b];
+  const int code_bytes = lz_code_bytes(hdr, b, nb, payload_stride);
+  if (code_bytes < 2) return;                     // corrupt header: leave the block untouched
+  lz_decode_block_warp<Sym>(base + code_at, code_bytes,
                             reinterpret_cast<Sym*>(raw + s * raw_bytes + off), bytes / (int)sizeof(Sym), smem[warp], lane);
 }
 
@@ -684,7 +691,8 @@ void lz_decode_cpu(const uint8_t* payload, uint8_t* raw, long long slices, long 
     const uint8_t* base = payload + s * payload_stride;
     const uint32_t* hdr = reinterpret_cast<const uint32_t*>(base);
     for (long long b = 0; b < nb; ++b)
-      lz_decode_one(base + lz_header_bytes(nb) + hdr[1 + b], raw + s * raw_bytes, raw_bytes, b, sym);
+      if (lz_code_bytes(hdr, b, nb, payload_stride) > 0)
+        lz_decode_one(base + lz_header_bytes(nb) + hdr[1 + b], raw + s * raw_bytes, raw_bytes, b, sym);
   }
 }
 

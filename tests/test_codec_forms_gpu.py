@@ -98,3 +98,28 @@ def test_codecs_take_tensors_off_the_vector_boundary(name, dtype):
         room = torch.empty(a.wires[0].numel() + 1, dtype=torch.uint8, device='cuda')
         moved = codecs.Packed([room[1:].view_as(a.wires[0]).copy_(a.wires[0])] + a.wires[1:], a.meta)
         assert torch.equal(codec.decompress(moved), codec.decompress(b))
+
+
+@pytest.mark.parametrize('device', ['cpu', 'cuda'])
+@pytest.mark.parametrize('damage', ['far', 'long', 'backwards'])
+def test_lz_blocks_with_a_damaged_header_are_left_alone(device, damage):
+    """Offsets that point outside the slice, or enclose no code, are not followed; the other blocks decode."""
+    lib = _lib()
+    raw = torch.randint(0, 3, (2, 4 * 2048), generator=torch.Generator().manual_seed(1)).to(torch.uint8).to(device)
+    payload, sizes = lib.lz_encode(raw, 2)
+    head = payload.view(torch.int32)[1]          # {blocks, offset of block 0, 1, 2, 3, end}
+    good = {'far': [0, 1], 'long': [0, 1, 2], 'backwards': [0, 2, 3]}[damage]
+    if damage == 'far':                          # block 2 and what follows it
+        head[4] = head[5] = 0x7ffffff0
+    elif damage == 'long':
+        head[5] = head[5] + 100000
+    else:                                        # block 1 would end before it begins, block 2 starts where it did
+        head[2] = head[3] + 4
+    out = lib.lz_decode(payload, sizes, raw.size(1), 2)
+    assert torch.equal(out[0], raw[0])
+    for b in good:
+        if damage == 'backwards' and b == 0:
+            continue                             # its code now runs into block 1's
+        assert torch.equal(out[1, b * 2048:(b + 1) * 2048], raw[1, b * 2048:(b + 1) * 2048])
+    with pytest.raises(RuntimeError, match='header'):
+        lib.lz_decode(payload[:, :16].contiguous(), sizes, raw.size(1), 2)
