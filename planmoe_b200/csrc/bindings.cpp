@@ -1265,6 +1265,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def_readwrite("perm_local_first", &GemmOpts::perm_local_first)
       .def_readwrite("copy_nblk", &GemmOpts::copy_nblk)
       .def_readwrite("rows_used", &GemmOpts::rows_used)
+      .def_readwrite("colsum", &GemmOpts::colsum)
       .def_readwrite("trace_ptr", &GemmOpts::trace_ptr)
       .def_readwrite("dq_ptr", &GemmOpts::dq_ptr)
       .def_readwrite("dq_arrival_ptr", &GemmOpts::dq_arrival_ptr)
