@@ -1,4 +1,4 @@
-// Entry points of kernels/gemm_local.cu for the GEMM launcher.
+// Entry points of kernels/gemm_local.cu and kernels/gemm_stream.cu for the GEMM launcher.
 #pragma once
 
 #include "planmoe.h"
@@ -27,5 +27,19 @@ bool local_gemm_takes(int epilogue, bool a_mn, bool b_mn);
 // even, all resident at once.
 cudaError_t launch_local_gemm(int epilogue, bool a_mn, bool b_mn, const CUtensorMap& ta, const CUtensorMap& tb,
                              const CUtensorMap& td, const CUtensorMap& tx, const LocalGemm& p, int ctas, cudaStream_t stream);
+
+// kernels/gemm_stream.cu: at most 128 rows a group, B MN-major, D = act(A . B + bias), aux (optional) = act'.
+struct StreamGemm {
+  int groups, M, N, K;
+  int activation, split;         // split: CTAs that share a tile's contraction (set by the launch)
+  const __nv_bfloat16* bias;     // [groups][N], on 16 bytes, or null
+  __nv_bfloat16* D; long long d_row_stride, d_group_stride;
+  __nv_bfloat16* aux; long long aux_row_stride, aux_group_stride;
+  const int* rows_used;          // [groups] rows in use, or null; the rows of a group without any are zeros
+  unsigned long long budget_ns;
+  int* status;
+};
+int stream_gemm_box(int M);      // rows of the A map's box
+cudaError_t launch_stream_gemm(const CUtensorMap& ta, const CUtensorMap& tb, StreamGemm p, int sms, cudaStream_t stream);
 
 }  // namespace planmoe
