@@ -146,6 +146,15 @@ __device__ __forceinline__ bool wait_flag_ge(const unsigned long long* flag, uns
   }
 }
 
+// ---- chained launches (launch.cuh) ----
+// What every kernel that is launched so does before it touches global memory: wait until the kernels before it have completed
+// and their writes are visible, then let the next one of the stream be brought onto the SMs as this one's blocks leave them.
+// In this order, so that at most one kernel is ahead of the one that runs.  Without the launch attribute both do nothing.
+__device__ __forceinline__ void chain_begin() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // ---- shared-memory barriers and the bulk-copy engine (cp.async.bulk, no tensor map) ----
 // Bulk copies move 16-byte-aligned byte ranges between global and shared memory without occupying
 // threads: a load completes on an mbarrier (complete_tx), stores are tracked in per-thread bulk groups.

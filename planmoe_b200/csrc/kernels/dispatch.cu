@@ -19,6 +19,7 @@
 
 #include "planmoe.h"
 #include "kernels/common.cuh"
+#include "kernels/launch.cuh"
 
 namespace planmoe {
 
@@ -213,6 +214,7 @@ gather_rows_kernel(const void* __restrict__ disp_, const float* __restrict__ sca
                    const int* __restrict__ idx, const int* __restrict__ loc,
                    const float* __restrict__ gates, T* __restrict__ out, int K, int S, int M,
                    int C, WaitGeom w, long long group_rows, bool round_gates) {
+  chain_begin();
   __shared__ int ok_s;
   if (w.flags != nullptr) {
     if (threadIdx.x == 0) ok_s = 1;
@@ -337,14 +339,13 @@ void launch_gather_rows(const void* disp, const float* scale_bias, const int* id
   int ctas = (S + kRowWarps - 1) / kRowWarps;
   if (ctas > 148 * 8) ctas = 148 * 8;
   if (ctas < 1) ctas = 1;
-  if (scale_bias != nullptr && group_rows > 0)
-    gather_rows_kernel<T, 2, 8><<<ctas, kRowThreads, 0, stream>>>(disp, scale_bias, idx, loc, gates, out, K, S, M, C, w, group_rows, round_gates);
-  else if (scale_bias != nullptr)
-    gather_rows_kernel<T, 1, 8><<<ctas, kRowThreads, 0, stream>>>(disp, scale_bias, idx, loc, gates, out, K, S, M, C, w, 0, round_gates);
-  else if (K <= 2)
-    gather_rows_kernel<T, 0, 2><<<ctas, kRowThreads, 0, stream>>>(disp, scale_bias, idx, loc, gates, out, K, S, M, C, w, 0, round_gates);
+  auto kern = scale_bias != nullptr ? (group_rows > 0 ? gather_rows_kernel<T, 2, 8> : gather_rows_kernel<T, 1, 8>)
+            : K <= 2 ? gather_rows_kernel<T, 0, 2> : gather_rows_kernel<T, 0, 8>;
+  if (scale_bias == nullptr) group_rows = 0;
+  if (wait != nullptr)                             // flags of other ranks: as the last one on the stream, not ahead of its turn
+    kern<<<ctas, kRowThreads, 0, stream>>>(disp, scale_bias, idx, loc, gates, out, K, S, M, C, w, group_rows, round_gates);
   else
-    gather_rows_kernel<T, 0, 8><<<ctas, kRowThreads, 0, stream>>>(disp, scale_bias, idx, loc, gates, out, K, S, M, C, w, 0, round_gates);
+    launch_chained(kern, ctas, kRowThreads, 0, stream, disp, scale_bias, idx, loc, gates, out, K, S, M, C, w, group_rows, round_gates);
 }
 
 // dgates[k][t] = <disp[slot_k(t)], dy[t]>.  With `scaled` != null the same pass also writes the
@@ -482,6 +483,7 @@ template <bool SCALE, bool Q8>
 __global__ void __launch_bounds__(kRowThreads)
 slots_fill_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ slot_map, const float* __restrict__ gates,
                   const int* __restrict__ used, __nv_bfloat16* __restrict__ out, int K, int S, int M, int E, int C) {
+  chain_begin();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nvec = M / 8;
   const long long rows = (long long)E * C;
@@ -538,6 +540,7 @@ slots_gate_grad_kernel(const __nv_bfloat16* __restrict__ disp, const __nv_bfloat
                        const int* __restrict__ idx, const int* __restrict__ loc, const float* __restrict__ gates,
                        const int* __restrict__ used, float* __restrict__ dgates, __nv_bfloat16* __restrict__ ddisp, int K,
                        int S, int M, int E, int C) {
+  chain_begin();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nvec = M / 8;
   const long long items = (long long)S + (long long)E * kSlotBlock;
@@ -612,6 +615,7 @@ slots_gate_grad_q8_kernel(const unsigned char* __restrict__ disp, const float2* 
                           const __nv_bfloat16* __restrict__ dy, const int* __restrict__ idx, const int* __restrict__ loc,
                           const float* __restrict__ gates, const int* __restrict__ used, float* __restrict__ dgates,
                           __nv_bfloat16* __restrict__ ddisp, int K, int S, int M, int E, int C) {
+  chain_begin();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nvec = M / 8;
   const long long items = (long long)S + (long long)E * kSlotBlock, slots = (long long)E * C;
@@ -669,15 +673,14 @@ unsigned row_grid(long long rows) {
 void launch_slots_fill(const void* x, const int* slot_map, const float* gates, const int* used, void* out, int K, int S,
                        int M, int E, int C, bool int8, cudaStream_t stream) {
   auto kern = int8 ? slots_fill_kernel<false, true> : gates != nullptr ? slots_fill_kernel<true, false> : slots_fill_kernel<false, false>;
-  kern<<<row_grid((long long)E * C), kRowThreads, 0, stream>>>(reinterpret_cast<const __nv_bfloat16*>(x), slot_map, gates,
+  launch_chained(kern, row_grid((long long)E * C), kRowThreads, 0, stream, reinterpret_cast<const __nv_bfloat16*>(x), slot_map, gates,
                                                                used, reinterpret_cast<__nv_bfloat16*>(out), K, S, M, E, C);
 }
 
 void launch_slots_gate_grad_q8(const void* disp, const float* disp_scales, const void* dy, const int* idx, const int* loc,
                                const float* gates, const int* used, float* dgates, void* ddisp, int K, int S, int M, int E,
                                int C, cudaStream_t stream) {
-  slots_gate_grad_q8_kernel<<<row_grid((long long)S + (long long)E * kSlotBlock), kRowThreads, 0, stream>>>(
-      reinterpret_cast<const unsigned char*>(disp), reinterpret_cast<const float2*>(disp_scales),
+  launch_chained(slots_gate_grad_q8_kernel, row_grid((long long)S + (long long)E * kSlotBlock), kRowThreads, 0, stream, reinterpret_cast<const unsigned char*>(disp), reinterpret_cast<const float2*>(disp_scales),
       reinterpret_cast<const __nv_bfloat16*>(dy), idx, loc, gates, used, dgates, reinterpret_cast<__nv_bfloat16*>(ddisp), K, S, M,
       E, C);
 }
@@ -686,8 +689,7 @@ void launch_slots_gate_grad(const void* disp, const void* dy, const int* idx, co
                             const int* used, float* dgates, void* ddisp, int K, int S, int M, int E, int C,
                             cudaStream_t stream) {
   auto kern = K <= 1 ? slots_gate_grad_kernel<1> : K <= 2 ? slots_gate_grad_kernel<2> : slots_gate_grad_kernel<4>;
-  kern<<<row_grid((long long)S + (long long)E * kSlotBlock), kRowThreads, 0, stream>>>(
-      reinterpret_cast<const __nv_bfloat16*>(disp), reinterpret_cast<const __nv_bfloat16*>(dy), idx, loc, gates, used, dgates,
+  launch_chained(kern, row_grid((long long)S + (long long)E * kSlotBlock), kRowThreads, 0, stream, reinterpret_cast<const __nv_bfloat16*>(disp), reinterpret_cast<const __nv_bfloat16*>(dy), idx, loc, gates, used, dgates,
       reinterpret_cast<__nv_bfloat16*>(ddisp), K, S, M, E, C);
 }
 

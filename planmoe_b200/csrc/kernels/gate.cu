@@ -17,6 +17,7 @@
 
 #include "planmoe.h"
 #include "kernels/common.cuh"
+#include "kernels/launch.cuh"
 
 namespace planmoe {
 
@@ -57,6 +58,7 @@ gate_stats_kernel(const T* __restrict__ logits, int S, int E, int K, int nblk,
                   int* __restrict__ slot_map, long long slots,
                   const int* __restrict__ perm)   // token at each position of the slot order, or null: token order
 {
+  chain_begin();
   __shared__ int warp_cnt[kGateWarps][kMaxK][kMaxE];
   __shared__ float score_sum[kGateWarps][kMaxE];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -146,6 +148,7 @@ gate_assign_kernel(int S, int E, int K, int C, int normalize, float eps,
                    const int* __restrict__ perm,
                    int* __restrict__ copies)      // [3][K][S]: idx, loc and gates (fp32) once more, or null
 {
+  chain_begin();
   __shared__ int base[kMaxK][kMaxE];
   __shared__ float red[kMaxE];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -245,6 +248,7 @@ gate_bwd_kernel(const T* __restrict__ logits, int S, int E, int K, int normalize
                 const float* __restrict__ dl_aux,                                 // [1] or null
                 const __nv_bfloat16* __restrict__ dl_aux_bf16,                    // [1] or null
                 const int* __restrict__ top1_count, T* __restrict__ dlogits) {
+  chain_begin();
   const int t = blockIdx.x * kGateBwdThreads + threadIdx.x;
   if (t >= S) return;
   float p[ME];
@@ -317,9 +321,9 @@ void launch_gate_forward(const T* logits, int S, int E, int K, int C, bool norma
   const int nblk = (S + kGateThreads - 1) / kGateThreads;
   auto stats = E <= 8 ? gate_stats_kernel<T, 8, SCORES> : E <= 16 ? gate_stats_kernel<T, 16, SCORES>
              : E <= 32 ? gate_stats_kernel<T, 32, SCORES> : gate_stats_kernel<T, 64, SCORES>;
-  stats<<<nblk, kGateThreads, 0, stream>>>(logits, S, E, K, nblk, idx, raw_gate, ws_rank, ws_blk_count, ws_blk_score,
+  launch_chained(stats, nblk, kGateThreads, 0, stream, logits, S, E, K, nblk, idx, raw_gate, ws_rank, ws_blk_count, ws_blk_score,
                                            slot_map, slot_map != nullptr ? (long long)E * C : 0, perm);
-  gate_assign_kernel<<<nblk, kGateThreads, 0, stream>>>(S, E, K, C, normalize ? 1 : 0, eps, idx,
+  launch_chained(gate_assign_kernel, nblk, kGateThreads, 0, stream, S, E, K, C, normalize ? 1 : 0, eps, idx,
                                                       raw_gate, ws_rank, ws_blk_count, ws_blk_score,
                                                       nblk, loc, gates, slot_map, top1_count, used, l_aux,
                                                       reinterpret_cast<__nv_bfloat16*>(l_aux_bf16), perm, copies);
@@ -332,7 +336,7 @@ void launch_gate_backward(const T* logits, int S, int E, int K, bool normalize, 
   const int nblk = (S + kGateBwdThreads - 1) / kGateBwdThreads;
   auto bwd = E <= 8 ? gate_bwd_kernel<T, 8, SCORES> : E <= 16 ? gate_bwd_kernel<T, 16, SCORES>
            : E <= 32 ? gate_bwd_kernel<T, 32, SCORES> : gate_bwd_kernel<T, 64, SCORES>;
-  bwd<<<nblk, kGateBwdThreads, 0, stream>>>(logits, S, E, K, normalize ? 1 : 0, eps, idx, dgates, dl_aux,
+  launch_chained(bwd, nblk, kGateBwdThreads, 0, stream, logits, S, E, K, normalize ? 1 : 0, eps, idx, dgates, dl_aux,
                                          reinterpret_cast<const __nv_bfloat16*>(dl_aux_bf16), top1_count, dlogits);
 }
 
@@ -347,6 +351,7 @@ int gate_workspace_blocks(int S) { return (S + kGateThreads - 1) / kGateThreads;
 template <class T>
 __global__ void __launch_bounds__(256)
 importance_key_kernel(const T* __restrict__ logits, int S, int E, float* __restrict__ key) {
+  chain_begin();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= S) return;
   const T* row = logits + (size_t)t * E;
@@ -368,6 +373,7 @@ constexpr int kRankTile = 4096;
 template <int TOK>
 __global__ void __launch_bounds__(256)
 importance_rank_kernel(const float* __restrict__ key, int S, int* __restrict__ rank, int* __restrict__ perm) {
+  chain_begin();
   __shared__ __align__(16) float tile[kRankTile];
   const int part = threadIdx.x & 7;
   const int t0 = blockIdx.x * 32 * TOK;           // a CTA's tokens lie in one tile
@@ -424,9 +430,9 @@ importance_rank_kernel(const float* __restrict__ key, int S, int* __restrict__ r
 template <class T>
 void launch_importance_order(const T* logits, int S, int E, float* key, int* rank, int* perm, cudaStream_t stream) {
   if (S <= 0) return;
-  importance_key_kernel<T><<<(S + 255) / 256, 256, 0, stream>>>(logits, S, E, key);
-  if (S >= 64 * 148) importance_rank_kernel<2><<<(S + 63) / 64, 256, 0, stream>>>(key, S, rank, perm);
-  else importance_rank_kernel<1><<<(S + 31) / 32, 256, 0, stream>>>(key, S, rank, perm);
+  launch_chained(importance_key_kernel<T>, (S + 255) / 256, 256, 0, stream, logits, S, E, key);
+  if (S >= 64 * 148) launch_chained(importance_rank_kernel<2>, (S + 63) / 64, 256, 0, stream, key, S, rank, perm);
+  else launch_chained(importance_rank_kernel<1>, (S + 31) / 32, 256, 0, stream, key, S, rank, perm);
 }
 template void launch_importance_order<float>(const float*, int, int, float*, int*, int*, cudaStream_t);
 template void launch_importance_order<__nv_bfloat16>(const __nv_bfloat16*, int, int, float*, int*, int*, cudaStream_t);

@@ -14,6 +14,7 @@
 
 #include "planmoe.h"
 #include "kernels/common.cuh"
+#include "kernels/launch.cuh"
 
 #include <type_traits>
 
@@ -47,6 +48,7 @@ template <int NT, int MT, bool W_BF16>
 __global__ void __launch_bounds__(kProjWarps * 32)
 gate_project_kernel(const __nv_bfloat16* __restrict__ x, const void* __restrict__ w_, float* __restrict__ logits, int S, int E,
                     int M, int round_bf16) {
+  chain_begin();
   __shared__ float part[kProjWarps][16 * MT][NT * 8 + 1];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3;
   const int t0 = blockIdx.x * 16 * MT;
@@ -155,6 +157,7 @@ template <int EB>
 __global__ void __launch_bounds__(256)
 gate_wgrad_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ dl, float* __restrict__ partial, int S, int E,
                   int M, int chunk_tokens) {
+  chain_begin();
   __shared__ float2 d_s[kWgradTokens][EB];
   __shared__ float red[8][256];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -227,6 +230,7 @@ __global__ void __launch_bounds__(256, MAXK <= 2 ? 4 : 2)
 gather_gate_kernel(const void* __restrict__ slots_, const float2* __restrict__ scales, const int* __restrict__ idx, const int* __restrict__ loc,
                    const float* __restrict__ gates, const float* __restrict__ dl, const void* __restrict__ w_,
                    __nv_bfloat16* __restrict__ dx, int K, int S, int M, int E, int C) {
+  chain_begin();
   constexpr bool GATED = FORM == kGatherGated, Q8 = FORM == kGatherInt8;
   extern __shared__ __align__(16) float gather_smem[];
   float* w_s = gather_smem;        // [E][first four, last four of eight columns][32 lanes][4]: no bank conflicts
@@ -338,11 +342,11 @@ void project_nt(const void* x, const void* w, float* logits, int S, int E, int M
   const __nv_bfloat16* xb = reinterpret_cast<const __nv_bfloat16*>(x);
   if constexpr (NT > 1) {
     if (S >= kProjWide) {
-      gate_project_kernel<NT, 2, W_BF16><<<(S + 31) / 32, kProjWarps * 32, 0, stream>>>(xb, w, logits, S, E, M, round_bf16);
+      launch_chained(gate_project_kernel<NT, 2, W_BF16>, (S + 31) / 32, kProjWarps * 32, 0, stream, xb, w, logits, S, E, M, round_bf16);
       return;
     }
   }
-  gate_project_kernel<NT, 1, W_BF16><<<(S + 15) / 16, kProjWarps * 32, 0, stream>>>(xb, w, logits, S, E, M, round_bf16);
+  launch_chained(gate_project_kernel<NT, 1, W_BF16>, (S + 15) / 16, kProjWarps * 32, 0, stream, xb, w, logits, S, E, M, round_bf16);
 }
 
 }  // namespace
@@ -371,10 +375,10 @@ void launch_gate_wgrad(const void* x, const float* dl, float* partial, int S, in
   const int n = gate_wgrad_chunks(S, M), tokens = (S + n - 1) / n;
   const dim3 grid((M + 255) / 256, n);
   const __nv_bfloat16* xb = reinterpret_cast<const __nv_bfloat16*>(x);
-  if (E <= 2) gate_wgrad_kernel<2><<<grid, 256, 0, stream>>>(xb, dl, partial, S, E, M, tokens);
-  else if (E <= 4) gate_wgrad_kernel<4><<<grid, 256, 0, stream>>>(xb, dl, partial, S, E, M, tokens);
-  else if (E <= 8) gate_wgrad_kernel<8><<<grid, 256, 0, stream>>>(xb, dl, partial, S, E, M, tokens);
-  else gate_wgrad_kernel<16><<<grid, 256, 0, stream>>>(xb, dl, partial, S, E, M, tokens);
+  if (E <= 2) launch_chained(gate_wgrad_kernel<2>, grid, 256, 0, stream, xb, dl, partial, S, E, M, tokens);
+  else if (E <= 4) launch_chained(gate_wgrad_kernel<4>, grid, 256, 0, stream, xb, dl, partial, S, E, M, tokens);
+  else if (E <= 8) launch_chained(gate_wgrad_kernel<8>, grid, 256, 0, stream, xb, dl, partial, S, E, M, tokens);
+  else launch_chained(gate_wgrad_kernel<16>, grid, 256, 0, stream, xb, dl, partial, S, E, M, tokens);
 }
 
 void launch_gather_gate(const void* slots, const float* scales, const int* idx, const int* loc, const float* gates,
@@ -392,7 +396,7 @@ void launch_gather_gate(const void* slots, const float* scales, const int* idx, 
   auto kern = scales != nullptr ? pick(std::integral_constant<int, kGatherInt8>{})
             : gates != nullptr  ? pick(std::integral_constant<int, kGatherGated>{})
                                 : pick(std::integral_constant<int, kGatherPlain>{});
-  kern<<<grid, 256, smem, stream>>>(slots, reinterpret_cast<const float2*>(scales), idx, loc, gates, dl, w, db, K, S, M, E, C);
+  launch_chained(kern, grid, 256, smem, stream, slots, reinterpret_cast<const float2*>(scales), idx, loc, gates, dl, w, db, K, S, M, E, C);
 }
 
 }  // namespace planmoe

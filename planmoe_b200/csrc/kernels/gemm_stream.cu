@@ -88,6 +88,7 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   tc_fence_after();
   const uint32_t tmem = ctl->tmem_base;
 
+  chain_begin();
   // this CTA's K blocks; none where the group holds no token
   const int kb_total = (p.K + BK - 1) / BK, per = (kb_total + p.split - 1) / p.split;
   const int kb0 = rank * per;
@@ -221,11 +222,13 @@ cudaError_t launch_rows(const CUtensorMap& ta, const CUtensorMap& tb, const Stre
   cfg.blockDim = dim3(kStreamThreads, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = (unsigned)p.split; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;     // see launch.cuh
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   return cudaLaunchKernelEx(&cfg, kern, ta, tb, p);
 }
 
