@@ -222,11 +222,11 @@ std::vector<Tensor> importance_order_op(const Tensor& logits) {
   TORCH_CHECK(logits.is_cuda() && logits.dim() == 2 && logits.is_contiguous());
   const int S = logits.size(0), E = logits.size(1);
   c10::cuda::CUDAGuard guard(logits.device());
-  Tensor key = torch::empty({S}, logits.options().dtype(at::kFloat));
+  Tensor ws = torch::empty({importance_workspace(S)}, logits.options().dtype(at::kLong));
   Tensor rank = torch::empty({S}, logits.options().dtype(at::kInt)), perm = torch::empty({S}, logits.options().dtype(at::kInt));
   DISPATCH_FLOAT(logits, "importance_order", [&] {
-    launch_importance_order<scalar_t>(reinterpret_cast<const scalar_t*>(logits.data_ptr()), S, E, key.data_ptr<float>(),
-                                      rank.data_ptr<int>(), perm.data_ptr<int>(), cur_stream());
+    launch_importance_order<scalar_t>(reinterpret_cast<const scalar_t*>(logits.data_ptr()), S, E,
+                                      reinterpret_cast<unsigned long long*>(ws.data_ptr()), rank.data_ptr<int>(), perm.data_ptr<int>(), cur_stream());
   });
   return {rank, perm};
 }
@@ -908,11 +908,13 @@ std::tuple<std::vector<Tensor>, int64_t> local_moe_forward_op(
   {
     Stage st(stages, "fwd.gate_topk_scan");
     if (prio) {
-      order = torch::empty({3, S}, iopt);         // keys, ranks, permutation
-      int* o = order.data_ptr<int>();
+      const int64_t words = importance_workspace(S);
+      order = torch::empty({words + S}, x.options().dtype(at::kLong));        // sorted tiles, ranks and permutation
+      unsigned long long* const ws64 = reinterpret_cast<unsigned long long*>(order.data_ptr());
+      int* const o = reinterpret_cast<int*>(ws64 + words);
       count_launch(2);
-      launch_importance_order<float>(logits.data_ptr<float>(), S, E, reinterpret_cast<float*>(o), o + S, o + 2 * S, cur_stream());
-      perm = o + 2 * S;
+      launch_importance_order<float>(logits.data_ptr<float>(), S, E, ws64, o, o + S, cur_stream());
+      perm = o + S;
     }
     const bool dynamic = capacity < 0, map_later = dynamic || (int8 && capacity % 32 != 0);
     if (!map_later) r.slot_map = torch::empty({E * capacity}, iopt);

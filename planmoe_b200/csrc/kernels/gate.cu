@@ -345,9 +345,13 @@ int gate_workspace_blocks(int S) { return (S + kGateThreads - 1) / kGateThreads;
 // ---- batch-prioritised routing: the order in which tokens claim slots -------------------------------
 // The reference sorts tokens by the score of their best expert, highest first (importance = -max softmax
 // score, PlanMoE/impls/fast_dispatch.py:135-138,153-154), and scans locations in that order.  Here the order
-// comes from a counting rank: key[t] = max_e softmax(logits[t])[e] = 1 / sum_e exp(l[t][e] - max_e l[t]);
+// comes from a rank: key[t] = max_e softmax(logits[t])[e] = 1 / sum_e exp(l[t][e] - max_e l[t]);
 // rank[t] = number of tokens that go before t (larger key, or the same key and a lower index), perm = rank^-1.
-// S^2 comparisons on fp32 keys staged through shared memory: exact, stable and free of sort libraries.
+// Few tokens: S^2 comparisons on fp32 keys staged through shared memory.  Many: sorted tiles.  Both are exact, stable and the same
+// work whatever the keys are.  (us for 4096, 16384 and 65536 tokens: counting 14 - 16, 46 - 48, 500; tiles 12 - 20, 27 - 35, 95 - 128,
+// for two and sixteen experts.)
+constexpr int kSortTokens = 8192;
+
 template <class T>
 __global__ void __launch_bounds__(256)
 importance_key_kernel(const T* __restrict__ logits, int S, int E, float* __restrict__ key) {
@@ -363,80 +367,147 @@ importance_key_kernel(const T* __restrict__ logits, int S, int E, float* __restr
   key[t] = k > 0.f ? k : 0.f;                     // NaN scores go last: ranks stay a permutation
 }
 
-// 32 tokens per CTA and pass, eight threads per token: each thread counts over an eighth of every key tile, the eight
+// 32 tokens per CTA, eight threads per token: each thread counts over an eighth of every key tile, the eight
 // counts are added by shuffles.  Ties need the index only in the tile that holds the token: every key of an earlier tile
 // goes before it from equality on, every key of a later one only when it is larger, so that a comparison is one test and
-// one add, on four keys per load.  Two tokens a thread share the loads once there are tokens enough for all SMs, and
-// a tile of 4096 keys leaves few barriers.  (16384 tokens: 115 us with the full test on single keys, 55 us with one token a
-// thread and tiles of 1024.)
-constexpr int kRankTile = 4096;
-template <int TOK>
+// one add, on four keys per load.  A tile of 4096 keys leaves few barriers.
+constexpr int kCountTile = 4096;
 __global__ void __launch_bounds__(256)
-importance_rank_kernel(const float* __restrict__ key, int S, int* __restrict__ rank, int* __restrict__ perm) {
+importance_count_kernel(const float* __restrict__ key, int S, int* __restrict__ rank, int* __restrict__ perm) {
   chain_begin();
-  __shared__ __align__(16) float tile[kRankTile];
+  __shared__ __align__(16) float tile[kCountTile];
   const int part = threadIdx.x & 7;
-  const int t0 = blockIdx.x * 32 * TOK;           // a CTA's tokens lie in one tile
-  float mine[TOK];
-  int before[TOK];
-#pragma unroll
-  for (int j = 0; j < TOK; ++j) {
-    const int t = t0 + j * 32 + (threadIdx.x >> 3);
-    mine[j] = t < S ? key[t] : 0.f;
-    before[j] = 0;
-  }
-  for (int base = 0; base < S; base += kRankTile) {
+  const int t0 = blockIdx.x * 32, t = t0 + (threadIdx.x >> 3);   // a CTA's tokens lie in one tile
+  const float mine = t < S ? key[t] : 0.f;
+  int before = 0;
+  for (int base = 0; base < S; base += kCountTile) {
     __syncthreads();
-    for (int i = threadIdx.x; i < kRankTile; i += blockDim.x) tile[i] = base + i < S ? key[base + i] : -INFINITY;
+    for (int i = threadIdx.x; i < kCountTile; i += blockDim.x) tile[i] = base + i < S ? key[base + i] : -INFINITY;
     __syncthreads();
     const int own = t0 - base;
-    const int n = min(kRankTile, S - base);       // keys are positive: the padding behind the last one never counts
-    if (own >= 0 && own < kRankTile) {
-      for (int i = part; i < n; i += 8) {
-#pragma unroll
-        for (int j = 0; j < TOK; ++j) {
-          const int t = t0 + j * 32 + (threadIdx.x >> 3);
-          before[j] += (tile[i] > mine[j] || (tile[i] == mine[j] && base + i < t)) ? 1 : 0;
-        }
-      }
+    const int n = min(kCountTile, S - base);      // keys are positive: the padding behind the last one never counts
+    if (own >= 0 && own < kCountTile) {
+      for (int i = part; i < n; i += 8) before += (tile[i] > mine || (tile[i] == mine && base + i < t)) ? 1 : 0;
     } else if (own > 0) {
 #pragma unroll 4
       for (int i = part * 4; i < n; i += 32) {    // an earlier tile is full
         const float4 k = *reinterpret_cast<const float4*>(tile + i);
-#pragma unroll
-        for (int j = 0; j < TOK; ++j)
-          before[j] += (k.x >= mine[j]) + (k.y >= mine[j]) + (k.z >= mine[j]) + (k.w >= mine[j]);
+        before += (k.x >= mine) + (k.y >= mine) + (k.z >= mine) + (k.w >= mine);
       }
     } else {
 #pragma unroll 4
       for (int i = part * 4; i < n; i += 32) {
         const float4 k = *reinterpret_cast<const float4*>(tile + i);
-#pragma unroll
-        for (int j = 0; j < TOK; ++j)
-          before[j] += (k.x > mine[j]) + (k.y > mine[j]) + (k.z > mine[j]) + (k.w > mine[j]);
+        before += (k.x > mine) + (k.y > mine) + (k.z > mine) + (k.w > mine);
       }
     }
   }
-#pragma unroll
-  for (int j = 0; j < TOK; ++j) {
-    before[j] += __shfl_xor_sync(0xffffffffu, before[j], 1);
-    before[j] += __shfl_xor_sync(0xffffffffu, before[j], 2);
-    before[j] += __shfl_xor_sync(0xffffffffu, before[j], 4);
-    const int t = t0 + j * 32 + (threadIdx.x >> 3);
-    if (part == 0 && t < S) { rank[t] = before[j]; perm[before[j]] = t; }
-  }
+  before += __shfl_xor_sync(0xffffffffu, before, 1);
+  before += __shfl_xor_sync(0xffffffffu, before, 2);
+  before += __shfl_xor_sync(0xffffffffu, before, 4);
+  if (part == 0 && t < S) { rank[t] = before; perm[before] = t; }
 }
 
+// Key and index make one 64-bit word, so that no two are equal and smaller goes first.  Blocks sort tiles of 1024 words; a
+// token's rank is then its place in its own tile plus, by binary search, how many words of every other tile are smaller.
+constexpr int kSortTile = 1024;
+constexpr int kSortThreads = kSortTile / 2;
+
 template <class T>
-void launch_importance_order(const T* logits, int S, int E, float* key, int* rank, int* perm, cudaStream_t stream) {
-  if (S <= 0) return;
-  launch_chained(importance_key_kernel<T>, (S + 255) / 256, 256, 0, stream, logits, S, E, key);
-  if (S >= 64 * 148) launch_chained(importance_rank_kernel<2>, (S + 63) / 64, 256, 0, stream, key, S, rank, perm);
-  else launch_chained(importance_rank_kernel<1>, (S + 31) / 32, 256, 0, stream, key, S, rank, perm);
+__global__ void __launch_bounds__(kSortThreads)
+importance_sort_kernel(const T* __restrict__ logits, int S, int E, unsigned long long* __restrict__ sorted) {
+  chain_begin();
+  __shared__ unsigned long long w[2][kSortTile];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t0 = blockIdx.x * kSortTile;
+  // Two words a thread, 32 places apart: distances below 32 by shuffle, 32 in the thread, the ten larger ones in shared memory.
+  const int i0 = warp * 64 + lane;
+  unsigned long long x[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int t = t0 + i0 + 32 * h;
+    x[h] = ~0ull;                                 // behind the last token: behind every token
+    if (t < S) {
+      const T* row = logits + (size_t)t * E;
+      float mx = -INFINITY;
+#pragma unroll 8
+      for (int e = 0; e < E; ++e) mx = fmaxf(mx, to_f32(row[e]));
+      float sum = 0.f;
+#pragma unroll 8
+      for (int e = 0; e < E; ++e) sum += expf(to_f32(row[e]) - mx);
+      float k = 1.f / sum;
+      k = k > 0.f ? k : 0.f;                      // NaN scores go last
+      x[h] = ((unsigned long long)~__float_as_uint(k) << 32) | (unsigned)t;    // positive floats compare as their bits
+    }
+  }
+  int buf = 0;
+#pragma unroll
+  for (int k = 2; k <= kSortTile; k <<= 1) {
+#pragma unroll
+    for (int j = k >> 1; j > 0; j >>= 1) {
+      unsigned long long y[2];
+      if (j == 32) {
+        y[0] = x[1]; y[1] = x[0];
+      } else if (j < 32) {
+        y[0] = __shfl_xor_sync(0xffffffffu, x[0], j); y[1] = __shfl_xor_sync(0xffffffffu, x[1], j);
+      } else {                                    // two buffers: one barrier a stage
+        w[buf][i0] = x[0]; w[buf][i0 + 32] = x[1];
+        __syncthreads();
+        y[0] = w[buf][i0 ^ j]; y[1] = w[buf][(i0 + 32) ^ j];
+        buf ^= 1;
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int i = i0 + 32 * h;
+        const bool smaller = ((i & j) == 0) == ((i & k) == 0);
+        x[h] = (x[h] < y[h]) == smaller ? x[h] : y[h];
+      }
+    }
+  }
+  sorted[t0 + i0] = x[0];
+  sorted[t0 + i0 + 32] = x[1];
 }
-template void launch_importance_order<float>(const float*, int, int, float*, int*, int*, cudaStream_t);
-template void launch_importance_order<__nv_bfloat16>(const __nv_bfloat16*, int, int, float*, int*, int*, cudaStream_t);
-template void launch_importance_order<__half>(const __half*, int, int, float*, int*, int*, cudaStream_t);
+
+constexpr int kRankThreads = 128;
+__global__ void __launch_bounds__(kRankThreads)
+importance_rank_kernel(const unsigned long long* __restrict__ sorted, int S, int* __restrict__ rank, int* __restrict__ perm) {
+  chain_begin();
+  const int i = blockIdx.x * kRankThreads + threadIdx.x;        // a place in a sorted tile: neighbours search alike
+  const int tiles = (S + kSortTile - 1) / kSortTile, own = i / kSortTile;
+  const unsigned long long word = sorted[i];
+  if (word == ~0ull) return;
+  int before = i - own * kSortTile;
+#pragma unroll 8
+  for (int tile = 0; tile < tiles; ++tile) {
+    const unsigned long long* s = sorted + (size_t)tile * kSortTile;
+    int n = 0;                                    // words of the tile that are smaller
+#pragma unroll
+    for (int step = kSortTile / 2; step > 0; step >>= 1) n += s[n + step - 1] < word ? step : 0;
+    n += s[n] < word ? 1 : 0;
+    before += tile == own ? 0 : n;
+  }
+  const int t = (int)(unsigned)word;
+  rank[t] = before;
+  perm[before] = t;
+}
+
+long long importance_workspace(int S) { return (long long)((S + kSortTile - 1) / kSortTile) * kSortTile; }
+
+template <class T>
+void launch_importance_order(const T* logits, int S, int E, unsigned long long* ws, int* rank, int* perm, cudaStream_t stream) {
+  if (S <= 0) return;
+  if (S < kSortTokens) {
+    float* key = reinterpret_cast<float*>(ws);
+    launch_chained(importance_key_kernel<T>, (S + 255) / 256, 256, 0, stream, logits, S, E, key);
+    launch_chained(importance_count_kernel, (S + 31) / 32, 256, 0, stream, key, S, rank, perm);
+    return;
+  }
+  const int tiles = (S + kSortTile - 1) / kSortTile;
+  launch_chained(importance_sort_kernel<T>, tiles, kSortThreads, 0, stream, logits, S, E, ws);
+  launch_chained(importance_rank_kernel, tiles * (kSortTile / kRankThreads), kRankThreads, 0, stream, ws, S, rank, perm);
+}
+template void launch_importance_order<float>(const float*, int, int, unsigned long long*, int*, int*, cudaStream_t);
+template void launch_importance_order<__nv_bfloat16>(const __nv_bfloat16*, int, int, unsigned long long*, int*, int*, cudaStream_t);
+template void launch_importance_order<__half>(const __half*, int, int, unsigned long long*, int*, int*, cudaStream_t);
 
 // slot map of a permuted token order back to token ids: owner = position * K + k -> perm[position] * K + k
 __global__ void remap_slot_map_kernel(int* __restrict__ slot_map, long long n, const int* __restrict__ perm, int K) {
