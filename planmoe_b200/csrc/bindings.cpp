@@ -351,6 +351,8 @@ Tensor route_scores_backward_op(const c10::optional<Tensor>& scores, const c10::
   return out;
 }
 
+#include "routing_nodes.h"
+
 Tensor cumsum_sub_one_op(const Tensor& x) {
   count_launch(2);
   TORCH_CHECK(x.is_cuda() && x.dim() == 2 && x.scalar_type() == at::kInt && x.is_contiguous());
@@ -585,11 +587,11 @@ std::vector<Tensor> colsum2_op(const Tensor& xa, const Tensor& xb, int64_t fold,
 }
 
 // ---- one rank: a pass of the layer, or of its experts, in one call --------------------------------
-// A stage of the pass for the per-stage timers: `stages` is None, or a callable that makes a context manager of a name.
+// A stage of the pass for the per-stage timers: `stages` is None (or null, without the interpreter), or a callable that makes a context manager of a name.
 struct Stage {
   py::object cm;
   Stage(const py::object& stages, const char* name) {
-    if (!stages.is_none()) { cm = stages(name); cm.attr("__enter__")(); }
+    if (stages && !stages.is_none()) { cm = stages(name); cm.attr("__enter__")(); }
   }
   ~Stage() {
     if (!cm) return;
@@ -965,6 +967,9 @@ std::vector<Tensor> local_moe_backward_op(const c10::optional<Tensor>& dy, const
   return local_backward(*dy, x, r, w1, w2, xs, dact, h, ys, scales, need, &g, dl_aux, stages);
 }
 
+#include "layer_node.h"
+#include "layer32.h"
+
 // rows [R, M] -> uint8 [R, M + 16]: M quantised bytes + {scale, low, 0, 0} (the wire rows of the fused send)
 Tensor int8_rows_encode_op(const Tensor& x) {
   count_launch(1);
@@ -1198,6 +1203,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("local_forward", &local_forward_op);
   m.def("local_backward", &local_backward_op);
   m.def("local_moe_forward", &local_moe_forward_op);
+  m.def("local_layer_node", &local_layer_node);
   m.def("local_moe_backward", &local_moe_backward_op);
   m.attr("gate_max_experts") = kProjMaxE;
   // whether the environment leaves a single rank to the direct path (read at every call, like all of these switches)
@@ -1209,6 +1215,11 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("importance_order", &importance_order_op);
   m.def("remap_slot_map", &remap_slot_map_op);
   m.def("gate_backward", &gate_backward_op);
+  m.def("route_scores_node", &route_scores_node);
+  m.def("scatter_node", &scatter_node);
+  m.def("gather_picks_node", &gather_picks_node);
+  m.def("layer32_forward", &layer32_forward_op);
+  m.def("layer32_backward", &layer32_backward_op);
   m.def("route_scores", &route_scores_op);
   m.def("route_scores_backward", &route_scores_backward_op);
   m.def("cumsum_sub_one", &cumsum_sub_one_op);

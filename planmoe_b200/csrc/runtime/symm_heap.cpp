@@ -91,28 +91,19 @@ class SymmHeap {
   std::vector<void*> opened_;
 };
 
-// Host-mapped int32[8] that kernels write error codes to; the host reads it without a sync of
-// its own (after the stream has been synchronised by the caller).
-class StatusWord {
- public:
-  StatusWord() {
-    check(cudaHostAlloc(reinterpret_cast<void**>(&host_), sizeof(int) * 8, cudaHostAllocMapped), "cudaHostAlloc");
-    std::memset(host_, 0, sizeof(int) * 8);
-    check(cudaHostGetDevicePointer(reinterpret_cast<void**>(&dev_), host_, 0), "cudaHostGetDevicePointer");
-  }
-  ~StatusWord() {
-    if (host_ != nullptr) cudaFreeHost(host_);
-  }
-  unsigned long long device_ptr() const { return reinterpret_cast<unsigned long long>(dev_); }
-  std::vector<int> read() const { return std::vector<int>(host_, host_ + 8); }
-  void clear() { std::memset(host_, 0, sizeof(int) * 8); }
-
- private:
-  int* host_ = nullptr;
-  int* dev_ = nullptr;
-};
-
 }  // namespace
+
+namespace planmoe {
+StatusWord::StatusWord() {
+  check(cudaHostAlloc(reinterpret_cast<void**>(&host_), sizeof(int) * 8, cudaHostAllocMapped), "cudaHostAlloc");
+  std::memset(host_, 0, sizeof(int) * 8);
+  check(cudaHostGetDevicePointer(reinterpret_cast<void**>(&dev_), host_, 0), "cudaHostGetDevicePointer");
+}
+StatusWord::~StatusWord() {
+  if (host_ != nullptr) cudaFreeHost(host_);
+}
+void StatusWord::clear() { std::memset(host_, 0, sizeof(int) * 8); }
+}  // namespace planmoe
 
 void bind_symm_heap(py::module_& m) {
   py::class_<SymmHeap>(m, "SymmHeap")
@@ -127,7 +118,8 @@ void bind_symm_heap(py::module_& m) {
       .def("size", &SymmHeap::size)
       .def_property_readonly("rank", &SymmHeap::rank)
       .def_property_readonly("world", &SymmHeap::world);
-  py::class_<StatusWord>(m, "StatusWord")
+  using planmoe::StatusWord;
+  py::class_<StatusWord, std::shared_ptr<StatusWord>>(m, "StatusWord")
       .def(py::init<>())
       .def("device_ptr", &StatusWord::device_ptr)
       .def("read", &StatusWord::read)

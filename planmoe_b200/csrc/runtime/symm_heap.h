@@ -12,4 +12,27 @@
 
 #include <pybind11/pybind11.h>
 
+#include <vector>
+
+namespace planmoe {
+
+// Host-mapped int32[8] that kernels write error codes to; the host reads it without a sync of
+// its own (after the stream has been synchronised by the caller).
+class StatusWord {
+ public:
+  StatusWord();
+  ~StatusWord();
+  StatusWord(const StatusWord&) = delete;
+  StatusWord& operator=(const StatusWord&) = delete;
+  unsigned long long device_ptr() const { return reinterpret_cast<unsigned long long>(dev_); }
+  std::vector<int> read() const { return std::vector<int>(host_, host_ + 8); }
+  void clear();
+
+ private:
+  int* host_ = nullptr;
+  int* dev_ = nullptr;
+};
+
+}  // namespace planmoe
+
 void bind_symm_heap(pybind11::module_& m);

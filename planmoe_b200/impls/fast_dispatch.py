@@ -96,55 +96,6 @@ def _gates_of(gates_all, normalize_gate):
     return gates_s
 
 
-class _RouteScores(torch.autograd.Function):
-    """Top-k, gates, locations, slot map and the value of the GShard loss of fp32 scores in two launches; the gates'
-    gradient in one.  Gradients and slots use ``own``, a second copy of picks, locations and gates: the caller may change the
-    lists of a plan in place."""
-
-    @staticmethod
-    def forward(ctx, scores, top_k, capacity, normalize):
-        ctx.set_materialize_grads(False)
-        idx, loc, slot_map, top1, loss, own, *gates = native.lib().route_scores(scores, top_k, capacity, normalize)
-        ctx.save_for_backward(scores, own, top1)
-        ctx.normalize = normalize
-        ctx.mark_non_differentiable(loss, top1, idx, loc, slot_map, own)
-        return (loss, top1, idx, loc, slot_map, own, *gates)
-
-    @staticmethod
-    def backward(ctx, _loss, _top1, _idx, _loc, _map, _own, *dgates):
-        if all(d is None for d in dgates):
-            return None, None, None, None
-        scores, own, top1 = ctx.saved_tensors
-        picks = own[0]
-        if torch.is_grad_enabled():             # create_graph: the same gradient as differentiable operations
-            pairs = [(g, d) for g, d in zip(_gates_of(scores.gather(1, picks.t().long()), ctx.normalize), dgates)
-                     if d is not None]
-            return torch.autograd.grad([g for g, _ in pairs], scores, [d for _, d in pairs], create_graph=True)[0], \
-                None, None, None
-        return native.lib().route_scores_backward(scores, picks, list(dgates), None, top1, scores.size(0), ctx.normalize), \
-            None, None, None
-
-
-class _RouteLoss(torch.autograd.Function):
-    """The GShard loss that ``_RouteScores`` computed, as a node of its own: its backward can run before, after or without
-    the gates'.  It is linear in the scores, sum_t sum_e scores[t, e] * top1[e] * E / S^2: their values may change before
-    the backward."""
-
-    @staticmethod
-    def forward(ctx, scores, value, top1):
-        ctx.save_for_backward(top1)
-        ctx.shape = scores.shape
-        return value.detach()                   # its own tensor on the value's memory
-
-    @staticmethod
-    def backward(ctx, dloss):
-        top1, = ctx.saved_tensors
-        S, E = ctx.shape
-        if torch.is_grad_enabled():
-            return (dloss * (E / (S * S)) * top1.to(dloss.dtype)).expand(S, E), None, None
-        return native.lib().route_scores_backward(None, None, [], dloss, top1, S, False), None, None
-
-
 def _route_on_kernels(scores, top_k, loss_fn):
     """Whether the routing kernels take this call.  They pick from fp32 scores (a tie goes to the lower expert id) and
     know the GShard loss; other losses and types, batch-prioritised order, function transforms (vmap, forward-mode),
@@ -152,11 +103,7 @@ def _route_on_kernels(scores, top_k, loss_fn):
     return (scores.is_cuda and scores.dtype == torch.float32 and scores.dim() == 2 and scores.size(0) > 0
             and 1 <= scores.size(1) <= 64 and 1 <= top_k <= 4 and scores.size(0) * top_k < 2 ** 31
             and (loss_fn is None or loss_fn is losses.gshard_loss)
-            and type(scores) in (torch.Tensor, torch.nn.Parameter) and gating.use_fast_cumsum
-            and not torch._C._are_functorch_transforms_active()
-            and torch.autograd.forward_ad._current_level < 0
-            and not torch.compiler.is_compiling() and not torch.jit.is_tracing()
-            and torch.utils._python_dispatch._get_current_dispatch_mode() is None)
+            and gating.use_fast_cumsum and D.plain_autograd(scores))
 
 
 def _align(capacity, alignment):
@@ -171,8 +118,11 @@ def extract_critical(scores, top_k, loss_fn=losses.gshard_loss, capacity_factor=
     if not batch_prioritized_routing and _route_on_kernels(scores, top_k, loss_fn):
         capacity = _align(top_k * int(capacity_factor * per_expert), alignment) if capacity_factor > 0 else 0
         scores = scores.contiguous()
-        l_loss, top1, idx, loc, slot_map, own, *gates_s = _RouteScores.apply(scores, top_k, capacity, bool(normalize_gate))
-        l_loss = _RouteLoss.apply(scores, l_loss, top1) if loss_fn is not None else None
+        # top-k, gates, locations, slot map and loss in two launches; gradients and slots use ``own``, a second copy of picks,
+        # locations and gates: the caller may change the lists of a plan in place
+        idx, loc, slot_map, _top1, _value, own, *gates_s = native.lib().route_scores_node(scores, top_k, capacity, bool(normalize_gate),
+                                                                                         loss_fn is not None)
+        l_loss = gates_s.pop() if loss_fn is not None else None
         if capacity_factor <= 0:
             peak = simple_all_reduce(loc.max(), group=group, op=torch.distributed.ReduceOp.MAX)
             capacity = int(peak) + 1

@@ -382,6 +382,13 @@ class MOELayer(torch.nn.Module):
 
     def _generic_forward(self, x, gctx, top_k, cf, degree, reserve_shape, comm_name=None):
         comm_name = comm_name or self.comm_name
+        from ..ops import layer32
+        if layer32.takes(self, gctx, x, top_k, cf, comm_name, reserve_shape):
+            y, l_aux, capacity = layer32.forward(self, x, gctx, top_k, cf, degree)
+            if self.auto_parallel:
+                self.use_model_parallel = True              # what the general rule says with one shard
+            self.last_stats = dict(capacity=capacity, degree=degree, path='generic', comm=comm_name)
+            return y, l_aux
         if x.is_cuda:
             with torch.autocast('cuda', enabled=False):
                 logits_dtype, crit, l_aux = self._route(x, gctx, top_k, cf, degree)

@@ -238,6 +238,15 @@ class _GatherPicks(torch.autograd.Function):
         return (ddisp, None, None, *dg)
 
 
+def plain_autograd(*tensors):
+    """Whether a call's gradients, if any, are those of ordinary reverse-mode autograd, which the C++ nodes know: no function
+    transform (vmap, functional gradients), no forward-mode, no tracing, no dispatch mode, no tensor subclass."""
+    return (not torch._C._are_functorch_transforms_active() and torch.autograd.forward_ad._current_level < 0
+            and not torch.compiler.is_compiling() and not torch.jit.is_tracing()
+            and torch.utils._python_dispatch._get_current_dispatch_mode() is None
+            and all(type(t) in (torch.Tensor, torch.nn.Parameter) for t in tensors))
+
+
 def picks_ok(x, plan, gates):
     """Whether gates go to the kernels pick by pick: fp32 gates of every token for data of the CUDA kernels."""
     return (x.is_cuda and _native_ok(x) and _vector_rows(x) and len(gates) == plan.K
@@ -249,11 +258,15 @@ def scatter_picks(x, plan, rows, gates):
 
 
 def gather_picks(disp, plan, rows, gates):
+    if len(gates) <= 4 and plain_autograd(disp, *gates):
+        return native.lib().gather_picks_node(disp, plan.idx, plan.loc, rows, list(gates), plan._slot_map, plan.E, plan.C)
     return _GatherPicks.apply(disp, plan, rows, *gates)
 
 
 def scatter(x, plan, gates=None):
     """Differentiable encode: ``[S, M] -> [E*C, M]`` (w.r.t. ``x`` and ``gates``)."""
+    if gates is None and x.is_cuda and _native_ok(x) and x.dim() == 2 and _vector_rows(x) and plain_autograd(x):
+        return native.lib().scatter_node(x, plan.idx, plan.loc, plan.slot_map, plan.E, plan.C)
     if _native_ok(x):
         return _Scatter.apply(x, gates, plan)
     return scatter_torch(x, plan, gates)

@@ -40,6 +40,7 @@ import torch
 import torch.nn.functional as F
 
 from . import native
+from .dispatch import plain_autograd
 from .gemm import ACT_CODES, EPI_BIAS_ACT, EPI_DACT, EPI_PUSH, EPI_STORE, grouped_gemm
 from ..parallel import transport as T
 from ..utils import stage_timer
@@ -578,7 +579,12 @@ def _local_layer(layer, st, x, gctx, top_k, capacity, align):
              status=st.tr.status)
     args = (native.aligned(x), w, ex.batched_fc1_w, ex.batched_fc1_bias, ex.batched_fc2_w, ex.batched_fc2_bias)
     if _needs_node(args):
-        y, l_aux = _LocalLayer.apply(*args, m)
+        if not stage_timer.enabled() and plain_autograd(*args):
+            (y, l_aux, *m['routing']), m['capacity'] = native.lib().local_layer_node(
+                *args, m['K'], m['capacity'], m['round_up'], m['normalize'], m['bf16_logits'], m['prio'], m['act'], m['postscore'], m['int8'],
+                m['budget_ms'], m['status'])
+        else:
+            y, l_aux = _LocalLayer.apply(*args, m)
     else:
         (y, l_aux, *saved, loc), m['capacity'] = _local_layer_forward(*args, m, False)
         m['routing'] = saved[4], loc
