@@ -397,6 +397,7 @@ Tensor int8_decode_op(const Tensor& q, const Tensor& scale, const Tensor& bias, 
 struct GemmOpts {
   int64_t epilogue = 0, activation = 0;
   c10::optional<Tensor> bias, aux, out;
+  c10::optional<Tensor> q8_out, q8_scales;      // kEpiStoreQ8: uint8 [groups * M, N], fp32 [N / 128, groups * M, 2]
   // flag gate
   int64_t gate_flags_ptr = 0, gate_rows = 0, gate_want = 0, gate_want_ptr = 0;
   int64_t gate_mode = 0, gate_nblk = 0, perm_w = 0, perm_seg_rows = 0, perm_local_first = 0;
@@ -450,7 +451,11 @@ Tensor grouped_gemm_op(const Tensor& A, bool a_mn, const Tensor& B, bool b_mn, c
   g.epilogue = o.epilogue; g.activation = o.activation;
 
   Tensor out;
-  if (o.epilogue != kEpiPush) {
+  if (o.epilogue == kEpiStoreQ8) {
+    out = o.q8_out.value();
+    g.D = out.data_ptr(); g.d_row_stride = g.N; g.d_group_stride = (long long)g.M * g.N;
+    g.q8_scales = o.q8_scales.value().data_ptr<float>();
+  } else if (o.epilogue != kEpiPush) {
     if (o.out.has_value() && o.out->defined()) {
       out = *o.out;
       TORCH_CHECK(out.scalar_type() == at::kBFloat16 && out.stride(-1) == 1 && out.dim() == 3);
@@ -620,33 +625,25 @@ static void local_check(const Tensor& x, const LocalRoute& r, const Tensor& w1) 
   TORCH_CHECK(!r.int8 || (r.postscore && r.C % 32 == 0 && x.size(1) % 128 == 0), "int8 rows: post-score, 128-column groups, whole slices");
 }
 
-// The expert GEMM whose epilogue writes int8 rows ([E * C, N] bytes and a (scale, low) pair per 128 columns and row) for one
-// rank: the push epilogue with this rank's own memory as the destination, addressed from a base of zero, and a flag that
-// nobody waits for.
-struct Int8Out { Tensor rows, scales; };
-static Int8Out local_gemm_int8(const Tensor& a, const Tensor& w, bool w_mn, const c10::optional<Tensor>& bias, const LocalRoute& r) {
-  const int64_t E = a.size(0), N = w_mn ? w.size(2) : w.size(1);
-  TORCH_CHECK(N % 128 == 0, "int8 rows: 128-column groups");
-  Int8Out out{torch::empty({E * r.C, N}, a.options().dtype(at::kByte)),
-              torch::empty({N / 128, E * r.C, 2}, a.options().dtype(at::kFloat))};
-  Tensor base = torch::zeros({2}, a.options().dtype(at::kLong));     // the base address, the flag
-  GemmOpts o;
-  o.epilogue = kEpiPush; o.budget_ms = r.budget_ms; o.status_ptr = r.status_ptr; o.bias = bias;
-  o.heap_bases_ptr = reinterpret_cast<int64_t>(base.data_ptr());
-  o.heap_bases_host = {0};
-  o.push_flag_off = o.heap_bases_ptr + 8;
-  o.push_data_off = reinterpret_cast<int64_t>(out.rows.data_ptr());
-  o.push_scale_off = reinterpret_cast<int64_t>(out.scales.data_ptr());
-  o.push_q8 = 1; o.push_rows = o.push_C = r.C; o.chunk_groups = E;
-  grouped_gemm_op(a, false, w, w_mn, o);
-  return out;
-}
-
 static GemmOpts local_opts(const LocalRoute& r, int64_t epilogue) {
   GemmOpts o;
   o.epilogue = epilogue; o.activation = r.act; o.budget_ms = r.budget_ms; o.status_ptr = r.status_ptr;
   o.rows_used = r.used;
   return o;
+}
+
+// The expert GEMM whose epilogue writes int8 rows: [E * C, N] bytes and a (scale, low) pair per 128 columns and row.
+struct Int8Out { Tensor rows, scales; };
+static Int8Out local_gemm_int8(const Tensor& a, const Tensor& w, bool w_mn, const c10::optional<Tensor>& bias, const LocalRoute& r) {
+  const int64_t E = a.size(0), N = w_mn ? w.size(2) : w.size(1);
+  TORCH_CHECK(N % 128 == 0 && r.C % 32 == 0 && a.size(1) == r.C, "int8 rows: 128-column groups, slices of 32 rows");
+  Int8Out out{torch::empty({E * r.C, N}, a.options().dtype(at::kByte)),
+              torch::empty({N / 128, E * r.C, 2}, a.options().dtype(at::kFloat))};
+  GemmOpts o = local_opts(r, kEpiStoreQ8);
+  o.bias = bias;
+  o.q8_out = out.rows; o.q8_scales = out.scales;
+  grouped_gemm_op(a, false, w, w_mn, o);
+  return out;
 }
 
 // {y [S, O], xs [E, C, M], dact [E, C, H], h [E, C, H], ys [E, C, O], scales}; without `want_grad` no derivative is saved

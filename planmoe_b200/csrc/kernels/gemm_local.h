@@ -16,6 +16,7 @@ struct LocalGemm {
   const __nv_bfloat16* bias;     // [groups][N] or null
   const int* rows_used;          // [groups] token rows in use (M dim, or the contraction of a weight gradient), or null
   float* colsum;                 // see GemmArgs
+  float* q8_scales;              // kEpiStoreQ8
   unsigned long long budget_ns;
   int* status;
 };
@@ -23,7 +24,8 @@ struct LocalGemm {
 // Whether the kernel exists for an epilogue and operand layouts.
 bool local_gemm_takes(int epilogue, bool a_mn, bool b_mn);
 
-// `ta` / `tb`: boxes of 128 (K-major) or 64 (MN-major) rows; `td`: D, `tx`: the activation derivative, 64 x 32 boxes.  `ctas`:
+// `ta` / `tb`: boxes of 128 (K-major) or 64 (MN-major) rows; `td`: D, `tx`: the activation derivative, 64 x 32 boxes
+// (kEpiStoreQ8: D as uint8 [groups * M][N], 128 x 32 boxes).  `ctas`:
 // even, all resident at once.
 cudaError_t launch_local_gemm(int epilogue, bool a_mn, bool b_mn, const CUtensorMap& ta, const CUtensorMap& tb,
                              const CUtensorMap& td, const CUtensorMap& tx, const LocalGemm& p, int ctas, cudaStream_t stream);

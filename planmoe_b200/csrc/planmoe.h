@@ -65,9 +65,7 @@ void launch_gate_grad(const T* disp, const T* dy, const int* idx, const int* loc
 
 // ---- one rank: tokens straight into the experts' slots ----
 // Of an expert's C slots only the first used[e] hold tokens.  What computes on slots does so in blocks of at most
-// kSlotBlock rows and stops behind the block with the last token; the rows of that block behind it are zeros.  The exception
-// is the GEMM that writes int8 rows: its push epilogue covers all slots, and what it makes of rows that hold nothing is never
-// gathered.
+// kSlotBlock rows and stops behind the block with the last token; the rows of that block behind it are zeros.
 constexpr int kSlotBlock = 256;
 // out[e * C + c] = (gate *) row of the token that holds the slot; int8 (without gates): the row as an int8 transfer
 // delivers it
@@ -162,6 +160,7 @@ enum GemmEpilogue : int {
   kEpiBiasAct = 1,  // t = acc + bias ; D = act(t) ; aux = act'(t)
   kEpiDAct = 2,     // D = acc * aux      (aux = a saved activation derivative)
   kEpiPush = 3,     // (acc + bias) stored into the origin ranks' combine buffers + flags
+  kEpiStoreQ8 = 4,  // D = uint8 rows of (acc + bias), a (scale, low) pair per 128 columns and row; local operands only
 };
 enum Activation : int { kActIdentity = 0, kActRelu = 1, kActGelu = 2, kActSilu = 3 };
 
@@ -182,6 +181,7 @@ struct GemmArgs {
   int epilogue, activation;
   void* D; long long d_row_stride, d_group_stride;          // bf16 output
   void* aux; long long aux_row_stride, aux_group_stride;    // bf16 activation derivative (in or out)
+  float* q8_scales;                // kEpiStoreQ8: fp32 [N / 128][groups * M][2]; D is then uint8 [groups * M][N]
   const void* bias; long long bias_group_stride;            // bf16 [groups][N] or null
   // flag-gated A rows (A is a receive buffer filled by peers): rows [s*gate_rows, (s+1)*gate_rows)
   // of every group become readable when gate_flags[s] >= gate_want.
