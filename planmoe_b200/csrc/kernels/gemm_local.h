@@ -30,7 +30,8 @@ bool local_gemm_takes(int epilogue, bool a_mn, bool b_mn);
 cudaError_t launch_local_gemm(int epilogue, bool a_mn, bool b_mn, const CUtensorMap& ta, const CUtensorMap& tb,
                              const CUtensorMap& td, const CUtensorMap& tx, const LocalGemm& p, int ctas, cudaStream_t stream);
 
-// kernels/gemm_stream.cu: at most 128 rows a group, B MN-major, D = act(A . B + bias), aux (optional) = act'.
+// kernels/gemm_stream.cu: at most kStreamRows rows a group, B MN-major, D = act(A . B + bias), aux (optional) = act'.
+constexpr int kStreamRows = 32;
 struct StreamGemm {
   int groups, M, N, K;
   int activation, split;         // split: CTAs that share a tile's contraction (set by the launch)
@@ -41,7 +42,8 @@ struct StreamGemm {
   unsigned long long budget_ns;
   int* status;
 };
-int stream_gemm_box(int M);      // rows of the A map's box
+bool stream_gemm_pays(int groups, int M, int N, int sms);
+// `ta`: boxes of kStreamRows rows, `tb`: of 64
 cudaError_t launch_stream_gemm(const CUtensorMap& ta, const CUtensorMap& tb, StreamGemm p, int sms, cudaStream_t stream);
 
 }  // namespace planmoe

@@ -1,12 +1,11 @@
-// Grouped bf16 GEMM for a handful of rows a group: y[g] = act(x[g] . w[g] + b[g]) with at most 128 rows, w [K, N] with N
+// Grouped bf16 GEMM for a handful of rows a group: y[g] = act(x[g] . w[g] + b[g]) with at most 32 rows, w [K, N] with N
 // contiguous.  A decoding step or a small batch meets every expert's weights; reading them is all the work there is.
 //
-// What bounded it before (one CTA per 128 x 256 tile over the whole contraction, gemm_tcgen05.cu): too few CTAs with loads in
-// flight.  16 tokens, 8 experts of 1024 x 4096, top-2: 128 CTAs in the first GEMM (25 us for 67 MB of weights), 32 in the second
-// (36 us); they take 21 us each now.  Here a cluster of up to eight CTAs shares a tile and splits its contraction; each keeps a partial sum in TMEM, lays it
-// out in shared memory, and adds up a share of the columns over the cluster's shared memories in CTA order, so that results do
-// not depend on timing.  With at most 32 rows a stage is 36 KiB and two CTAs fit on an SM.  Groups without a token read no
-// weights: their rows are zeros, so that the bias is all there is.
+// One CTA per 128 x 256 tile over the whole contraction (gemm_tcgen05.cu) leaves SMs without loads in flight where there are few
+// tiles: 8 experts of 4096 x 1024 are 32 CTAs.  Here a cluster of up to eight CTAs shares a tile and splits its contraction; each
+// keeps a partial sum in TMEM, lays it out in shared memory, and adds up a share of the columns over the cluster's shared
+// memories in CTA order, so that results do not depend on timing.  Two CTAs fit on an SM.  Groups without a token read no
+// weights: their rows are zeros, so that the bias is all there is.  For which launches: stream_gemm_pays.
 //
 //   warp 0      TMA producer       warp 1   MMA issuer (tcgen05.mma.cta_group::1, 128 x 256 x 16; rows behind the tile's are
 //                                           whatever lies behind them in shared memory and are never read back)
@@ -17,8 +16,6 @@
 #include "kernels/gemm_local.h"
 #include "kernels/gemm_tc.cuh"
 
-#include <climits>
-
 namespace planmoe {
 
 namespace {
@@ -28,16 +25,14 @@ constexpr int kMaxSplit = 8;
 constexpr uint32_t kBBytes = BN * BK * 2;          // 32 KiB
 constexpr int kPartRow = BN + 4;                   // floats between rows of a partial sum: lanes on different banks
 
-template <int ROWS> struct StreamGeo {             // ROWS: rows of the A box, 32 or 128
-  static constexpr uint32_t kABytes = ROWS * BK * 2, kStage = kABytes + kBBytes;
-  static constexpr int kStages = ROWS == 32 ? 3 : 4;
-  static constexpr uint32_t kRing = kStages * kStage, kTotal = kRing + 256;
-  static_assert(ROWS * kPartRow * 4 <= kRing, "the partial sum takes the ring's place");
-  static_assert(kABytes + 128 * 128 <= kStage, "the MMA reads 128 rows from the stage's start");
-};
+constexpr uint32_t kABytes = kStreamRows * BK * 2, kStage = kABytes + kBBytes;
+constexpr int kStages = 3;
+constexpr uint32_t kRing = kStages * kStage, kSmemTotal = kRing + 256;
+static_assert(kStreamRows * kPartRow * 4 <= kRing, "the partial sum takes the ring's place");
+static_assert(kABytes + 128 * 128 <= kStage, "the MMA reads 128 rows from the stage's start");
 
 struct StreamCtl {
-  uint64_t full[4], empty[4], acc_full;
+  uint64_t full[kStages], empty[kStages], acc_full;
   uint32_t tmem_base;
   volatile int abort;
 };
@@ -58,23 +53,21 @@ __device__ __forceinline__ void act8(const pair_t* x, uint4& out, uint4& deriv) 
   deriv = make_uint4(pack_pair(d[0]), pack_pair(d[1]), pack_pair(d[2]), pack_pair(d[3]));
 }
 
-template <int ROWS>
 __global__ void __launch_bounds__(kStreamThreads)
 stream_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const StreamGemm p) {
-  using G = StreamGeo<ROWS>;
   extern __shared__ __align__(1024) uint8_t smem[];
   if ((smem_u32(smem) & 1023u) != 0u) {            // swizzled tiles need 1024-byte aligned stages
     if (threadIdx.x == 0) report_status(p.status, kStatusBadArgument, 1024, (int)(smem_u32(smem) & 1023u), 0);
     return;                                        // same address in every CTA: the whole grid returns
   }
-  StreamCtl* const ctl = reinterpret_cast<StreamCtl*>(smem + G::kRing);
+  StreamCtl* const ctl = reinterpret_cast<StreamCtl*>(smem + kRing);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = (int)cluster_ctarank();
   const int nt_count = (p.N + BN - 1) / BN, tile = (int)blockIdx.x / p.split;
   const int g = tile / nt_count, n0 = (tile - g * nt_count) * BN;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < G::kStages; ++s) { mbar_init(smem_u32(&ctl->full[s]), 1); mbar_init(smem_u32(&ctl->empty[s]), 1); }
+    for (int s = 0; s < kStages; ++s) { mbar_init(smem_u32(&ctl->full[s]), 1); mbar_init(smem_u32(&ctl->empty[s]), 1); }
     mbar_init(smem_u32(&ctl->acc_full), 1);
     ctl->abort = 0;
     fence_barrier_init();
@@ -103,15 +96,15 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
       ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&ctl->empty[stage]), phase ^ 1u, &ctl->abort, p.budget_ns, p.status, 0, stage));
       if (!ok) break;
       if (leader) {
-        const uint32_t full = smem_u32(&ctl->full[stage]), sa = smem_u32(smem) + stage * G::kStage, sb = sa + G::kABytes;
+        const uint32_t full = smem_u32(&ctl->full[stage]), sa = smem_u32(smem) + stage * kStage, sb = sa + kABytes;
         const int k0 = (kb0 + kb) * BK;
-        mbar_expect_tx(full, G::kStage);
+        mbar_expect_tx(full, kStage);
         tma_load_4d<1>(sa, &tmA, full, k0, 0, g, 0);
 #pragma unroll
         for (int h = 0; h < BN / 64; ++h) tma_load_4d<1>(sb + h * (64 * BK * 2), &tmB, full, n0 + h * 64, k0, g, 0);
       }
       __syncwarp();
-      if (++stage == G::kStages) { stage = 0; phase ^= 1u; }
+      if (++stage == kStages) { stage = 0; phase ^= 1u; }
     }
     if (!ok) __nanosleep(200000);                  // let copies already in flight land before teardown
     __syncwarp();
@@ -125,7 +118,7 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
       if (!ok) break;
       tc_fence_after();
       if (leader) {
-        const uint32_t sa = smem_u32(smem) + stage * G::kStage, sb = sa + G::kABytes;
+        const uint32_t sa = smem_u32(smem) + stage * kStage, sb = sa + kABytes;
 #pragma unroll
         for (int k = 0; k < BK / UMMA_K; ++k)
           umma_bf16<1>(tmem, make_desc(sa + k * (UMMA_K * 2), 16, 1024), make_desc(sb + k * (UMMA_K * 128), 64 * BK * 2, 1024), idesc,
@@ -133,7 +126,7 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
         umma_commit<1>(smem_u32(&ctl->empty[stage]));
       }
       __syncwarp();
-      if (++stage == G::kStages) { stage = 0; phase ^= 1u; }
+      if (++stage == kStages) { stage = 0; phase ^= 1u; }
     }
     if (ok && kbs > 0 && leader) umma_commit<1>(smem_u32(&ctl->acc_full));
     __syncwarp();
@@ -211,16 +204,28 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   cluster_sync_all();                              // nobody leaves while its partial sum may still be read
 }
 
-template <int ROWS>
-cudaError_t launch_rows(const CUtensorMap& ta, const CUtensorMap& tb, const StreamGemm& p, unsigned ctas, cudaStream_t stream) {
-  auto kern = stream_gemm_kernel<ROWS>;
-  constexpr int smem = (int)StreamGeo<ROWS>::kTotal;
-  static const cudaError_t configured = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+}  // namespace
+
+// Few rows and tiles for at most a third of the SMs.  us with 8 rows a group, one CTA a tile and split: 32 tiles (8 x 4096 x 1024) 34
+// and 16, 16 tiles (1 x 4096 x 4096) 34 and 16, 8 tiles (4 x 2048 x 512) 19 and 8; 64 tiles 21 and 25 (8 x 2048 x 2048) or 37 and 31 (32 x
+// 4096 x 512); 128 tiles (8 x 1024 x 4096) 15 and 21.  With 64 rows the partial sums cost more than the split gives (8 x 4096 x 1024: 35
+// and 43).
+bool stream_gemm_pays(int groups, int M, int N, int sms) {
+  return M <= kStreamRows && 3ll * groups * ((N + BN - 1) / BN) <= sms;
+}
+
+// Splits until there are two CTAs for every SM, with at least four K blocks each: what a split adds is the exchange of its
+// partial sum.
+cudaError_t launch_stream_gemm(const CUtensorMap& ta, const CUtensorMap& tb, StreamGemm p, int sms, cudaStream_t stream) {
+  const int tiles = p.groups * ((p.N + BN - 1) / BN), kbs = (p.K + BK - 1) / BK;       // few, see stream_gemm_pays
+  p.split = 1;
+  while (p.split < kMaxSplit && tiles * p.split < 2 * sms && kbs >= 8 * p.split) p.split *= 2;
+  static const cudaError_t configured = cudaFuncSetAttribute(stream_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemTotal);
   if (configured != cudaSuccess) return configured;
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(ctas, 1, 1);
+  cfg.gridDim = dim3((unsigned)(tiles * p.split), 1, 1);
   cfg.blockDim = dim3(kStreamThreads, 1, 1);
-  cfg.dynamicSmemBytes = smem;
+  cfg.dynamicSmemBytes = kSmemTotal;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -229,23 +234,7 @@ cudaError_t launch_rows(const CUtensorMap& ta, const CUtensorMap& tb, const Stre
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  return cudaLaunchKernelEx(&cfg, kern, ta, tb, p);
-}
-
-}  // namespace
-
-int stream_gemm_box(int M) { return M <= 32 ? 32 : 128; }
-
-// Splits until there are two CTAs for every SM, with at least four K blocks each: what a split adds is the exchange of its
-// partial sum.
-cudaError_t launch_stream_gemm(const CUtensorMap& ta, const CUtensorMap& tb, StreamGemm p, int sms, cudaStream_t stream) {
-  const long long tiles = (long long)p.groups * ((p.N + BN - 1) / BN);
-  const int kbs = (p.K + BK - 1) / BK;
-  p.split = 1;
-  while (p.split < kMaxSplit && tiles * p.split < 2ll * sms && kbs >= 8 * p.split) p.split *= 2;
-  if (tiles * p.split > INT_MAX) return cudaErrorInvalidValue;
-  const unsigned ctas = (unsigned)(tiles * p.split);
-  return stream_gemm_box(p.M) == 32 ? launch_rows<32>(ta, tb, p, ctas, stream) : launch_rows<128>(ta, tb, p, ctas, stream);
+  return cudaLaunchKernelEx(&cfg, stream_gemm_kernel, ta, tb, p);
 }
 
 }  // namespace planmoe

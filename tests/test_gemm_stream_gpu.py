@@ -8,10 +8,10 @@ from test_gemm_local_gpu import _close, _rand
 
 pytestmark = pytest.mark.gpu
 
-# rows on both sides of the two box sizes; contractions of one K block, of fewer blocks than splits, ragged, of many rounds of the
-# ring; ragged columns; one tile and more tiles than the SMs hold
-SHAPES = [(1, 1, 8, 8), (2, 8, 64, 256), (3, 31, 520, 264), (8, 32, 1024, 4096), (8, 8, 4096, 1024), (4, 33, 72, 1032), (5, 100, 2056, 520),
-          (2, 128, 4096, 256), (64, 16, 256, 2048)]
+# contractions of one K block, of fewer blocks than splits, ragged, of many rounds of the ring; ragged columns; the most rows and
+# tiles that are split, and one more of either
+SHAPES = [(1, 1, 8, 8), (2, 8, 64, 256), (3, 31, 520, 264), (4, 32, 1024, 3000), (8, 8, 4096, 1024), (4, 32, 72, 1032), (1, 32, 2056, 12288),
+          (4, 33, 72, 1032), (1, 16, 256, 12800), (64, 16, 256, 2048)]
 
 
 @pytest.mark.parametrize('G,M,K,N', SHAPES)
@@ -33,7 +33,7 @@ def test_rows(G, M, K, N, act):
     _close(torch.where(away, aux.double(), deriv), deriv, 4 * K)
 
 
-@pytest.mark.parametrize('M', [7, 32, 96])
+@pytest.mark.parametrize('M', [7, 32])
 def test_groups_without_a_token_read_no_weights(M):
     G, K, N = 6, 1032, 776
     used = torch.tensor([0, M, 1, 0, M // 2, 0])
