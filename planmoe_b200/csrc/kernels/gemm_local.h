@@ -34,7 +34,7 @@ cudaError_t launch_local_gemm(int epilogue, bool a_mn, bool b_mn, const CUtensor
 constexpr int kStreamRows = 32;
 struct StreamGemm {
   int groups, M, N, K;
-  int activation, split;         // split: CTAs that share a tile's contraction (set by the launch)
+  int activation;
   const __nv_bfloat16* bias;     // [groups][N], on 16 bytes, or null
   __nv_bfloat16* D; long long d_row_stride, d_group_stride;
   __nv_bfloat16* aux; long long aux_row_stride, aux_group_stride;
@@ -44,6 +44,6 @@ struct StreamGemm {
 };
 bool stream_gemm_pays(int groups, int M, int N, int sms);
 // `ta`: boxes of kStreamRows rows, `tb`: of 64
-cudaError_t launch_stream_gemm(const CUtensorMap& ta, const CUtensorMap& tb, StreamGemm p, int sms, cudaStream_t stream);
+cudaError_t launch_stream_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const StreamGemm& p, cudaStream_t stream);
 
 }  // namespace planmoe

@@ -1,4 +1,4 @@
-"""The grouped GEMM for a handful of rows: splits of the contraction, edges of its tiles, groups without a token."""
+"""The grouped GEMM for a handful of rows: edges of its tiles, groups without a token."""
 
 import pytest
 import torch
@@ -8,8 +8,8 @@ from test_gemm_local_gpu import _close, _rand
 
 pytestmark = pytest.mark.gpu
 
-# contractions of one K block, of fewer blocks than splits, ragged, of many rounds of the ring; ragged columns; the most rows and
-# tiles that are split, and one more of either
+# contractions of one K block, of fewer blocks than the ring has stages, ragged, of many rounds of the ring; ragged columns; the most
+# rows and tiles that it takes, and one more of either
 SHAPES = [(1, 1, 8, 8), (2, 8, 64, 256), (3, 31, 520, 264), (4, 32, 1024, 3000), (8, 8, 4096, 1024), (4, 32, 72, 1032), (1, 32, 2056, 12288),
           (4, 33, 72, 1032), (1, 16, 256, 12800), (64, 16, 256, 2048)]
 
@@ -44,3 +44,17 @@ def test_groups_without_a_token_read_no_weights(M):
     check_status()
     want = a.double() @ b.double().nan_to_num() + bias.double().unsqueeze(1)
     _close(got, want, K)
+
+
+@pytest.mark.parametrize('G,M,K,N', SHAPES)
+@pytest.mark.parametrize('act', ['gelu', 'identity'])
+def test_bits_of_the_kernel_for_more_rows(G, M, K, N, act):
+    """Every output adds its products up in the same order, so that a small batch and a large one agree."""
+    a, b, bias = _rand(G, M, K, seed=1), _rand(G, K, N, seed=2), _rand(G, N, seed=3)
+
+    def run(**how):
+        aux = torch.full((G, M, N), float('nan'), dtype=torch.bfloat16, device='cuda')
+        return grouped_gemm(a, False, b, True, EPI_BIAS_ACT, ACT_CODES[act], bias=bias, aux=aux, **how), aux
+    got, want = run(), run(cta_group=1)
+    check_status()
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
