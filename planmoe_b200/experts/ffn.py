@@ -26,27 +26,35 @@ _KNOWN_ACTS = {
 }
 
 
+_KNOWN_MODULES = {torch.nn.ReLU: 'relu', torch.nn.GELU: 'gelu', torch.nn.SiLU: 'silu', torch.nn.Identity: 'identity'}
+
+
+def _identity(x):
+    return x
+
+
+_ACT_FNS = {'relu': F.relu, 'gelu': F.gelu, 'silu': F.silu, 'identity': _identity}
+_KNOWN_ACTS[_identity] = 'identity'
+
+
 def activation_name(fn):
-    """Name of a fusable activation ('relu' | 'gelu' | 'silu' | 'identity') or None."""
+    """Name of a fusable activation ('relu' | 'gelu' | 'silu' | 'identity') or None.  A module counts as what its class computes:
+    one with a forward of its own, from a subclass or put in place, is no known one."""
     if fn is None:
         return 'relu'
     if isinstance(fn, str):
-        return fn if fn in ('relu', 'gelu', 'silu', 'identity') else None
-    if isinstance(fn, torch.nn.ReLU):
-        return 'relu'
-    if isinstance(fn, torch.nn.GELU) and getattr(fn, 'approximate', 'none') == 'none':
-        return 'gelu'
-    if isinstance(fn, torch.nn.SiLU):
-        return 'silu'
-    if isinstance(fn, torch.nn.Identity):
-        return 'identity'
+        return fn if fn in _ACT_FNS else None
+    if isinstance(fn, torch.nn.Module):
+        if 'forward' in fn.__dict__ or type(fn).__call__ is not torch.nn.Module.__call__:
+            return None
+        for cls, name in _KNOWN_MODULES.items():
+            if isinstance(fn, cls) and type(fn).forward is cls.forward:
+                return name if getattr(fn, 'approximate', 'none') == 'none' else None
+        return None
     try:
         return _KNOWN_ACTS.get(fn)
     except TypeError:
         return None
-
-
-_ACT_FNS = {'relu': F.relu, 'gelu': F.gelu, 'silu': F.silu, 'identity': lambda x: x}
 
 
 class FusedExpertsNetwork(torch.nn.Module):
@@ -68,6 +76,13 @@ class FusedExpertsNetwork(torch.nn.Module):
                 assert self.act_name is not None, "Unknown activation name: %s" % activation_fn
                 activation_fn = _ACT_FNS[self.act_name]
             self.activation_fn = activation_fn
+
+    @property
+    def fused_act(self):
+        """Name of the activation that a kernel may compute in the place of ``activation_fn`` as it is now, or None: the attribute
+        can be replaced at any time, ``act_name`` says what the constructor was given."""
+        fn = self.activation_fn
+        return None if self.act_name is None or fn is None or isinstance(fn, str) else activation_name(fn)
 
     def update(self, ctx):
         """Allocate the batched parameters for ``ctx`` (the owning MoE layer)."""
@@ -107,7 +122,7 @@ class FusedExpertsNetwork(torch.nn.Module):
 
 
     def fused_ok(self, x):
-        return (x.is_cuda and x.dtype == torch.bfloat16 and self.act_name is not None
+        return (x.is_cuda and x.dtype == torch.bfloat16 and self.fused_act is not None
                 and self.batched_fc1_w.dtype == torch.bfloat16 and self.sharded_count == 1
                 and x.size(-1) % 64 == 0 and self.batched_fc1_w.size(2) % 64 == 0
                 and self.batched_fc2_w.size(2) % 64 == 0
@@ -120,7 +135,7 @@ class FusedExpertsNetwork(torch.nn.Module):
         b1, b2 = self.batched_fc1_bias, self.batched_fc2_bias
         if self.fused_ok(x):
             from ..ops import gemm
-            return gemm.expert_ffn(x, w1, b1, w2, b2, self.act_name)
+            return gemm.expert_ffn(x, w1, b1, w2, b2, self.fused_act)
 
         zero_group = getattr(ctx, 'ffn_zero_group', None) if ctx is not None else None
         if zero_group is not None and not ctx.use_model_parallel:

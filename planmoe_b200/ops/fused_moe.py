@@ -574,7 +574,7 @@ def _linear_gate(layer, gctx, x):
 def _local_layer(layer, st, x, gctx, top_k, capacity, align):
     ex, w = layer.experts, gctx.wg.weight
     m = dict(K=top_k, capacity=capacity, round_up=lambda peak: _capacity_step(peak, align), normalize=layer.normalize_gate,
-             bf16_logits=not gctx.fp32_gate, prio=layer.batch_prioritized_routing, act=ACT_CODES[ex.act_name],
+             bf16_logits=not gctx.fp32_gate, prio=layer.batch_prioritized_routing, act=ACT_CODES[ex.fused_act],
              postscore=layer.is_postscore, int8=layer.compress_name == 'int8', budget_ms=st.tr.budget_ms,
              status=st.tr.status)
     args = (native.aligned(x), w, ex.batched_fc1_w, ex.batched_fc1_bias, ex.batched_fc2_w, ex.batched_fc2_bias)
@@ -709,11 +709,11 @@ def forward(layer, x, gctx, top_k, capacity_factor, degree):
     args = (gates, ex.batched_fc1_w, ex.batched_fc1_bias, ex.batched_fc2_w, ex.batched_fc2_bias)
     if local:
         y = _local_experts(x, *args, dict(idx=idx, loc=loc, slot_map=slot_map, used=used, C=capacity,
-                                          act=ACT_CODES[ex.act_name], postscore=layer.is_postscore, int8=q8,
+                                          act=ACT_CODES[ex.fused_act], postscore=layer.is_postscore, int8=q8,
                                           budget_ms=st.tr.budget_ms, status=st.tr.status))
     else:
         meta = dict(state=st, idx=idx, loc=loc, slot_map=slot_map, E=E, C=capacity, degree=degree, K=top_k,
-                    act=ACT_CODES[ex.act_name], postscore=layer.is_postscore, q8=q8)
+                    act=ACT_CODES[ex.fused_act], postscore=layer.is_postscore, q8=q8)
         y = _FusedExperts.apply(native.aligned(x), *args, meta)
     _note_stats(layer, st, q8, idx, loc, E, capacity, degree, x, local)
     return y, l_aux.to(logits.dtype)

@@ -41,10 +41,14 @@ class _Layer32(torch.autograd.Function):
         return (*native.lib().layer32_backward(dy, dloss, x, wg, w1, w2, saved, *ctx.args, list(need)), *(None,) * 5)
 
 
+def _no_hooks(fn):
+    return not isinstance(fn, torch.nn.Module) or not (fn._forward_hooks or fn._forward_pre_hooks or fn._backward_hooks or fn._backward_pre_hooks)
+
+
 def takes(layer, gctx, x, top_k, cf, comm_name, reserve_shape):
     """Whether a call of the generic path is one that the node knows: one rank, fp32 throughout, a plain linear gate, FFN
-    experts without hooks, GShard loss, token order, gates applied after the experts, a positive capacity factor; products in full
-    fp32 and outside autocast; ordinary reverse-mode autograd."""
+    experts with a known activation, no hooks on any of them, GShard loss, token order, gates applied after the experts, a
+    positive capacity factor; products in full fp32 and outside autocast; ordinary reverse-mode autograd."""
     from ..experts.ffn import FusedExpertsNetwork
     from ..gates.top import LinearTopKGate
     from . import fused_moe
@@ -57,7 +61,8 @@ def takes(layer, gctx, x, top_k, cf, comm_name, reserve_shape):
             or layer.batch_prioritized_routing or layer.collect_stats or len(reserve_shape) != 1 or stage_timer.enabled()):
         return False
     if (not fused_moe._unhooked(ex, FusedExpertsNetwork) or not fused_moe._unhooked(gctx, LinearTopKGate)
-            or not fused_moe._unhooked(gctx.wg, torch.nn.Linear) or ex.act_name is None or ex.skip_expert
+            or not fused_moe._unhooked(gctx.wg, torch.nn.Linear) or ex.skip_expert or ex.fused_act is None
+            or not _no_hooks(ex.activation_fn)
             or 'expert_local' in layer.__dict__ or nnm._global_forward_hooks or nnm._global_forward_pre_hooks
             or nnm._global_backward_hooks or nnm._global_backward_pre_hooks):
         return False
@@ -93,7 +98,7 @@ def forward(layer, x, gctx, top_k, cf, degree):
     capacity += -capacity % (4 * degree)
     ex, normalize = layer.experts, bool(layer.normalize_gate)
     args = (native.aligned(x), gctx.wg.weight, *(getattr(ex, n) for n in _EXPERT_PARAMS))
-    more = (top_k, capacity, normalize, ACT_CODES[ex.act_name])
+    more = (top_k, capacity, normalize, ACT_CODES[ex.fused_act])
     if torch.is_grad_enabled() and any(t.requires_grad for t in args):
         y, loss = _Layer32.apply(*args, _as_operations(ex.activation_fn, top_k, cf, degree, normalize), *more)
     else:
