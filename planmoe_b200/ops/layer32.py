@@ -74,7 +74,8 @@ def takes(layer, gctx, x, top_k, cf, comm_name, reserve_shape):
             and 1 <= min(int(top_k), E) <= 4 and x.size(0) * top_k < 2 ** 31 and ps[2].size(2) % 4 == 0
             and ps[3].size(1) == ps[2].size(2) and wg.size(1) == x.size(1) == ps[0].size(1)
             and all(p.dtype == torch.float32 and p.device == x.device for p in (wg, *ps))
-            and not torch.is_autocast_enabled('cuda') and not torch.backends.cuda.matmul.allow_tf32
+            # the legacy flag, allow_tf32, cannot be read once TF32 was chosen by this switch, which follows the legacy ones
+            and not torch.is_autocast_enabled('cuda') and torch.backends.cuda.matmul.fp32_precision in ('none', 'ieee')
             and plain_autograd(x, wg, *ps))
 
 

@@ -103,3 +103,32 @@ def test_other_calls_stay_where_they_were(monkeypatch, what):
         with torch.autocast('cuda', enabled=what == 'autocast'):
             layer(x)
     assert took and not any(took)
+
+
+@pytest.mark.parametrize('where', ['matmul', 'all'])
+@pytest.mark.parametrize('precision', ['tf32', 'ieee'])
+def test_fp32_precision_switches(monkeypatch, where, precision):
+    """The present switches (the legacy flag cannot be read once one of them is set to TF32): full precision takes the node."""
+    holder = torch.backends.cuda.matmul if where == 'matmul' else torch.backends
+    layer = _layer(4, 2, 1.0, 'gelu', 64, 32)
+    x = torch.randn(40, 64, device='cuda')
+    took, before = _watch(monkeypatch), [(h, h.fp32_precision) for h in (torch.backends, torch.backends.cuda.matmul)]
+
+    def run():
+        layer.zero_grad(set_to_none=True)
+        xin = x.clone().requires_grad_()
+        y = layer(xin)
+        (y.square().sum() + y.l_aux).backward()
+        return [y.detach(), y.l_aux.detach(), xin.grad] + [p.grad for p in layer.parameters()]
+    try:
+        torch.backends.cuda.matmul.fp32_precision = 'none'       # products follow the switch for all operations
+        holder.fp32_precision = precision
+        got = run()
+        assert took == [precision == 'ieee']
+        monkeypatch.setattr(layer32, 'takes', lambda *a: False)
+        want = run()
+    finally:
+        for h, value in before:
+            h.fp32_precision = value
+    for a, b in zip(got, want):                          # sums of up to 64 terms in another order; TF32: the same operations
+        torch.testing.assert_close(a, b, rtol=1e-5, atol=2e-5)
