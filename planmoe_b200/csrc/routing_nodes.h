@@ -13,12 +13,44 @@ Tensor vector_rows(const Tensor& t) {
   return reinterpret_cast<uintptr_t>(c.data_ptr()) % 16 == 0 ? c : c.clone();
 }
 
+// Encode, decode and the gates' gradient as differentiable operations, for a gradient of a gradient.  Sums are fp32 and gates are
+// rounded to the data's type, as in the kernels.
+struct PickOps {
+  const Tensor &idx, &loc;
+  int64_t E, C;
+  variable_list gates;                             // one a pick, or none at all
+
+  Tensor kept(int64_t k) const { return ((loc[k] < C).logical_and_(loc[k] >= 0).logical_and_(idx[k] >= 0)).unsqueeze(1); }
+  Tensor slot(int64_t k) const { return (idx[k].to(at::kLong) * C + loc[k].to(at::kLong)).clamp(0, E * C - 1); }
+  Tensor weighted(const Tensor& rows, int64_t k, at::ScalarType dtype) const {
+    const Tensor r = at::where(kept(k), rows.to(at::kFloat), at::zeros({}, rows.options().dtype(at::kFloat)));
+    return gates.empty() ? r : r * gates[k].to(dtype).to(at::kFloat).unsqueeze(1);
+  }
+  Tensor scatter(const Tensor& x) const {
+    Tensor out = at::zeros({E * C, x.size(1)}, x.options().dtype(at::kFloat));
+    for (int64_t k = 0; k < idx.size(0); ++k) out = out.index_add(0, slot(k), weighted(x, k, x.scalar_type()));
+    return out.to(x.scalar_type());
+  }
+  Tensor gather(const Tensor& disp) const {
+    Tensor out;
+    for (int64_t k = 0; k < idx.size(0); ++k) {
+      const Tensor r = weighted(disp.index_select(0, slot(k)), k, disp.scalar_type());
+      out = out.defined() ? out + r : r;
+    }
+    return out.to(disp.scalar_type());
+  }
+  Tensor gate_grad(const Tensor& disp, const Tensor& dy, int64_t k) const {
+    return PickOps{idx, loc, E, C, {}}.weighted(disp.index_select(0, slot(k)), k, at::kFloat).mul(dy.to(at::kFloat)).sum(1);
+  }
+};
+
 // Tokens [S, M] -> slots [E * C, M], without gates.
 struct ScatterNode : torch::autograd::Function<ScatterNode> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& idx, const Tensor& loc, const Tensor& slot_map,
                         int64_t E, int64_t C) {
     ctx->set_materialize_grads(false);
     ctx->save_for_backward({idx, loc});
+    ctx->saved_data["E"] = E;
     ctx->saved_data["C"] = C;
     return dispatch_scatter_op(vector_rows(x), slot_map, c10::nullopt, idx.size(0), E * C, false);
   }
@@ -26,14 +58,22 @@ struct ScatterNode : torch::autograd::Function<ScatterNode> {
     variable_list out(6);
     if (!grads[0].defined()) return out;
     const variable_list saved = ctx->get_saved_variables();
-    out[0] = dispatch_gather_op(vector_rows(grads[0]), saved[0], saved[1], c10::nullopt, ctx->saved_data["C"].toInt(), false);
+    const int64_t C = ctx->saved_data["C"].toInt();
+    if (at::GradMode::is_enabled())                // create_graph
+      out[0] = PickOps{saved[0], saved[1], ctx->saved_data["E"].toInt(), C, {}}.gather(grads[0]);
+    else
+      out[0] = dispatch_gather_op(vector_rows(grads[0]), saved[0], saved[1], c10::nullopt, C, false);
     return out;
   }
 };
 
+// In-place changes of a tensor so far; those of inference tensors are not counted.
+int64_t version_of(const Tensor& t) { return t.is_inference() ? 0 : (int64_t)t._version(); }
+
 // Slots [E * C, M] -> tokens [S, M], weighted by fp32 `rows` [K, S], which the kernels round to the data's type; the gradient
 // of the gates goes to the picks' own tensors g0 .. g3, the first K of which are there.  No `slot_map`: made when the
-// backward needs it.
+// backward needs it.  The gates are kept beside the saved tensors: a gradient uses `rows`, whatever has become of them since, and
+// only a gradient of a gradient, which runs through their history, wants them as they were.
 using OptTensor = c10::optional<Tensor>;
 struct GatherPicksNode : torch::autograd::Function<GatherPicksNode> {
   static constexpr int kGates = 4, kInputs = 1 + kGates + 6;
@@ -43,6 +83,12 @@ struct GatherPicksNode : torch::autograd::Function<GatherPicksNode> {
     ctx->save_for_backward({disp, idx, loc, rows, slot_map.value_or(Tensor())});
     ctx->saved_data["E"] = E;
     ctx->saved_data["C"] = C;
+    std::vector<Tensor> gates;
+    std::vector<int64_t> made;
+    for (const OptTensor* g : {&g0, &g1, &g2, &g3})
+      if (g->has_value()) { gates.push_back(**g); made.push_back(version_of(**g)); }
+    ctx->saved_data["gates"] = std::move(gates);
+    ctx->saved_data["made"] = std::move(made);
     return dispatch_gather_op(vector_rows(disp), idx, loc, rows, C, disp.scalar_type() != at::kFloat);
   }
   static variable_list backward(AutogradContext* ctx, const variable_list& grads) {
@@ -52,6 +98,17 @@ struct GatherPicksNode : torch::autograd::Function<GatherPicksNode> {
     const variable_list saved = ctx->get_saved_variables();
     const Tensor &disp = saved[0], &idx = saved[1], &loc = saved[2], &rows = saved[3];
     const int64_t K = idx.size(0);
+    if (at::GradMode::is_enabled()) {              // create_graph
+      const std::vector<Tensor> gates = ctx->saved_data["gates"].toTensorVector();
+      const std::vector<int64_t> made = ctx->saved_data["made"].toIntVector();
+      for (int64_t k = 0; k < K; ++k)
+        TORCH_CHECK(version_of(gates[k]) == made[k], "gates needed for the gradient of a gradient have been modified by an inplace operation");
+      const PickOps ops{idx, loc, E, C, gates};
+      out[0] = ops.scatter(grads[0]);
+      for (int64_t k = 0; k < K; ++k)
+        if (ctx->needs_input_grad(1 + k)) out[1 + k] = ops.gate_grad(disp, grads[0], k);
+      return out;
+    }
     const Tensor dy = vector_rows(grads[0]);
     const Tensor map = saved[4].defined() ? saved[4] : build_slot_map_op(idx, loc, E, C);
     out[0] = dispatch_scatter_op(dy, map, rows, K, E * C, disp.scalar_type() != at::kFloat);

@@ -85,11 +85,11 @@ def gather_torch(disp, plan, gates=None):
 
 
 def gate_grad_torch(disp, dy, plan):
-    res = []
+    res, acc = [], torch.promote_types(disp.dtype, torch.float32)
     for k in range(plan.K):
         valid = (plan.loc[k] < plan.C) & (plan.idx[k] >= 0)
         slot = (plan.idx[k].long() * plan.C + plan.loc[k].long()).clamp_(0, plan.E * plan.C - 1)
-        res.append((disp[slot].float() * dy.float()).sum(-1) * valid)
+        res.append((disp[slot].to(acc) * dy.to(acc)).sum(-1) * valid)
     return torch.stack(res)
 
 
@@ -147,6 +147,21 @@ def _gates_for(x, gates):
     return gates.detach().to(torch.float32 if x.is_cuda else x.dtype).contiguous()
 
 
+class _Live:
+    """Gates that a node was given, for a gradient of its gradient: they go into that as they are, with their history, where the
+    gradient itself uses a copy of their values."""
+
+    def __init__(self, gates):
+        self.made = [(g, None if g.is_inference() else g._version) for g in gates]
+
+    def get(self):
+        if any(v is not None and g._version != v for g, v in self.made):
+            raise RuntimeError("gates needed for the gradient of a gradient have been modified by an inplace operation")
+        return [g for g, _ in self.made]
+
+
+# Under create_graph the functions below answer with differentiable operations: encode and decode are each other's adjoint.
+
 class _Scatter(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, gates, plan):
@@ -154,17 +169,20 @@ class _Scatter(torch.autograd.Function):
         g = _gates_for(x, gates)
         ctx.save_for_backward(x if gates is not None else None, g)
         ctx.gdtype = gates.dtype if gates is not None else None
+        ctx.live = _Live([gates]) if gates is not None else None
         return _scatter(x, plan, g)
 
     @staticmethod
     def backward(ctx, ddisp):
         x, g = ctx.saved_tensors
         plan = ctx.plan
+        want_gates = g is not None and ctx.needs_input_grad[1]
+        if torch.is_grad_enabled():
+            return (gather(ddisp, plan, ctx.live.get()[0] if g is not None else None),
+                    gate_grad_torch(ddisp, x, plan).to(ctx.gdtype) if want_gates else None, None)
         ddisp = _rows(ddisp)
         dx = _gather(ddisp, plan, g)
-        dg = None
-        if g is not None and ctx.needs_input_grad[1]:
-            dg = _gate_grad(ddisp, x, plan).to(ctx.gdtype)
+        dg = _gate_grad(ddisp, x, plan).to(ctx.gdtype) if want_gates else None
         return dx, dg, None
 
 
@@ -175,17 +193,20 @@ class _Gather(torch.autograd.Function):
         g = _gates_for(disp, gates)
         ctx.save_for_backward(disp if gates is not None else None, g)
         ctx.gdtype = gates.dtype if gates is not None else None
+        ctx.live = _Live([gates]) if gates is not None else None
         return _gather(disp, plan, g)
 
     @staticmethod
     def backward(ctx, dy):
         disp, g = ctx.saved_tensors
         plan = ctx.plan
+        want_gates = g is not None and ctx.needs_input_grad[1]
+        if torch.is_grad_enabled():
+            return (scatter(dy, plan, ctx.live.get()[0] if g is not None else None),
+                    gate_grad_torch(disp, dy, plan).to(ctx.gdtype) if want_gates else None, None)
         dy = _rows(dy)
         ddisp = _scatter(dy, plan, g)
-        dg = None
-        if g is not None and ctx.needs_input_grad[1]:
-            dg = _gate_grad(disp, dy, plan).to(ctx.gdtype)
+        dg = _gate_grad(disp, dy, plan).to(ctx.gdtype) if want_gates else None
         return ddisp, dg, None
 
 
@@ -198,6 +219,7 @@ class _ScatterPicks(torch.autograd.Function):
         ctx.plan, ctx.round = plan, x.dtype != torch.float32
         ctx.set_materialize_grads(False)
         ctx.save_for_backward(x, rows)
+        ctx.live = _Live(gates)
         return native.lib().dispatch_scatter(_rows(x), plan.slot_map, rows, plan.K, plan.E * plan.C, ctx.round)
 
     @staticmethod
@@ -206,11 +228,13 @@ class _ScatterPicks(torch.autograd.Function):
         plan = ctx.plan
         if ddisp is None:
             return (None,) * (3 + plan.K)
+        want_gates = any(ctx.needs_input_grad[3:])
+        if torch.is_grad_enabled():
+            dg = gate_grad_torch(ddisp, x, plan).unbind(0) if want_gates else [None] * plan.K
+            return (gather(ddisp, plan, torch.stack(ctx.live.get()).to(x.dtype)), None, None, *dg)
         ddisp = _rows(ddisp)
         dx = native.lib().dispatch_gather(ddisp, plan.idx, plan.loc, rows, plan.C, ctx.round)
-        dg = [None] * plan.K
-        if any(ctx.needs_input_grad[3:]):
-            dg = _gate_grad(ddisp, x, plan).unbind(0)
+        dg = _gate_grad(ddisp, x, plan).unbind(0) if want_gates else [None] * plan.K
         return (dx, None, None, *dg)
 
 
@@ -222,6 +246,7 @@ class _GatherPicks(torch.autograd.Function):
         ctx.plan, ctx.round = plan, disp.dtype != torch.float32
         ctx.set_materialize_grads(False)
         ctx.save_for_backward(disp, rows)
+        ctx.live = _Live(gates)
         return native.lib().dispatch_gather(_rows(disp), plan.idx, plan.loc, rows, plan.C, ctx.round)
 
     @staticmethod
@@ -230,11 +255,13 @@ class _GatherPicks(torch.autograd.Function):
         plan = ctx.plan
         if dy is None:
             return (None,) * (3 + plan.K)
+        want_gates = any(ctx.needs_input_grad[3:])
+        if torch.is_grad_enabled():
+            dg = gate_grad_torch(disp, dy, plan).unbind(0) if want_gates else [None] * plan.K
+            return (scatter(dy, plan, torch.stack(ctx.live.get()).to(disp.dtype)), None, None, *dg)
         dy = _rows(dy)
         ddisp = native.lib().dispatch_scatter(dy, plan.slot_map, rows, plan.K, plan.E * plan.C, ctx.round)
-        dg = [None] * plan.K
-        if any(ctx.needs_input_grad[3:]):
-            dg = _gate_grad(disp, dy, plan).unbind(0)
+        dg = _gate_grad(disp, dy, plan).unbind(0) if want_gates else [None] * plan.K
         return (ddisp, None, None, *dg)
 
 
