@@ -9,6 +9,7 @@
 
 #include <climits>
 #include <torch/extension.h>
+#include <torch/csrc/autograd/functions/basic_ops.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAStream.h>
 #include <c10/cuda/CUDAGuard.h>

@@ -3,6 +3,9 @@
 // forward-mode and tracing.  Included by bindings.cpp behind local_moe_forward_op and local_moe_backward_op.
 #pragma once
 
+static const char* const kSecondOrder =
+    "the gradient was computed by kernels and cannot be differentiated twice; PLANMOE_GEMM=cublas makes a layer of operations that can";
+
 // What a pass is done with; capacity, idx and loc are set by the forward.
 struct LayerArgs {
   int64_t K, capacity;
@@ -20,6 +23,23 @@ struct StatusHolder : torch::CustomClassHolder {
   explicit StatusHolder(std::shared_ptr<StatusWord> w) : word(std::move(w)) {}
 };
 
+// Results of a backward under create_graph (ops/native.py, first_order): the same values, which raise when they are
+// differentiated by what they depend on.
+static variable_list once(variable_list found, const std::vector<variable_list>& depends) {
+  const size_t n = found.size();
+  bool any = false;
+  for (Tensor& t : found) {
+    any = any || t.defined();
+    if (t.defined()) t = t.detach();
+  }
+  for (const variable_list& list : depends)
+    for (const Tensor& t : list)
+      if (t.defined() && t.requires_grad()) found.push_back(t);
+  if (any && found.size() > n) found = torch::autograd::DelayedError(kSecondOrder, (int64_t)found.size())(std::move(found));
+  found.resize(n);
+  return found;
+}
+
 struct LayerNode : torch::autograd::Function<LayerNode> {
   static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& wg, const Tensor& w1, const Tensor& b1,
                                const Tensor& w2, const Tensor& b2, LayerArgs* a) {
@@ -29,6 +49,7 @@ struct LayerNode : torch::autograd::Function<LayerNode> {
                                                     (int64_t)a->status->device_ptr(), true, py::none());
     a->capacity = capacity; a->idx = t[6]; a->loc = t[14];
     ctx->save_for_backward({x, wg, w1, w2, t[2], t[3], t[4], t[5], t[6], t[7], t[8], t[9], t[10], t[11], t[12], t[13]});
+    ctx->saved_data["also"] = std::vector<Tensor>{b1, b2};
     ctx->saved_data["act"] = a->act;
     ctx->saved_data["flags"] = (int64_t)(a->postscore | a->int8 << 1 | a->normalize << 2 | a->bf16_logits << 3);
     ctx->saved_data["budget_ms"] = a->budget_ms;
@@ -50,7 +71,7 @@ struct LayerNode : torch::autograd::Function<LayerNode> {
                                                         s[2], s[3], s[4], s[5], s[11], s[12], s[13], s[14], opt(s[15]),
                                                         (flags & 4) != 0, (flags & 8) != 0, need, py::object());
     for (int i = 0; i < 6; ++i) out[i] = d[i];
-    return out;
+    return at::GradMode::is_enabled() ? once(std::move(out), {grads, s, ctx->saved_data["also"].toTensorVector()}) : out;
   }
 };
 

@@ -280,6 +280,7 @@ class _FusedGate(torch.autograd.Function):
     def forward(ctx, logits, top_k, capacity, normalize):
         lib = native.lib()
         ctx.set_materialize_grads(False)
+        ctx.also = (logits,) if not logits.is_contiguous() else ()
         logits = logits.contiguous()
         idx, loc, gates, slot_map, top1, l_aux, used = lib.gate_forward_used(logits, top_k, capacity, normalize)
         ctx.save_for_backward(logits, idx, top1)
@@ -288,6 +289,7 @@ class _FusedGate(torch.autograd.Function):
         return gates, l_aux.view(()), idx, loc, slot_map, used
 
     @staticmethod
+    @native.first_order
     def backward(ctx, dgates, dl_aux, *_):
         logits, idx, top1 = ctx.saved_tensors
         lib = native.lib()
@@ -372,11 +374,13 @@ class _FusedExperts(torch.autograd.Function):
 
         ctx.meta, ctx.bs = meta, bs
         ctx.save_for_backward(x, gates_f, w1, w2, dact, h)
+        ctx.also = (gates, b1, b2)
         ctx.dims = (W, rank, E, C, d, K, E_l, Cc, S, M, H, O, R)
         ctx.lease = _Lease(bs)
         return out
 
     @staticmethod
+    @native.first_order
     def backward(ctx, dout):
         lib = native.lib()
         meta, bs = ctx.meta, ctx.bs
@@ -483,9 +487,11 @@ class _LocalExperts(torch.autograd.Function):
         y, xs, dact, h, ys, scales = _local_forward(x, gates, w1, b1, w2, b2, meta, True)
         ctx.save_for_backward(x, gates, w1, w2, xs, dact, h, ys, scales, meta['idx'], meta['loc'], meta['slot_map'], meta['used'])
         ctx.meta = {k: meta[k] for k in ('C', 'act', 'postscore', 'int8', 'budget_ms', 'status')}
+        ctx.also = (b1, b2)
         return y
 
     @staticmethod
+    @native.first_order
     def backward(ctx, dy):
         x, gates, w1, w2, xs, dact, h, ys, scales, idx, loc, slot_map, used = ctx.saved_tensors
         route = _local_route(gates, dict(ctx.meta, idx=idx, loc=loc, slot_map=slot_map, used=used))
@@ -527,10 +533,12 @@ class _LocalLayer(torch.autograd.Function):
         (y, l_aux, *saved, loc), m['capacity'] = _local_layer_forward(x, wg, w1, b1, w2, b2, m, True)
         m['routing'] = saved[4], loc
         ctx.save_for_backward(x, wg, w1, w2, *saved)
+        ctx.also = (b1, b2)
         ctx.m = {k: m[k] for k in ('act', 'postscore', 'int8', 'normalize', 'bf16_logits', 'budget_ms', 'status')}
         return y, l_aux
 
     @staticmethod
+    @native.first_order
     def backward(ctx, dy, dl_aux):
         x, wg, w1, w2, logits, top1, slot_map, used, idx, loc, gates, xs, dact, h, ys, scales = ctx.saved_tensors
         m = ctx.m

@@ -72,6 +72,7 @@ def grouped_gemm(A, a_mn, B, b_mn, epilogue=EPI_STORE, activation=0, bias=None, 
 class _ExpertFFN(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w1, b1, w2, b2, act):
+        ctx.also = (b1, b2) if x.is_contiguous() else (x, b1, b2)
         x = x.contiguous()
         G, R, _ = x.shape
         H = w1.size(2)
@@ -83,6 +84,7 @@ class _ExpertFFN(torch.autograd.Function):
         return y
 
     @staticmethod
+    @native.first_order
     def backward(ctx, dy):
         x, w1, w2, pre, h = ctx.saved_tensors
         dy = dy.contiguous()

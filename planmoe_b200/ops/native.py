@@ -9,6 +9,7 @@ GPU code paths call ``lib()`` so that a missing extension is a loud error, never
 fallback to eager PyTorch.
 """
 
+import functools
 import importlib
 import os
 
@@ -52,6 +53,32 @@ def aligned(t):
     contiguous view may start anywhere in its storage."""
     t = t.contiguous()
     return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
+def first_order(backward):
+    """For the backward of an autograd function that runs kernels and has no gradient of its own.  Under create_graph its results
+    are the same and raise when they are differentiated, by whatever they depend on: the incoming gradients, the saved inputs and
+    those that the forward names in ``ctx.also``.  (``torch.autograd.function.once_differentiable`` looks at the incoming
+    gradients alone, and an engine that is asked for certain inputs does not come by its error.)"""
+    @functools.wraps(backward)
+    def run(ctx, *grads):
+        import torch
+        if not torch.is_grad_enabled():
+            return backward(ctx, *grads)
+        with torch.no_grad():
+            found = backward(ctx, *grads)
+        found = found if isinstance(found, tuple) else (found,)
+        values = [t.detach() for t in found if t is not None]
+        on = [t for t in (*grads, *ctx.saved_tensors, *getattr(ctx, 'also', ())) if t is not None and t.requires_grad]
+        if not values or not on:
+            return found
+        made = iter(torch._C._functions.DelayedError(SECOND_ORDER, len(values) + len(on))(*values, *on))
+        return tuple(None if t is None else next(made) for t in found)
+    return run
+
+
+SECOND_ORDER = ("the gradient was computed by kernels and cannot be differentiated twice; PLANMOE_GEMM=cublas makes a layer of "
+                "operations that can")
 
 
 def force_python_fallback():

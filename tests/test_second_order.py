@@ -8,6 +8,7 @@ import torch.nn.functional as F
 from planmoe_b200 import moe
 from planmoe_b200.impls.fast_dispatch import extract_critical, fast_decode, fast_encode
 from planmoe_b200.ops import dispatch as D
+from planmoe_b200.ops import gemm
 
 S, M, E, C = 9, 4, 3, 4
 
@@ -142,3 +143,39 @@ def test_fp32_layer_twice(monkeypatch, fused):
     got = twice(ours, [x.clone().requires_grad_()] + params)
     want = twice(plain, [t.detach().double().requires_grad_() for t in [x] + params])
     _close(got, want, 1e-5)                              # some twenty fp32 roundings of sums of up to 64 terms
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('path', ['layer', 'timers', 'experts', 'exchange', 'ffn', 'gate'])
+def test_no_second_derivative_is_an_error(monkeypatch, path):
+    """First derivatives under create_graph are the ordinary ones; using their graph raises."""
+    from planmoe_b200.utils import stage_timer
+    if path == 'exchange':
+        monkeypatch.setenv('PLANMOE_LOCAL', '0')
+    layer = _layer(torch.bfloat16, **({'is_gshard_loss': False} if path == 'experts' else {}))
+    if path == 'timers':
+        stage_timer.enable()
+    x = torch.randn(40, 64, device='cuda', dtype=torch.bfloat16)
+    ex = layer.experts
+
+    def run(create):
+        xin = x.clone().requires_grad_()
+        if path == 'ffn':
+            y = gemm.expert_ffn(xin.view(4, 10, 64), ex.batched_fc1_w, ex.batched_fc1_bias, ex.batched_fc2_w, ex.batched_fc2_bias, 'gelu')
+        elif path == 'gate':
+            from planmoe_b200.ops.fused_moe import fused_gate
+            y = fused_gate(xin, 2, 8, True)[0]
+        else:
+            y = layer(xin)
+        w = xin if path == 'gate' else ex.batched_fc1_w
+        return torch.autograd.grad(y.float().square().sum(), [xin, w], create_graph=create), xin
+    try:
+        (want, _), (got, xin) = run(False), run(True)
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+        # by anything that the gradients depend on, also beside terms that are sound
+        more = {'gate': [], 'ffn': [ex.batched_fc1_bias, ex.batched_fc2_w]}.get(path, [ex.batched_fc2_bias, layer.gates[0].wg.weight])
+        for by in [xin] + more:
+            with pytest.raises(RuntimeError, match='differentiated twice'):
+                torch.autograd.grad(got[0].float().square().sum() + by.float().square().sum(), by, retain_graph=True)
+    finally:
+        stage_timer.enable(False)
