@@ -147,12 +147,18 @@ __device__ __forceinline__ bool wait_flag_ge(const unsigned long long* flag, uns
 }
 
 // ---- chained launches (launch.cuh) ----
-// What every kernel that is launched so does before it touches global memory: wait until the kernels before it have completed
-// and their writes are visible, then let the next one of the stream be brought onto the SMs as this one's blocks leave them.
-// In this order, so that at most one kernel is ahead of the one that runs.  Without the launch attribute both do nothing.
+// What a kernel of one rank that may be launched so does before it touches global memory: wait until the kernels before it have
+// completed and their writes are visible, then let the next one of the stream be brought onto the SMs as this one's blocks leave
+// them.  In this order, so that at most one kernel is ahead of the one that runs.  The wait does nothing in a launch without the
+// attribute; the release counts in every launch, for a next one that has the attribute.
+// A kernel that waits for other ranks, sends or pushes to them waits here but does not release: what follows it takes no place on
+// an SM before it has completed, so that a kernel of another stream that a peer waits for finds the room that it would find
+// without chained launches.
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void chain_begin() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  chain_wait();
+  chain_release();
 }
 
 // ---- shared-memory barriers and the bulk-copy engine (cp.async.bulk, no tensor map) ----

@@ -214,7 +214,8 @@ gather_rows_kernel(const void* __restrict__ disp_, const float* __restrict__ sca
                    const int* __restrict__ idx, const int* __restrict__ loc,
                    const float* __restrict__ gates, T* __restrict__ out, int K, int S, int M,
                    int C, WaitGeom w, long long group_rows, bool round_gates) {
-  chain_begin();
+  chain_wait();
+  if (w.flags == nullptr) chain_release();         // not ahead of other ranks' flags
   __shared__ int ok_s;
   if (w.flags != nullptr) {
     if (threadIdx.x == 0) ok_s = 1;

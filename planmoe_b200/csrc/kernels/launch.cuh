@@ -7,9 +7,12 @@ namespace planmoe {
 
 // Launches `kern`, which calls chain_begin() before it touches global memory, so that its blocks may take their places while the
 // kernel before it ends (programmatic dependent launch).  Without that, 2.5 us lie between one kernel's end and the next one's
-// work, in a pass of up to eighteen launches.  Only grids of at most one block per SM: blocks of a larger one would crowd onto
-// the SMs that come free first, and a kernel that is one wave of the chip then lasts as long as the fullest SM (16384 tokens,
-// 16 experts, with the row kernels chained too: 569 us a pass, without 546).
+// work, in a pass of up to eighteen launches.  Only grids of at most one block per SM: blocks of a larger one may crowd onto the
+// SMs that come free first, and nothing is gained (three runs each, us a pass as it is and with the row kernels chained too:
+// inference of 16384 tokens with 16 experts 583 - 591 and 588 - 595, training on 8192 tokens with two 778 - 790 and 788 - 802).
+// The GEMM kernels of one rank, whose grids are resident at once, set the attribute themselves.
+// Kernels that deal with other ranks are neither launched so nor let the next one start early (chain_begin); others may be in a
+// pass of several ranks, too: gates, column sums, weight gradients.
 constexpr unsigned kChainedBlocks = 148;
 
 template <class... Params, class... Args>
