@@ -18,6 +18,7 @@
 
 #include "planmoe.h"
 #include "kernels/common.cuh"
+#include "kernels/launch.cuh"
 
 namespace planmoe {
 
@@ -115,11 +116,8 @@ void launch_xfer(const void* src_base, const long long* msgs, int n_msgs, int ct
   if (n_msgs <= 0) return;
   if (ctas_per_msg < 1) ctas_per_msg = 1;
   constexpr int smem = kXferSlots * kXferSlotBytes;
-  static bool configured = false;
-  if (!configured) {
-    cudaFuncSetAttribute(xfer_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    configured = true;
-  }
+  static std::atomic<unsigned long long> told{0};
+  allow_smem(xfer_kernel, smem, told);             // without it the launch fails and says so
   dim3 grid(ctas_per_msg, n_msgs);
   xfer_kernel<<<grid, 32, smem, stream>>>(reinterpret_cast<const unsigned char*>(src_base), msgs, n_msgs, heap_bases,
                                         flag_off, wait_flags, wait_idx, n_wait, want, budget_ns, status,

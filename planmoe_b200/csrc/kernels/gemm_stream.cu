@@ -4,10 +4,9 @@
 // Tiles of 128 x 256 (gemm_tcgen05.cu) leave SMs without loads in flight where there are few of them: 8 experts of 4096 x 1024 are 32
 // CTAs.  Here a tile is 64 columns wide, the narrowest that the weights' swizzled layout has, and its CTA goes through the whole
 // contraction: four times the CTAs, no sum that is shared between them, and outputs whose products are added up in the same order
-// as there, bit for bit.  (Splitting the contraction of a wide tile over a cluster rounds differently; it took 17.0 us where this takes 18.3, 8 x 4096 x 1024, and
-// 19.7 for 12.0, 5 x 2048 x 2048.)  Two CTAs
-// fit on an SM.  Groups without a token read no weights: their rows are zeros, so that the bias is all there is.  For which
-// launches: stream_gemm_pays.
+// as there, bit for bit.  (The contraction of a wide tile split over a cluster rounds differently; it took 17.0 us where this takes
+// 18.3, 8 x 4096 x 1024, and 19.7 for 12.0, 5 x 2048 x 2048.)  Two CTAs fit on an SM.  Groups without a token read no weights: their
+// rows are zeros, so that the bias is all there is.  For which launches: stream_gemm_pays.
 //
 //   warp 0      TMA producer; then the accumulators, TMEM to shared memory
 //   warp 1      MMA issuer (tcgen05.mma.cta_group::1, 128 x 64 x 16; rows behind the tile's are whatever lies behind them in
@@ -18,6 +17,7 @@
 #include "planmoe.h"
 #include "kernels/gemm_local.h"
 #include "kernels/gemm_tc.cuh"
+#include "kernels/launch.cuh"
 
 namespace planmoe {
 
@@ -190,8 +190,8 @@ bool stream_gemm_pays(int groups, int M, int N, int sms) {
 }
 
 cudaError_t launch_stream_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const StreamGemm& p, cudaStream_t stream) {
-  static const cudaError_t configured = cudaFuncSetAttribute(stream_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemTotal);
-  if (configured != cudaSuccess) return configured;
+  static std::atomic<unsigned long long> told{0};
+  if (const cudaError_t e = allow_smem(stream_gemm_kernel, (int)kSmemTotal, told); e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)(p.groups * ((p.N + kStreamCols - 1) / kStreamCols)), 1, 1);      // few, see stream_gemm_pays
   cfg.blockDim = dim3(kStreamThreads, 1, 1);

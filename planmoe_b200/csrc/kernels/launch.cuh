@@ -3,7 +3,23 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
+
 namespace planmoe {
+
+// Lets `kern` have `bytes` of dynamic shared memory.  The limit is the present device's, not the process's: `done`, a static of the
+// call's place, has a bit for each device that has been told (one beyond the 64th is told every time).
+template <class Kern>
+cudaError_t allow_smem(Kern* kern, int bytes, std::atomic<unsigned long long>& done) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
+  if (done.load(std::memory_order_relaxed) & bit) return cudaSuccess;
+  e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_relaxed);
+  return e;
+}
 
 // Launches `kern`, which calls chain_begin() before it touches global memory, so that its blocks may take their places while the
 // kernel before it ends (programmatic dependent launch).  Without that, 2.5 us lie between one kernel's end and the next one's
