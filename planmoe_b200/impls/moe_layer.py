@@ -383,7 +383,7 @@ class MOELayer(torch.nn.Module):
     def _generic_forward(self, x, gctx, top_k, cf, degree, reserve_shape, comm_name=None):
         comm_name = comm_name or self.comm_name
         from ..ops import layer32
-        if layer32.takes(self, gctx, x, top_k, cf, comm_name, reserve_shape):
+        if layer32.takes(self, gctx, x, top_k, cf, degree, comm_name, reserve_shape):
             y, l_aux, capacity = layer32.forward(self, x, gctx, top_k, cf, degree)
             if self.auto_parallel:
                 self.use_model_parallel = True              # what the general rule says with one shard

@@ -45,15 +45,18 @@ def _no_hooks(fn):
     return not isinstance(fn, torch.nn.Module) or not (fn._forward_hooks or fn._forward_pre_hooks or fn._backward_hooks or fn._backward_pre_hooks)
 
 
-def takes(layer, gctx, x, top_k, cf, comm_name, reserve_shape):
+def takes(layer, gctx, x, top_k, cf, degree, comm_name, reserve_shape):
     """Whether a call of the generic path is one that the node knows: one rank, fp32 throughout, a plain linear gate, FFN
-    experts with a known activation, no hooks on any of them, GShard loss, token order, gates applied after the experts, a
-    positive capacity factor; products in full fp32 and outside autocast; ordinary reverse-mode autograd."""
+    experts with a known activation, no hooks on any of them, no more chunks than there are transfers for, GShard loss, token
+    order, gates applied after the experts, a positive capacity factor; products in full fp32 and outside autocast; ordinary
+    reverse-mode autograd."""
     from ..experts.ffn import FusedExpertsNetwork
     from ..gates.top import LinearTopKGate
+    from ..impls.communicate import AllToAllStatus
     from . import fused_moe
     from torch.nn.modules import module as nnm
-    if not (x.is_cuda and x.dtype == torch.float32 and x.dim() == 2 and x.size(0) > 0 and x.size(1) % 4 == 0 and cf > 0):
+    if not (x.is_cuda and x.dtype == torch.float32 and x.dim() == 2 and x.size(0) > 0 and x.size(1) % 4 == 0 and cf > 0
+            and 1 <= degree <= AllToAllStatus.max_num_split):
         return False
     ex = layer.experts
     if (layer.world_size != 1 or layer.sharded_count != 1 or layer.experts_type != 'ffn' or layer.compress_name != 'no'
@@ -93,6 +96,8 @@ def _as_operations(act, top_k, cf, degree, normalize):
 
 def forward(layer, x, gctx, top_k, cf, degree):
     """``(y, l_aux, capacity)``"""
+    from ..impls.communicate import AllToAllStatus
+    AllToAllStatus.init(layer.group, degree, 1)          # what the chunked transfers of later calls read
     E, S = layer.num_global_experts, x.size(0)
     top_k = min(int(top_k), E)
     capacity = top_k * int(cf * ((S + E - 1) // E))

@@ -132,3 +132,13 @@ def test_fp32_precision_switches(monkeypatch, where, precision):
             h.fp32_precision = value
     for a, b in zip(got, want):                          # sums of up to 64 terms in another order; TF32: the same operations
         torch.testing.assert_close(a, b, rtol=1e-5, atol=2e-5)
+
+
+def test_more_chunks_than_transfers_are_refused():
+    layer = _layer(4, 2, 1.0, 'relu', 64, 32)
+    x = torch.randn(600, 64, device='cuda')
+    from planmoe_b200.impls.communicate import AllToAllStatus
+    layer(x, a2a_ffn_overlap_degree=AllToAllStatus.max_num_split)
+    assert (AllToAllStatus.num_split, AllToAllStatus.split_dim) == (AllToAllStatus.max_num_split, 1)
+    with pytest.raises(AssertionError):
+        layer(x, a2a_ffn_overlap_degree=2 * AllToAllStatus.max_num_split)
