@@ -47,12 +47,14 @@ def _no_hooks(fn):
 
 def takes(layer, gctx, x, top_k, cf, degree, comm_name, reserve_shape):
     """Whether a call of the generic path is one that the node knows: one rank, fp32 throughout, a plain linear gate, FFN
-    experts with a known activation, no hooks on any of them, no more chunks than there are transfers for, GShard loss, token
-    order, gates applied after the experts, a positive capacity factor; products in full fp32 and outside autocast; ordinary
-    reverse-mode autograd."""
+    experts with a known activation, no hooks on any of them, no more chunks than there are transfers for, the
+    built-in transfers (which move nothing here) and methods, GShard loss, token order, gates applied after the experts, a
+    positive capacity factor; products in full fp32 and outside autocast; ordinary reverse-mode autograd."""
     from ..experts.ffn import FusedExpertsNetwork
     from ..gates.top import LinearTopKGate
     from ..impls.communicate import AllToAllStatus
+    from ..impls.moe_layer import MOELayer
+    from ..parallel import codecs, comms
     from . import fused_moe
     from torch.nn.modules import module as nnm
     if not (x.is_cuda and x.dtype == torch.float32 and x.dim() == 2 and x.size(0) > 0 and x.size(1) % 4 == 0 and cf > 0
@@ -60,13 +62,15 @@ def takes(layer, gctx, x, top_k, cf, degree, comm_name, reserve_shape):
         return False
     ex = layer.experts
     if (layer.world_size != 1 or layer.sharded_count != 1 or layer.experts_type != 'ffn' or layer.compress_name != 'no'
-            or comm_name not in ('naive', 'pipe', 'hetu', 'dd') or not layer.is_gshard_loss or not layer.is_postscore
+            or codecs.factory('no') is not codecs.NoCompressor or comm_name not in ('naive', 'pipe', 'hetu', 'dd')
+            or comms.factory(comm_name) not in comms.BUILTIN or not layer.is_gshard_loss or not layer.is_postscore
             or layer.batch_prioritized_routing or layer.collect_stats or len(reserve_shape) != 1 or stage_timer.enabled()):
         return False
     if (not fused_moe._unhooked(ex, FusedExpertsNetwork) or not fused_moe._unhooked(gctx, LinearTopKGate)
             or not fused_moe._unhooked(gctx.wg, torch.nn.Linear) or ex.skip_expert or ex.fused_act is None
             or not _no_hooks(ex.activation_fn)
-            or 'expert_local' in layer.__dict__ or nnm._global_forward_hooks or nnm._global_forward_pre_hooks
+            or any(n in layer.__dict__ or getattr(type(layer), n) is not getattr(MOELayer, n) for n in ('expert_local', '_route'))
+            or nnm._global_forward_hooks or nnm._global_forward_pre_hooks
             or nnm._global_backward_hooks or nnm._global_backward_pre_hooks):
         return False
     wg = gctx.wg.weight

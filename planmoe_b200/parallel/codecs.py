@@ -202,6 +202,11 @@ class NativeCompressor(AbstractCompressor):
         return raw.view(dtype).view(shape)
 
 
+def factory(name):
+    """What makes the codec of a name, or None: one of a native module, or unknown."""
+    return _REGISTRY.get(name)
+
+
 def get_compressor(name):
     factory = _REGISTRY.get(name)
     if factory is not None:

@@ -265,6 +265,11 @@ class NativeComm(AbstractComm):
         return self._handle(t).all_to_all(t)
 
 
+def factory(name):
+    """What makes the algorithm of a name, or None: one of a native module, or unknown."""
+    return _REGISTRY.get(name)
+
+
 def get_comm(name, group=None):
     factory = _REGISTRY.get(name)
     if factory is None:

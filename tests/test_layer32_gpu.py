@@ -142,3 +142,40 @@ def test_more_chunks_than_transfers_are_refused():
     assert (AllToAllStatus.num_split, AllToAllStatus.split_dim) == (AllToAllStatus.max_num_split, 1)
     with pytest.raises(AssertionError):
         layer(x, a2a_ffn_overlap_degree=2 * AllToAllStatus.max_num_split)
+
+
+@pytest.mark.parametrize('what', ['expert_local', 'route', 'comm', 'codec'])
+def test_parts_of_the_generic_path_put_in_place(monkeypatch, what):
+    """A subclass's methods and algorithms registered under a built-in name are the ones that run."""
+    from planmoe_b200.impls.moe_layer import MOELayer
+    from planmoe_b200.parallel import codecs, comms
+    seen = []
+
+    class Local(MOELayer):
+        def expert_local(self, x, reserve_shape):
+            seen.append('expert_local')
+            return super().expert_local(x, reserve_shape)
+
+    class Route(MOELayer):
+        def _route(self, *a):
+            seen.append('route')
+            return super()._route(*a)
+
+    class Comm(comms.NaiveComm):
+        def all_to_all(self, t):
+            seen.append('comm')
+            return super().all_to_all(t)
+
+    class Codec(codecs.NoCompressor):
+        def compress(self, *a, **k):
+            seen.append('codec')
+            return super().compress(*a, **k)
+    layer = _layer(4, 2, 1.0, 'relu', 64, 32)
+    if what in ('expert_local', 'route'):
+        layer.__class__ = {'expert_local': Local, 'route': Route}[what]
+    elif what == 'comm':
+        monkeypatch.setitem(comms._REGISTRY, 'naive', Comm)
+    else:
+        monkeypatch.setitem(codecs._REGISTRY, 'no', Codec)
+    layer(torch.randn(40, 64, device='cuda'))
+    assert what in seen
