@@ -48,8 +48,8 @@ def test_groups_without_a_token_read_no_weights(M):
 
 @pytest.mark.parametrize('G,M,K,N', SHAPES)
 @pytest.mark.parametrize('act', ['gelu', 'identity'])
-def test_bits_of_the_kernel_for_more_rows(G, M, K, N, act):
-    """Every output adds its products up in the same order, so that a small batch and a large one agree."""
+def test_bits_of_the_kernel_for_up_to_128_rows(G, M, K, N, act):
+    """Every output adds its products up in the order of the kernel for up to 128 rows."""
     a, b, bias = _rand(G, M, K, seed=1), _rand(G, K, N, seed=2), _rand(G, N, seed=3)
 
     def run(**how):
