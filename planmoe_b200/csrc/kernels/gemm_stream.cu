@@ -5,8 +5,8 @@
 // CTAs.  Here a tile is 64 columns wide, the narrowest that the weights' swizzled layout has, and its CTA goes through the whole
 // contraction: four times the CTAs, no sum that is shared between them, and outputs whose products are added up in the same order
 // as there, bit for bit.  (The contraction of a wide tile split over a cluster rounds differently; it took 17.0 us where this takes
-// 18.3, 8 x 4096 x 1024, and 19.7 for 12.0, 5 x 2048 x 2048.)  Two CTAs fit on an SM.  Groups without a token read no weights: their
-// rows are zeros, so that the bias is all there is.  For which launches: stream_gemm_pays.
+// 15.7, 8 x 4096 x 1024, 19.7 for 11.0, 5 x 2048 x 2048, and 12.4 for 14.8, 1 x 4096 x 4096.)  Two CTAs fit on an SM.  Groups without a
+// token read no weights: their rows are zeros, so that the bias is all there is.  For which launches: stream_gemm_pays.
 //
 //   warp 0      TMA producer; then the accumulators, TMEM to shared memory
 //   warp 1      MMA issuer (tcgen05.mma.cta_group::1, 128 x 64 x 16; rows behind the tile's are whatever lies behind them in
@@ -27,12 +27,16 @@ constexpr int kStreamThreads = 128;
 constexpr int kStreamCols = 64;
 constexpr int kAccRow = kStreamCols + 4;           // floats between rows of the accumulators in shared memory: lanes on different banks
 
-constexpr uint32_t kABytes = kStreamRows * BK * 2, kBBytes = kStreamCols * BK * 2, kStage = kABytes + kBBytes;
-constexpr int kStages = 8;
+// Two K blocks a stage: what bounds a CTA is the round of waiting, issuing and committing, not the bytes in flight (6, 8 or 9 stages
+// of one block take the same time).  us for stages x blocks of 8 x 1, 4 x 2, 2 x 4: 8 x 4096 x 1024 18.3, 15.7, 17.1; 1 x 4096 x 4096
+// 18.2, 14.8, 15.9; 12 x 2048 x 1024 12.1, 11.9, 13.2.
+constexpr int kPer = 2, kStages = 4;
+constexpr uint32_t kABytes = kStreamRows * BK * 2, kBBytes = kStreamCols * BK * 2, kBlockBytes = kABytes + kBBytes;
+constexpr uint32_t kStage = kPer * kBlockBytes;
 constexpr uint32_t kRing = kStages * kStage, kMmaRows = BM * BK * 2;
-constexpr uint32_t kPad = kMmaRows - kStage;       // the MMA reads 128 rows from the last stage's start, too
+constexpr uint32_t kPad = kMmaRows - kBlockBytes;  // the MMA reads 128 rows from the last block's start, too
 constexpr uint32_t kSmemTotal = kRing + kPad + 256;
-static_assert(kMmaRows > kStage && kStage % 1024 == 0, "ring");
+static_assert(kMmaRows > kBlockBytes && kStage % 1024 == 0, "ring");
 static_assert(kStreamRows == 32 && kStreamRows * kAccRow * 4 <= kRing, "one warp's TMEM lanes; they take the ring's place");
 static_assert(2 * (kSmemTotal + 1024) <= 233472, "two CTAs fit on an SM");
 
@@ -88,14 +92,20 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     const bool leader = elect_one();
     uint32_t stage = 0, phase = 0;
     bool ok = true;
-    for (int kb = 0; kb < kbs; ++kb) {
+    for (int kb = 0; kb < kbs; kb += kPer) {
       ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&ctl->empty[stage]), phase ^ 1u, &ctl->abort, p.budget_ns, p.status, 0, stage));
       if (!ok) break;
       if (leader) {
         const uint32_t full = smem_u32(&ctl->full[stage]), sa = smem_u32(smem) + stage * kStage;
-        mbar_expect_tx(full, kStage);
-        tma_load_4d<1>(sa, &tmA, full, kb * BK, 0, g, 0);
-        tma_load_4d<1>(sa + kABytes, &tmB, full, n0, kb * BK, g, 0);
+        const int n = min(kPer, kbs - kb);
+        mbar_expect_tx(full, n * kBlockBytes);
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+          if (j < n) {
+            tma_load_4d<1>(sa + j * kBlockBytes, &tmA, full, (kb + j) * BK, 0, g, 0);
+            tma_load_4d<1>(sa + j * kBlockBytes + kABytes, &tmB, full, n0, (kb + j) * BK, g, 0);
+          }
+        }
       }
       __syncwarp();
       if (++stage == kStages) { stage = 0; phase ^= 1u; }
@@ -128,16 +138,21 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     const bool leader = elect_one();
     uint32_t stage = 0, phase = 0;
     bool ok = true;
-    for (int kb = 0; kb < kbs; ++kb) {
+    for (int kb = 0; kb < kbs; kb += kPer) {
       ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&ctl->full[stage]), phase, &ctl->abort, p.budget_ns, p.status, 1, stage));
       if (!ok) break;
       tc_fence_after();
       if (leader) {
-        const uint32_t sa = smem_u32(smem) + stage * kStage, sb = sa + kABytes;
 #pragma unroll
-        for (int k = 0; k < BK / UMMA_K; ++k)
-          umma_bf16<1>(tmem, make_desc(sa + k * (UMMA_K * 2), 16, 1024), make_desc(sb + k * (UMMA_K * 128), 64 * BK * 2, 1024), idesc,
-                       (kb | k) != 0 ? 1u : 0u);
+        for (int j = 0; j < kPer; ++j) {
+          const uint32_t sa = smem_u32(smem) + stage * kStage + j * kBlockBytes, sb = sa + kABytes;
+          if (j < kbs - kb) {
+#pragma unroll
+            for (int k = 0; k < BK / UMMA_K; ++k)
+              umma_bf16<1>(tmem, make_desc(sa + k * (UMMA_K * 2), 16, 1024), make_desc(sb + k * (UMMA_K * 128), 64 * BK * 2, 1024), idesc,
+                           (kb | j | k) != 0 ? 1u : 0u);
+          }
+        }
         umma_commit<1>(smem_u32(&ctl->empty[stage]));
       }
       __syncwarp();
@@ -182,9 +197,10 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
 }  // namespace
 
 // Few rows, and at most a third of the SMs have a wide tile.  us with 8 rows a group and weights from HBM, tiles of 256 and of 64
-// columns (wide tiles, groups x contraction x columns): 8 (4 x 2048 x 512) 19.1 and 10.7, 16 (1 x 4096 x 4096) 34.6 and 18.2, 32 (8 x 4096
-// x 1024) 34.5 and 18.3, 40 (5 x 2048 x 2048) 20.1 and 12.0, 48 (48 x 512 x 256) 8.8 and 7.2.  64 wide tiles would gain, too (8 x 2048 x
-// 2048: 21.0 and 13.6), 128 lose (8 x 1024 x 4096: 15.3 and 17.3): there the wide ones are loads enough for the chip.
+// columns (wide tiles, groups x contraction x columns): 8 (4 x 2048 x 512) 19.1 and 9.0, 16 (1 x 4096 x 4096) 34.6 and 14.8, 32 (8 x 4096
+// x 1024) 34.5 and 15.7, 40 (5 x 2048 x 2048) 20.1 and 11.0, 48 (48 x 512 x 256) 8.8 and 7.2.  With one K block a stage 64 wide tiles
+// would gain, too (8 x 2048 x 2048: 21.0 and 13.6), 128 lose (8 x 1024 x 4096: 15.3 and 17.3): there the wide ones are loads enough
+// for the chip.
 bool stream_gemm_pays(int groups, int M, int N, int sms) {
   return M <= kStreamRows && 3ll * groups * ((N + BN - 1) / BN) <= sms;
 }
